@@ -14,6 +14,8 @@ namespace {
 // With path counts sigma = m * 2^(512 k), q is kept as (1 + delta) / m
 // (FP64) and a successor's term is scaled by 2^(512 (k_v - k_w)).
 // ----------------------------------------------------------------------------
+constexpr int32_t BACK_HEAVY = 4096;  // entries above this take a CTA each
+
 struct BCtl {
     int32_t L0;       // deepest level; levels L0 .. 1 finalise their predecessors
     int32_t src;      // source of this sweep (excluded from the BC sum)
@@ -59,7 +61,7 @@ __device__ __forceinline__ void bc_finish_vertex(int32_t v, QT<EXT> s, const mgo
 // Level L-1 entries pull (1+delta)/sigma from their level-L successors.
 // q of the successors was written by other blocks in the previous level,
 // so it is loaded through L2 (the persistent kernel runs every level in one
-// launch).  Entries above PUSH_HEAVY are listed for bc_back_heavy_level.
+// launch).  Entries above BACK_HEAVY are listed for bc_back_heavy_level.
 template <bool EXT>
 __device__ __forceinline__ void bc_back_level(const Args &a, int32_t L, int32_t src, int32_t *hcount, QT<EXT> *q,
                                               float *delta, float *bcacc, int32_t *heavy_list)
@@ -80,7 +82,7 @@ __device__ __forceinline__ void bc_back_level(const Args &a, int32_t L, int32_t 
         for (int i = b0 + gwarp; i < b1; i += nwarps) {
             const int32_t v = a.queue[i];
             const int32_t b = a.row[v], e = a.row[v + 1];
-            if (e - b > PUSH_HEAVY) {
+            if (e - b > BACK_HEAVY) {
                 if (lane == 0) heavy_list[atomicAdd(hcount, 1)] = v;
                 continue;
             }
@@ -103,7 +105,7 @@ __device__ __forceinline__ void bc_back_level(const Args &a, int32_t L, int32_t 
             start = a.row[v];
             deg = a.row[v + 1] - start;
             if (EXT) kv = a.sigma[v].k;
-            if (deg > PUSH_HEAVY) {
+            if (deg > BACK_HEAVY) {
                 int h = atomicAdd(hcount, 1);
                 heavy_list[h] = v;
                 deg = 0;

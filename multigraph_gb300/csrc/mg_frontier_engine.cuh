@@ -11,8 +11,8 @@
 // pass of its body is four launches with fixed grids:
 //   k_sparse_levels  (cooperative, persistent) every consecutive push level:
 //            frontier queue -> neighbours (warp load-balanced search over the
-//            degrees of 32 queue entries; vertices above PUSH_HEAVY split over
-//            the whole grid), claims / relaxes destinations with the
+//            degrees of 32 queue entries; vertices above PUSH_HEAVY cut into
+//            chunks that teams of warps share), claims / relaxes destinations with the
 //            operator hooks, appends the next queue with warp-aggregated
 //            atomics and sets the next-frontier bitmap; one grid barrier
 //            per level, after which every block takes the end-of-level
@@ -44,9 +44,23 @@
 namespace {
 
 constexpr int MODE_PUSH = 0, MODE_PULL = 1;
-constexpr int32_t PUSH_HEAVY = 4096;
+// Frontier vertices above PUSH_HEAVY out-edges are listed as chunks of
+// PUSH_CHUNK edges (at most PUSH_CHUNKS a vertex), which a push level spreads
+// over teams of warps; the rest go one or more to a warp.  A 32-edge step is
+// a chain of dependent L2 accesses of 2-3 us, so what counts is the longest
+// run of steps in one warp: with one warp for any vertex of up to 4096
+// edges, the first level of a traversal from a hub took 317 us on R-MAT 20
+// (a 3,400-edge source: 100+ steps); with the chunks it is one step.
+constexpr int32_t PUSH_HEAVY = 128;
+constexpr int32_t PUSH_CHUNK = 512;
+constexpr int32_t PUSH_CHUNKS = 1024;
 constexpr int THREADS = 256;
-constexpr int PTHREADS = 1024;  // persistent kernels: 2 CTAs of 1024 per SM (fewer barrier arrivals)
+// persistent kernels: blocks of 1024 threads, and for the push phase one
+// block per SM: 152 arrivals at the grid barrier instead of 304, and 64
+// registers a thread instead of 32 with spills in the edge loops (lattice
+// BFS 5.8 -> 4.8 us a level at 100 K vertices, 8.5 -> 7.9 at 16.8 M; R-MAT
+// pushes 5-15 % faster)
+constexpr int PTHREADS = 1024;
 // grid barrier words (2 + GRID_SYNC_GROUPS), the barrier error flag, the BC
 // path-count overflow flag, rounded up
 constexpr size_t BAR_BYTES = 4 * (2 + mgd::GRID_SYNC_GROUPS + 1 + 7);
@@ -60,7 +74,7 @@ struct FCtl {
     int32_t cur;        // current bitmap buffer 0..2
     int32_t qoff, qsize;  // current queue slice
     int32_t nqoff, nq;    // next queue slice (nq: atomic counter)
-    int32_t hcur, nhcur;  // heavy list sizes: current / next (atomic)
+    int32_t hcur, nhcur;  // heavy chunk list sizes: current / next (atomic)
     int32_t hpar;         // heavy list parity
     int32_t status;       // 0 ok, 1 iteration cap
     int32_t pull_iters;
@@ -95,7 +109,9 @@ struct Args {
     uint32_t *visited;
     int32_t words;
     int32_t *queue;
-    int32_t *heavy;      // 2 * n (parity)
+    int4 *heavy;         // 2 * hcap chunks (parity): vertex, first edge, end
+    int32_t hcap;
+    int32_t has_heavy;   // some vertex may have more than PUSH_HEAVY out-edges
     int32_t *lvl_off;
     FCtl *ctl;
     unsigned *bar;       // grid barrier words of the persistent kernels
@@ -104,7 +120,7 @@ struct Args {
     struct LevelCnt *cnt;  // persistent push phase: per-level counters, 4 rotating slots
 };
 
-// Counters one push level produces (next queue size, heavy entries, next
+// Counters one push level produces (next queue size, heavy chunks, next
 // frontier's out-edges).  The persistent push phase keeps them in 4 slots
 // by level mod 4, so every block can read level L's counters after the one
 // barrier while level L+1 appends to the next slot; block 0 clears slot
@@ -139,24 +155,57 @@ __device__ __forceinline__ void warp_add64(long long *dst, long long v)
     if (mgd::lane() == 0 && v) atomicAdd((unsigned long long *)dst, (unsigned long long)v);
 }
 
+// Edges per chunk of a heavy vertex: PUSH_CHUNK, or more (a multiple of 32)
+// where that would make more than PUSH_CHUNKS chunks.
+__device__ __forceinline__ int32_t push_chunk(int32_t deg)
+{
+    return max(PUSH_CHUNK, (((deg - 1) / PUSH_CHUNKS + 1) + 31) & ~31);
+}
+
+// chunks that the heavy list can hold at most: a vertex above PUSH_HEAVY
+// edges has at most deg / PUSH_CHUNK + 1 of them
+inline int32_t heavy_cap(int64_t m) { return (int32_t)(m / PUSH_CHUNK + m / (PUSH_HEAVY + 1) + 2); }
+
+// The chunks of the lanes' heavy vertices (deg <= PUSH_HEAVY: none) to the
+// list `out`: one atomic a warp, the chunks spread over the lanes; all lanes
+// of the warp call.
+__device__ __forceinline__ void list_heavy(int4 *out, int32_t *count, int32_t v, int32_t begin, int32_t deg)
+{
+    const int lane = mgd::lane();
+    const int32_t ch = push_chunk(deg), nc = deg > PUSH_HEAVY ? (deg - 1) / ch + 1 : 0;
+    const int incl = mgd::warp_scan_incl(nc);
+    const int total = __shfl_sync(0xffffffffu, incl, 31);
+    int32_t base = 0;
+    if (lane == 0) base = atomicAdd(count, total);
+    base = __shfl_sync(0xffffffffu, base, 0);
+    for (int k0 = 0; k0 < total; k0 += 32) {
+        const int k = min(k0 + lane, total - 1);
+        const int own = mgd::owner_lane(incl - nc, k);
+        const int i = k - __shfl_sync(0xffffffffu, incl - nc, own);
+        const int32_t u = __shfl_sync(0xffffffffu, v, own), b = __shfl_sync(0xffffffffu, begin, own),
+                      d = __shfl_sync(0xffffffffu, deg, own), c = __shfl_sync(0xffffffffu, ch, own);
+        if (k0 + lane < total) out[base + k] = make_int4(u, b + i * c, b + min(d, (i + 1) * c), 0);
+    }
+}
+
 // record a newly reached vertex in the next frontier (push sweeps; all lanes
 // call).  A relaxed operator has already set the vertex's bit when it
 // improved it.
-template <class Op>
+template <class Op, bool HEAVY>
 __device__ __forceinline__ void emit_next(const Args &a, const FCtl &c, int nextbuf, bool found, int32_t v,
                                           long long &dsum, int32_t *nq, int32_t *nhcur)
 {
     int slot = mgd::warp_append(nq, found);
+    int32_t b = 0, dg = 0;
     if (found) {
         a.queue[c.nqoff + slot] = v;
         if (Op::kLevelSync) mgd::bm_set(bm_buf(a, nextbuf), v);
-        int32_t dg = a.row[v + 1] - a.row[v];
+        b = a.row[v];
+        dg = a.row[v + 1] - b;
         dsum += dg;
-        if (dg > PUSH_HEAVY) {
-            int h = atomicAdd(nhcur, 1);
-            a.heavy[(size_t)(c.hpar ^ 1) * a.n + h] = v;
-        }
     }
+    if (HEAVY && __any_sync(0xffffffffu, dg > PUSH_HEAVY))
+        list_heavy(a.heavy + (size_t)(c.hpar ^ 1) * a.hcap, nhcur, v, b, dg);
 }
 
 // ----------------------------------------------------------------------------
@@ -193,7 +242,7 @@ __device__ __forceinline__ bool push_edge(const Args &a, int it1, int32_t v, int
 // path counts were written by other blocks in the previous level, so they
 // are loaded through L2 (__ldcg): the persistent kernel runs many levels in
 // one launch.
-template <class Op>
+template <class Op, bool HEAVY>
 __device__ __forceinline__ void push_level(const Args &a, const FCtl &c, LevelCnt *lc)
 {
     const int it1 = c.iter + 1;
@@ -207,26 +256,29 @@ __device__ __forceinline__ void push_level(const Args &a, const FCtl &c, LevelCn
     const int gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
     long long scanned = 0, dsum = 0;
-    // heavy frontier vertices: every thread of the grid strides over their edges
-    for (int h = 0; h < c.hcur; h++) {
-        int32_t u = __ldcg(&a.heavy[(size_t)c.hpar * a.n + h]);
-        int32_t b = a.row[u], e = a.row[u + 1];
-        int32_t pi = __ldcg(&a.label[u]);
-        const mgops::PathCount pd = Op::kPathCounts ? mgops::pc_load_cg(&a.sigma[u]) : mgops::pc_zero();
-        if (Op::kPathCounts && !a.bc_ext && pd.m >= mgops::PC_PLAIN_MAX) *a.bc_ovf = 1;
-        int32_t span = e - b;
-        int32_t rounds = (span + gridDim.x * blockDim.x - 1) / (gridDim.x * blockDim.x);
-        for (int r = 0; r < rounds; r++) {
-            int32_t k = b + r * gridDim.x * blockDim.x + blockIdx.x * blockDim.x + threadIdx.x;
-            bool found = false;
-            int32_t v = 0;
-            if (k < e) {
-                v = a.col[k];
-                found = push_edge<Op>(a, it1, v, pi, pd, Op::kWeighted ? a.wt[k] : 0, bm_buf(a, nextbuf));
+    // chunks of heavy frontier vertices: a warp each, or a team of warps when
+    // there are fewer chunks than warps
+    if (HEAVY && c.hcur > 0) {
+        const int tw = c.hcur >= nwarps ? 1 : nwarps / c.hcur;
+        const int4 *list = a.heavy + (size_t)c.hpar * a.hcap;
+        for (int h = gwarp / tw; h < c.hcur; h += nwarps / tw) {
+            const int4 it = __ldcg(&list[h]);
+            const int32_t u = it.x, e = it.z;
+            const int32_t pi = __ldcg(&a.label[u]);
+            const mgops::PathCount pd = Op::kPathCounts ? mgops::pc_load_cg(&a.sigma[u]) : mgops::pc_zero();
+            if (Op::kPathCounts && !a.bc_ext && pd.m >= mgops::PC_PLAIN_MAX) *a.bc_ovf = 1;
+            for (int32_t k0 = it.y + (gwarp % tw) * 32; k0 < e; k0 += tw * 32) {
+                const int32_t k = k0 + lane;
+                bool found = false;
+                int32_t v = 0;
+                if (k < e) {
+                    v = a.col[k];
+                    found = push_edge<Op>(a, it1, v, pi, pd, Op::kWeighted ? a.wt[k] : 0, bm_buf(a, nextbuf));
+                }
+                emit_next<Op, HEAVY>(a, c, nextbuf, found, v, dsum, &lc->nq, &lc->nhcur);
             }
-            emit_next<Op>(a, c, nextbuf, found, v, dsum, &lc->nq, &lc->nhcur);
+            if (lane == 0 && gwarp % tw == 0) scanned += e - it.y;
         }
-        scanned += (threadIdx.x == 0 && blockIdx.x == 0) ? span : 0;
     }
     // light frontier vertices: vpw per warp (32, or fewer when the frontier
     // would leave warps idle), load-balanced over their edges
@@ -243,7 +295,7 @@ __device__ __forceinline__ void push_level(const Args &a, const FCtl &c, LevelCn
             u = __ldcg(&a.queue[c.qoff + base + lane]);
             start = a.row[u];
             deg = a.row[u + 1] - start;
-            if (deg > PUSH_HEAVY) deg = 0;
+            if (HEAVY && deg > PUSH_HEAVY) deg = 0;
             pi = __ldcg(&a.label[u]);
             if (Op::kPathCounts) {
                 pd = mgops::pc_load_cg(&a.sigma[u]);
@@ -267,7 +319,7 @@ __device__ __forceinline__ void push_level(const Args &a, const FCtl &c, LevelCn
                 v = a.col[e];
                 found = push_edge<Op>(a, it1, v, opi, opd, Op::kWeighted ? a.wt[e] : 0, bm_buf(a, nextbuf));
             }
-            emit_next<Op>(a, c, nextbuf, found, v, dsum, &lc->nq, &lc->nhcur);
+            emit_next<Op, HEAVY>(a, c, nextbuf, found, v, dsum, &lc->nq, &lc->nhcur);
         }
     }
     warp_add64(&lc->nfe, dsum);
@@ -517,36 +569,53 @@ __global__ void __launch_bounds__(THREADS) k_pull(Args a)
 
 // ----------------------------------------------------------------------------
 // compact: after a pull sweep, the next frontier's bitmap -> queue slice,
-// edge count and heavy list.  Each warp takes 32 bitmap words (1024
-// vertices) and reserves its queue slots with one atomicAdd.
+// edge count and heavy list.  A block takes every gridDim-th word of the
+// bitmap (hub-first ids: the first words hold the heavy vertices, whose
+// chunks take the time), its words dealt out to its warps in turn, and
+// reserves its queue slots with one atomicAdd; a warp goes through its words
+// a lane per vertex, so the row offsets come in coalesced.
 // ----------------------------------------------------------------------------
 __global__ void __launch_bounds__(THREADS) k_compact(Args a)
 {
     const FCtl c = *a.ctl;
     if (c.mode != MODE_PULL || c.more == 0) return;
+    constexpr int NW = THREADS / 32;
+    __shared__ int s_cnt[NW], s_base;
     const uint32_t *nb = bm_buf(a, (c.cur + 1) % 3);
-    const int lane = mgd::lane();
-    const int gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int nwarps = (gridDim.x * blockDim.x) >> 5;
+    const int lane = mgd::lane(), warp = threadIdx.x >> 5;
+    int4 *heavy = a.heavy + (size_t)(c.hpar ^ 1) * a.hcap;
     long long dsum = 0;
-    for (int32_t w0 = gwarp * 32; w0 < a.words; w0 += nwarps * 32) {
-        const int32_t wi = w0 + lane;
-        uint32_t bits = wi < a.words ? nb[wi] : 0u;
-        const int cnt = __popc(bits);
-        const int incl = mgd::warp_scan_incl(cnt);
-        const int total = __shfl_sync(0xffffffffu, incl, 31);
-        int base = 0;
-        if (lane == 31 && total) base = atomicAdd(&a.ctl->nq, total);
-        base = __shfl_sync(0xffffffffu, base, 31) + incl - cnt;
-        while (bits) {
-            const int b = __ffs(bits) - 1;
-            bits &= bits - 1;
-            const int32_t v = wi * 32 + b;
-            a.queue[c.nqoff + base++] = v;
-            const int32_t dg = a.row[v + 1] - a.row[v];
-            dsum += dg;
-            if (dg > PUSH_HEAVY) a.heavy[(size_t)(c.hpar ^ 1) * a.n + atomicAdd(&a.ctl->nhcur, 1)] = v;
+    for (int64_t w0 = blockIdx.x; w0 < a.words; w0 += (int64_t)gridDim.x * THREADS) {
+        const int64_t wi = w0 + (int64_t)(lane * NW + warp) * gridDim.x;
+        const uint32_t bits = wi < a.words ? nb[wi] : 0u;
+        const int total = __reduce_add_sync(0xffffffffu, __popc(bits));
+        if (lane == 0) s_cnt[warp] = total;
+        __syncthreads();
+        int base = 0, all = 0;
+        for (int k = 0; k < NW; k++) {
+            base += k < warp ? s_cnt[k] : 0;
+            all += s_cnt[k];
         }
+        if (threadIdx.x == 0 && all) s_base = atomicAdd(&a.ctl->nq, all);
+        __syncthreads();
+        base += s_base;
+        unsigned full = __ballot_sync(0xffffffffu, bits != 0);
+        while (full) {
+            const int j = __ffs(full) - 1;
+            full &= full - 1;
+            const uint32_t word = __shfl_sync(0xffffffffu, bits, j);
+            const int32_t v = (int32_t)(w0 + (int64_t)(j * NW + warp) * gridDim.x) * 32 + lane;
+            int32_t rb = 0, dg = 0;
+            if ((word >> lane) & 1u) {
+                a.queue[c.nqoff + base + __popc(word & ((1u << lane) - 1u))] = v;
+                rb = a.row[v];
+                dg = a.row[v + 1] - rb;
+                dsum += dg;
+            }
+            base += __popc(word);
+            if (a.has_heavy && __any_sync(0xffffffffu, dg > PUSH_HEAVY)) list_heavy(heavy, &a.ctl->nhcur, v, rb, dg);
+        }
+        __syncthreads();   // s_cnt / s_base are reused
     }
     warp_add64(&a.ctl->nf_edges, dsum);
 }
@@ -654,8 +723,10 @@ __device__ __forceinline__ FCtl block_load_ctl(const FCtl *p)
     return c;
 }
 
-template <class Op>
-__global__ void __launch_bounds__(PTHREADS, 2) k_sparse_levels(Args a)
+// HEAVY: the graph may have vertices above PUSH_HEAVY out-edges (graphs that
+// have none run without the chunk code and its votes).
+template <class Op, bool HEAVY>
+__global__ void __launch_bounds__(PTHREADS, 1) k_sparse_levels(Args a)
 {
     __shared__ FCtl s_c;
     __shared__ int4 s_cnt;
@@ -675,7 +746,7 @@ __global__ void __launch_bounds__(PTHREADS, 2) k_sparse_levels(Args a)
             z->nhcur = 0;
             z->nfe = 0;
         }
-        push_level<Op>(a, s_c, lc);
+        push_level<Op, HEAVY>(a, s_c, lc);
         if (!mgd::grid_sync(a.bar, a.bar_err, a.bar_never)) break;
         if (threadIdx.x == 0) {
             s_cnt = __ldcg(reinterpret_cast<const int4 *>(lc));  // nq, nhcur, nfe (lo, hi)
@@ -707,40 +778,54 @@ __global__ void __launch_bounds__(PTHREADS, 2) k_sparse_levels(Args a)
 // init: source
 // ----------------------------------------------------------------------------
 // sources: srcs[0..nsrc) when srcs is non-null, else the single `src`
-// (several sources = one traversal of a disjoint union of graphs)
+// (several sources = one traversal of a disjoint union of graphs), a thread
+// each of one block (one thread walking 30 sources took 33 us)
+constexpr int INIT_THREADS = 256;
 template <class Op>
-__global__ void k_init(Args a, int32_t src, const int32_t *srcs, int32_t nsrc, int dirmode, int alpha, int beta,
-                       int max_iter)
+__global__ void __launch_bounds__(INIT_THREADS) k_init(Args a, int32_t src, const int32_t *srcs, int32_t nsrc,
+                                                       int dirmode, int alpha, int beta, int max_iter)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+    __shared__ int s_q;
+    __shared__ unsigned long long s_ve;
     FCtl *c = a.ctl;
-    std::memset(c, 0, sizeof(FCtl));
-    c->more = 1;
-    c->archive = Op::kLevelSync;
-    c->max_iter = max_iter;
-    c->dirmode = dirmode;
-    c->alpha = alpha;
-    c->beta = beta;
-    c->mode = (dirmode == MG_DIR_PULL) ? MODE_PULL : MODE_PUSH;
-    int32_t q = 0;
-    long long ve = 0;
-    for (int32_t i = 0; i < (srcs ? nsrc : 1); i++) {
-        int32_t s = srcs ? srcs[i] : src;
-        if (!mgd::bm_set(a.visited, s)) continue;  // duplicate source
-        a.label[s] = Op::source_value();
-        if (Op::kPathCounts) a.sigma[s] = mgops::pc_one();
-        mgd::bm_set(a.bm, s);  // buffer 0 is the current frontier
-        a.queue[q++] = s;
-        int32_t d = a.row[s + 1] - a.row[s];
-        ve += d;
-        if (d > PUSH_HEAVY) a.heavy[c->hcur++] = s;
+    if (threadIdx.x == 0) {
+        s_q = 0;
+        s_ve = 0;
+        std::memset(c, 0, sizeof(FCtl));
+        c->more = 1;
+        c->archive = Op::kLevelSync;
+        c->max_iter = max_iter;
+        c->dirmode = dirmode;
+        c->alpha = alpha;
+        c->beta = beta;
+        c->mode = (dirmode == MG_DIR_PULL) ? MODE_PULL : MODE_PUSH;
+        *a.fmin = INT32_MAX;
     }
-    c->qoff = 0;
-    c->qsize = q;
-    c->nqoff = Op::kLevelSync ? q : a.n;
-    c->visited_edges = ve;
-    if (Op::kLevelSync) { a.lvl_off[0] = 0; a.lvl_off[1] = q; c->nlevels = 1; }
-    *a.fmin = INT32_MAX;
+    __syncthreads();
+    const int32_t count = srcs ? nsrc : 1;
+    for (int32_t i0 = threadIdx.x & ~31; i0 < count; i0 += INIT_THREADS) {
+        const int32_t i = i0 + mgd::lane();
+        const int32_t s = i < count ? (srcs ? srcs[i] : src) : -1;
+        int32_t b = 0, d = 0;
+        if (s >= 0 && mgd::bm_set(a.visited, s)) {  // (a duplicate source is queued once)
+            a.label[s] = Op::source_value();
+            if (Op::kPathCounts) a.sigma[s] = mgops::pc_one();
+            mgd::bm_set(a.bm, s);  // buffer 0 is the current frontier
+            a.queue[atomicAdd(&s_q, 1)] = s;
+            b = a.row[s];
+            d = a.row[s + 1] - b;
+            atomicAdd(&s_ve, (unsigned long long)d);
+        }
+        if (a.has_heavy && __any_sync(0xffffffffu, d > PUSH_HEAVY)) list_heavy(a.heavy, &c->hcur, s, b, d);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const int32_t q = s_q;
+        c->qsize = q;
+        c->nqoff = Op::kLevelSync ? q : a.n;
+        c->visited_edges = (long long)s_ve;
+        if (Op::kLevelSync) { a.lvl_off[0] = 0; a.lvl_off[1] = q; c->nlevels = 1; }
+    }
 }
 
 // ----------------------------------------------------------------------------
@@ -792,7 +877,7 @@ mg_status ensure_ws(mg_graph *g)
     MG_TRY(dev_alloc(w->bm, 3 * words * 4));
     MG_TRY(dev_alloc(w->visited, words * 4));
     MG_TRY(dev_alloc(w->queue, 2 * n * 4));
-    MG_TRY(dev_alloc(w->heavy, 2 * n * 4));
+    MG_TRY(dev_alloc(w->heavy, 2 * (size_t)heavy_cap(g->ne) * sizeof(int4)));
     MG_TRY(dev_alloc(w->ctl, sizeof(FCtl)));
     MG_TRY(dev_alloc(w->lvl_off, (n + 3) * 4));
     MG_TRY(dev_alloc(w->bar, BAR_BYTES));
@@ -801,9 +886,12 @@ mg_status ensure_ws(mg_graph *g)
     int &cg = w->coop_grid[&OpTag<Op>::id];
     if (cg == 0) {
         int per_sm = 0;
-        MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sparse_levels<Op>, PTHREADS, 0));
+        if (g->relabeled)
+            MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sparse_levels<Op, true>, PTHREADS, 0));
+        else
+            MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sparse_levels<Op, false>, PTHREADS, 0));
         if (per_sm < 1) return fail(MG_ERR_CUDA, "persistent push kernel does not fit on an SM");
-        cg = std::min(per_sm, 2) * g->num_sms;
+        cg = g->num_sms;
     }
     return MG_OK;
 }
@@ -822,7 +910,8 @@ mg_status launch_sparse_levels(const Args &a, int grid, cudaStream_t st)
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    MG_CUDA(cudaLaunchKernelEx(&cfg, k_sparse_levels<Op>, a));
+    if (a.has_heavy) MG_CUDA(cudaLaunchKernelEx(&cfg, k_sparse_levels<Op, true>, a));
+    else MG_CUDA(cudaLaunchKernelEx(&cfg, k_sparse_levels<Op, false>, a));
     return MG_OK;
 }
 
@@ -849,7 +938,9 @@ inline Args make_args(mg_graph *g)
     a.visited = w->visited.as<uint32_t>();
     a.words = (std::max(g->nv, 1) + 31) / 32;
     a.queue = w->queue.as<int32_t>();
-    a.heavy = w->heavy.as<int32_t>();
+    a.heavy = w->heavy.as<int4>();
+    a.hcap = heavy_cap(g->ne);
+    a.has_heavy = g->relabeled;  // (graphs with a degree of 128 or more are relabeled)
     a.lvl_off = w->lvl_off.as<int32_t>();
     a.ctl = w->ctl.as<FCtl>();
     a.bar = w->bar.as<unsigned>();
@@ -901,7 +992,7 @@ mg_status frontier_run_impl(mg_graph *g, int32_t src, const int32_t *srcs_host, 
     if (Op::kPathCounts) MG_CUDA(cudaMemsetAsync(a.sigma, 0, n * sizeof(mgops::PathCount), s));
     int max_iter = opt.max_iter > 0 ? opt.max_iter : (Op::kLevelSync ? g->nv + 2 : 4 * g->nv + 16);
     int alpha = opt.alpha > 0 ? opt.alpha : (Op::kLevelSync ? 15 : 4), beta = opt.beta > 0 ? opt.beta : 18;
-    k_init<Op><<<1, 32, 0, s>>>(a, src, srcs_dev, nsrc, opt.direction, alpha, beta, max_iter);
+    k_init<Op><<<1, INIT_THREADS, 0, s>>>(a, src, srcs_dev, nsrc, opt.direction, alpha, beta, max_iter);
     MG_CUDA(cudaGetLastError());
     const void *tag = &OpTag<Op>::id;
     const int coop = w->coop_grid[tag];
