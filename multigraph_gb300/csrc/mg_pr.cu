@@ -879,185 +879,346 @@ __global__ void __launch_bounds__(THREADS) k_wpr_grad(int32_t n, const int32_t *
     }
 }
 
-// personalised PageRank, 32 seeds per pass: lane = seed, X / C are [n][32]
-// for the current seed block (one 128 B line per vertex).  Rows with more
-// than PPR_HEAVY in-edges are split into PPR_HEAVY-edge chunks (warp per
-// chunk, partial sums per chunk) and combined in order by k_ppr_heavy.
+// ---------------------------------------------------------------------------
+// Personalised PageRank, up to 32 seeds per pass.  X / C are [n][4 LPR]: a
+// vertex's values for the pass's seeds lie side by side, four seeds (a
+// float4) a lane, LPR lanes a vertex (1, 2, 4 or 8: the fewest that hold the
+// pass's seeds), 32 / LPR rows a warp at a time.  With the hub-first order
+// the rows of a warp have similar lengths; they run in step over the longest
+// one.  Rows with more than PPR_HEAVY in-edges are split into PPR_HEAVY-edge
+// chunks (partial sums per chunk) that k_ppr_close combines in order.
+//
+// What bounds the sweep is bytes in flight towards L2 (4 GB of gathers on
+// R-MAT 20, L2 and L1 both under half of their rates): eight 16-byte gathers
+// a lane in 64 registers keep 128 KB in flight per SM, where one 4-byte
+// gather of eight edges a lane in 32 registers kept 55 KB.
+// R-MAT 20, 32 seeds: 527 -> 358 us per sweep (11.5 TB/s of gathers).
+//
+// Sums run in a fixed order that does not depend on LPR (pairwise over eight
+// consecutive edges, the eights compensated in order), so a hub's total does
+// not drift between sweeps.
+// ---------------------------------------------------------------------------
 constexpr int32_t PPR_HEAVY = 256;
+constexpr int PPR_THREADS = 512;       // two blocks per SM at 64 registers
+constexpr int PPR_PER_SM = 2;
+constexpr int PPR_CLOSE_THREADS = 512;
+constexpr int PPR_CLOSE_PER_SM = 2;
 
 struct PPCtl {
-    int32_t more, iter, cur, status, max_iter, pad;
+    int32_t more, iter, cur, status, max_iter, nseed;
+    int32_t done;            // blocks of k_ppr_close that have finished this sweep
+    int32_t pad;
     double resid[32];
 };
 
 struct PPArgs {
     int32_t n;
     const int32_t *prow, *pcol, *outrow;
-    const int32_t *seeds;
-    int32_t nseed;
+    int32_t *seeds;          // [32] the pass's seeds (-1: none)
     const int32_t *hchunk;   // (row, begin, end)
     int32_t nhchunks;
     const int32_t *hrows, *hrow_chunk;
     int32_t nhrows;
-    float *X0, *C0, *X1, *C1;
-    float *hpart;            // [nhchunks][32]
-    double *bpart;           // [2*grid][32][2]
+    float4 *X[2], *C[2];
+    float4 *hpart;           // [nhchunks][LPR]
+    double2 *bpart;          // [sweep + close blocks][32] (residual, dangling mass)
     double *dang;            // [32] dangling mass of the current iterate
     PPCtl *ctl;
     float damping;
 };
 
-__global__ void k_ppr_init(PPArgs a, int32_t max_iter)
+// start of a pass (X[0] and C[0] are zero): one block of 32 threads
+__global__ void k_ppr_init(PPArgs a, const int32_t *seeds, int32_t nseed, int32_t width, int32_t max_iter)
 {
-    const size_t total = (size_t)a.n * 32;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        int32_t v = (int32_t)(i >> 5);
-        int s = (int)(i & 31);
-        float x = (s < a.nseed && a.seeds[s] == v) ? 1.0f : 0.0f;
-        a.X0[i] = x;
-        int32_t od = a.outrow[v + 1] - a.outrow[v];
-        a.C0[i] = od > 0 ? x / (float)od : 0.0f;
+    const int s = threadIdx.x;
+    const int32_t v = s < nseed ? seeds[s] : -1;
+    a.seeds[s] = v;
+    double dg = 0.0;
+    if (v >= 0) {
+        const int32_t od = a.outrow[v + 1] - a.outrow[v];
+        reinterpret_cast<float *>(a.X[0])[(size_t)v * width + s] = 1.0f;
+        reinterpret_cast<float *>(a.C[0])[(size_t)v * width + s] = od > 0 ? 1.0f / (float)od : 0.0f;
+        dg = od == 0 ? 1.0 : 0.0;
     }
-    if (blockIdx.x == 0 && threadIdx.x < 32) {
-        int s = threadIdx.x;
-        double dg = 0.0;
-        if (s < a.nseed) { int32_t v = a.seeds[s]; dg = (a.outrow[v + 1] == a.outrow[v]) ? 1.0 : 0.0; }
-        a.dang[s] = dg;
-        if (s == 0) {
-            std::memset(a.ctl, 0, sizeof(PPCtl));
-            a.ctl->more = 1;
-            a.ctl->max_iter = max_iter;
+    a.dang[s] = dg;
+    if (s == 0) {
+        std::memset(a.ctl, 0, sizeof(PPCtl));
+        a.ctl->more = 1;
+        a.ctl->max_iter = max_iter;
+        a.ctl->nseed = nseed;
+    }
+}
+
+__device__ __forceinline__ float4 f4_add(float4 a, float4 b)
+{
+    return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
+}
+
+// four compensated adds (mgd::kahan_add)
+__device__ __forceinline__ void f4_kahan(float4 &t, float4 &r, float4 x)
+{
+    mgd::kahan_add(t.x, r.x, x.x);
+    mgd::kahan_add(t.y, r.y, x.y);
+    mgd::kahan_add(t.z, r.z, x.z);
+    mgd::kahan_add(t.w, r.w, x.w);
+}
+
+// Per-lane state of the sweep: the lane's seeds, and compensated sums of the
+// residual and the dangling mass.
+struct PprLane {
+    int32_t seed[4];
+    float r[4], rc[4], d[4], dc[4];
+};
+
+template <int LPR>
+__device__ __forceinline__ PprLane ppr_lane(const PPArgs &a)
+{
+    PprLane l;
+    const int gl = threadIdx.x & (LPR - 1);
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        l.seed[k] = a.seeds[gl * 4 + k];
+        l.r[k] = l.rc[k] = l.d[k] = l.dc[k] = 0.0f;
+    }
+    return l;
+}
+
+// row v's update from its gathered sum s (this lane's four seeds)
+template <int LPR, bool DANG>
+__device__ __forceinline__ void ppr_apply(const PPArgs &a, int cur, int32_t v, float4 s4, PprLane &l)
+{
+    const int gl = threadIdx.x & (LPR - 1);
+    const size_t at = (size_t)v * LPR + gl;
+    const int32_t od = __ldg(&a.outrow[v + 1]) - __ldg(&a.outrow[v]);
+    // the iterate is streamed; L2 is kept for the contributions
+    const float4 xo4 = __ldcs(&a.X[cur][at]);
+    const float s[4] = {s4.x, s4.y, s4.z, s4.w}, xo[4] = {xo4.x, xo4.y, xo4.z, xo4.w};
+    float xn[4], cn[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        float base = 0.0f;
+        if (v == l.seed[k]) base = (1.0f - a.damping) + a.damping * (float)a.dang[gl * 4 + k];
+        xn[k] = base + a.damping * s[k];
+        cn[k] = od > 0 ? xn[k] / (float)od : 0.0f;
+        mgd::kahan_add(l.r[k], l.rc[k], fabsf(xn[k] - xo[k]));
+        if (DANG && od == 0) mgd::kahan_add(l.d[k], l.dc[k], xn[k]);
+    }
+    __stcs(&a.X[cur ^ 1][at], make_float4(xn[0], xn[1], xn[2], xn[3]));
+    a.C[cur ^ 1][at] = make_float4(cn[0], cn[1], cn[2], cn[3]);
+}
+
+// Sum of C over the columns [b, e) for this lane's seeds.  All lanes of the
+// warp call (a group without a row passes b == e) and run over the longest
+// of their ranges; the next eight ids are loaded ahead of the current
+// gathers.
+template <int LPR>
+__device__ __forceinline__ float4 ppr_gather(const float4 *__restrict__ C, const int32_t *__restrict__ pcol, int32_t b,
+                                             int32_t e)
+{
+    constexpr int IPL = 8 / LPR;   // ids a lane loads of eight
+    const int gl = threadIdx.x & (LPR - 1);
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f), low = acc;
+    const int32_t rounds = (int32_t)__reduce_max_sync(0xffffffffu, (unsigned)((e - b + 7) >> 3));
+    int32_t id[IPL];
+#pragma unroll
+    for (int k = 0; k < IPL; k++) {
+        const int32_t p = b + gl + k * LPR;
+        id[k] = p < e ? __ldcs(&pcol[p]) : -1;
+    }
+    for (int32_t r = 0; r < rounds; r++) {
+        float4 t[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            const int32_t u = __shfl_sync(0xffffffffu, id[j / LPR], j % LPR, LPR);
+            t[j] = u >= 0 ? C[(size_t)u * LPR + gl] : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        b += 8;
+#pragma unroll
+        for (int k = 0; k < IPL; k++) {
+            const int32_t p = b + gl + k * LPR;
+            id[k] = p < e ? __ldcs(&pcol[p]) : -1;
+        }
+        f4_kahan(acc, low, f4_add(f4_add(f4_add(t[0], t[1]), f4_add(t[2], t[3])),
+                                  f4_add(f4_add(t[4], t[5]), f4_add(t[6], t[7]))));
+    }
+    return acc;
+}
+
+// the block's residual and dangling sums of every seed to bpart[slot]
+template <int LPR, int NT>
+__device__ __forceinline__ void ppr_block_partials(const PPArgs &a, int slot, const PprLane &l)
+{
+    __shared__ double sr[NT / 32][4 * LPR], sd[NT / 32][4 * LPR];
+    const int lane = mgd::lane(), warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        double r = (double)l.r[k] - (double)l.rc[k], d = (double)l.d[k] - (double)l.dc[k];
+#pragma unroll
+        for (int o = 16; o >= LPR; o >>= 1) {
+            r += __shfl_xor_sync(0xffffffffu, r, o);
+            d += __shfl_xor_sync(0xffffffffu, d, o);
+        }
+        if (lane < LPR) {
+            sr[warp][lane * 4 + k] = r;
+            sd[warp][lane * 4 + k] = d;
         }
     }
-}
-
-__device__ __forceinline__ void ppr_apply(const PPArgs &a, const PPCtl &c, int32_t v, float s, int lane, float dang,
-                                          int32_t seed, double &resid, double &dnext)
-{
-    const float *Xc = c.cur ? a.X1 : a.X0;
-    float *Xn = c.cur ? a.X0 : a.X1;
-    float *Cn = c.cur ? a.C0 : a.C1;
-    float base = (v == seed) ? (1.0f - a.damping) + a.damping * dang : 0.0f;
-    float xn = base + a.damping * s;
-    float xo = Xc[(size_t)v * 32 + lane];
-    Xn[(size_t)v * 32 + lane] = xn;
-    int32_t od = a.outrow[v + 1] - a.outrow[v];
-    Cn[(size_t)v * 32 + lane] = od > 0 ? xn / (float)od : 0.0f;
-    if (od == 0) dnext += xn;
-    resid += fabsf(xn - xo);
-}
-
-__device__ __forceinline__ void ppr_block_partials(const PPArgs &a, int slot, double resid, double dnext)
-{
-    __shared__ double sr[THREADS / 32][32], sd[THREADS / 32][32];
-    const int lane = mgd::lane();
-    sr[threadIdx.x >> 5][lane] = resid;
-    sd[threadIdx.x >> 5][lane] = dnext;
     __syncthreads();
     if (threadIdx.x < 32) {
-        double R = 0, D = 0;
-        for (int w = 0; w < THREADS / 32; w++) { R += sr[w][threadIdx.x]; D += sd[w][threadIdx.x]; }
-        a.bpart[((size_t)slot * 32 + threadIdx.x) * 2] = R;
-        a.bpart[((size_t)slot * 32 + threadIdx.x) * 2 + 1] = D;
+        double R = 0.0, D = 0.0;
+        if (threadIdx.x < 4 * LPR)
+            for (int w = 0; w < NT / 32; w++) {
+                R += sr[w][threadIdx.x];
+                D += sd[w][threadIdx.x];
+            }
+        a.bpart[(size_t)slot * 32 + threadIdx.x] = make_double2(R, D);
     }
 }
 
-// gather sum of C[u][lane] over [b, e)
-__device__ __forceinline__ float ppr_gather(const float *Cc, const int32_t *pcol, int32_t b, int32_t e, int lane)
+template <int LPR, bool DANG>
+__global__ void __launch_bounds__(PPR_THREADS, PPR_PER_SM) k_ppr_sweep(PPArgs a)
 {
-    float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
-    int32_t p = b;
-    for (; p + 8 <= e; p += 8) {
-        int32_t u[8];
-#pragma unroll
-        for (int j = 0; j < 8; j++) u[j] = pcol[p + j];
-        float t[8];
-#pragma unroll
-        for (int j = 0; j < 8; j++) t[j] = Cc[(size_t)u[j] * 32 + lane];
-        s0 += t[0] + t[4];
-        s1 += t[1] + t[5];
-        s2 += t[2] + t[6];
-        s3 += t[3] + t[7];
+    if (a.ctl->more == 0) return;
+    constexpr int RPW = 32 / LPR;   // rows a warp
+    const int cur = a.ctl->cur;
+    const float4 *C = a.C[cur];
+    const int gl = threadIdx.x & (LPR - 1), grp = mgd::lane() / LPR;
+    const int gwarp = (blockIdx.x * PPR_THREADS + threadIdx.x) >> 5;
+    const int nwarps = (gridDim.x * PPR_THREADS) >> 5;
+    PprLane l = ppr_lane<LPR>(a);
+    // chunks of heavy rows first: the longest
+    for (int32_t c0 = gwarp * RPW; c0 < a.nhchunks; c0 += nwarps * RPW) {
+        const int32_t ch = c0 + grp;
+        const bool ok = ch < a.nhchunks;
+        const int32_t b = ok ? __ldg(&a.hchunk[3 * ch + 1]) : 0, e = ok ? __ldg(&a.hchunk[3 * ch + 2]) : 0;
+        const float4 s = ppr_gather<LPR>(C, a.pcol, b, e);
+        if (ok) a.hpart[(size_t)ch * LPR + gl] = s;
     }
-    for (; p < e; p++) s0 += Cc[(size_t)pcol[p] * 32 + lane];
-    return (s0 + s1) + (s2 + s3);
+    // the next rows' offsets are loaded ahead of the current rows' gathers
+    int32_t v = gwarp * RPW + grp;
+    int32_t b = v < a.n ? __ldg(&a.prow[v]) : 0, e = v < a.n ? __ldg(&a.prow[v + 1]) : 0;
+    for (int32_t v0 = gwarp * RPW; v0 < a.n; v0 += nwarps * RPW) {
+        const int32_t vn = v + nwarps * RPW;
+        const int32_t bn = vn < a.n ? __ldg(&a.prow[vn]) : 0, en = vn < a.n ? __ldg(&a.prow[vn + 1]) : 0;
+        const bool row = v < a.n && e - b <= PPR_HEAVY;
+        const float4 s = ppr_gather<LPR>(C, a.pcol, b, row ? e : b);
+        if (row) ppr_apply<LPR, DANG>(a, cur, v, s, l);
+        v = vn;
+        b = bn;
+        e = en;
+    }
+    ppr_block_partials<LPR, PPR_THREADS>(a, blockIdx.x, l);
 }
 
-__global__ void __launch_bounds__(THREADS) k_ppr_sweep(PPArgs a)
+// Closes a sweep: the heavy rows (a warp each: its lane groups take every
+// (32 / LPR)-th chunk, combined by a fixed xor tree), then the last block to
+// arrive adds up every block's residual and dangling sums (a warp per share
+// of the slots, fixed order) and updates the loop state.  (One warp adding
+// 2,432 slots one after another took 300 us of an 830 us sweep.)
+template <int LPR, bool DANG>
+__global__ void __launch_bounds__(PPR_CLOSE_THREADS, PPR_CLOSE_PER_SM) k_ppr_close(PPArgs a, int sweep_blocks, float tol,
+                                                                 cudaGraphConditionalHandle h, int use_cond)
 {
-    const PPCtl c = *a.ctl;
-    if (c.more == 0) return;
-    const float *Cc = c.cur ? a.C1 : a.C0;
-    const int lane = mgd::lane();
-    const int gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int nwarps = (gridDim.x * blockDim.x) >> 5;
-    const int32_t seed = lane < a.nseed ? a.seeds[lane] : -1;
-    const float dang = (float)a.dang[lane];
-    double resid = 0.0, dnext = 0.0;
-    for (int32_t v = gwarp; v < a.n; v += nwarps) {
-        int32_t b = a.prow[v], e = a.prow[v + 1];
-        if (e - b > PPR_HEAVY) continue;  // warp-uniform
-        float s = ppr_gather(Cc, a.pcol, b, e, lane);
-        ppr_apply(a, c, v, s, lane, dang, seed, resid, dnext);
-    }
-    for (int32_t ch = gwarp; ch < a.nhchunks; ch += nwarps) {
-        int32_t b = a.hchunk[3 * ch + 1], e = a.hchunk[3 * ch + 2];
-        a.hpart[(size_t)ch * 32 + lane] = ppr_gather(Cc, a.pcol, b, e, lane);
-    }
-    ppr_block_partials(a, blockIdx.x, resid, dnext);
-}
-
-__global__ void __launch_bounds__(THREADS) k_ppr_heavy(PPArgs a)
-{
-    const PPCtl c = *a.ctl;
-    if (c.more == 0) return;
-    const int lane = mgd::lane();
-    const int gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int nwarps = (gridDim.x * blockDim.x) >> 5;
-    const int32_t seed = lane < a.nseed ? a.seeds[lane] : -1;
-    const float dang = (float)a.dang[lane];
-    double resid = 0.0, dnext = 0.0;
-    for (int32_t i = gwarp; i < a.nhrows; i += nwarps) {
-        int32_t v = a.hrows[i];
-        float s = 0.0f;
-        for (int32_t k = a.hrow_chunk[i]; k < a.hrow_chunk[i + 1]; k++) s += a.hpart[(size_t)k * 32 + lane];
-        ppr_apply(a, c, v, s, lane, dang, seed, resid, dnext);
-    }
-    ppr_block_partials(a, gridDim.x + blockIdx.x, resid, dnext);
-}
-
-__global__ void k_ppr_finish(PPArgs a, int nslots, float tol, cudaGraphConditionalHandle h, int use_cond)
-{
-    const int lane = threadIdx.x;  // 32 threads, lane = seed
     PPCtl *ctl = a.ctl;
-    int more = ctl->more;
-    if (more) {
-        double R = 0, D = 0;
-        for (int b = 0; b < nslots; b++) {
-            R += a.bpart[((size_t)b * 32 + lane) * 2];
-            D += a.bpart[((size_t)b * 32 + lane) * 2 + 1];
-        }
-        ctl->resid[lane] = R;
-        a.dang[lane] = D;
-        int cont = (lane < a.nseed) && (R > (double)tol);
-        cont = __any_sync(0xffffffffu, cont);
-        if (lane == 0) {
-            ctl->iter += 1;
-            ctl->cur ^= 1;
-            if (cont && ctl->iter >= ctl->max_iter) { ctl->status = 1; cont = 0; }
-            ctl->more = cont;
-        }
-        more = cont;
+    if (ctl->more == 0) {
+        if (blockIdx.x == 0 && threadIdx.x == 0 && use_cond) cudaGraphSetConditional(h, 0u);
+        return;
     }
-    if (lane == 0 && use_cond) cudaGraphSetConditional(h, more ? 1u : 0u);
+    constexpr int RPW = 32 / LPR, NW = PPR_CLOSE_THREADS / 32;
+    const int cur = ctl->cur;
+    const int gl = threadIdx.x & (LPR - 1), grp = mgd::lane() / LPR, warp = threadIdx.x >> 5;
+    const int gwarp = blockIdx.x * NW + warp;
+    PprLane l = ppr_lane<LPR>(a);
+    for (int32_t i = gwarp; i < a.nhrows; i += gridDim.x * NW) {
+        const int32_t v = __ldg(&a.hrows[i]), k1 = __ldg(&a.hrow_chunk[i + 1]);
+        int32_t k = __ldg(&a.hrow_chunk[i]) + grp;
+        float4 s = make_float4(0.f, 0.f, 0.f, 0.f), low = s;
+        for (; k + 3 * RPW < k1; k += 4 * RPW) {
+            float4 t[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) t[j] = __ldcs(&a.hpart[(size_t)(k + j * RPW) * LPR + gl]);
+            f4_kahan(s, low, f4_add(f4_add(t[0], t[1]), f4_add(t[2], t[3])));
+        }
+        for (; k < k1; k += RPW) f4_kahan(s, low, __ldcs(&a.hpart[(size_t)k * LPR + gl]));
+#pragma unroll
+        for (int o = LPR; o < 32; o <<= 1)
+            s = f4_add(s, make_float4(__shfl_xor_sync(0xffffffffu, s.x, o), __shfl_xor_sync(0xffffffffu, s.y, o),
+                                      __shfl_xor_sync(0xffffffffu, s.z, o), __shfl_xor_sync(0xffffffffu, s.w, o)));
+        if (grp == 0) ppr_apply<LPR, DANG>(a, cur, v, s, l);
+    }
+    ppr_block_partials<LPR, PPR_CLOSE_THREADS>(a, sweep_blocks + blockIdx.x, l);
+    __shared__ int s_last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(&ctl->done, 1) == (int)gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __shared__ double tr[NW][32], td[NW][32];
+    const int lane = mgd::lane(), nslots = sweep_blocks + gridDim.x;
+    double R = 0.0, D = 0.0;
+    int b = warp;
+    for (; b + 3 * NW < nslots; b += 4 * NW) {
+        double2 t[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) t[j] = __ldcg(&a.bpart[(size_t)(b + j * NW) * 32 + lane]);
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            R += t[j].x;
+            D += t[j].y;
+        }
+    }
+    for (; b < nslots; b += NW) {
+        const double2 t = __ldcg(&a.bpart[(size_t)b * 32 + lane]);
+        R += t.x;
+        D += t.y;
+    }
+    tr[warp][lane] = R;
+    td[warp][lane] = D;
+    __syncthreads();
+    if (warp != 0) return;
+    for (int w = 1; w < NW; w++) {
+        R += tr[w][lane];
+        D += td[w][lane];
+    }
+    ctl->resid[lane] = R;
+    a.dang[lane] = D;
+    int more = __any_sync(0xffffffffu, lane < ctl->nseed && R > (double)tol);
+    if (lane == 0) {
+        ctl->iter += 1;
+        ctl->cur = cur ^ 1;
+        ctl->done = 0;
+        if (more && ctl->iter >= ctl->max_iter) {
+            ctl->status = 1;
+            more = 0;
+        }
+        ctl->more = more;
+        if (use_cond) cudaGraphSetConditional(h, more ? 1u : 0u);
+    }
 }
 
-__global__ void k_ppr_store(int32_t n, const float *X, int32_t nseed, int32_t s0, float *out)
+// The pass's result rows out[s0 + s][v] in caller order: 32 caller vertices
+// at a time through a shared-memory tile, so both the 16 LPR byte rows of X
+// and the result rows move in whole lines.  old2new null: the ids are equal.
+__global__ void __launch_bounds__(THREADS) k_ppr_store(int32_t n, const float *X, int32_t width, const int32_t *old2new,
+                                                       int32_t nseed, float *out)
 {
-    const size_t total = (size_t)n * 32;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        int s = (int)(i & 31);
-        if (s < nseed) out[(size_t)(s0 + s) * n + (i >> 5)] = X[i];
+    __shared__ float tile[THREADS / 32][32][33];
+    float (*t)[33] = tile[threadIdx.x >> 5];
+    const int lane = mgd::lane();
+    const int32_t gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+    for (int64_t v0 = (int64_t)gwarp * 32; v0 < n; v0 += (int64_t)nwarps * 32) {
+        const int cnt = (int)min((int64_t)32, n - v0);
+        int32_t src = 0;
+        if (lane < cnt) src = old2new ? __ldg(&old2new[v0 + lane]) : (int32_t)(v0 + lane);
+        for (int k = 0; k < cnt; k++) {
+            const int32_t u = __shfl_sync(0xffffffffu, src, k);
+            if (lane < width) t[k][lane] = __ldcs(&X[(size_t)u * width + lane]);
+        }
+        __syncwarp();
+        if (lane < cnt)
+            for (int s = 0; s < nseed; s++) __stcs(&out[(size_t)s * n + v0 + lane], t[lane][s]);
+        __syncwarp();
     }
 }
 
@@ -1072,8 +1233,8 @@ struct PrWS {
 };
 
 struct PprWS {
-    mgi::DevBuf X0, X1, C0, C1, seeds, ctl, bpart, dang, hpart, out;
-    mgi::LoopGraph lg;
+    mgi::DevBuf X0, X1, C0, C1, seeds, gseeds, ctl, bpart, dang, hpart, out;
+    mgi::LoopGraph lg[8];   // by lanes per row and dangling vertices
 };
 
 struct WprWS {};
@@ -1097,9 +1258,10 @@ void free_ppr_ws(mg_graph *g)
 {
     if (!g->ppws) return;
     PprWS *w = g->ppws;
-    DevBuf *bufs[] = {&w->X0, &w->X1, &w->C0, &w->C1, &w->seeds, &w->ctl, &w->bpart, &w->dang, &w->hpart, &w->out};
+    DevBuf *bufs[] = {&w->X0, &w->X1, &w->C0, &w->C1, &w->seeds, &w->gseeds, &w->ctl, &w->bpart, &w->dang,
+                      &w->hpart, &w->out};
     for (DevBuf *b : bufs) dev_free(*b);
-    w->lg.destroy();
+    for (auto &l : w->lg) l.destroy();
     delete w;
     g->ppws = nullptr;
 }
@@ -1441,6 +1603,56 @@ mg_status mg_wpagerank_backward(mg_graph *g, const float *g_host, const mg_opts 
     return copy_out(g, grad_w_out, w->grad_caller.p, (size_t)g->ne * 4);
 }
 
+}  // extern "C"
+
+// one pass of up to 4 LPR seeds: sweeps until every seed's L1 change is at
+// most tol
+template <int LPR, bool DANG>
+static mg_status ppr_pass(mg_graph *g, const PPArgs &a, const int32_t *seeds_dev, int32_t nseed, const mg_opts &opt,
+                          float tol, int32_t max_iter, PPCtl &hc)
+{
+    PprWS *w = g->ppws;
+    cudaStream_t s = g->stream;
+    const size_t bytes = (size_t)std::max(g->nv, 1) * LPR * 16;
+    const int grid = launch_grid(g, PPR_THREADS, PPR_PER_SM), close_grid = launch_grid(g, PPR_CLOSE_THREADS, PPR_CLOSE_PER_SM);
+    MG_CUDA(cudaMemsetAsync(a.X[0], 0, bytes, s));
+    MG_CUDA(cudaMemsetAsync(a.C[0], 0, bytes, s));
+    k_ppr_init<<<1, 32, 0, s>>>(a, seeds_dev, nseed, 4 * LPR, max_iter);
+    MG_CUDA(cudaGetLastError());
+    Profiler &P = g->prof;
+    const int sl = P.slot("ppr_pull"), sc = P.slot("ppr_close");
+    BodyFn body = [&](cudaStream_t st, cudaGraphConditionalHandle h, int use_cond) -> mg_status {
+        P.begin(sl);
+        k_ppr_sweep<LPR, DANG><<<grid, PPR_THREADS, 0, st>>>(a);
+        P.end();
+        P.begin(sc);
+        k_ppr_close<LPR, DANG><<<close_grid, PPR_CLOSE_THREADS, 0, st>>>(a, grid, tol, h, use_cond);
+        P.end();
+        MG_CUDA(cudaGetLastError());
+        return MG_OK;
+    };
+    // the captured kernels take the whole PPArgs (pointers, counts, the
+    // heavy-row table, damping), the tolerance and the grids by value; the
+    // pass's seeds lie in a buffer, so every pass of a call replays one loop
+    const LoopKey key = LoopKey().add(a).add(tol).add(grid).add(close_grid);
+    const int slot = (LPR == 1 ? 0 : LPR == 2 ? 1 : LPR == 4 ? 2 : 3) * 2 + (DANG ? 1 : 0);
+    MG_TRY(run_loop(opt.profile ? MG_EXEC_HOST : opt.exec, opt.profile != 0, s, w->lg[slot], key, body, &a.ctl->more,
+                    g->pinned_flag, max_iter + 2));
+    MG_CUDA(cudaMemcpyAsync(&hc, a.ctl, sizeof(PPCtl), cudaMemcpyDeviceToHost, s));
+    MG_CUDA(cudaStreamSynchronize(s));
+    return MG_OK;
+}
+
+template <int LPR>
+static mg_status ppr_pass(mg_graph *g, const PPArgs &a, const int32_t *seeds_dev, int32_t nseed, const mg_opts &opt,
+                          float tol, int32_t max_iter, PPCtl &hc)
+{
+    return g->n_dangling > 0 ? ppr_pass<LPR, true>(g, a, seeds_dev, nseed, opt, tol, max_iter, hc)
+                             : ppr_pass<LPR, false>(g, a, seeds_dev, nseed, opt, tol, max_iter, hc);
+}
+
+extern "C" {
+
 mg_status mg_ppr_batch(mg_graph *g, const int32_t *seeds, int32_t nseeds, const mg_opts *o, float *out,
                        mg_run_info *info)
 {
@@ -1452,7 +1664,6 @@ mg_status mg_ppr_batch(mg_graph *g, const int32_t *seeds, int32_t nseeds, const 
     if (!g->ppws) g->ppws = new PprWS();
     PprWS *w = g->ppws;
     const size_t n = (size_t)std::max(g->nv, 1);
-    const int grid = launch_grid(g, THREADS, 8);
     cudaStream_t s = g->stream;
     // heavy-row chunk table for PPR (built once per graph from the pull offsets)
     if (g->ppr_nhchunks < 0) {
@@ -1478,15 +1689,19 @@ mg_status mg_ppr_batch(mg_graph *g, const int32_t *seeds, int32_t nseeds, const 
         g->ppr_nhchunks = (int32_t)(hc.size() / 3);
         g->ppr_nhrows = (int32_t)hr.size();
     }
-    MG_TRY(dev_alloc(w->X0, n * 32 * 4));
-    MG_TRY(dev_alloc(w->X1, n * 32 * 4));
-    MG_TRY(dev_alloc(w->C0, n * 32 * 4));
-    MG_TRY(dev_alloc(w->C1, n * 32 * 4));
+    // lanes per row: as many as the widest pass of this call needs
+    const int32_t widest = std::min(nseeds, 32);
+    const size_t width = widest > 16 ? 32 : widest > 8 ? 16 : widest > 4 ? 8 : 4;
+    MG_TRY(dev_alloc(w->X0, n * width * 4));
+    MG_TRY(dev_alloc(w->X1, n * width * 4));
+    MG_TRY(dev_alloc(w->C0, n * width * 4));
+    MG_TRY(dev_alloc(w->C1, n * width * 4));
     MG_TRY(dev_alloc(w->seeds, (size_t)std::max(nseeds, 1) * 4));
+    MG_TRY(dev_alloc(w->gseeds, 32 * 4));
     MG_TRY(dev_alloc(w->ctl, sizeof(PPCtl)));
-    MG_TRY(dev_alloc(w->bpart, (size_t)2 * grid * 32 * 2 * 8));
+    MG_TRY(dev_alloc(w->bpart, (size_t)g->num_sms * (PPR_PER_SM + PPR_CLOSE_PER_SM) * 32 * sizeof(double2)));
     MG_TRY(dev_alloc(w->dang, 32 * 8));
-    MG_TRY(dev_alloc(w->hpart, (size_t)std::max(g->ppr_nhchunks, 1) * 32 * 4));
+    MG_TRY(dev_alloc(w->hpart, (size_t)std::max(g->ppr_nhchunks, 1) * width * 4));
     MG_TRY(dev_alloc(w->out, (size_t)std::max(nseeds, 1) * n * 4));
     std::vector<int32_t> eseeds(seeds, seeds + nseeds);
     for (int32_t &v : eseeds) v = to_engine(g, v);
@@ -1497,54 +1712,37 @@ mg_status mg_ppr_batch(mg_graph *g, const int32_t *seeds, int32_t nseeds, const 
     std::memset(&a, 0, sizeof(a));
     a.n = g->nv;
     a.prow = g->trow; a.pcol = g->tcol; a.outrow = g->row.as<int32_t>();
+    a.seeds = w->gseeds.as<int32_t>();
     a.hchunk = g->ppr_hchunk.as<int32_t>(); a.nhchunks = g->ppr_nhchunks;
     a.hrows = g->ppr_hrows.as<int32_t>(); a.hrow_chunk = g->ppr_hrow_chunk.as<int32_t>(); a.nhrows = g->ppr_nhrows;
-    a.X0 = w->X0.as<float>(); a.X1 = w->X1.as<float>(); a.C0 = w->C0.as<float>(); a.C1 = w->C1.as<float>();
-    a.hpart = w->hpart.as<float>();
-    a.bpart = w->bpart.as<double>();
+    a.X[0] = w->X0.as<float4>(); a.X[1] = w->X1.as<float4>();
+    a.C[0] = w->C0.as<float4>(); a.C[1] = w->C1.as<float4>();
+    a.hpart = w->hpart.as<float4>();
+    a.bpart = w->bpart.as<double2>();
     a.dang = w->dang.as<double>();
     a.ctl = w->ctl.as<PPCtl>();
     a.damping = opt.damping > 0 ? opt.damping : 0.85f;
-    Profiler &P = g->prof;
-    const int sl = P.slot("ppr_pull"), sh = P.slot("ppr_heavy"), sf = P.slot("ppr_finish");
     int32_t total_iters = 0;
     double max_resid = 0.0;
     for (int32_t s0 = 0; s0 < nseeds; s0 += 32) {
-        a.nseed = std::min(32, nseeds - s0);
-        a.seeds = w->seeds.as<int32_t>() + s0;
-        k_ppr_init<<<grid, THREADS, 0, s>>>(a, max_iter);
-        BodyFn body = [&](cudaStream_t st, cudaGraphConditionalHandle h, int use_cond) -> mg_status {
-            P.begin(sl);
-            k_ppr_sweep<<<grid, THREADS, 0, st>>>(a);
-            P.end();
-            P.begin(sh);
-            k_ppr_heavy<<<grid, THREADS, 0, st>>>(a);
-            P.end();
-            P.begin(sf);
-            k_ppr_finish<<<1, 32, 0, st>>>(a, 2 * grid, tol, h, use_cond);
-            P.end();
-            MG_CUDA(cudaGetLastError());
-            return MG_OK;
-        };
-        // the captured kernels take the whole PPArgs (pointers, counts, the
-        // heavy-row table, damping), the tolerance and the grid by value
-        const LoopKey key = LoopKey().add(a).add(tol).add(grid);
-        MG_TRY(run_loop(opt.profile ? MG_EXEC_HOST : opt.exec, opt.profile != 0, s, w->lg, key, body, &a.ctl->more,
-                        g->pinned_flag, max_iter + 2));
+        const int32_t cnt = std::min(32, nseeds - s0);
+        const int32_t *sd = w->seeds.as<int32_t>() + s0;
         PPCtl hc;
-        MG_CUDA(cudaMemcpyAsync(&hc, w->ctl.p, sizeof(PPCtl), cudaMemcpyDeviceToHost, s));
-        MG_CUDA(cudaStreamSynchronize(s));
+        int32_t pass_width;
+        if (cnt > 16) { pass_width = 32; MG_TRY(ppr_pass<8>(g, a, sd, cnt, opt, tol, max_iter, hc)); }
+        else if (cnt > 8) { pass_width = 16; MG_TRY(ppr_pass<4>(g, a, sd, cnt, opt, tol, max_iter, hc)); }
+        else if (cnt > 4) { pass_width = 8; MG_TRY(ppr_pass<2>(g, a, sd, cnt, opt, tol, max_iter, hc)); }
+        else { pass_width = 4; MG_TRY(ppr_pass<1>(g, a, sd, cnt, opt, tol, max_iter, hc)); }
         if (hc.status) return fail(MG_ERR_ITER_LIMIT, "PPR did not converge in %d sweeps", max_iter);
         total_iters += hc.iter;
-        for (int i = 0; i < a.nseed; i++) max_resid = std::max(max_resid, hc.resid[i]);
-        const float *X = hc.cur ? a.X1 : a.X0;
-        k_ppr_store<<<grid, THREADS, 0, s>>>(g->nv, X, a.nseed, s0, w->out.as<float>());
+        for (int i = 0; i < cnt; i++) max_resid = std::max(max_resid, hc.resid[i]);
+        k_ppr_store<<<launch_grid(g, THREADS, 6), THREADS, 0, s>>>(
+            g->nv, (const float *)a.X[hc.cur], pass_width, g->relabeled ? g->old2new.as<int32_t>() : nullptr, cnt,
+            w->out.as<float>() + (size_t)s0 * g->nv);
         MG_CUDA(cudaGetLastError());
     }
-    const void *res = nullptr;
-    MG_TRY(to_caller(g, 7, w->out.p, 4, nseeds, &res));
     MG_TRY(end_run(g, opt, info));
     if (info) { info->iterations = total_iters; info->residual = max_resid; }
-    return copy_out(g, out, res, (size_t)nseeds * g->nv * 4);
+    return copy_out(g, out, w->out.p, (size_t)nseeds * g->nv * 4);
 }
 }  // extern "C"
