@@ -595,12 +595,56 @@ __global__ void k_sym_check(int32_t n, const int32_t *row, const int32_t *col, c
     wmin_flush(&sums[3], wlo);
 }
 
-// inverse of k_relabel_edges for per-edge payloads (engine order -> caller order)
-__global__ void k_unrelabel_edges(int32_t m, const int32_t *__restrict__ cpos, const uint32_t *__restrict__ src,
-                                  uint32_t *__restrict__ dst)
+// Edge values ct[u].x * (val[v] - ct[u].y) straight to caller order: a lane
+// per engine position (coalesced columns and positions, one gather of val
+// and one of ct, a scattered 4-byte store), four 32-position steps per warp
+// with every load of a step ahead of its stores.  (A warp per row kept the
+// hub rows on one warp each: 726 us on R-MAT 19 with the row totals; 2 x
+// 30 us now, and no engine-order copy to carry over.)
+__global__ void __launch_bounds__(256) k_edge_grad(int32_t m, const int32_t *row_new, const int32_t *pos_row,
+                                                   const int32_t *__restrict__ cpos, const int32_t *__restrict__ col,
+                                                   const float2 *__restrict__ ct, const float *__restrict__ val,
+                                                   float *__restrict__ out)
 {
-    for (int32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < m; p += gridDim.x * blockDim.x)
-        dst[__ldcs(&cpos[p])] = __ldcs(&src[p]);
+    const int lane = threadIdx.x & 31;
+    const int32_t nsteps = (m + 31) / 32;
+    const int32_t gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+    for (int32_t c0 = gwarp * RELABEL_ILP; c0 < nsteps; c0 += nwarps * RELABEL_ILP) {
+        int32_t q[RELABEL_ILP], u[RELABEL_ILP], rr[RELABEL_ILP], st[RELABEL_ILP];
+#pragma unroll
+        for (int j = 0; j < RELABEL_ILP; j++) {
+            const int64_t p = (int64_t)(c0 + j) * 32 + lane;
+            q[j] = p < m ? __ldcs(&cpos[p]) : -1;
+            u[j] = p < m ? __ldcs(&col[p]) : 0;
+        }
+        engine_rows(m, row_new, pos_row, c0, rr, st);
+        float x[RELABEL_ILP];
+        float2 r[RELABEL_ILP];
+#pragma unroll
+        for (int j = 0; j < RELABEL_ILP; j++) {
+            x[j] = __ldg(&val[u[j]]);
+            r[j] = __ldg(&ct[rr[j]]);
+        }
+#pragma unroll
+        for (int j = 0; j < RELABEL_ILP; j++)
+            if (q[j] >= 0) out[q[j]] = r[j].x * (x[j] - r[j].y);
+    }
+}
+
+// the same without relabeling (rows below 128 edges): an 8-lane group a row
+__global__ void __launch_bounds__(256) k_edge_grad_rows(int32_t n, const int32_t *__restrict__ row,
+                                                        const int32_t *__restrict__ col,
+                                                        const float2 *__restrict__ ct, const float *__restrict__ val,
+                                                        float *__restrict__ out)
+{
+    const int gl = threadIdx.x & 7;
+    for (int64_t u = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3; u < n;
+         u += ((int64_t)gridDim.x * blockDim.x) >> 3) {
+        const float2 r = __ldg(&ct[u]);
+        for (int32_t p = __ldg(&row[u]) + gl, e = __ldg(&row[u + 1]); p < e; p += 8)
+            __stcs(&out[p], r.x * (__ldg(&val[__ldcs(&col[p])]) - r.y));
+    }
 }
 
 // caller-order result: dst[r*n + v] = src[r*n + old2new[v]]
@@ -762,15 +806,15 @@ mg_status edges_to_engine(mg_graph *g, const void *src_caller, void *dst_engine)
     return MG_OK;
 }
 
-mg_status edges_to_caller(mg_graph *g, const void *src_engine, void *dst_caller)
+mg_status edge_grad_to_caller(mg_graph *g, const float2 *ct, const float *val, float *out)
 {
-    if (!g->relabeled) {
-        MG_CUDA(cudaMemcpyAsync(dst_caller, src_engine, (size_t)g->ne * 4, cudaMemcpyDeviceToDevice, g->stream));
-        return MG_OK;
-    }
     if (g->ne == 0) return MG_OK;
-    k_unrelabel_edges<<<g->num_sms * 8, 256, 0, g->stream>>>(g->ne, g->cpos.as<int32_t>(),
-                                                             (const uint32_t *)src_engine, (uint32_t *)dst_caller);
+    const int grid = g->num_sms * 8;
+    if (g->relabeled)
+        k_edge_grad<<<grid, 256, 0, g->stream>>>(g->ne, g->row.as<int32_t>(), g->pos_row.as<int32_t>(),
+                                                 g->cpos.as<int32_t>(), g->col.as<int32_t>(), ct, val, out);
+    else
+        k_edge_grad_rows<<<grid, 256, 0, g->stream>>>(g->nv, g->row.as<int32_t>(), g->col.as<int32_t>(), ct, val, out);
     MG_CUDA(cudaGetLastError());
     return MG_OK;
 }
@@ -861,6 +905,7 @@ static mg_status upload_arrays(mg_graph *g, const mg_host_graph *h, const HostLa
     }
     MG_TRY(upload_bins(g, L));
     g->hub.valid = false;  // new pull columns
+    g->col_version += 1;
     g->h_prow = L.prow;
     g->symmetric = L.symmetric;
     g->weights_symmetric = L.wsym;
@@ -1061,7 +1106,10 @@ mg_status mg_graph_commit(mg_graph *g)
             g->min_weight = wmin_decode(g->sym_host[3]);
             // PageRank's hub split follows the columns: rebuilt only when
             // some column id changed
-            if (g->sym_host[4] != 0) g->hub.valid = false;
+            if (g->sym_host[4] != 0) {
+                g->hub.valid = false;
+                g->col_version += 1;
+            }
             if (g->relabeled) {
                 // the staged arrays are now the current graph's caller-order CSR
                 std::swap(g->o_row, g->s_row);

@@ -185,6 +185,7 @@ struct mg_graph {
     mgi::DevBuf fw;
     bool has_fw = false;
     uint64_t fw_version = 0;       // bumped whenever fw or the CSR changes
+    uint64_t col_version = 1;      // bumped whenever the columns (or their order) may have changed
     // hub-first relabeling: the engines run on ids ordered by descending
     // log2 degree; results are mapped back before they leave the library
     bool relabeled = false;
@@ -234,7 +235,9 @@ mg_status vertices_to_engine(mg_graph *g, const void *src_caller, void *dst_engi
 mg_status cc_to_caller(mg_graph *g, const int32_t *parent, const void **out);
 // per-edge 4-byte payloads between caller CSR order and engine CSR order
 mg_status edges_to_engine(mg_graph *g, const void *src_caller, void *dst_engine);
-mg_status edges_to_caller(mg_graph *g, const void *src_engine, void *dst_caller);
+// out[caller position of (u, v)] = ct[u].x * (val[v] - ct[u].y) over every
+// edge, ct and val in engine ids
+mg_status edge_grad_to_caller(mg_graph *g, const float2 *ct, const float *val, float *out);
 // new degree bins / heavy chunks (heavy-row threshold, chunk edges, thread
 // bin cutoff) from the
 // host copy of the pull-side row offsets; drops the algorithm workspaces

@@ -847,36 +847,139 @@ __global__ void k_pr_ctl_init(PCtl *c, int32_t n, int32_t max_iter, float dampin
     pctl_derive(c);
 }
 
-// weighted: out-weight sums S[u] = sum_e w[e] (CSR order)
-__global__ void k_row_sums(int32_t n, const int32_t *row, const float *w, float *S)
+// Loop control for the adjoint: start mean of lambda = mean of g (for
+// dangling rows); the stopping threshold relative to |g|_1 (lambda scales
+// with g, and an absolute L1 threshold would sit below FP32 resolution for
+// large n).  part: (sum g, sum |g|) of each block of k_gvec_sums, added in
+// slot order.  (The host used to add g up while the GPU waited.)
+__global__ void __launch_bounds__(THREADS) k_gvec_sums(int32_t n, const float *g, double2 *part)
 {
-    for (int32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < n; u += gridDim.x * blockDim.x) {
-        float s = 0.0f;
-        for (int32_t p = row[u]; p < row[u + 1]; p++) s += w[p];
-        S[u] = s;
+    __shared__ double2 sp[THREADS / 32];
+    double a = 0.0, b = 0.0;
+    for (int32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
+        const double x = (double)g[v];
+        a += x;
+        b += fabs(x);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        a += __shfl_xor_sync(0xffffffffu, a, o);
+        b += __shfl_xor_sync(0xffffffffu, b, o);
+    }
+    if (mgd::lane() == 0) sp[threadIdx.x >> 5] = make_double2(a, b);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < THREADS / 32; w++) {
+            a += sp[w].x;
+            b += sp[w].y;
+        }
+        part[blockIdx.x] = make_double2(a, b);
     }
 }
 
-// adjoint edge scatter: grad[e] = d x_u / S_u * (lambda_v - t_u),
-// t_u = sum_k P_uk lambda_k recomputed over the row (warp per row)
-__global__ void __launch_bounds__(THREADS) k_wpr_grad(int32_t n, const int32_t *row, const int32_t *col,
-                                                      const float *w, const float *S, const float *x,
-                                                      const float *lam, float damping, float *grad)
+__global__ void k_adjoint_ctl_init(PCtl *c, int32_t n, int32_t max_iter, float damping, float tol, const double2 *part,
+                                   int nparts)
 {
-    const int lane = mgd::lane();
-    const int gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int nwarps = (gridDim.x * blockDim.x) >> 5;
-    for (int32_t u = gwarp; u < n; u += nwarps) {
-        int32_t b = row[u], e = row[u + 1];
-        float Su = S[u];
-        float t = 0.0f;
-        for (int32_t p = b + lane; p < e; p += 32) t += w[p] * lam[col[p]];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-        float coef = Su > 0.0f ? damping * x[u] / Su : 0.0f;
-        float tu = Su > 0.0f ? t / Su : 0.0f;
-        for (int32_t p = b + lane; p < e; p += 32) grad[p] = coef * (lam[col[p]] - tu);
+    double a = 0.0, b = 0.0;
+    for (int i = threadIdx.x; i < nparts; i += 32) {
+        const double2 p = part[i];
+        a += p.x;
+        b += p.y;
     }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        a += __shfl_xor_sync(0xffffffffu, a, o);
+        b += __shfl_xor_sync(0xffffffffu, b, o);
+    }
+    if (threadIdx.x != 0) return;
+    std::memset(c, 0, sizeof(PCtl));
+    c->more = 1;
+    c->max_iter = max_iter;
+    c->damping = damping;
+    c->tol = (float)(tol * fmax(b, 1e-30));
+    c->n = n;
+    c->lam_mean = n > 0 ? a / n : 0.0;
+    pctl_derive(c);
+}
+
+// Row totals over the degree bins of the pull rows (the graph is symmetric,
+// so they are the out-rows too) and CTA-sized chunks of the heavy rows, whose
+// partials k_row_total_heavy adds in order.  RowWeights: S[u] = sum_e w[e];
+// RowBack: the adjoint's row value t_u = sum_e w[e] lam[v] / S[u] and the
+// factor d x_u / S_u of its edges, ct[u] = (factor, t_u).  (A thread per row
+// for S kept one thread on a hub row: 1.3 ms on R-MAT 19; 30 us now.)
+struct RowWeights {
+    using T = float;
+    static constexpr bool kRowAware = false, kWeights = true;
+    float *S;
+    __device__ T identity() const { return 0.0f; }
+    __device__ bool skip(int32_t) const { return false; }
+    __device__ T edge(int32_t, int32_t, int32_t, int32_t w) const { return __int_as_float(w); }
+    __device__ T combine(T x, T y) const { return x + y; }
+    __device__ void flush() {}
+    __device__ void finish(int32_t u, T s) { S[u] = s; }
+};
+
+struct RowBack {
+    using T = float;
+    static constexpr bool kRowAware = false, kWeights = true;
+    const float *S, *x, *lam;
+    float damping;
+    float2 *ct;
+    __device__ T identity() const { return 0.0f; }
+    __device__ bool skip(int32_t) const { return false; }
+    __device__ T edge(int32_t, int32_t, int32_t v, int32_t w) const { return __int_as_float(w) * lam[v]; }
+    __device__ T combine(T x, T y) const { return x + y; }
+    __device__ void flush() {}
+    __device__ void finish(int32_t u, T s)
+    {
+        const float Su = S[u];
+        ct[u] = Su > 0.0f ? make_float2(damping * x[u] / Su, s / Su) : make_float2(0.0f, 0.0f);
+    }
+};
+
+template <class Op>
+__global__ void __launch_bounds__(THREADS) k_row_total(PArgs a, Op op)
+{
+    const int32_t *pwt = reinterpret_cast<const int32_t *>(a.pw);
+    mgd::bins_reduce(op, a.prow, a.pcol, pwt, a.wrows, a.nwrows, a.nwlong, a.trows, a.ntrows);
+    __shared__ float s_part[THREADS / 32];
+    for (int32_t ch = blockIdx.x; ch < a.nhchunks; ch += gridDim.x) {
+        const int32_t u = a.hchunk[3 * ch], b = a.hchunk[3 * ch + 1], e = a.hchunk[3 * ch + 2];
+        float acc = 0.0f;
+        for (int32_t p = b + threadIdx.x; p < e; p += THREADS)
+            acc += op.edge(p, u, __ldcs(&a.pcol[p]), __ldcs(&pwt[p]));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if (mgd::lane() == 0) s_part[threadIdx.x >> 5] = acc;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            float s = 0.0f;
+            for (int w = 0; w < THREADS / 32; w++) s += s_part[w];
+            a.hpart[ch] = s;
+        }
+        __syncthreads();
+    }
+}
+
+template <class Op>
+__global__ void __launch_bounds__(THREADS) k_row_total_heavy(PArgs a, Op op)
+{
+    for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < a.nhrows; i += gridDim.x * blockDim.x) {
+        float s = 0.0f;
+        for (int32_t k = a.hrow_chunk[i]; k < a.hrow_chunk[i + 1]; k++) s += a.hpart[k];
+        op.finish(a.hrows[i], s);
+    }
+}
+
+template <class Op>
+mg_status row_totals(const mg_graph *g, const PArgs &a, const Op &op)
+{
+    k_row_total<Op><<<a.nblocks, THREADS, 0, g->stream>>>(a, op);
+    if (a.nhrows > 0)
+        k_row_total_heavy<Op><<<(a.nhrows + THREADS - 1) / THREADS, THREADS, 0, g->stream>>>(a, op);
+    MG_CUDA(cudaGetLastError());
+    return MG_OK;
 }
 
 // ---------------------------------------------------------------------------
@@ -1225,8 +1328,11 @@ __global__ void __launch_bounds__(THREADS) k_ppr_store(int32_t n, const float *X
 }  // namespace
 
 struct PrWS {
-    mgi::DevBuf x0, x1, c0, c1, active, hpart, bpart, ctl, S, wT, gvec, grad, lam_keep, xkeep;
-    mgi::DevBuf wT_caller, gvec_caller, grad_caller;  // caller-order staging of a relabeled graph
+    mgi::DevBuf x0, x1, c0, c1, active, hpart, bpart, ctl, S, wT, gvec, lam_keep, xkeep;
+    mgi::DevBuf gvec_caller, grad_caller;  // caller-order vectors
+    mgi::DevBuf tpos;          // int32 [ne]: caller position of the reverse of each engine position's edge
+    mgi::DevBuf ct, gsum;      // adjoint: row factors and totals; partial sums of g
+    uint64_t tpos_version = 0; // col_version that tpos was built from (0: none)
     mgi::DevBuf q0, q1, qval;  // data-driven queue sweeps
     uint64_t wT_version = 0;  // fw_version that S and wT were derived from (0: none)
     mgi::LoopGraph lg[6];
@@ -1246,8 +1352,8 @@ void free_pr_ws(mg_graph *g)
     if (!g->pws) return;
     PrWS *w = g->pws;
     DevBuf *bufs[] = {&w->x0, &w->x1, &w->c0, &w->c1, &w->active, &w->hpart, &w->bpart, &w->ctl, &w->S,
-                      &w->wT, &w->gvec, &w->grad, &w->lam_keep, &w->xkeep, &w->wT_caller, &w->gvec_caller,
-                      &w->grad_caller, &w->q0, &w->q1, &w->qval};
+                      &w->wT, &w->gvec, &w->lam_keep, &w->xkeep, &w->gvec_caller, &w->grad_caller, &w->tpos,
+                      &w->ct, &w->gsum, &w->q0, &w->q1, &w->qval};
     for (DevBuf *b : bufs) dev_free(*b);
     for (auto &l : w->lg) l.destroy();
     delete w;
@@ -1422,11 +1528,12 @@ static mg_status pr_setup(mg_graph *g, PArgs &a, bool weighted_or_adj, int32_t l
     return MG_OK;
 }
 
-// transposed float weights: wT[pos of (v,u) in row v] = w[pos of (u,v) in row u].
-// One thread per edge: the owner row u of position p by binary search over
-// the row offsets, then u among row v's (ascending) columns.
-__global__ void k_transpose_weights(int32_t n, int32_t m, const int32_t *row, const int32_t *col, const float *w,
-                                    float *wT)
+// Reverse positions of a symmetric CSR: rev[pos of (v,u) in row v] = pos of
+// (u,v) in row u.  One thread per edge: the owner row u of position p by
+// binary search over the row offsets, then u among row v's (ascending)
+// columns.  Once per set of columns; a new set of weights then costs one
+// gather (the searches took 535 us per set on R-MAT 19, the gather 45).
+__global__ void k_reverse_positions(int32_t n, int32_t m, const int32_t *row, const int32_t *col, int32_t *rev)
 {
     for (int32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < m; p += gridDim.x * blockDim.x) {
         int32_t lo = 0, hi = n - 1;  // last u with row[u] <= p
@@ -1442,7 +1549,25 @@ __global__ void k_transpose_weights(int32_t n, int32_t m, const int32_t *row, co
             if (cm == u) { q = mid; break; }
             if (cm < u) a = mid + 1; else b = mid - 1;
         }
-        if (q >= 0) wT[q] = __ldg(&w[p]);
+        if (q >= 0) rev[q] = p;
+    }
+}
+
+// dst[p] = src[at[p]] (0 where at[p] is -1), four positions a thread in flight
+__global__ void __launch_bounds__(THREADS) k_gather_weights(int32_t m, const int32_t *__restrict__ at,
+                                                            const float *__restrict__ src, float *__restrict__ dst)
+{
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < m; p += 4 * stride) {
+        int32_t q[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) q[j] = p + j * stride < m ? __ldcs(&at[p + j * stride]) : -1;
+        float x[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) x[j] = q[j] >= 0 ? __ldg(&src[q[j]]) : 0.0f;
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            if (p + j * stride < m) __stcs(&dst[p + j * stride], x[j]);
     }
 }
 
@@ -1510,20 +1635,41 @@ mg_status mg_wpagerank(mg_graph *g, const mg_opts *o, float *x_out, mg_run_info 
     MG_TRY(dev_alloc(w->xkeep, n * 4));
     if (w->wT_version != g->fw_version) {
         // out-weight sums and transposed weights, once per set of weights
+        a.prow = g->row.as<int32_t>();
+        a.pcol = g->col.as<int32_t>();
+        a.pw = g->fw.as<float>();
+        MG_TRY(row_totals(g, a, RowWeights{a.S}));
+        a.prow = g->trow;
+        a.pcol = g->tcol;
         const int egrid = launch_grid(g, THREADS, 16);
-        k_row_sums<<<grid, THREADS, 0, s>>>(g->nv, g->row.as<int32_t>(), g->fw.as<float>(), a.S);
-        if (g->relabeled) {
-            // transposed weights are located in the caller's CSR (ascending
-            // columns), then carried to engine order like the column ids
-            MG_TRY(dev_alloc(w->wT_caller, m * 4 + 16));
-            k_transpose_weights<<<egrid, THREADS, 0, s>>>(g->nv, g->ne, g->o_row.as<int32_t>(),
-                                                          g->o_col.as<int32_t>(), g->o_fw.as<float>(),
-                                                          w->wT_caller.as<float>());
-            MG_TRY(edges_to_engine(g, w->wT_caller.p, w->wT.p));
-        } else {
-            k_transpose_weights<<<egrid, THREADS, 0, s>>>(g->nv, g->ne, g->row.as<int32_t>(), g->col.as<int32_t>(),
-                                                          g->fw.as<float>(), w->wT.as<float>());
+        if (w->tpos_version != g->col_version) {
+            // the reverse positions are found in the caller's CSR (ascending
+            // columns) and carried to engine order like the column ids
+            MG_TRY(dev_alloc(w->tpos, m * 4));
+            DevBuf rev;
+            int32_t *at = w->tpos.as<int32_t>();
+            if (g->relabeled) {
+                MG_TRY(dev_alloc(rev, m * 4));
+                at = rev.as<int32_t>();
+            }
+            const int32_t *crow = g->relabeled ? g->o_row.as<int32_t>() : g->row.as<int32_t>();
+            const int32_t *ccol = g->relabeled ? g->o_col.as<int32_t>() : g->col.as<int32_t>();
+            cudaError_t e = cudaMemsetAsync(at, 0xff, (size_t)g->ne * 4, s);
+            k_reverse_positions<<<egrid, THREADS, 0, s>>>(g->nv, g->ne, crow, ccol, at);
+            if (e == cudaSuccess) e = cudaGetLastError();
+            mg_status st = MG_OK;
+            if (g->relabeled && e == cudaSuccess) {
+                st = edges_to_engine(g, at, w->tpos.p);
+                e = cudaStreamSynchronize(s);
+            }
+            dev_free(rev);
+            MG_TRY(st);
+            MG_CUDA(e);
+            w->tpos_version = g->col_version;
         }
+        k_gather_weights<<<egrid, THREADS, 0, s>>>(g->ne, w->tpos.as<int32_t>(),
+                                                   g->relabeled ? g->o_fw.as<float>() : g->fw.as<float>(),
+                                                   w->wT.as<float>());
         MG_CUDA(cudaGetLastError());
         w->wT_version = g->fw_version;
     }
@@ -1557,33 +1703,25 @@ mg_status mg_wpagerank_backward(mg_graph *g, const float *g_host, const mg_opts 
     const int grid = a.nblocks;
     const size_t n = (size_t)std::max(g->nv, 1), m = (size_t)std::max(g->ne, 1);
     MG_TRY(dev_alloc(w->gvec, n * 4));
-    MG_TRY(dev_alloc(w->grad, m * 4));
+    MG_TRY(dev_alloc(w->ct, n * sizeof(float2)));
+    MG_TRY(dev_alloc(w->gsum, (size_t)g->num_sms * sizeof(double2)));
     MG_TRY(dev_alloc(w->lam_keep, n * 4));
     MG_TRY(dev_alloc(w->gvec_caller, n * 4));
     MG_TRY(dev_alloc(w->grad_caller, m * 4));
     if (g->nv) MG_CUDA(cudaMemcpyAsync(w->gvec_caller.p, g_host, (size_t)g->nv * 4, cudaMemcpyHostToDevice, s));
     MG_TRY(vertices_to_engine(g, w->gvec_caller.p, w->gvec.p));
-    k_row_sums<<<grid, THREADS, 0, s>>>(g->nv, g->row.as<int32_t>(), g->fw.as<float>(), a.S);
     // lambda = g + d * P lambda : rows of P are the CSR rows (out-edges) with weights w
     a.prow = g->row.as<int32_t>();
     a.pcol = g->col.as<int32_t>();
     a.pw = g->fw.as<float>();
     a.gvec = w->gvec.as<float>();
+    MG_TRY(row_totals(g, a, RowWeights{a.S}));
     float d = opt.damping > 0 ? opt.damping : 0.85f;
     float tol = opt.tol > 0 ? opt.tol : 1e-6f;
     int max_iter = opt.max_iter > 0 ? opt.max_iter : 10000;
-    // initial mean of lambda = mean of g (for dangling rows)
-    // and the stopping threshold, relative to |g|_1: lambda scales with g,
-    // and an absolute L1 threshold would sit below FP32 resolution for
-    // large n
-    double gm = 0.0, g1 = 0.0;
-    for (int32_t i = 0; i < g->nv; i++) {
-        gm += g_host[i];
-        g1 += std::fabs((double)g_host[i]);
-    }
-    gm = g->nv ? gm / g->nv : 0.0;
-    const float tol_abs = (float)(tol * std::max(g1, 1e-30));
-    k_pr_ctl_init<<<1, 32, 0, s>>>(a.ctl, g->nv, max_iter, d, tol_abs, 0.0, gm);
+    double2 *gsum = w->gsum.as<double2>();
+    k_gvec_sums<<<g->num_sms, THREADS, 0, s>>>(g->nv, w->gvec_caller.as<float>(), gsum);
+    k_adjoint_ctl_init<<<1, 32, 0, s>>>(a.ctl, g->nv, max_iter, d, tol, gsum, g->num_sms);
     k_pr_init<PrAdjoint><<<grid, THREADS, 0, s>>>(a, 0.0f);
     int cur = 0;
     MG_TRY(pr_loop<PrAdjoint>(g, a, opt, "wpr_adjoint", info, &cur));
@@ -1591,13 +1729,11 @@ mg_status mg_wpagerank_backward(mg_graph *g, const float *g_host, const mg_opts 
     MG_CUDA(cudaMemcpyAsync(w->lam_keep.p, lam, (size_t)g->nv * 4, cudaMemcpyDeviceToDevice, s));
     int sg = g->prof.slot("wpr_grad");
     g->prof.begin(sg);
-    k_wpr_grad<<<grid, THREADS, 0, s>>>(g->nv, g->row.as<int32_t>(), g->col.as<int32_t>(), g->fw.as<float>(), a.S,
-                                        w->xkeep.as<float>(), w->lam_keep.as<float>(), d, w->grad.as<float>());
+    MG_TRY(row_totals(g, a, RowBack{a.S, w->xkeep.as<float>(), w->lam_keep.as<float>(), d, w->ct.as<float2>()}));
+    MG_TRY(edge_grad_to_caller(g, w->ct.as<float2>(), w->lam_keep.as<float>(), w->grad_caller.as<float>()));
     g->prof.end();
-    MG_CUDA(cudaGetLastError());
     const void *lam_out = nullptr;
     MG_TRY(to_caller(g, MG_RES_DELTA, w->lam_keep.p, 4, 1, &lam_out));
-    MG_TRY(edges_to_caller(g, w->grad.p, w->grad_caller.p));
     MG_TRY(end_run(g, opt, info));
     MG_TRY(copy_out(g, lambda_out, lam_out, (size_t)g->nv * 4));
     return copy_out(g, grad_w_out, w->grad_caller.p, (size_t)g->ne * 4);
