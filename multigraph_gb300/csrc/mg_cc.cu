@@ -16,8 +16,8 @@
 //
 // Symmetric graphs skip most of the edges (neighbour sampling, as in
 // Sutton et al., "Optimizing Parallel Graph Connectivity Computation via
-// Subgraph Sampling", IPDPS 2018): every vertex first links to its first
-// SAMPLE_ROUNDS neighbours (the trees compressed after each round), the most frequent root
+// Subgraph Sampling", IPDPS 2018): every vertex first links to some of its
+// neighbours (the trees compressed after each round), the most frequent root
 // among 1024 sampled vertices is taken as the giant component, and only rows
 // whose vertex is outside it hook their remaining edges (in both
 // directions, so an edge with one end in the giant component is hooked from
@@ -50,36 +50,65 @@ __device__ __forceinline__ int32_t cc_find(volatile int32_t *parent, int32_t v)
     return v;
 }
 
+// The root, or an ancestor that was one a moment ago: up to NEAR_HOPS steps
+// through L1, then cc_find.  Every vertex of the giant tree ends at the same
+// word; read through L2 that word alone took 340 us of a compress on R-MAT
+// 20.  A copy in L1 can only be an older ancestor of the vertex, so the walk
+// still ends inside its tree, and no entry but a root's is its own parent
+// (roots never become roots again).
+constexpr int NEAR_HOPS = 12;
+__device__ __forceinline__ int32_t cc_find_near(int32_t *parent, int32_t v)
+{
+    for (int k = 0; k < NEAR_HOPS; k++) {
+        const int32_t p = __ldca(&parent[v]);
+        if (p == v) return v;
+        v = p;
+    }
+    return cc_find(parent, v);
+}
+
+// Links the trees of a and b.  The first finds may be out of date: equal
+// ancestors mean one tree all the same, and a link is made only by a
+// compare-and-swap on a word that still is a root (always larger under
+// smaller, so no cycle), else the finds are repeated through L2.
 __device__ __forceinline__ void cc_union(int32_t *parent, int32_t a, int32_t b)
 {
     volatile int32_t *vp = parent;
+    a = cc_find_near(parent, a);
+    b = cc_find_near(parent, b);
     for (;;) {
-        a = cc_find(vp, a);
-        b = cc_find(vp, b);
         if (!mgops::Cc::update_condition(a, b)) return;
         if (a < b) { int32_t t = a; a = b; b = t; }
         int32_t old = atomicCAS(&parent[a], a, b);  // link larger root under smaller
         if (old == a) return;
-        a = old;
+        a = cc_find(vp, old);
+        b = cc_find(vp, b);
     }
 }
 
 constexpr int SAMPLE_ROUNDS = 2;
 constexpr int MODE_SAMPLES = 1024;
+constexpr int LINK_FIRST = 8;   // neighbours looked at by the first link of a relabeled graph (one or two sectors)
 
-// link_first: the first neighbour below v starts the tree (a valid link:
-// parent < v); otherwise every vertex is its own tree
-__global__ void k_cc_init(int32_t n, const int32_t *row, const int32_t *col, int32_t *parent, int link_first)
+// The first `link` neighbours below v start the tree: v hangs under the
+// least of them (a valid link: parent < v), a plain store.  With hub-first
+// ids that is the neighbour of the highest degree, so the trees are a few
+// links deep: on R-MAT 16 with shuffled-round ids, linking to the first two
+// neighbours in caller order by atomic unions took 123 us and flattening
+// the chains it made 70 us; this takes 3 + 5.  Without hub-first ids (a
+// lattice) the least neighbour would chain whole columns: link 0, every
+// vertex its own tree.
+__global__ void k_cc_init(int32_t n, const int32_t *row, const int32_t *col, int32_t *parent, int link)
 {
     for (int32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
         int32_t p = mgops::Cc::initialize(v);
-        if (link_first && row[v + 1] > row[v]) p = min(p, col[row[v]]);
+        if (link > 0) {
+            const int32_t b = row[v], e = min(row[v + 1], b + link);
+            for (int32_t k = b; k < e; k++) p = min(p, col[k]);
+        }
         parent[v] = p;
     }
 }
-
-// link every vertex to its r-th neighbour
-__global__ void k_cc_sample(int32_t n, const int32_t *row, const int32_t *col, int32_t r, int32_t *parent);
 
 // The most frequent root among MODE_SAMPLES vertices of one graph of a
 // batch (block b samples caller ids [voff[b], voff[b+1]), the whole id range
@@ -90,22 +119,36 @@ __global__ void k_cc_sample(int32_t n, const int32_t *row, const int32_t *col, i
 __global__ void __launch_bounds__(MODE_SAMPLES) k_cc_mode(int32_t n, const int32_t *voff, const int32_t *old2new,
                                                           const int32_t *parent, uint32_t *giant_bm)
 {
-    __shared__ int32_t s_val[MODE_SAMPLES];
+    // samples counted in a shared-memory hash table (comparing every sample
+    // with every other took 22 us)
+    constexpr int SLOTS = 2 * MODE_SAMPLES;
+    __shared__ int32_t s_key[SLOTS];
+    __shared__ int s_num[SLOTS];
     __shared__ int32_t s_best[MODE_SAMPLES / 32], s_cnt[MODE_SAMPLES / 32];
     const int t = threadIdx.x;
     const int32_t lo = voff ? voff[blockIdx.x] : 0, hi = voff ? voff[blockIdx.x + 1] : n;
     const int32_t span = hi - lo;
     if (span <= 0) return;  // block-uniform
+    for (int i = t; i < SLOTS; i += MODE_SAMPLES) {
+        s_key[i] = -1;
+        s_num[i] = 0;
+    }
     // spread the samples over the id range
     int32_t v = lo + (int32_t)(((int64_t)t * span) / MODE_SAMPLES +
                                (((int64_t)t * 7919) % max(span / MODE_SAMPLES, 1)));
     v = min(max(v, lo), hi - 1);
     if (old2new) v = old2new[v];
-    s_val[t] = parent[v];
+    const int32_t mine = parent[v];
     __syncthreads();
-    const int32_t mine = s_val[t];
-    int cnt = 0;
-    for (int i = 0; i < MODE_SAMPLES; i++) cnt += (s_val[i] == mine);
+    int at = (int)(((uint32_t)mine * 2654435761u) >> 21) & (SLOTS - 1);
+    while (true) {  // at most MODE_SAMPLES keys: a free slot is always found
+        const int32_t k = atomicCAS(&s_key[at], -1, mine);
+        if (k == -1 || k == mine) break;
+        at = (at + 1) & (SLOTS - 1);
+    }
+    atomicAdd(&s_num[at], 1);
+    __syncthreads();
+    const int cnt = s_num[at];
     // block argmax of (cnt, -value)
     int32_t bv = mine;
     int bc = cnt;
@@ -124,6 +167,7 @@ __global__ void __launch_bounds__(MODE_SAMPLES) k_cc_mode(int32_t n, const int32
     }
 }
 
+// link every vertex to its r-th neighbour
 __global__ void k_cc_sample(int32_t n, const int32_t *row, const int32_t *col, int32_t r, int32_t *parent)
 {
     for (int32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
@@ -131,6 +175,47 @@ __global__ void k_cc_sample(int32_t n, const int32_t *row, const int32_t *col, i
         if (row[v + 1] - b > r) {
             const int32_t u = col[b + r];
             if (u != v) cc_union(parent, v, u);
+        }
+    }
+}
+
+// Every root (flat trees) that sees a smaller root among its first ROOT_SCAN
+// neighbours' hangs itself under the least one: a warp per root (a lane, for
+// a short row), a plain store to the root's own entry, so no two threads
+// write the same word.  (Roots only ever point at smaller roots, which may
+// move at the same time; the next compress flattens the chains.)  On
+// hub-first ids the roots left by the first link are hubs whose neighbours
+// mostly belong to the giant tree.  Linking every vertex to a neighbour by
+// atomic union instead sends one compare-and-swap per vertex to the few hot
+// roots: 118 us a round on R-MAT 16 and 950 us on R-MAT 20, against 13 and 18.
+constexpr int ROOT_SCAN = 256;
+__global__ void __launch_bounds__(THREADS) k_cc_roots(int32_t n, const int32_t *row, const int32_t *col,
+                                                      int32_t *parent)
+{
+    const int lane = threadIdx.x & 31;
+    for (int32_t base = blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < n; base += gridDim.x * blockDim.x) {
+        const int32_t v = base + lane;
+        const bool root = v < n && parent[v] == v;
+        int32_t b = 0, e = 0;
+        if (root) {
+            b = row[v];
+            e = min(row[v + 1], b + ROOT_SCAN);
+        }
+        if (e - b <= LINK_FIRST) {   // short rows a lane each
+            int32_t m = v;
+            for (int32_t k = b; k < e; k++) m = min(m, __ldcg(&parent[col[k]]));
+            if (root && m < v) parent[v] = m;
+            e = b;
+        }
+        unsigned todo = __ballot_sync(0xffffffffu, e > b);
+        while (todo) {
+            const int j = __ffs(todo) - 1;
+            todo &= todo - 1;
+            const int32_t r = base + j, eb = __shfl_sync(0xffffffffu, b, j), ee = __shfl_sync(0xffffffffu, e, j);
+            int32_t m = r;
+            for (int32_t k = eb + lane; k < ee; k += 32) m = min(m, __ldcg(&parent[col[k]]));
+            m = __reduce_min_sync(0xffffffffu, m);
+            if (lane == 0 && m < r) parent[r] = m;
         }
     }
 }
@@ -182,11 +267,8 @@ __global__ void __launch_bounds__(THREADS) k_cc_hook(int32_t n, const int32_t *p
 
 __global__ void k_cc_compress(int32_t n, int32_t *parent)
 {
-    volatile int32_t *vp = parent;
-    for (int32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-        int32_t r = cc_find(vp, v);
-        parent[v] = r;
-    }
+    for (int32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
+        parent[v] = cc_find_near(parent, v);
 }
 
 }  // namespace
@@ -231,17 +313,24 @@ mg_status cc_run(mg_graph *g, mg_run_info *info, const std::vector<int32_t> *vof
     Profiler &P = g->prof;
     const int si = P.slot("cc_init"), sh = P.slot("cc_hook"), sc = P.slot("cc_compress");
     const bool sample = g->symmetric;
+    const bool hub_link = sample && g->relabeled;
     P.begin(si);
-    k_cc_init<<<grid, THREADS, 0, s>>>(g->nv, g->trow, g->tcol, parent, sample ? 0 : 1);
+    k_cc_init<<<grid, THREADS, 0, s>>>(g->nv, g->trow, g->tcol, parent, hub_link ? LINK_FIRST : sample ? 0 : 1);
     P.end();
     if (sample) {
-        // singleton trees, then each sampling round links every vertex to
-        // its r-th neighbour and flattens the trees again, so no find walks
-        // a long chain (a lattice's first neighbours would chain rows)
         const int ss = P.slot("cc_sample"), sm = P.slot("cc_mode");
+        if (hub_link) {
+            P.begin(sc);
+            k_cc_compress<<<grid, THREADS, 0, s>>>(g->nv, parent);
+            P.end();
+        }
         for (int r = 0; r < SAMPLE_ROUNDS; r++) {
+            // each round links the trees and flattens them again, so no find
+            // walks a long chain: the roots among themselves on hub-first
+            // ids, else every vertex to its r-th neighbour
             P.begin(ss);
-            k_cc_sample<<<grid, THREADS, 0, s>>>(g->nv, g->trow, g->tcol, r, parent);
+            if (hub_link) k_cc_roots<<<grid, THREADS, 0, s>>>(g->nv, g->trow, g->tcol, parent);
+            else k_cc_sample<<<grid, THREADS, 0, s>>>(g->nv, g->trow, g->tcol, r, parent);
             P.end();
             P.begin(sc);
             k_cc_compress<<<grid, THREADS, 0, s>>>(g->nv, parent);
