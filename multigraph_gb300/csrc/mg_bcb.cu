@@ -21,7 +21,10 @@ __global__ void k_bb_init(BbArgs a, int32_t nsrc, int32_t dirmode, int32_t alpha
     const int32_t v = valid ? a.src[lane] : -1 - lane;
     const uint32_t same = __match_any_sync(0xffffffffu, v);
     const bool leader = valid && lane == __ffs(same) - 1;
-    if (valid) a.sig[(size_t)v * W + lane] = mgops::pc_one();
+    if (valid) {
+        if (a.mode == M_INT) a.cnt[0][(size_t)v * W + lane] = 1u;
+        else a.sig[(size_t)v * W + lane] = mgops::pc_one();
+    }
     const uint32_t leaders = __ballot_sync(0xffffffffu, leader);
     unsigned long long deg = 0;
     int heavy = 0;
@@ -55,6 +58,7 @@ __global__ void k_bb_init(BbArgs a, int32_t nsrc, int32_t dirmode, int32_t alpha
         c.dense_levels = c.dense;
         a.off[0] = 0;
         a.off[1] = cnt;
+        a.lnfe[0] = deg;
         *a.ctl = c;
     }
 }
@@ -73,21 +77,32 @@ __global__ void __launch_bounds__(THREADS) k_bb_mark(BbArgs a)
     bb_mark_phase(a, c, a.off[c.d], a.off[c.d + 1], &a.ctl->k.ncand);
 }
 
-template <bool TP, bool EXT>
+template <bool TP, int M>
 __global__ void __launch_bounds__(THREADS) k_bb_pull(BbArgs a)
 {
     pdl_enter();
     const BbCtl c = *a.ctl;
-    if (c.more == 0) return;
-    bb_pull_phase<TP, EXT>(a, c, c.dense ? a.n : c.k.ncand);
+    if (c.more == 0 || c.dense == 2) return;
+    bb_pull_phase<TP, M>(a, c, c.dense ? a.n : c.k.ncand);
 }
 
+template <int M>
 __global__ void __launch_bounds__(THREADS) k_bb_heavy(BbArgs a)
 {
     pdl_enter();
     const BbCtl c = *a.ctl;
     if (c.more == 0) return;
-    bb_heavy_phase(a, c);
+    if (M == M_INT && c.dense == 2) bb_gather_heavy_phase(a, c);
+    else bb_heavy_phase<M>(a, c);
+}
+
+// dense level without masks (M_INT)
+__global__ void __launch_bounds__(GTHREADS, GPER_SM) k_bb_gather(BbArgs a)
+{
+    pdl_enter();
+    const BbCtl c = *a.ctl;
+    if (c.more == 0 || c.dense != 2) return;
+    bb_gather_phase(a, c);
 }
 
 // Archives level d+1 and, in the last block to finish, decides the next
@@ -107,8 +122,9 @@ __global__ void __launch_bounds__(THREADS) k_bb_compact(BbArgs a, cudaGraphCondi
     const LvlCnt k = n.k;
     const int32_t d = n.d;
     int32_t off_d2;
-    bb_decide(n, k, n.ovf, a.off[d + 1], off_d2, a.m);
+    bb_decide(n, k, n.ovf, a.off[d + 1], off_d2, a.m, a.mode);
     a.off[d + 2] = off_d2;
+    a.lnfe[d + 1] = k.nfe;
     n.k = LvlCnt{0, 0, 0, 0, 0ull};
     n.done = 0;
     *cp = n;
@@ -129,22 +145,33 @@ __global__ void k_bbb_start(BbArgs a)
     if (run) bbb_start_phase(a, L);
 }
 
-template <bool TP, bool EXT>
+template <bool TP, int M>
 __global__ void __launch_bounds__(THREADS) k_bbb_pull(BbArgs a)
 {
     pdl_enter();
     const BbCtl c = *a.ctl;
     if (c.more == 0) return;
-    bbb_pull_phase<TP, EXT>(a, c.L);
+    if (!TP && back_gathers(a, c.L)) return;
+    bbb_pull_phase<TP, M>(a, c.L);
 }
 
-template <bool EXT>
+// backward level without masks (M_INT)
+__global__ void __launch_bounds__(GTHREADS, GPER_SM) k_bbb_gather(BbArgs a)
+{
+    pdl_enter();
+    const BbCtl c = *a.ctl;
+    if (c.more == 0 || !back_gathers(a, c.L)) return;
+    bbb_gather_phase(a, c.L);
+}
+
+template <int M>
 __global__ void __launch_bounds__(THREADS, 8) k_bbb_heavy(BbArgs a)
 {
     pdl_enter();
     const BbCtl c = *a.ctl;
     if (c.more == 0) return;
-    bbb_heavy_phase<EXT>(a, c.L);
+    if (M == M_INT && back_gathers(a, c.L)) bbb_gather_heavy_phase(a, c.L);
+    else bbb_heavy_phase<M>(a, c.L);
 }
 
 // End of backward level L (masks cleared / scattered); the last block to
@@ -181,6 +208,12 @@ __global__ void __launch_bounds__(THREADS) k_bbb_next(BbArgs a, cudaGraphConditi
 // level: pull | barrier | heavy | barrier | next | barrier.  The phase
 // bodies are the per-level kernels' own.  A barrier timeout sets status 3.
 
+// One block of 1024 threads per SM: a grid barrier's cost is its arrivals
+// (608 to 760 blocks of 256 before), and 64 registers a thread leave no
+// spills (32 sources on a 480 x 397 lattice, forward levels 15.8 ->
+// 13.3 ms, backward 13.5 -> 12.7 ms).
+constexpr int PTHREADS = 1024;
+
 __device__ __forceinline__ LvlCnt load_cnt_l2(const LvlCnt *k)
 {
     LvlCnt r;
@@ -192,8 +225,8 @@ __device__ __forceinline__ LvlCnt load_cnt_l2(const LvlCnt *k)
     return r;
 }
 
-template <bool TP, bool EXT>
-__global__ void __launch_bounds__(THREADS) k_bb_levels(BbArgs a, int heavy)
+template <bool TP, int M>
+__global__ void __launch_bounds__(PTHREADS, 1) k_bb_levels(BbArgs a, int heavy)
 {
     __shared__ BbCtl s_c;
     __shared__ int32_t s_off[2];
@@ -214,10 +247,10 @@ __global__ void __launch_bounds__(THREADS) k_bb_levels(BbArgs a, int heavy)
         bb_mark_phase(a, c, b0, b1, &k->ncand);
         if (!(ok = mgd::grid_sync(a.bar, a.bar_err))) break;
         const int32_t ncand = __ldcg(&k->ncand);
-        bb_pull_phase<TP, EXT>(a, c, ncand);
+        bb_pull_phase<TP, M>(a, c, ncand);
         if (!(ok = mgd::grid_sync(a.bar, a.bar_err))) break;
         if (heavy) {
-            bb_heavy_phase(a, c);
+            bb_heavy_phase<M>(a, c);
             if (!(ok = mgd::grid_sync(a.bar, a.bar_err))) break;
         }
         bb_compact_phase(a, c, b0, b1, ncand, k);
@@ -225,7 +258,7 @@ __global__ void __launch_bounds__(THREADS) k_bb_levels(BbArgs a, int heavy)
         if (threadIdx.x == 0) {
             BbCtl n = c;
             int32_t off_d2;
-            bb_decide(n, load_cnt_l2(k), __ldcg(&a.ctl->ovf), b1, off_d2, a.m);
+            bb_decide(n, load_cnt_l2(k), __ldcg(&a.ctl->ovf), b1, off_d2, a.m, M);
             if (blockIdx.x == 0) a.off[c.d + 2] = off_d2;
             s_c = n;
             s_off[0] = b1;
@@ -246,8 +279,8 @@ __global__ void __launch_bounds__(THREADS) k_bb_levels(BbArgs a, int heavy)
     }
 }
 
-template <bool TP, bool EXT>
-__global__ void __launch_bounds__(THREADS) k_bbb_levels(BbArgs a, int heavy)
+template <bool TP, int M>
+__global__ void __launch_bounds__(PTHREADS, 1) k_bbb_levels(BbArgs a, int heavy)
 {
     __shared__ BbCtl s_c;
     if (threadIdx.x == 0) s_c = load_ctl_l2(a.ctl);
@@ -256,10 +289,10 @@ __global__ void __launch_bounds__(THREADS) k_bbb_levels(BbArgs a, int heavy)
     bool ok = true;
     int32_t L = s_c.L;
     for (; L >= 1; L--) {
-        bbb_pull_phase<TP, EXT>(a, L);
+        bbb_pull_phase<TP, M>(a, L);
         if (!(ok = mgd::grid_sync(a.bar, a.bar_err))) break;
         if (heavy) {
-            bbb_heavy_phase<EXT>(a, L);
+            bbb_heavy_phase<M>(a, L);
             if (!(ok = mgd::grid_sync(a.bar, a.bar_err))) break;
         }
         bbb_next_phase(a, L);
@@ -278,7 +311,7 @@ mg_status launch_coop(K kernel, int grid, cudaStream_t st, const BbArgs &a, int 
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(THREADS);
+    cfg.blockDim = dim3(PTHREADS);
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;
@@ -289,9 +322,10 @@ mg_status launch_coop(K kernel, int grid, cudaStream_t st, const BbArgs &a, int 
     return MG_OK;
 }
 
-__global__ void k_bb_to_float(int32_t n, const double *bc, float *out)
+__global__ void k_bb_to_float(int32_t n, const float2 *bc, float *out)
 {
-    for (int32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) out[v] = (float)bc[v];
+    for (int32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
+        out[v] = bc[v].x + bc[v].y;
 }
 
 }  // namespace
@@ -299,6 +333,7 @@ __global__ void k_bb_to_float(int32_t n, const double *bc, float *out)
 
 struct BcWS {
     mgi::DevBuf vis, fm, cbm, cand, arch, amask, off, sig, q, hpart, hmask, bc, bcf, fheavy, src, ctl, bar, pcnt;
+    mgi::DevBuf lnfe, gpart;
     mgi::LoopGraph fwd, bwd;
     int coop_f = 0, coop_b = 0;   // resident grids of the persistent sweeps (0: not sized yet)
 };
@@ -314,7 +349,7 @@ void free_bc_ws(mg_graph *g)
     BcWS *w = g->bws;
     DevBuf *bufs[] = {&w->vis, &w->fm, &w->cbm, &w->cand, &w->arch, &w->amask, &w->off, &w->sig,
                       &w->q, &w->hpart, &w->hmask, &w->bc, &w->bcf, &w->fheavy, &w->src, &w->ctl,
-                      &w->bar, &w->pcnt};
+                      &w->bar, &w->pcnt, &w->lnfe, &w->gpart};
     for (DevBuf *b : bufs) dev_free(*b);
     w->fwd.destroy();
     w->bwd.destroy();
@@ -344,8 +379,18 @@ mg_status bc_batched(mg_graph *g, const int32_t *src_engine, int32_t nsrc, const
     MG_TRY(dev_alloc(w->arch, cap * 4));
     MG_TRY(dev_alloc(w->amask, cap * 4));
     MG_TRY(dev_alloc(w->off, (n + 4) * 4));
-    MG_TRY(dev_alloc(w->sig, cap * sizeof(mgops::PathCount)));
+    // Low-degree graphs (average degree <= TP_AVG_DEG, e.g. lattices) reach
+    // counts past 2^29 within a few dozen levels: they start in M_PLAIN; the
+    // others in M_INT
+    const bool tp = (int64_t)g->ne <= (int64_t)TP_AVG_DEG * g->nv;
+    const int mode = g->bc_ext ? M_EXT : (tp || g->bcb_no_int) ? M_PLAIN : M_INT;
+    MG_TRY(dev_alloc(w->sig, mode == M_INT ? 2 * cap * 4 : cap * sizeof(mgops::PathCount)));
     MG_TRY(dev_alloc(w->q, cap * 8));
+    MG_TRY(dev_alloc(w->lnfe, (n + 4) * 8));
+    if (mode == M_INT) {
+        MG_TRY(ppr_chunks(g));
+        MG_TRY(dev_alloc(w->gpart, (size_t)std::max(g->ppr_nhchunks, 1) * W * 8));
+    }
     MG_TRY(dev_alloc(w->hpart, nch * W * sizeof(mgops::PathCount)));
     MG_TRY(dev_alloc(w->hmask, nch * 4));
     MG_TRY(dev_alloc(w->bc, n * 8));
@@ -375,10 +420,18 @@ mg_status bc_batched(mg_graph *g, const int32_t *src_engine, int32_t nsrc, const
     a.off = w->off.as<int32_t>();
     a.sig = w->sig.as<mgops::PathCount>();
     a.q = w->q.p;
+    a.mode = mode;
+    a.lnfe = w->lnfe.as<unsigned long long>();
+    if (mode == M_INT) {
+        a.cnt[0] = w->sig.as<uint32_t>(); a.cnt[1] = a.cnt[0] + cap;
+        a.qp[0] = w->q.as<float>(); a.qp[1] = a.qp[0] + cap;
+        a.gchunk = g->ppr_hchunk.as<int32_t>(); a.ngchunks = g->ppr_nhchunks;
+        a.grows = g->ppr_hrows.as<int32_t>(); a.grow_chunk = g->ppr_hrow_chunk.as<int32_t>(); a.ngrows = g->ppr_nhrows;
+        a.gpart = w->gpart.p;
+    }
     a.hpart = w->hpart.as<mgops::PathCount>();
-    a.ext = g->bc_ext ? 1 : 0;
     a.hmask = w->hmask.as<uint32_t>();
-    a.bc = w->bc.as<double>();
+    a.bc = w->bc.as<float2>();
     a.fheavy = w->fheavy.as<int32_t>();
     a.src = w->src.as<int32_t>();
     a.ctl = w->ctl.as<BbCtl>();
@@ -395,13 +448,13 @@ mg_status bc_batched(mg_graph *g, const int32_t *src_engine, int32_t nsrc, const
     // kernels with the thread path; their grids are what stays resident
     // (the thread path costs registers), so no CTA waits for a second wave.
     // Denser graphs keep one warp per row at eight CTAs per SM.
-    const bool tp = (int64_t)g->ne <= (int64_t)TP_AVG_DEG * g->nv;
     int occ_f = 8, occ_b = 8;
+    const bool ext = mode == M_EXT;
     if (tp) {
-        if (a.ext) MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_f, k_bb_pull<true, true>, THREADS, 0));
-        else MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_f, k_bb_pull<true, false>, THREADS, 0));
-        if (a.ext) MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_b, k_bbb_pull<true, true>, THREADS, 0));
-        else MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_b, k_bbb_pull<true, false>, THREADS, 0));
+        if (ext) MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_f, k_bb_pull<true, M_EXT>, THREADS, 0));
+        else MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_f, k_bb_pull<true, M_PLAIN>, THREADS, 0));
+        if (ext) MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_b, k_bbb_pull<true, M_EXT>, THREADS, 0));
+        else MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_b, k_bbb_pull<true, M_PLAIN>, THREADS, 0));
     }
     const int grid_f = launch_grid(g, THREADS, std::max(1, std::min(8, occ_f)));
     const int grid_b = launch_grid(g, THREADS, std::max(1, std::min(8, occ_b)));
@@ -409,49 +462,59 @@ mg_status bc_batched(mg_graph *g, const int32_t *src_engine, int32_t nsrc, const
     // grids are what stays resident
     if (tp && w->coop_f == 0) {
         int of = 0, ob = 0, ofx = 0, obx = 0;
-        MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&of, k_bb_levels<true, false>, THREADS, 0));
-        MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ofx, k_bb_levels<true, true>, THREADS, 0));
-        MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ob, k_bbb_levels<true, false>, THREADS, 0));
-        MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&obx, k_bbb_levels<true, true>, THREADS, 0));
-        const int pf = std::min({of, ofx, 8}), pb = std::min({ob, obx, 8});
-        if (pf < 1 || pb < 1) return fail(MG_ERR_CUDA, "persistent batched BC kernels do not fit on an SM");
-        w->coop_f = pf * g->num_sms;
-        w->coop_b = pb * g->num_sms;
+        MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&of, k_bb_levels<true, M_PLAIN>, PTHREADS, 0));
+        MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ofx, k_bb_levels<true, M_EXT>, PTHREADS, 0));
+        MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ob, k_bbb_levels<true, M_PLAIN>, PTHREADS, 0));
+        MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&obx, k_bbb_levels<true, M_EXT>, PTHREADS, 0));
+        if (std::min({of, ofx, ob, obx}) < 1)
+            return fail(MG_ERR_CUDA, "persistent batched BC kernels do not fit on an SM");
+        w->coop_f = w->coop_b = g->num_sms;
     }
     const bool persist = tp;
     const int coop_f = w->coop_f, coop_b = w->coop_b;
     const int alpha = opt.alpha > 0 ? opt.alpha : 15;
     const int max_levels = g->nv + 2;
     // heavy-row folds only on graphs that have heavy rows
-    const bool heavy = g->nhrows > 0;
+    const bool heavy = g->nhrows > 0 || a.ngrows > 0;
+    const int grid_g = launch_grid(g, GTHREADS, GPER_SM);
     Profiler &P = g->prof;
     const int s_mark = P.slot("bcb_mark"), s_pull = P.slot("bcb_pull"), s_heavy = P.slot("bcb_heavy");
     const int s_comp = P.slot("bcb_compact_decide");
     const int s_bp = P.slot("bcb_back"), s_bh = P.slot("bcb_back_heavy"), s_bn = P.slot("bcb_back_next");
+    const int s_gather = mode == M_INT ? P.slot("bcb_gather") : -1, s_bg = mode == M_INT ? P.slot("bcb_back_gather") : -1;
     const int s_lv = persist ? P.slot("bcb_levels") : -1, s_blv = persist ? P.slot("bcb_back_levels") : -1;
     BodyFn fwd = [&](cudaStream_t st, cudaGraphConditionalHandle h, int use_cond) -> mg_status {
         if (persist) {
             MG_CUDA(cudaMemsetAsync(a.pcnt, 0, 4 * sizeof(LvlCnt), st));
             P.begin(s_lv);
-            if (a.ext) MG_TRY(launch_coop(k_bb_levels<true, true>, coop_f, st, a, (int)heavy));
-            else MG_TRY(launch_coop(k_bb_levels<true, false>, coop_f, st, a, (int)heavy));
+            if (ext) MG_TRY(launch_coop(k_bb_levels<true, M_EXT>, coop_f, st, a, (int)heavy));
+            else MG_TRY(launch_coop(k_bb_levels<true, M_PLAIN>, coop_f, st, a, (int)heavy));
             P.end();
         }
         P.begin(s_mark);
         k_bb_mark<<<grid, THREADS, 0, st>>>(a);
         P.end();
         P.begin(s_pull);
-        if (a.ext) {
-            if (tp) MG_TRY(launch_pdl(k_bb_pull<true, true>, grid_f, THREADS, st, a));
-            else MG_TRY(launch_pdl(k_bb_pull<false, true>, grid_f, THREADS, st, a));
+        if (mode == M_INT) {
+            MG_TRY(launch_pdl(k_bb_pull<false, M_INT>, grid_f, THREADS, st, a));
+        } else if (ext) {
+            if (tp) MG_TRY(launch_pdl(k_bb_pull<true, M_EXT>, grid_f, THREADS, st, a));
+            else MG_TRY(launch_pdl(k_bb_pull<false, M_EXT>, grid_f, THREADS, st, a));
         } else {
-            if (tp) MG_TRY(launch_pdl(k_bb_pull<true, false>, grid_f, THREADS, st, a));
-            else MG_TRY(launch_pdl(k_bb_pull<false, false>, grid_f, THREADS, st, a));
+            if (tp) MG_TRY(launch_pdl(k_bb_pull<true, M_PLAIN>, grid_f, THREADS, st, a));
+            else MG_TRY(launch_pdl(k_bb_pull<false, M_PLAIN>, grid_f, THREADS, st, a));
         }
         P.end();
+        if (mode == M_INT) {
+            P.begin(s_gather);
+            MG_TRY(launch_pdl(k_bb_gather, grid_g, GTHREADS, st, a));
+            P.end();
+        }
         if (heavy) {
             P.begin(s_heavy);
-            MG_TRY(launch_pdl(k_bb_heavy, grid, THREADS, st, a));
+            if (mode == M_INT) MG_TRY(launch_pdl(k_bb_heavy<M_INT>, grid, THREADS, st, a));
+            else if (ext) MG_TRY(launch_pdl(k_bb_heavy<M_EXT>, grid, THREADS, st, a));
+            else MG_TRY(launch_pdl(k_bb_heavy<M_PLAIN>, grid, THREADS, st, a));
             P.end();
         }
         P.begin(s_comp);
@@ -462,18 +525,26 @@ mg_status bc_batched(mg_graph *g, const int32_t *src_engine, int32_t nsrc, const
     };
     BodyFn bwd = [&](cudaStream_t st, cudaGraphConditionalHandle h, int use_cond) -> mg_status {
         P.begin(s_bp);
-        if (a.ext) {
-            if (tp) k_bbb_pull<true, true><<<grid_b, THREADS, 0, st>>>(a);
-            else k_bbb_pull<false, true><<<grid_b, THREADS, 0, st>>>(a);
+        if (mode == M_INT) {
+            k_bbb_pull<false, M_INT><<<grid_b, THREADS, 0, st>>>(a);
+        } else if (ext) {
+            if (tp) k_bbb_pull<true, M_EXT><<<grid_b, THREADS, 0, st>>>(a);
+            else k_bbb_pull<false, M_EXT><<<grid_b, THREADS, 0, st>>>(a);
         } else {
-            if (tp) k_bbb_pull<true, false><<<grid_b, THREADS, 0, st>>>(a);
-            else k_bbb_pull<false, false><<<grid_b, THREADS, 0, st>>>(a);
+            if (tp) k_bbb_pull<true, M_PLAIN><<<grid_b, THREADS, 0, st>>>(a);
+            else k_bbb_pull<false, M_PLAIN><<<grid_b, THREADS, 0, st>>>(a);
         }
         P.end();
+        if (mode == M_INT) {
+            P.begin(s_bg);
+            MG_TRY(launch_pdl(k_bbb_gather, grid_g, GTHREADS, st, a));
+            P.end();
+        }
         if (heavy) {
             P.begin(s_bh);
-            if (a.ext) MG_TRY(launch_pdl(k_bbb_heavy<true>, grid, THREADS, st, a));
-            else MG_TRY(launch_pdl(k_bbb_heavy<false>, grid, THREADS, st, a));
+            if (mode == M_INT) MG_TRY(launch_pdl(k_bbb_heavy<M_INT>, grid, THREADS, st, a));
+            else if (ext) MG_TRY(launch_pdl(k_bbb_heavy<M_EXT>, grid, THREADS, st, a));
+            else MG_TRY(launch_pdl(k_bbb_heavy<M_PLAIN>, grid, THREADS, st, a));
             P.end();
         }
         P.begin(s_bn);
@@ -485,17 +556,22 @@ mg_status bc_batched(mg_graph *g, const int32_t *src_engine, int32_t nsrc, const
     // every by-value argument of the captured kernels
     const LoopKey key = LoopKey().add(a).add(grid).add(grid_f).add(grid_b).add(heavy).add(tp).add(coop_f);
     const LoopKey key_b = LoopKey(key).add(1);
-    const int mode = opt.profile ? MG_EXEC_HOST : opt.exec;
+    const int exec_mode = opt.profile ? MG_EXEC_HOST : opt.exec;
     int32_t levels = 0, dense_levels = 0;
     for (int32_t g0 = 0; g0 < nsrc; g0 += W) {
         const int32_t cnt = std::min<int32_t>(W, nsrc - g0);
         MG_CUDA(cudaMemcpyAsync(w->src.p, src_engine + g0, (size_t)cnt * 4, cudaMemcpyHostToDevice, s));
+        if (mode == M_INT) {
+            // mask-free levels read unreached vertices' counts and q as zero
+            MG_CUDA(cudaMemsetAsync(a.cnt[0], 0, 2 * cap * 4, s));
+            MG_CUDA(cudaMemsetAsync(a.qp[0], 0, 2 * cap * 4, s));
+        }
         MG_CUDA(cudaMemsetAsync(a.vis, 0, n * 4, s));
         MG_CUDA(cudaMemsetAsync(a.fm0, 0, 3 * n * 4, s));
         MG_CUDA(cudaMemsetAsync(a.bar, 0, 64, s));
         k_bb_init<<<1, 32, 0, s>>>(a, cnt, opt.direction, alpha, max_levels);
         MG_CUDA(cudaGetLastError());
-        MG_TRY(run_loop(mode, opt.profile != 0, s, w->fwd, key, fwd, &a.ctl->more, g->pinned_flag, max_levels + 2));
+        MG_TRY(run_loop(exec_mode, opt.profile != 0, s, w->fwd, key, fwd, &a.ctl->more, g->pinned_flag, max_levels + 2));
         k_bbb_start<<<grid, THREADS, 0, s>>>(a);
         MG_CUDA(cudaGetLastError());
         if (persist) {
@@ -503,11 +579,11 @@ mg_status bc_batched(mg_graph *g, const int32_t *src_engine, int32_t nsrc, const
             // from zero: this grid differs from the forward one)
             MG_CUDA(cudaMemsetAsync(a.bar, 0, 64, s));
             P.begin(s_blv);
-            if (a.ext) MG_TRY(launch_coop(k_bbb_levels<true, true>, coop_b, s, a, (int)heavy));
-            else MG_TRY(launch_coop(k_bbb_levels<true, false>, coop_b, s, a, (int)heavy));
+            if (ext) MG_TRY(launch_coop(k_bbb_levels<true, M_EXT>, coop_b, s, a, (int)heavy));
+            else MG_TRY(launch_coop(k_bbb_levels<true, M_PLAIN>, coop_b, s, a, (int)heavy));
             P.end();
         } else {
-            MG_TRY(run_loop(mode, opt.profile != 0, s, w->bwd, key_b, bwd, &a.ctl->more, g->pinned_flag,
+            MG_TRY(run_loop(exec_mode, opt.profile != 0, s, w->bwd, key_b, bwd, &a.ctl->more, g->pinned_flag,
                             max_levels + 2));
         }
         BbCtl hc;
@@ -516,10 +592,12 @@ mg_status bc_batched(mg_graph *g, const int32_t *src_engine, int32_t nsrc, const
         if (hc.status == 1) return fail(MG_ERR_ITER_LIMIT, "batched BC: level cap %d reached", max_levels);
         if (hc.status == 3) return fail(MG_ERR_CUDA, "batched BC: grid barrier of a persistent sweep timed out");
         if (hc.status != 0) return fail(MG_ERR_CUDA, "batched BC: level archive overflow");
-        if (hc.ovf && !g->bc_ext) {
-            // a path count passed FP64's comfortable range: this graph's BC
-            // runs use extended path counts from now on, starting over here
-            g->bc_ext = true;
+        if (hc.ovf && mode != M_EXT) {
+            // a path count passed 2^29 (M_INT) or FP64's comfortable range:
+            // this graph's batched BC runs take the next form from now on,
+            // starting over here
+            if (mode == M_INT) g->bcb_no_int = true;
+            else g->bc_ext = true;
             return bc_batched(g, src_engine, nsrc, opt, info, bc_dev);
         }
         levels += hc.nlevels;

@@ -9,12 +9,18 @@
 //
 //   vis[v]   bit s set once v has been reached from source s
 //   fm[v]    bit s set when v is on source s's current frontier
-//   sig[v*32+s]  path count of v from source s (mgops::PathCount: FP64
-//                mantissa m and a 2^512 scale k; plain FP64 until a count
-//                reaches mgops::PC_PLAIN_MAX = 2^90, then the run repeats
-//                in extended mode)
-//   q[v*32+s]    (1 + delta_s[v]) / m   (backward; FP32 with plain counts,
-//                FP64 with extended ones)
+//   path counts  of v from source s, in one of three forms; a count that does
+//                not fit sets a flag and the run repeats in the next form:
+//                  M_INT   uint32 below INT_LIMIT = 2^29, so that eight add
+//                          up in 32 bits, summed in 64 (exact); graphs above
+//                          TP_AVG_DEG start here
+//                  M_PLAIN FP64 below mgops::PC_PLAIN_MAX = 2^90
+//                          (low-degree graphs start here)
+//                  M_EXT   mgops::PathCount, FP64 mantissa with a 2^512 scale
+//                M_INT keeps two arrays [n][32], one per level parity
+//                (cnt[level & 1]); the others one PathCount array sig
+//   q[v*32+s]    (1 + delta_s[v]) / count   (backward; FP32, FP64 in M_EXT;
+//                M_INT: qp[level & 1])
 //   archive  (vertex, mask) entries, grouped by level: entry (v, M) at
 //            level d means v is at distance d from exactly the sources in M
 //
@@ -43,6 +49,21 @@
 // with the per-vertex score bc[u] += sum of delta_s[u] over the entry's
 // sources (u excluded as its own source); k_bbb_next then clears level
 // L+1's masks, scatters level L-1's into the third buffer and steps L.
+//
+// Dense levels in M_INT (frontier out-edges above m / GATHER_FWD, resp.
+// level out-edges above m / GATHER_BACK) need no masks at all.  An unreached
+// row's reached in-neighbours are all on the frontier (a neighbour one level
+// up would have reached it before), so the row's new counts are the plain
+// sums of its in-neighbours' counts -- zero where unreached -- once the
+// counts being written this level sit in another array: the parity arrays.
+// The backward sums are the same over q (levels below L+1 still hold zero).
+// k_bb_gather / k_bbb_gather then read a neighbour's 32 values as one line,
+// eight lanes a row with a 16-byte load each, eight edges in flight (the
+// layout of personalised PageRank's sweep), where the masked path tests,
+// shuffles and loads one neighbour after another.  R-MAT 20, us per dense
+// level: forward 1,340 -> 330, backward 1,280 -> 330.  FP64 is out of both
+// paths: GB300's FP64 pipe was 60 % busy in the forward sums and 48 % in the
+// backward finish (its score sums are pairs of FP32 now).
 //
 // On low-degree graphs (average degree <= 8) both pull kernels first give
 // each row / entry with at most 8 edges and at most 4 sources at this level
@@ -77,6 +98,14 @@ constexpr int32_t MARK_HEAVY = 2048;  // frontier entries above this out-degree 
 constexpr int TDEG = 8;
 constexpr int TBITS = 4;
 constexpr int TP_AVG_DEG = 8;  // graphs up to this average degree use the thread path
+enum { M_INT = 0, M_PLAIN = 1, M_EXT = 2 };  // path-count forms
+constexpr unsigned long long INT_LIMIT = 1ull << 29;
+// levels summed without masks: forward when the frontier's out-edges exceed
+// m / GATHER_FWD (most edges of a row then hit), backward when the level's
+// entries hold more than m / GATHER_BACK edges
+constexpr unsigned long long GATHER_FWD = 4, GATHER_BACK = 8;
+constexpr int GTHREADS = 512;  // mask-free kernels: two blocks per SM at 64 registers
+constexpr int GPER_SM = 2;
 
 // what one forward level counts (atomics): candidates of a sparse level,
 // entries archived for the next level, their heavy entries and out-edges
@@ -92,7 +121,7 @@ struct BbCtl {
     int32_t more;
     int32_t d;          // forward level being expanded
     int32_t cur;        // fm buffer holding level d
-    int32_t dense;      // this level pulls over every row
+    int32_t dense;      // this level pulls over every row (2: without masks)
     int32_t nfh;        // heavy frontier entries at level d
     int32_t nlevels;    // levels 0..nlevels-1 archived (set when the forward sweep ends)
     int32_t L;          // backward level
@@ -111,7 +140,7 @@ struct BbCtl {
 
 // the next level from level d's counters; off_d2 = archive offset of level d+2
 __device__ __forceinline__ void bb_decide(BbCtl &n, const LvlCnt &k, int32_t ovf, int32_t off_d1, int32_t &off_d2,
-                                          int32_t m)
+                                          int32_t m, int32_t mode)
 {
     off_d2 = off_d1 + k.nnew;
     if (k.status) n.status = k.status;
@@ -132,6 +161,7 @@ __device__ __forceinline__ void bb_decide(BbCtl &n, const LvlCnt &k, int32_t ovf
         else if (n.dirmode == MG_DIR_PULL) n.dense = 1;
         else n.dense = n.nfe_cur * (unsigned long long)n.alpha > (unsigned long long)m;
         n.dense_levels += n.dense;
+        if (n.dense && mode == M_INT && n.nfe_cur * GATHER_FWD > (unsigned long long)m) n.dense = 2;
     }
 }
 
@@ -156,9 +186,16 @@ struct BbArgs {
     mgops::PathCount *sig;
     void *q;                     // float (plain counts) or double (extended) per (v, source)
     mgops::PathCount *hpart;     // per chunk x 32 lanes (backward reuses it as double)
-    int32_t ext;                 // extended path counts
+    int32_t mode;                // M_INT / M_PLAIN / M_EXT
+    uint32_t *cnt[2];            // M_INT: counts by level parity
+    float *qp[2];                // M_INT: q by level parity
+    unsigned long long *lnfe;    // out-edges of every level's entries
+    // rows above GCHUNK edges in GCHUNK-edge chunks (mask-free levels)
+    const int32_t *gchunk, *grows, *grow_chunk;
+    int32_t ngchunks, ngrows;
+    void *gpart;                 // [ngchunks][32] partial sums (uint64 / float)
     uint32_t *hmask;
-    double *bc;                  // score accumulator (all groups)
+    float2 *bc;                  // scores (all groups): sum as an unevaluated pair high + low
     int32_t *fheavy;
     const int32_t *src;          // the group's sources (engine ids), W entries
     BbCtl *ctl;
@@ -209,6 +246,33 @@ __device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long x)
     for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
     return x;
 }
+
+// (hi, lo) += x, exact up to the rounding of lo (TwoSum)
+__device__ __forceinline__ void pair_add(float &hi, float &lo, float x)
+{
+    const float s = hi + x, bp = s - hi;
+    lo += (hi - (s - bp)) + (x - bp);
+    hi = s;
+}
+
+// the score of u += (hi, lo)
+__device__ __forceinline__ void score_add(const BbArgs &a, int32_t u, float hi, float lo)
+{
+    float2 b = a.bc[u];
+    pair_add(b.x, b.y, hi);
+    b.y += lo;
+    a.bc[u] = b;
+}
+
+// a path count of each form: its sum while a row is pulled
+template <int M>
+struct SumOf {
+    using T = mgops::PathCount;
+};
+template <>
+struct SumOf<M_INT> {
+    using T = unsigned long long;
+};
 
 // ---------------------------------------------------------------------------
 // forward
@@ -278,15 +342,17 @@ __device__ __forceinline__ void bb_mark_phase(const BbArgs &a, const BbCtl &c, i
 }
 
 // One row's in-edges [b, e) against the frontier masks: lane s returns the
-// sum of sig over in-neighbours on source s's frontier; *hit gets the union
-// of the masks that hit (restricted to `want`).
-template <bool EXT>
-__device__ __forceinline__ mgops::PathCount pull_span(const BbArgs &a, const uint32_t *fcur, int32_t b, int32_t e,
-                                                      uint32_t want, uint32_t &hit)
+// sum of the counts over in-neighbours on source s's frontier (level d);
+// *hit gets the union of the masks that hit (restricted to `want`).
+template <int M>
+__device__ __forceinline__ typename SumOf<M>::T pull_span(const BbArgs &a, const uint32_t *fcur, int32_t d, int32_t b,
+                                                          int32_t e, uint32_t want, uint32_t &hit)
 {
     const int lane = mgd::lane();
     mgops::PathCount acc = mgops::pc_zero();  // extended counts
     double accp = 0.0;                        // plain counts
+    unsigned long long acci = 0;              // integer counts
+    const uint32_t *cnt = a.cnt[d & 1];
     uint32_t newm = 0;
     for (int32_t base = b; base < e; base += 32) {
         const int32_t p = base + lane;
@@ -297,30 +363,61 @@ __device__ __forceinline__ mgops::PathCount pull_span(const BbArgs &a, const uin
             f = fcur[u] & want;
         }
         unsigned hits = __ballot_sync(0xffffffffu, f != 0);
-        while (hits) {
-            const int j = __ffs(hits) - 1;
-            hits &= hits - 1;
-            const int32_t uj = __shfl_sync(0xffffffffu, u, j);
-            const uint32_t fj = __shfl_sync(0xffffffffu, f, j);
-            newm |= fj;
-            if ((fj >> lane) & 1u) {
-                if (EXT) acc = mgops::pc_add(acc, a.sig[(size_t)uj * W + lane], true);
-                else accp += a.sig[(size_t)uj * W + lane].m;
+        if constexpr (M == M_INT) {
+            // four hits' loads in flight
+            while (hits) {
+                uint32_t x[4] = {0, 0, 0, 0};
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    if (hits) {
+                        const int j = __ffs(hits) - 1;
+                        hits &= hits - 1;
+                        const int32_t uj = __shfl_sync(0xffffffffu, u, j);
+                        const uint32_t fj = __shfl_sync(0xffffffffu, f, j);
+                        newm |= fj;
+                        if ((fj >> lane) & 1u) x[k] = cnt[(size_t)uj * W + lane];
+                    }
+                }
+#pragma unroll
+                for (int k = 0; k < 4; k++) acci += x[k];
+            }
+        } else {
+            while (hits) {
+                const int j = __ffs(hits) - 1;
+                hits &= hits - 1;
+                const int32_t uj = __shfl_sync(0xffffffffu, u, j);
+                const uint32_t fj = __shfl_sync(0xffffffffu, f, j);
+                newm |= fj;
+                if ((fj >> lane) & 1u) {
+                    if (M == M_EXT) acc = mgops::pc_add(acc, a.sig[(size_t)uj * W + lane], true);
+                    else accp += a.sig[(size_t)uj * W + lane].m;
+                }
             }
         }
     }
     hit = newm;
-    if (!EXT) acc.m = accp;
-    return acc;
+    if constexpr (M == M_INT) {
+        return acci;
+    } else {
+        if (M == M_PLAIN) acc.m = accp;
+        return acc;
+    }
 }
 
-__device__ __forceinline__ void settle_row(const BbArgs &a, uint32_t *fnext, int32_t v, uint32_t newm,
-                                           mgops::PathCount acc)
+// row v reached at level d + 1 from the sources in newm
+template <int M>
+__device__ __forceinline__ void settle_row(const BbArgs &a, uint32_t *fnext, int32_t d, int32_t v, uint32_t newm,
+                                           typename SumOf<M>::T acc)
 {
     const int lane = mgd::lane();
     if ((newm >> lane) & 1u) {
-        a.sig[(size_t)v * W + lane] = acc;
-        if (!a.ext && acc.m >= mgops::PC_PLAIN_MAX) a.ctl->ovf = 1;
+        if constexpr (M == M_INT) {
+            a.cnt[(d + 1) & 1][(size_t)v * W + lane] = (uint32_t)acc;
+            if (acc >= INT_LIMIT) a.ctl->ovf = 1;
+        } else {
+            a.sig[(size_t)v * W + lane] = acc;
+            if (M == M_PLAIN && acc.m >= mgops::PC_PLAIN_MAX) a.ctl->ovf = 1;
+        }
     }
     if (lane == 0) {
         a.vis[v] |= newm;
@@ -349,10 +446,10 @@ __device__ __forceinline__ bool pull_row_thread(const BbArgs &a, const uint32_t 
         mgops::PathCount acc = mgops::pc_zero();
         for (int32_t p = b; p < e; p++) {
             const int32_t u = __ldg(&a.tcol[p]);
-            if ((fcur[u] >> s) & 1u) acc = mgops::pc_add(acc, a.sig[(size_t)u * W + s], a.ext != 0);
+            if ((fcur[u] >> s) & 1u) acc = mgops::pc_add(acc, a.sig[(size_t)u * W + s], a.mode == M_EXT);
         }
         a.sig[(size_t)v * W + s] = acc;
-        if (!a.ext && acc.m >= mgops::PC_PLAIN_MAX) a.ctl->ovf = 1;
+        if (a.mode != M_EXT && acc.m >= mgops::PC_PLAIN_MAX) a.ctl->ovf = 1;
     }
     a.vis[v] |= newm;
     fnext[v] = newm;
@@ -360,7 +457,7 @@ __device__ __forceinline__ bool pull_row_thread(const BbArgs &a, const uint32_t 
 }
 
 // level d -> d+1 over nrows rows (every row when dense, else the candidates)
-template <bool TP, bool EXT>
+template <bool TP, int M>
 __device__ __forceinline__ void bb_pull_phase(const BbArgs &a, const BbCtl &c, int32_t nrows)
 {
     const int lane = mgd::lane();
@@ -391,8 +488,8 @@ __device__ __forceinline__ void bb_pull_phase(const BbArgs &a, const BbCtl &c, i
                 const int32_t b = __ldg(&a.trow[vj]), e = __ldg(&a.trow[vj + 1]);
                 if (e - b > a.heavy_deg) continue;  // chunk path below
                 uint32_t newm;
-                const mgops::PathCount acc = pull_span<EXT>(a, fcur, b, e, wj, newm);
-                if (newm) settle_row(a, fnext, vj, newm, acc);
+                const auto acc = pull_span<M>(a, fcur, c.d, b, e, wj, newm);
+                if (newm) settle_row<M>(a, fnext, c.d, vj, newm, acc);
             }
         }
     } else {
@@ -403,8 +500,8 @@ __device__ __forceinline__ void bb_pull_phase(const BbArgs &a, const BbCtl &c, i
             const int32_t b = __ldg(&a.trow[v]), e = __ldg(&a.trow[v + 1]);
             if (e - b > a.heavy_deg) continue;  // chunk path below
             uint32_t newm;
-            const mgops::PathCount acc = pull_span<EXT>(a, fcur, b, e, want, newm);
-            if (newm) settle_row(a, fnext, v, newm, acc);
+            const auto acc = pull_span<M>(a, fcur, c.d, b, e, want, newm);
+            if (newm) settle_row<M>(a, fnext, c.d, v, newm, acc);
         }
     }
     for (int32_t ch = gwarp; ch < a.nhchunks; ch += nwarps) {
@@ -412,13 +509,14 @@ __device__ __forceinline__ void bb_pull_phase(const BbArgs &a, const BbCtl &c, i
         uint32_t want = ~a.vis[v] & c.gmask;
         if (!c.dense && !mgd::bm_test(a.cbm, v)) want = 0;
         uint32_t newm = 0;
-        mgops::PathCount acc = mgops::pc_zero();
-        if (want) acc = pull_span<EXT>(a, fcur, b, e, want, newm);
-        if (newm) a.hpart[(size_t)ch * W + lane] = acc;
+        typename SumOf<M>::T acc{};
+        if (want) acc = pull_span<M>(a, fcur, c.d, b, e, want, newm);
+        if (newm) reinterpret_cast<typename SumOf<M>::T *>(a.hpart)[(size_t)ch * W + lane] = acc;
         if (lane == 0) a.hmask[ch] = newm;
     }
 }
 
+template <int M>
 __device__ __forceinline__ void bb_heavy_phase(const BbArgs &a, const BbCtl &c)
 {
     const int lane = mgd::lane();
@@ -428,13 +526,16 @@ __device__ __forceinline__ void bb_heavy_phase(const BbArgs &a, const BbCtl &c)
     for (int32_t i = gwarp; i < a.nhrows; i += nwarps) {
         const int32_t v = __ldg(&a.hrows[i]), k0 = __ldg(&a.hrow_chunk[i]), k1 = __ldg(&a.hrow_chunk[i + 1]);
         uint32_t newm = 0;
-        mgops::PathCount acc = mgops::pc_zero();
+        typename SumOf<M>::T acc{};
+        const auto *part = reinterpret_cast<const typename SumOf<M>::T *>(a.hpart);
         for (int32_t k = k0; k < k1; k++) {
             const uint32_t hm = a.hmask[k];
             newm |= hm;
-            if ((hm >> lane) & 1u) acc = mgops::pc_add(acc, a.hpart[(size_t)k * W + lane], a.ext != 0);
+            if (!((hm >> lane) & 1u)) continue;
+            if constexpr (M == M_INT) acc += part[(size_t)k * W + lane];
+            else acc = mgops::pc_add(acc, part[(size_t)k * W + lane], M == M_EXT);
         }
-        if (newm) settle_row(a, fnext, v, newm, acc);
+        if (newm) settle_row<M>(a, fnext, c.d, v, newm, acc);
     }
 }
 
@@ -495,32 +596,34 @@ __device__ __forceinline__ void bbb_start_phase(const BbArgs &a, int32_t L)
     }
 }
 
-template <bool EXT>
-using QT = typename std::conditional<EXT, double, float>::type;
+template <int M>
+using QT = typename std::conditional<M == M_EXT, double, float>::type;
 
-template <bool EXT>
-__device__ __forceinline__ QT<EXT> *q_of(const BbArgs &a)
+// q of level L's vertices
+template <int M>
+__device__ __forceinline__ QT<M> *q_of(const BbArgs &a, int32_t L)
 {
-    return reinterpret_cast<QT<EXT> *>(a.q);
+    if constexpr (M == M_INT) return a.qp[L & 1];
+    else return reinterpret_cast<QT<M> *>(a.q);
 }
 
 // successor v's term for lane s of an entry whose count has scale ku
-template <bool EXT>
-__device__ __forceinline__ QT<EXT> back_term(const BbArgs &a, int32_t v, int s, int32_t ku)
+template <int M>
+__device__ __forceinline__ QT<M> back_term(const BbArgs &a, int32_t L, int32_t v, int s, int32_t ku)
 {
-    QT<EXT> t = q_of<EXT>(a)[(size_t)v * W + s];
-    if (EXT) t *= (QT<EXT>)mgops::pc_scale(ku - a.sig[(size_t)v * W + s].k);
+    QT<M> t = q_of<M>(a, L + 1)[(size_t)v * W + s];
+    if (M == M_EXT) t *= (QT<M>)mgops::pc_scale(ku - a.sig[(size_t)v * W + s].k);
     return t;
 }
 
 // successors' q summed for the sources in `want`: out-edges [b, e); ku is
 // this lane's scale of the entry's path count
-template <bool EXT>
-__device__ __forceinline__ QT<EXT> back_span(const BbArgs &a, const uint32_t *nxt, const int32_t *col, int32_t b,
-                                             int32_t e, uint32_t want, int32_t ku)
+template <int M>
+__device__ __forceinline__ QT<M> back_span(const BbArgs &a, const uint32_t *nxt, int32_t L, const int32_t *col,
+                                           int32_t b, int32_t e, uint32_t want, int32_t ku)
 {
     const int lane = mgd::lane();
-    QT<EXT> acc = 0;
+    QT<M> acc = 0;
     for (int32_t base = b; base < e; base += 32) {
         const int32_t p = base + lane;
         int32_t v = 0;
@@ -535,67 +638,105 @@ __device__ __forceinline__ QT<EXT> back_span(const BbArgs &a, const uint32_t *nx
             hits &= hits - 1;
             const int32_t vj = __shfl_sync(0xffffffffu, v, j);
             const uint32_t fj = __shfl_sync(0xffffffffu, f, j);
-            if ((fj >> lane) & 1u) acc += back_term<EXT>(a, vj, lane, ku);
+            if ((fj >> lane) & 1u) acc += back_term<M>(a, L, vj, lane, ku);
         }
     }
     return acc;
 }
 
 // lane's scale of u's path count (0 in plain mode)
-template <bool EXT>
+template <int M>
 __device__ __forceinline__ int32_t lane_scale(const BbArgs &a, int32_t u, uint32_t msk)
 {
     const int lane = mgd::lane();
-    return (EXT && ((msk >> lane) & 1u)) ? a.sig[(size_t)u * W + lane].k : 0;
+    return (M == M_EXT && ((msk >> lane) & 1u)) ? a.sig[(size_t)u * W + lane].k : 0;
 }
 
-template <bool EXT>
-__device__ __forceinline__ void back_finish(const BbArgs &a, int32_t u, uint32_t msk, QT<EXT> s)
+// delta = count * sum and q = (1 + delta) / count of one (vertex, source);
+// as if formed in FP64 and rounded once.  Integer counts below 2^24 (nearly
+// all) stay in FP32: the product of two FP32 numbers rounds once, and the
+// quotient is corrected by its remainder (1 + delta as an exact pair).
+template <int M>
+__device__ __forceinline__ float back_delta(typename SumOf<M>::T count, QT<M> s, QT<M> &q)
+{
+    if constexpr (M == M_INT) {
+        if (count < (1ull << 24)) {
+            const float sg = (float)(uint32_t)count;
+            const float dv = sg * s;
+            float hi = 1.0f, lo = 0.0f;
+            pair_add(hi, lo, dv);
+            const float q0 = __fdiv_rn(hi, sg);
+            q = q0 + __fdividef(fmaf(-q0, sg, hi) + lo, sg);
+            return dv;
+        }
+        const double sg = (double)count;
+        const float dv = (float)(sg * (double)s);
+        q = (float)((1.0 + (double)dv) / sg);
+        return dv;
+    } else {
+        const float dv = (float)(count.m * (double)s);
+        q = (QT<M>)((1.0 + (double)dv) / count.m);
+        return dv;
+    }
+}
+
+// the (vertex, source) count at level L
+template <int M>
+__device__ __forceinline__ typename SumOf<M>::T count_at(const BbArgs &a, int32_t L, int32_t u, int s)
+{
+    if constexpr (M == M_INT) return a.cnt[L & 1][(size_t)u * W + s];
+    else return a.sig[(size_t)u * W + s];
+}
+
+template <int M>
+__device__ __forceinline__ void back_finish(const BbArgs &a, int32_t L, int32_t u, uint32_t msk, QT<M> s)
 {
     const int lane = mgd::lane();
-    double contrib = 0.0;
+    float hi = 0.0f, lo = 0.0f;
     if ((msk >> lane) & 1u) {
-        const double sg = a.sig[(size_t)u * W + lane].m;
-        const float dv = (float)(sg * (double)s);
-        q_of<EXT>(a)[(size_t)u * W + lane] = (QT<EXT>)((1.0 + (double)dv) / sg);
-        if (__ldg(&a.src[lane]) != u) contrib = (double)dv;
+        const float dv = back_delta<M>(count_at<M>(a, L, u, lane), s, q_of<M>(a, L)[(size_t)u * W + lane]);
+        if (__ldg(&a.src[lane]) != u) hi = dv;
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) contrib += __shfl_xor_sync(0xffffffffu, contrib, o);
-    if (lane == 0) a.bc[u] += contrib;
+    for (int o = 16; o > 0; o >>= 1) {
+        const float h = __shfl_xor_sync(0xffffffffu, hi, o), l = __shfl_xor_sync(0xffffffffu, lo, o);
+        pair_add(hi, lo, h);
+        lo += l;
+    }
+    if (lane == 0) score_add(a, u, hi, lo);
 }
 
 // One thread, one level-L entry (u, msk) with at most TDEG out-edges and
 // at most TBITS sources: back_span and back_finish for each source of the
 // entry in turn (the same sums in the same edge order; the entry's score
 // contributions are added in source order).
-template <bool EXT>
-__device__ __forceinline__ bool back_entry_thread(const BbArgs &a, const uint32_t *nxt, int32_t u, uint32_t msk)
+template <int M>
+__device__ __forceinline__ bool back_entry_thread(const BbArgs &a, const uint32_t *nxt, int32_t L, int32_t u,
+                                                  uint32_t msk)
 {
     if (__popc(msk) > TBITS) return false;
     const int32_t b = __ldg(&a.row[u]), e = __ldg(&a.row[u + 1]);
     if (e - b > TDEG) return false;
-    double contrib = 0.0;
+    float hi = 0.0f, lo = 0.0f;
     uint32_t mm = msk;
     while (mm) {
         const int s = __ffs(mm) - 1;
         mm &= mm - 1;
         const mgops::PathCount su = a.sig[(size_t)u * W + s];
-        QT<EXT> acc = 0;
+        QT<M> acc = 0;
         for (int32_t p = b; p < e; p++) {
             const int32_t v = __ldg(&a.col[p]);
-            if ((nxt[v] >> s) & 1u) acc += back_term<EXT>(a, v, s, su.k);
+            if ((nxt[v] >> s) & 1u) acc += back_term<M>(a, L, v, s, su.k);
         }
-        const float dv = (float)(su.m * (double)acc);
-        q_of<EXT>(a)[(size_t)u * W + s] = (QT<EXT>)((1.0 + (double)dv) / su.m);
-        if (__ldg(&a.src[s]) != u) contrib += (double)dv;
+        const float dv = back_delta<M>(su, acc, q_of<M>(a, L)[(size_t)u * W + s]);
+        if (__ldg(&a.src[s]) != u) pair_add(hi, lo, dv);
     }
-    a.bc[u] += contrib;
+    score_add(a, u, hi, lo);
     return true;
 }
 
 // backward level L: every level-L entry from its level-(L+1) successors
-template <bool TP, bool EXT>
+template <bool TP, int M>
 __device__ __forceinline__ void bbb_pull_phase(const BbArgs &a, int32_t L)
 {
     const int lane = mgd::lane();
@@ -616,7 +757,7 @@ __device__ __forceinline__ void bbb_pull_phase(const BbArgs &a, int32_t L)
             if (lane < vpw && i < hi) {
                 u = a.arch[i];
                 msk = a.amask[i];
-                deferred = !back_entry_thread<EXT>(a, nxt, u, msk);
+                deferred = !back_entry_thread<M>(a, nxt, L, u, msk);
             }
             unsigned dm = __ballot_sync(0xffffffffu, deferred);
             while (dm) {
@@ -626,8 +767,8 @@ __device__ __forceinline__ void bbb_pull_phase(const BbArgs &a, int32_t L)
                 const uint32_t mj = __shfl_sync(0xffffffffu, msk, j);
                 const int32_t b = __ldg(&a.row[uj]), e = __ldg(&a.row[uj + 1]);
                 if (e - b > a.heavy_deg) continue;  // chunk path below
-                const QT<EXT> sj = back_span<EXT>(a, nxt, a.col, b, e, mj, lane_scale<EXT>(a, uj, mj));
-                back_finish<EXT>(a, uj, mj, sj);
+                const QT<M> sj = back_span<M>(a, nxt, L, a.col, b, e, mj, lane_scale<M>(a, uj, mj));
+                back_finish<M>(a, L, uj, mj, sj);
             }
         }
     } else {
@@ -636,37 +777,37 @@ __device__ __forceinline__ void bbb_pull_phase(const BbArgs &a, int32_t L)
             const uint32_t msk = a.amask[i];
             const int32_t b = __ldg(&a.row[u]), e = __ldg(&a.row[u + 1]);
             if (e - b > a.heavy_deg) continue;  // chunk path below
-            const QT<EXT> s = back_span<EXT>(a, nxt, a.col, b, e, msk, lane_scale<EXT>(a, u, msk));
-            back_finish<EXT>(a, u, msk, s);
+            const QT<M> s = back_span<M>(a, nxt, L, a.col, b, e, msk, lane_scale<M>(a, u, msk));
+            back_finish<M>(a, L, u, msk, s);
         }
     }
     // heavy rows: the in-row chunks double as out-row chunks (symmetric graphs)
-    QT<EXT> *hp = reinterpret_cast<QT<EXT> *>(a.hpart);
+    QT<M> *hp = reinterpret_cast<QT<M> *>(a.hpart);
     for (int32_t ch = gwarp; ch < a.nhchunks; ch += nwarps) {
         const int32_t u = __ldg(&a.hchunk[3 * ch]);
         const uint32_t msk = cur[u];
         if (msk == 0) continue;
-        hp[(size_t)ch * W + lane] = back_span<EXT>(a, nxt, a.tcol, __ldg(&a.hchunk[3 * ch + 1]), __ldg(&a.hchunk[3 * ch + 2]), msk,
-                                                   lane_scale<EXT>(a, u, msk));
+        hp[(size_t)ch * W + lane] = back_span<M>(a, nxt, L, a.tcol, __ldg(&a.hchunk[3 * ch + 1]), __ldg(&a.hchunk[3 * ch + 2]), msk,
+                                                   lane_scale<M>(a, u, msk));
     }
 }
 
 // heavy rows: chunk partials folded in chunk order (graphs with heavy rows)
-template <bool EXT>
+template <int M>
 __device__ __forceinline__ void bbb_heavy_phase(const BbArgs &a, int32_t L)
 {
     const int lane = mgd::lane();
     const int gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
     const uint32_t *cur = fmb_of(a, L);
-    const QT<EXT> *hp = reinterpret_cast<const QT<EXT> *>(a.hpart);
+    const QT<M> *hp = reinterpret_cast<const QT<M> *>(a.hpart);
     for (int32_t i = gwarp; i < a.nhrows; i += nwarps) {
         const int32_t u = __ldg(&a.hrows[i]);
         const uint32_t msk = cur[u];
         if (msk == 0) continue;
-        QT<EXT> s = 0;
+        QT<M> s = 0;
         for (int32_t k = __ldg(&a.hrow_chunk[i]); k < __ldg(&a.hrow_chunk[i + 1]); k++) s += hp[(size_t)k * W + lane];
-        back_finish<EXT>(a, u, msk, s);
+        back_finish<M>(a, L, u, msk, s);
     }
 }
 
@@ -682,6 +823,274 @@ __device__ __forceinline__ void bbb_next_phase(const BbArgs &a, int32_t L)
     if (L >= 2) {
         uint32_t *prv = fmb_of(a, L - 1);
         for (int32_t i = a.off[L - 1] + gtid; i < a.off[L]; i += stride) prv[a.arch[i]] = a.amask[i];
+    }
+}
+
+
+// ---------------------------------------------------------------------------
+// mask-free levels (M_INT): eight lanes a row, four sources (16 bytes) a lane
+// ---------------------------------------------------------------------------
+constexpr int GL = 8;              // lanes a row
+constexpr int32_t GCHUNK = 256;    // rows above this many edges go in chunks
+
+// Sum over the columns [b, e) of the rows val[col][..] (this lane's four
+// sources) through add(t[8]).  All lanes of the warp call (a group without
+// work passes b == e) and run over the longest of their ranges; the next
+// eight ids are loaded ahead of the current gathers.
+template <class V, class Add>
+__device__ __forceinline__ void gather_rows(const V *__restrict__ val, const int32_t *__restrict__ col, int32_t b,
+                                            int32_t e, Add add)
+{
+    const int gl = threadIdx.x & (GL - 1);
+    const int32_t rounds = (int32_t)__reduce_max_sync(0xffffffffu, (unsigned)((e - b + GL - 1) / GL));
+    int32_t id = b + gl < e ? __ldcs(&col[b + gl]) : -1;
+    for (int32_t r = 0; r < rounds; r++) {
+        V t[GL];
+#pragma unroll
+        for (int j = 0; j < GL; j++) {
+            const int32_t u = __shfl_sync(0xffffffffu, id, j, GL);
+            t[j] = u >= 0 ? val[(size_t)u * GL + gl] : V{};
+        }
+        b += GL;
+        id = b + gl < e ? __ldcs(&col[b + gl]) : -1;
+        add(t);
+    }
+}
+
+struct Sum4 {
+    unsigned long long x = 0, y = 0, z = 0, w = 0;
+    __device__ __forceinline__ void add(const uint4 (&t)[GL])
+    {
+        x += ((t[0].x + t[1].x) + (t[2].x + t[3].x)) + ((t[4].x + t[5].x) + (t[6].x + t[7].x));
+        y += ((t[0].y + t[1].y) + (t[2].y + t[3].y)) + ((t[4].y + t[5].y) + (t[6].y + t[7].y));
+        z += ((t[0].z + t[1].z) + (t[2].z + t[3].z)) + ((t[4].z + t[5].z) + (t[6].z + t[7].z));
+        w += ((t[0].w + t[1].w) + (t[2].w + t[3].w)) + ((t[4].w + t[5].w) + (t[6].w + t[7].w));
+    }
+};
+
+// row v's new counts (this lane's four sums): stored for the sources that
+// had not reached v, the row's masks updated (all eight lanes of the row's
+// group call)
+__device__ __forceinline__ void gather_settle(const BbArgs &a, uint32_t *fnext, int32_t d, int32_t v, uint32_t want,
+                                              const Sum4 &s, unsigned gmask)
+{
+    const int gl = threadIdx.x & (GL - 1);
+    const unsigned long long x[4] = {s.x, s.y, s.z, s.w};
+    uint32_t m = 0;
+    uint32_t *out = a.cnt[(d + 1) & 1] + (size_t)v * W + gl * 4;
+    bool over = false;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const uint32_t bit = 1u << (gl * 4 + k);
+        if (x[k] != 0 && (want & bit)) {
+            m |= bit;
+            out[k] = (uint32_t)x[k];
+            over |= x[k] >= INT_LIMIT;
+        }
+    }
+    if (over) a.ctl->ovf = 1;
+    const uint32_t newm = __reduce_or_sync(gmask, m);
+    if (gl == 0 && newm) {
+        a.vis[v] |= newm;
+        fnext[v] = newm;
+    }
+}
+
+__device__ __forceinline__ unsigned group_mask() { return 0xffu << (mgd::lane() & ~(GL - 1)); }
+
+__device__ __forceinline__ void bb_gather_phase(const BbArgs &a, const BbCtl &c)
+{
+    constexpr int RPW = 32 / GL;
+    const int gl = threadIdx.x & (GL - 1), grp = mgd::lane() / GL;
+    const int gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int nwarps = (gridDim.x * blockDim.x) >> 5;
+    const uint4 *val = reinterpret_cast<const uint4 *>(a.cnt[c.d & 1]);
+    uint32_t *fnext = fm_of(a, c.cur ^ 1);
+    const unsigned gm = group_mask();
+    ulonglong2 *part = reinterpret_cast<ulonglong2 *>(a.gpart);
+    for (int32_t c0 = gwarp * RPW; c0 < a.ngchunks; c0 += nwarps * RPW) {
+        const int32_t ch = c0 + grp;
+        int32_t b = 0, e = 0;
+        if (ch < a.ngchunks && (~a.vis[__ldg(&a.gchunk[3 * ch])] & c.gmask)) {
+            b = __ldg(&a.gchunk[3 * ch + 1]);
+            e = __ldg(&a.gchunk[3 * ch + 2]);
+        }
+        Sum4 s;
+        gather_rows(val, a.tcol, b, e, [&](const uint4 (&t)[GL]) { s.add(t); });
+        if (e > b) {
+            part[(size_t)ch * 16 + gl * 2] = make_ulonglong2(s.x, s.y);
+            part[(size_t)ch * 16 + gl * 2 + 1] = make_ulonglong2(s.z, s.w);
+        }
+    }
+    // the next row's mask and offsets are loaded ahead of this row's gathers
+    int32_t v = gwarp * RPW + grp;
+    uint32_t want = v < a.n ? ~a.vis[v] & c.gmask : 0u;
+    int32_t b = v < a.n ? __ldg(&a.trow[v]) : 0, e = v < a.n ? __ldg(&a.trow[v + 1]) : 0;
+    for (int32_t v0 = gwarp * RPW; v0 < a.n; v0 += nwarps * RPW) {
+        const int32_t vn = v + nwarps * RPW;
+        const uint32_t wn = vn < a.n ? ~a.vis[vn] & c.gmask : 0u;
+        const int32_t bn = vn < a.n ? __ldg(&a.trow[vn]) : 0, en = vn < a.n ? __ldg(&a.trow[vn + 1]) : 0;
+        const bool row = want != 0 && e - b <= GCHUNK;
+        Sum4 s;
+        gather_rows(val, a.tcol, b, row ? e : b, [&](const uint4 (&t)[GL]) { s.add(t); });
+        if (row) gather_settle(a, fnext, c.d, v, want, s, gm);
+        v = vn;
+        want = wn;
+        b = bn;
+        e = en;
+    }
+}
+
+// rows above GCHUNK edges: their chunks' sums
+__device__ __forceinline__ void bb_gather_heavy_phase(const BbArgs &a, const BbCtl &c)
+{
+    constexpr int RPW = 32 / GL;
+    const int gl = threadIdx.x & (GL - 1), grp = mgd::lane() / GL;
+    const int gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int nwarps = (gridDim.x * blockDim.x) >> 5;
+    uint32_t *fnext = fm_of(a, c.cur ^ 1);
+    const ulonglong2 *part = reinterpret_cast<const ulonglong2 *>(a.gpart);
+    for (int32_t i = gwarp; i < a.ngrows; i += nwarps) {
+        const int32_t v = __ldg(&a.grows[i]);
+        const uint32_t want = ~a.vis[v] & c.gmask;
+        if (want == 0) continue;   // warp-uniform
+        Sum4 s;
+        for (int32_t k = __ldg(&a.grow_chunk[i]) + grp, k1 = __ldg(&a.grow_chunk[i + 1]); k < k1; k += RPW) {
+            const ulonglong2 p = __ldcs(&part[(size_t)k * 16 + gl * 2]), r = __ldcs(&part[(size_t)k * 16 + gl * 2 + 1]);
+            s.x += p.x;
+            s.y += p.y;
+            s.z += r.x;
+            s.w += r.y;
+        }
+#pragma unroll
+        for (int o = GL; o < 32; o <<= 1) {
+            s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
+            s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+            s.z += __shfl_xor_sync(0xffffffffu, s.z, o);
+            s.w += __shfl_xor_sync(0xffffffffu, s.w, o);
+        }
+        if (grp == 0) gather_settle(a, fnext, c.d, v, want, s, 0xffu);
+    }
+}
+
+__device__ __forceinline__ bool back_gathers(const BbArgs &a, int32_t L)
+{
+    return a.mode == M_INT && __ldcg(&a.lnfe[L]) * GATHER_BACK > (unsigned long long)a.m;
+}
+
+__device__ __forceinline__ void f4_sum8(float4 &acc, const float4 (&t)[GL])
+{
+    acc.x += ((t[0].x + t[1].x) + (t[2].x + t[3].x)) + ((t[4].x + t[5].x) + (t[6].x + t[7].x));
+    acc.y += ((t[0].y + t[1].y) + (t[2].y + t[3].y)) + ((t[4].y + t[5].y) + (t[6].y + t[7].y));
+    acc.z += ((t[0].z + t[1].z) + (t[2].z + t[3].z)) + ((t[4].z + t[5].z) + (t[6].z + t[7].z));
+    acc.w += ((t[0].w + t[1].w) + (t[2].w + t[3].w)) + ((t[4].w + t[5].w) + (t[6].w + t[7].w));
+}
+
+// entry (u, msk) of level L from its successors' sums: q of this lane's
+// sources and the row's score (the eight lanes of the group call)
+__device__ __forceinline__ void gather_finish(const BbArgs &a, int32_t L, int32_t u, uint32_t msk, float4 sum,
+                                              const int4 &src, unsigned gm)
+{
+    const int gl = threadIdx.x & (GL - 1);
+    const uint4 c4 = *reinterpret_cast<const uint4 *>(a.cnt[L & 1] + (size_t)u * W + gl * 4);
+    const uint32_t c[4] = {c4.x, c4.y, c4.z, c4.w};
+    const float s[4] = {sum.x, sum.y, sum.z, sum.w};
+    const int32_t sr[4] = {src.x, src.y, src.z, src.w};
+    float *out = a.qp[L & 1] + (size_t)u * W + gl * 4;
+    float hi = 0.0f, lo = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+        if ((msk >> (gl * 4 + k)) & 1u) {
+            const float dv = back_delta<M_INT>(c[k], s[k], out[k]);
+            if (sr[k] != u) pair_add(hi, lo, dv);
+        }
+#pragma unroll
+    for (int o = GL / 2; o > 0; o >>= 1) {
+        const float h = __shfl_xor_sync(gm, hi, o), l = __shfl_xor_sync(gm, lo, o);
+        pair_add(hi, lo, h);
+        lo += l;
+    }
+    if (gl == 0) score_add(a, u, hi, lo);
+}
+
+__device__ __forceinline__ int4 lane_sources(const BbArgs &a)
+{
+    return *reinterpret_cast<const int4 *>(a.src + (threadIdx.x & (GL - 1)) * 4);
+}
+
+__device__ __forceinline__ void bbb_gather_phase(const BbArgs &a, int32_t L)
+{
+    constexpr int RPW = 32 / GL;
+    const int gl = threadIdx.x & (GL - 1), grp = mgd::lane() / GL;
+    const int gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int nwarps = (gridDim.x * blockDim.x) >> 5;
+    const float4 *val = reinterpret_cast<const float4 *>(a.qp[(L + 1) & 1]);
+    const uint32_t *cur = fmb_of(a, L);
+    const unsigned gm = group_mask();
+    float4 *part = reinterpret_cast<float4 *>(a.gpart);
+    for (int32_t c0 = gwarp * RPW; c0 < a.ngchunks; c0 += nwarps * RPW) {
+        const int32_t ch = c0 + grp;
+        int32_t b = 0, e = 0;
+        if (ch < a.ngchunks && cur[__ldg(&a.gchunk[3 * ch])]) {
+            b = __ldg(&a.gchunk[3 * ch + 1]);
+            e = __ldg(&a.gchunk[3 * ch + 2]);
+        }
+        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+        gather_rows(val, a.tcol, b, e, [&](const float4 (&t)[GL]) { f4_sum8(s, t); });
+        if (e > b) part[(size_t)ch * GL + gl] = s;
+    }
+    const int4 src = lane_sources(a);
+    const int32_t lo = a.off[L], hi = a.off[L + 1];
+    int32_t i = lo + gwarp * RPW + grp;
+    int32_t u = i < hi ? a.arch[i] : 0;
+    uint32_t msk = i < hi ? a.amask[i] : 0u;
+    int32_t b = __ldg(&a.trow[u]), e = __ldg(&a.trow[u + 1]);
+    for (int32_t i0 = lo + gwarp * RPW; i0 < hi; i0 += nwarps * RPW) {
+        const int32_t in = i + nwarps * RPW;
+        const int32_t un = in < hi ? a.arch[in] : 0;
+        const uint32_t mn = in < hi ? a.amask[in] : 0u;
+        const bool row = msk != 0 && e - b <= GCHUNK;
+        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+        gather_rows(val, a.tcol, b, row ? e : b, [&](const float4 (&t)[GL]) { f4_sum8(s, t); });
+        const int32_t bn = __ldg(&a.trow[un]), en = __ldg(&a.trow[un + 1]);
+        if (row) gather_finish(a, L, u, msk, s, src, gm);
+        i = in;
+        u = un;
+        msk = mn;
+        b = bn;
+        e = en;
+    }
+}
+
+__device__ __forceinline__ void bbb_gather_heavy_phase(const BbArgs &a, int32_t L)
+{
+    constexpr int RPW = 32 / GL;
+    const int gl = threadIdx.x & (GL - 1), grp = mgd::lane() / GL;
+    const int gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int nwarps = (gridDim.x * blockDim.x) >> 5;
+    const uint32_t *cur = fmb_of(a, L);
+    const float4 *part = reinterpret_cast<const float4 *>(a.gpart);
+    const int4 src = lane_sources(a);
+    for (int32_t r = gwarp; r < a.ngrows; r += nwarps) {
+        const int32_t u = __ldg(&a.grows[r]);
+        const uint32_t msk = cur[u];
+        if (msk == 0) continue;   // warp-uniform
+        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int32_t k = __ldg(&a.grow_chunk[r]) + grp, k1 = __ldg(&a.grow_chunk[r + 1]); k < k1; k += RPW) {
+            const float4 p = __ldcs(&part[(size_t)k * GL + gl]);
+            s.x += p.x;
+            s.y += p.y;
+            s.z += p.z;
+            s.w += p.w;
+        }
+#pragma unroll
+        for (int o = GL; o < 32; o <<= 1) {
+            s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
+            s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+            s.z += __shfl_xor_sync(0xffffffffu, s.z, o);
+            s.w += __shfl_xor_sync(0xffffffffu, s.w, o);
+        }
+        if (grp == 0) gather_finish(a, L, u, msk, s, src, 0xffu);
     }
 }
 

@@ -155,6 +155,7 @@ struct mg_graph {
     int32_t nv = 0, ne = 0;
     bool symmetric = true;         // transpose == graph (pull uses the same arrays)
     bool bc_ext = false;           // BC path counts overflowed plain FP64 once: extended from then on
+    bool bcb_no_int = false;       // batched BC: path counts passed 2^29 once: FP64 counts from then on
     bool weights_symmetric = true; // weight of (u,v) == weight of (v,u)
     // CSR (push side, out-edges)
     mgi::DevBuf row, col, wt;
@@ -178,7 +179,8 @@ struct mg_graph {
     std::vector<int32_t> h_prow;   // pull-side row offsets (engine order), for re-binning
     int32_t n_dangling = 0;        // vertices with out-degree 0
     int32_t min_weight = 0;        // smallest integer edge weight
-    // PPR heavy rows: rows with in-degree > PPR_HEAVY split in PPR_CHUNK pieces
+    // pull rows above 256 in-edges in 256-edge chunks (personalised PageRank,
+    // batched BC's mask-free levels): mgi::ppr_chunks
     mgi::DevBuf ppr_hchunk, ppr_hrows, ppr_hrow_chunk;
     int32_t ppr_nhchunks = -1, ppr_nhrows = 0;
     // float edge weights for weighted PageRank (CSR order)
@@ -242,6 +244,8 @@ mg_status edge_grad_to_caller(mg_graph *g, const float2 *ct, const float *val, f
 // bin cutoff) from the
 // host copy of the pull-side row offsets; drops the algorithm workspaces
 mg_status rebin(mg_graph *g, int32_t heavy, int32_t chunk, int32_t tbin);
+// the table of rows above 256 in-edges (once per layout)
+mg_status ppr_chunks(mg_graph *g);
 // batched multi-source BC over engine-id sources (symmetric graphs); the
 // float scores in engine order stay in the graph's BC workspace
 mg_status bc_batched(mg_graph *g, const int32_t *src_engine, int32_t nsrc, const mg_opts &opt, mg_run_info *info,

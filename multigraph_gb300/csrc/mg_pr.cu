@@ -1741,6 +1741,33 @@ mg_status mg_wpagerank_backward(mg_graph *g, const float *g_host, const mg_opts 
 
 }  // extern "C"
 
+// heavy-row chunk table (built once per layout from the pull offsets)
+mg_status mgi::ppr_chunks(mg_graph *g)
+{
+    if (g->ppr_nhchunks >= 0) return MG_OK;
+    const std::vector<int32_t> &pr = g->h_prow;
+    std::vector<int32_t> hc, hr, hrc{0};
+    for (int32_t v = 0; v < g->nv; v++) {
+        if (pr[v + 1] - pr[v] <= PPR_HEAVY) continue;
+        hr.push_back(v);
+        for (int32_t b = pr[v]; b < pr[v + 1]; b += PPR_HEAVY) {
+            hc.push_back(v); hc.push_back(b); hc.push_back(std::min(pr[v + 1], b + PPR_HEAVY));
+        }
+        hrc.push_back((int32_t)(hc.size() / 3));
+    }
+    cudaStream_t s = g->stream;
+    MG_TRY(dev_alloc(g->ppr_hchunk, std::max<size_t>(hc.size(), 3) * 4));
+    MG_TRY(dev_alloc(g->ppr_hrows, std::max<size_t>(hr.size(), 1) * 4));
+    MG_TRY(dev_alloc(g->ppr_hrow_chunk, hrc.size() * 4));
+    if (!hc.empty()) MG_CUDA(cudaMemcpyAsync(g->ppr_hchunk.p, hc.data(), hc.size() * 4, cudaMemcpyHostToDevice, s));
+    if (!hr.empty()) MG_CUDA(cudaMemcpyAsync(g->ppr_hrows.p, hr.data(), hr.size() * 4, cudaMemcpyHostToDevice, s));
+    MG_CUDA(cudaMemcpyAsync(g->ppr_hrow_chunk.p, hrc.data(), hrc.size() * 4, cudaMemcpyHostToDevice, s));
+    MG_CUDA(cudaStreamSynchronize(s));
+    g->ppr_nhchunks = (int32_t)(hc.size() / 3);
+    g->ppr_nhrows = (int32_t)hr.size();
+    return MG_OK;
+}
+
 // one pass of up to 4 LPR seeds: sweeps until every seed's L1 change is at
 // most tol
 template <int LPR, bool DANG>
@@ -1801,30 +1828,7 @@ mg_status mg_ppr_batch(mg_graph *g, const int32_t *seeds, int32_t nseeds, const 
     PprWS *w = g->ppws;
     const size_t n = (size_t)std::max(g->nv, 1);
     cudaStream_t s = g->stream;
-    // heavy-row chunk table for PPR (built once per graph from the pull offsets)
-    if (g->ppr_nhchunks < 0) {
-        std::vector<int32_t> pr(n + 1);
-        MG_CUDA(cudaMemcpyAsync(pr.data(), g->trow, (size_t)(g->nv + 1) * 4, cudaMemcpyDeviceToHost, s));
-        MG_CUDA(cudaStreamSynchronize(s));
-        std::vector<int32_t> hc, hr, hrc{0};
-        for (int32_t v = 0; v < g->nv; v++) {
-            if (pr[v + 1] - pr[v] <= PPR_HEAVY) continue;
-            hr.push_back(v);
-            for (int32_t b = pr[v]; b < pr[v + 1]; b += PPR_HEAVY) {
-                hc.push_back(v); hc.push_back(b); hc.push_back(std::min(pr[v + 1], b + PPR_HEAVY));
-            }
-            hrc.push_back((int32_t)(hc.size() / 3));
-        }
-        MG_TRY(dev_alloc(g->ppr_hchunk, std::max<size_t>(hc.size(), 3) * 4));
-        MG_TRY(dev_alloc(g->ppr_hrows, std::max<size_t>(hr.size(), 1) * 4));
-        MG_TRY(dev_alloc(g->ppr_hrow_chunk, hrc.size() * 4));
-        if (!hc.empty()) MG_CUDA(cudaMemcpyAsync(g->ppr_hchunk.p, hc.data(), hc.size() * 4, cudaMemcpyHostToDevice, s));
-        if (!hr.empty()) MG_CUDA(cudaMemcpyAsync(g->ppr_hrows.p, hr.data(), hr.size() * 4, cudaMemcpyHostToDevice, s));
-        MG_CUDA(cudaMemcpyAsync(g->ppr_hrow_chunk.p, hrc.data(), hrc.size() * 4, cudaMemcpyHostToDevice, s));
-        MG_CUDA(cudaStreamSynchronize(s));
-        g->ppr_nhchunks = (int32_t)(hc.size() / 3);
-        g->ppr_nhrows = (int32_t)hr.size();
-    }
+    MG_TRY(ppr_chunks(g));
     // lanes per row: as many as the widest pass of this call needs
     const int32_t widest = std::min(nseeds, 32);
     const size_t width = widest > 16 ? 32 : widest > 8 ? 16 : widest > 4 ? 8 : 4;
