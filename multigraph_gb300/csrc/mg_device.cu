@@ -928,7 +928,7 @@ static void destroy_graph(mg_graph *g)
     hub_free(g);
     DevBuf *bufs[] = {&g->row, &g->col, &g->wt, &g->trow_own, &g->tcol_own, &g->twt_own,
                       &g->hchunk, &g->hrows, &g->hrow_chunk, &g->fw, &g->o_fw, &g->ppr_hchunk, &g->ppr_hrows,
-                      &g->ppr_hrow_chunk, &g->o_row, &g->o_col, &g->o_wt, &g->old2new, &g->new2old,
+                      &g->ppr_hrow_chunk, &g->ppr_hchunk_at, &g->o_row, &g->o_col, &g->o_wt, &g->old2new, &g->new2old,
                       &g->wrows, &g->trows, &g->pos_row, &g->cpos, &g->sym_sums, &g->s_row,
                       &g->s_col, &g->s_wt};
     for (DevBuf *b : bufs) dev_free(*b);

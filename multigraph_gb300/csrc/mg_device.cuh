@@ -7,6 +7,7 @@
 
 #include "mg_bins.cuh"
 
+#include <cstdlib>
 #include <functional>
 #include <string>
 #include <vector>
@@ -181,8 +182,9 @@ struct mg_graph {
     int32_t min_weight = 0;        // smallest integer edge weight
     // pull rows above 256 in-edges in 256-edge chunks (personalised PageRank,
     // batched BC's mask-free levels): mgi::ppr_chunks
-    mgi::DevBuf ppr_hchunk, ppr_hrows, ppr_hrow_chunk;
+    mgi::DevBuf ppr_hchunk, ppr_hrows, ppr_hrow_chunk, ppr_hchunk_at;  // (.._at: each chunk's place in hrows)
     int32_t ppr_nhchunks = -1, ppr_nhrows = 0;
+    int32_t short_rows = 0;        // (the same table) first of the short rows at the end of the order
     // float edge weights for weighted PageRank (CSR order)
     mgi::DevBuf fw;
     bool has_fw = false;
@@ -226,6 +228,14 @@ mg_status begin_run(mg_graph *g, const mg_opts *o, mg_opts &opt, mg_run_info *in
 mg_status end_run(mg_graph *g, const mg_opts &opt, mg_run_info *info);
 mg_status copy_out(mg_graph *g, void *host, const void *dev, size_t bytes);
 int launch_grid(const mg_graph *g, int threads, int per_sm);
+// failure injection for tests (MG_FAIL_BARRIER=1): the persistent kernels'
+// barriers never complete, their bounded waits run out and the run reports
+// an error
+inline int fail_barrier()
+{
+    const char *fb = std::getenv("MG_FAIL_BARRIER");
+    return (fb && fb[0] == '1') ? 1 : 0;
+}
 // caller ids <-> engine ids (identity unless the graph was relabeled)
 int32_t to_engine(const mg_graph *g, int32_t v);
 // result in engine order (rows x nv elements of elem = 4 or 8 bytes) -> a
@@ -301,12 +311,13 @@ __device__ __forceinline__ void kahan_add(float &t, float &r, float x)
 // Warp-wide sum of the lanes' compensated sums (t - r), every lane gets the
 // total: an xor tree whose adds carry their exact rounding errors (TwoSum),
 // so the total rounds about once.  TwoSum is exact in either operand order,
-// so every lane forms the same value.
+// so every lane forms the same value.  G < 32: over groups of G lanes.
+template <int G = 32>
 __device__ __forceinline__ float warp_sum_comp(float t, float r)
 {
     float v = t - r, c = 0.0f;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
+    for (int o = G / 2; o > 0; o >>= 1) {
         const float vo = __shfl_xor_sync(0xffffffffu, v, o);
         const float co = __shfl_xor_sync(0xffffffffu, c, o);
         const float u = v + vo;

@@ -946,10 +946,7 @@ inline Args make_args(mg_graph *g)
     a.bar = w->bar.as<unsigned>();
     a.cnt = w->cnt.as<LevelCnt>();
     a.bar_err = reinterpret_cast<int *>(w->bar.as<unsigned>() + 2 + mgd::GRID_SYNC_GROUPS);
-    // failure injection for tests: the persistent kernels' barriers never
-    // complete, their bounded waits run out and the run reports an error
-    const char *fb = std::getenv("MG_FAIL_BARRIER");
-    a.bar_never = (fb && fb[0] == '1') ? 1 : 0;
+    a.bar_never = mgi::fail_barrier();
     return a;
 }
 

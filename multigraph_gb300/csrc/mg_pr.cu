@@ -123,8 +123,9 @@ constexpr int NPART = 5;       // partials per block slot
 constexpr int SPARSE_ALPHA = 16;  // queue sweeps once active in-edges < m / SPARSE_ALPHA
 
 // ---------------------------------------------------------------------------
-// PageRank operators: the engine (k_pr_light / k_pr_apply / k_prd_*) is a
-// template over one of these.  Hooks:
+// PageRank operators: the engine (k_pr_light / k_pr_apply / k_prd_*, k_pr_all)
+// is a template over one of these.  Row state that another block may have
+// written earlier in the same launch (k_pr_all) is read through L2.  Hooks:
 //   apply(a, c, v, s, any, dang)  row v's update from its gathered sum s:
 //                                 writes the next iterate and contribution,
 //                                 returns |change|, sets any when the row
@@ -185,7 +186,7 @@ struct PrTopology {
                                                   float &dang)
     {
         const int cur = c.cur, nxt = cur ^ 1;
-        const float xo = a.x[cur][v];
+        const float xo = __ldcg(&a.x[cur][v]);
         const int32_t od = a.outrow[v + 1] - a.outrow[v];
         const float xn = c.base + c.damping * s;
         a.x[nxt][v] = xn;
@@ -229,7 +230,7 @@ struct PrWeighted {
                                                   float &dang)
     {
         const int cur = c.cur, nxt = cur ^ 1;
-        const float xo = a.x[cur][v];
+        const float xo = __ldcg(&a.x[cur][v]);
         const float xn = c.base + c.damping * s;
         a.x[nxt][v] = xn;
         const float Su = a.S[v];
@@ -251,7 +252,7 @@ struct PrAdjoint {
         const float Su = a.S[v];
         const float t = Su > 0.0f ? s / Su : c.lam_meanf;
         const float xn = a.gvec[v] + c.damping * t;
-        const float xo = a.c[cur][v];
+        const float xo = __ldcg(&a.c[cur][v]);
         a.c[nxt][v] = xn;
         dang = xn;  // sum of lambda for the mean
         return fabsf(xn - xo);
@@ -700,6 +701,225 @@ __global__ void __launch_bounds__(THREADS) k_pr_apply(PArgs a, cudaGraphConditio
     }
     block_partials<Op::kDataDriven>(a, a.nblocks + blockIdx.x, (float)resid, (float)dangs, any, act, dfz);
     close_sweep<Op>(a, c, a.nblocks + gridDim.x, h, use_cond);
+}
+
+// ---------------------------------------------------------------------------
+// Small graphs: the whole run -- start values, every sweep, the result in
+// caller order -- in one cooperative launch, a grid barrier per sweep.
+// A sweep of the other layouts costs two launches, 152 stagings of up to
+// 224 KB and a reduction over 1,216 blocks: 33 us on R-MAT 16 (1.8 M edges)
+// whatever the size.  Here rows of up to ALL_CHUNK in-edges take eight lanes
+// each (four rows a warp), the short rows at the end of the hub-first order
+// (fewer than ALL_SHORT in-edges; every row of a low-degree graph) a thread,
+// longer ones a warp per ALL_CHUNK-edge chunk, the last chunk to finish
+// adding up the row (chunk order, so the sum does not depend on who is last).
+// Contributions are gathered through L1 (the barrier's fence makes the other
+// blocks' values visible there): the hubs' few sectors read by every edge
+// straight from L2 took the R-MAT 16 sweep from 18 to 48 us.  Sums are
+// compensated as in the segmented layout.  After the barrier every block
+// adds up the 152 blocks' partial sums itself and comes to the same
+// decision.  Only for forms that are continuous in the sums' rounding
+// (normalised, weighted, adjoint): the data-driven form freezes and PR_T
+// holds a row by comparing its change with a threshold, where one last bit
+// can decide.  R-MAT 16: 30 -> 18 us per sweep, 320 x 311 lattice 18 -> 7 us.
+// ---------------------------------------------------------------------------
+constexpr int ALL_THREADS = 1024;
+constexpr int32_t ALL_CHUNK = 256;
+constexpr int32_t ALL_SHORT = 16;
+// Up to this many edges; past them the other layouts' sweeps, whose blocks
+// are resident twice as densely, are the faster ones.  us per sweep, here /
+// segmented / gather: R-MAT 17 (3.7 M edges) 25 / 32 / 36, R-MAT 19 of edge
+// factor 6 (6.0 M) 35 / 38 / 39, R-MAT 18 (7.6 M) 40 / 39 / 42, R-MAT 19
+// (15.5 M) 84 / 41 / 57.  Graphs of short rows only: 1500 x 1400 lattice
+// (8.6 M) 21 / 48 / 30.
+constexpr int64_t ALL_MAX_EDGES = 6 << 20, ALL_MAX_EDGES_SHORT = 12 << 20;
+
+struct PrAllArgs {
+    const int32_t *chunk, *chunk_at, *rows, *row_chunk;  // rows above ALL_CHUNK edges (mgi::ppr_chunks)
+    int32_t nchunks;
+    int32_t split;          // rows [0, split) take eight lanes, the others a thread each
+    int32_t *arrive;        // [rows] chunks finished (zero before the launch, only grows)
+    float *part;            // [chunks] partial sums
+    double *bsum;           // [2][grid][3] blocks' sums by sweep parity
+    unsigned *bar;          // grid barrier word (zero before the launch), error word
+    int *bar_err;
+    int bar_never;
+    const int32_t *old2new; // null: engine ids are the caller's
+    float *out;             // result in caller order (null: left in x[cur] / c[cur])
+    float x0;
+};
+
+template <class Op>
+__global__ void __launch_bounds__(ALL_THREADS, 1) k_pr_all(PArgs a, PrAllArgs z)
+{
+    static_assert(!Op::kDataDriven, "rows are never skipped here");
+    constexpr unsigned FULL = 0xffffffffu;
+    constexpr int NW = ALL_THREADS / 32;
+    __shared__ PCtl s_c;
+    __shared__ double s_r[NW], s_d[NW];
+    __shared__ int s_a[NW];
+    const int lane = mgd::lane(), warp = threadIdx.x >> 5, gl = lane & 7, grp = lane >> 3;
+    const int gwarp = blockIdx.x * NW + warp, nwarps = gridDim.x * NW;
+    const int32_t *pw = reinterpret_cast<const int32_t *>(a.pw);
+    if (threadIdx.x == 0) s_c = *a.ctl;
+    for (int32_t v = blockIdx.x * ALL_THREADS + threadIdx.x; v < a.n; v += gridDim.x * ALL_THREADS)
+        pr_init_row<Op>(a, v, z.x0);
+    bool ok = mgd::grid_sync(z.bar, z.bar_err, z.bar_never);
+    const double base0 = (1.0 - (double)s_c.damping) / a.n, basek = (double)s_c.damping / a.n;
+    while (ok && s_c.more) {
+        PrRowOp<Op> op{a, s_c};
+        const float *cc = a.c[s_c.cur];
+        for (int32_t ch = gwarp; ch < z.nchunks; ch += nwarps) {
+            const int32_t v = __ldg(&z.chunk[3 * ch]), b = __ldg(&z.chunk[3 * ch + 1]), e = __ldg(&z.chunk[3 * ch + 2]);
+            float s = 0.0f, r = 0.0f, t[ALL_CHUNK / 32];
+#pragma unroll
+            for (int j = 0; j < ALL_CHUNK / 32; j++) {
+                const int32_t p = b + lane + 32 * j;
+                t[j] = p < e ? cc[__ldg(&a.pcol[p])] : 0.0f;
+                if (Op::kWeights && p < e) t[j] *= __int_as_float(__ldg(&pw[p]));
+            }
+#pragma unroll
+            for (int j = 0; j < ALL_CHUNK / 32; j++) mgd::kahan_add(s, r, t[j]);
+            s = mgd::warp_sum_comp(s, r);
+            const int32_t at = __ldg(&z.chunk_at[ch]), k0 = __ldg(&z.row_chunk[at]), k1 = __ldg(&z.row_chunk[at + 1]);
+            int last = 0;
+            if (lane == 0) {
+                __stcg(&z.part[ch], s);
+                __threadfence();
+                last = (atomicAdd(&z.arrive[at], 1) + 1) % (k1 - k0) == 0;
+            }
+            if (__shfl_sync(FULL, last, 0)) {
+                __threadfence();
+                s = r = 0.0f;
+                for (int32_t k = k0 + lane; k < k1; k += 32) mgd::kahan_add(s, r, __ldcg(&z.part[k]));
+                s = mgd::warp_sum_comp(s, r);
+                if (lane == 0) op.finish_row(v, s);
+            }
+        }
+        // the next rows' offsets are loaded ahead of the current rows' sums
+        int32_t v = gwarp * 4 + grp;
+        int32_t b = v < z.split ? __ldg(&a.prow[v]) : 0, e = v < z.split ? __ldg(&a.prow[v + 1]) : 0;
+        for (int32_t v0 = gwarp * 4; v0 < z.split; v0 += nwarps * 4) {
+            const int32_t vn = v + nwarps * 4;
+            const int32_t bn = vn < z.split ? __ldg(&a.prow[vn]) : 0, en = vn < z.split ? __ldg(&a.prow[vn + 1]) : 0;
+            const bool row = v < z.split && e - b <= ALL_CHUNK;
+            const int32_t len = row ? e - b : 0;
+            const int32_t rounds = (int32_t)__reduce_max_sync(FULL, (unsigned)((len + 31) >> 5));
+            float s = 0.0f, r = 0.0f;
+            for (int32_t k = 0; k < rounds; k++) {
+                float t[4];
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const int32_t i = k * 32 + j * 8 + gl;
+                    t[j] = i < len ? cc[__ldg(&a.pcol[b + i])] : 0.0f;
+                    if (Op::kWeights && i < len) t[j] *= __int_as_float(__ldg(&pw[b + i]));
+                }
+#pragma unroll
+                for (int j = 0; j < 4; j++) mgd::kahan_add(s, r, t[j]);
+            }
+            s = mgd::warp_sum_comp<8>(s, r);
+            if (row && gl == 0) op.finish_row(v, s);
+            v = vn;
+            b = bn;
+            e = en;
+        }
+        for (int32_t w = z.split + gwarp * 32 + lane; w < a.n; w += nwarps * 32) {
+            const int32_t wb = __ldg(&a.prow[w]), we = __ldg(&a.prow[w + 1]);
+            if (we - wb > ALL_CHUNK) continue;   // (a directed graph's long in-rows: chunks above)
+            const int32_t len = we - wb;
+            float s = 0.0f, r = 0.0f;
+            for (int32_t k = 0; k < len; k += 4) {
+                float t[4];
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    t[j] = k + j < len ? cc[__ldg(&a.pcol[wb + k + j])] : 0.0f;
+                    if (Op::kWeights && k + j < len) t[j] *= __int_as_float(__ldg(&pw[wb + k + j]));
+                }
+#pragma unroll
+                for (int j = 0; j < 4; j++) mgd::kahan_add(s, r, t[j]);
+            }
+            op.finish_row(w, s - r);
+        }
+        // the block's sums, FP32 within a warp as in block_partials, FP64 across
+        float r = op.resid, dg = op.dangs;
+        int any = op.any;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            r += __shfl_xor_sync(FULL, r, o);
+            dg += __shfl_xor_sync(FULL, dg, o);
+        }
+        any = __any_sync(FULL, any);
+        if (lane == 0) {
+            s_r[warp] = (double)r;
+            s_d[warp] = (double)dg;
+            s_a[warp] = any;
+        }
+        __syncthreads();
+        double *bs = z.bsum + (size_t)(s_c.iter & 1) * gridDim.x * 3;
+        if (warp == 0) {
+            double R = s_r[lane], D = s_d[lane];
+            any = __any_sync(FULL, s_a[lane]);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                R += __shfl_xor_sync(FULL, R, o);
+                D += __shfl_xor_sync(FULL, D, o);
+            }
+            if (lane == 0) {
+                __stcg(&bs[blockIdx.x * 3], R);
+                __stcg(&bs[blockIdx.x * 3 + 1], D);
+                __stcg(&bs[blockIdx.x * 3 + 2], (double)any);
+            }
+        }
+        ok = mgd::grid_sync(z.bar, z.bar_err, z.bar_never);
+        if (!ok) break;
+        if (warp == 0) {
+            double R = 0.0, D = 0.0;
+            any = 0;
+            for (int i = lane; i < (int)gridDim.x; i += 32) {
+                R += __ldcg(&bs[i * 3]);
+                D += __ldcg(&bs[i * 3 + 1]);
+                any |= __ldcg(&bs[i * 3 + 2]) != 0.0;
+            }
+            any = __any_sync(FULL, any);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                R += __shfl_xor_sync(FULL, R, o);
+                D += __shfl_xor_sync(FULL, D, o);
+            }
+            if (lane == 0) {
+                s_c.iter += 1;
+                s_c.cur ^= 1;
+                s_c.resid = R;
+                s_c.any = any;
+                if (Op::kAdjoint) {
+                    s_c.lam_mean = D / a.n;
+                    s_c.lam_meanf = (float)s_c.lam_mean;
+                } else {
+                    s_c.dangling = D;
+                    s_c.base = (float)(base0 + basek * D);
+                }
+                int more = Op::more(any, R, s_c.tol) ? 1 : 0;
+                if (more && s_c.iter >= s_c.max_iter) {
+                    s_c.status = 1;
+                    more = 0;
+                }
+                s_c.more = more;
+            }
+        }
+        __syncthreads();
+    }
+    if (z.out && ok) {
+        const float *x = Op::kAdjoint ? a.c[s_c.cur] : a.x[s_c.cur];
+        for (int32_t i = blockIdx.x * ALL_THREADS + threadIdx.x; i < a.n; i += gridDim.x * ALL_THREADS)
+            z.out[i] = __ldcg(&x[z.old2new ? __ldg(&z.old2new[i]) : i]);
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        if (!ok) {
+            s_c.status = 3;
+            s_c.more = 0;
+        }
+        *a.ctl = s_c;
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1334,6 +1554,7 @@ struct PrWS {
     mgi::DevBuf ct, gsum;      // adjoint: row factors and totals; partial sums of g
     uint64_t tpos_version = 0; // col_version that tpos was built from (0: none)
     mgi::DevBuf q0, q1, qval;  // data-driven queue sweeps
+    mgi::DevBuf arrive, apart, bsum, bar;  // k_pr_all
     uint64_t wT_version = 0;  // fw_version that S and wT were derived from (0: none)
     mgi::LoopGraph lg[6];
 };
@@ -1353,7 +1574,8 @@ void free_pr_ws(mg_graph *g)
     PrWS *w = g->pws;
     DevBuf *bufs[] = {&w->x0, &w->x1, &w->c0, &w->c1, &w->active, &w->hpart, &w->bpart, &w->ctl, &w->S,
                       &w->wT, &w->gvec, &w->lam_keep, &w->xkeep, &w->gvec_caller, &w->grad_caller, &w->tpos,
-                      &w->ct, &w->gsum, &w->q0, &w->q1, &w->qval};
+                      &w->ct, &w->gsum, &w->q0, &w->q1, &w->qval, &w->arrive,
+                      &w->apart, &w->bsum, &w->bar};
     for (DevBuf *b : bufs) dev_free(*b);
     for (auto &l : w->lg) l.destroy();
     delete w;
@@ -1374,6 +1596,23 @@ void free_ppr_ws(mg_graph *g)
 
 void free_wpr_ws(mg_graph *g) { (void)g; }
 
+
+// what the loop control block says after a run: info, the iterate's index,
+// the status as an error
+static mg_status pr_outcome(mg_graph *g, const PCtl &hc, bool dd, int32_t max_iter, mg_run_info *info, int *final_cur)
+{
+    if (info) {
+        info->iterations = hc.iter;
+        info->pull_iterations = dd ? hc.dense_iters : hc.iter;   // sweeps over every row
+        info->residual = hc.resid;
+        info->edges_scanned = (int64_t)hc.iter * g->ne;
+    }
+    *final_cur = hc.cur;
+    if (hc.status == 3) return fail(MG_ERR_CUDA, "grid barrier of the persistent PageRank kernel timed out");
+    if (hc.status != 0)
+        return fail(MG_ERR_ITER_LIMIT, "PageRank did not converge in %d sweeps (residual %g)", max_iter, hc.resid);
+    return MG_OK;
+}
 
 // Runs sweeps of variant V until convergence; the result is x[ctl.cur]
 // (c[ctl.cur] for the adjoint).
@@ -1436,15 +1675,64 @@ static mg_status pr_loop(mg_graph *g, PArgs &a, const mg_opts &opt, const char *
     MG_CUDA(cudaMemcpyAsync(&hc, a.ctl, sizeof(PCtl), cudaMemcpyDeviceToHost, s));
     MG_CUDA(cudaStreamSynchronize(s));
     if (a.P) MG_TRY(hub_check(g));
-    if (info) {
-        info->iterations = hc.iter;
-        info->pull_iterations = Op::kDataDriven ? hc.dense_iters : hc.iter;   // sweeps over every row
-        info->residual = hc.resid;
-        info->edges_scanned = (int64_t)hc.iter * g->ne;
-    }
-    *final_cur = hc.cur;
-    if (hc.status != 0) return fail(MG_ERR_ITER_LIMIT, "PageRank did not converge in %d sweeps (residual %g)", max_iter, hc.resid);
-    return MG_OK;
+    return pr_outcome(g, hc, Op::kDataDriven, max_iter, info, final_cur);
+}
+
+// Whether a run takes the one-launch form.  A host-driven or profiled loop
+// and a layout the caller names keep their kernels.
+static bool pr_small(const mg_graph *g, const mg_opts &opt, bool named_layout)
+{
+    const bool short_rows = !g->relabeled && (int64_t)g->ne <= (int64_t)8 * g->nv;  // (as ppr_chunks)
+    return opt.exec == MG_EXEC_GRAPH && !opt.profile && !named_layout && g->nv > 0 &&
+           g->ne <= (short_rows ? ALL_MAX_EDGES_SHORT : ALL_MAX_EDGES);
+}
+
+// the one-launch form, after the control block's start values; out: result
+// in caller order, or null
+template <class Op>
+static mg_status pr_all(mg_graph *g, const PArgs &a, const mg_opts &opt, float x0, float *out, mg_run_info *info,
+                        int *final_cur)
+{
+    PrWS *w = g->pws;
+    cudaStream_t s = g->stream;
+    MG_TRY(ppr_chunks(g));
+    PrAllArgs z;
+    std::memset(&z, 0, sizeof(z));
+    const int grid = g->num_sms;
+    const size_t nrows = (size_t)std::max(g->ppr_nhrows, 1);
+    MG_TRY(dev_alloc(w->arrive, nrows * 4));
+    MG_TRY(dev_alloc(w->apart, (size_t)std::max(g->ppr_nhchunks, 1) * 4));
+    MG_TRY(dev_alloc(w->bsum, (size_t)grid * 2 * 3 * 8));
+    MG_TRY(dev_alloc(w->bar, 64));
+    z.chunk = g->ppr_hchunk.as<int32_t>(); z.chunk_at = g->ppr_hchunk_at.as<int32_t>();
+    z.rows = g->ppr_hrows.as<int32_t>(); z.row_chunk = g->ppr_hrow_chunk.as<int32_t>();
+    z.nchunks = g->ppr_nhchunks;
+    z.split = g->short_rows;
+    z.arrive = w->arrive.as<int32_t>();
+    z.part = w->apart.as<float>();
+    z.bsum = w->bsum.as<double>();
+    z.bar = w->bar.as<unsigned>();
+    z.bar_err = reinterpret_cast<int *>(z.bar + 8);
+    z.bar_never = fail_barrier();
+    z.old2new = g->relabeled ? g->old2new.as<int32_t>() : nullptr;
+    z.out = out;
+    z.x0 = x0;
+    MG_CUDA(cudaMemsetAsync(z.arrive, 0, nrows * 4, s));
+    MG_CUDA(cudaMemsetAsync(z.bar, 0, 64, s));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3(ALL_THREADS);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    MG_CUDA(cudaLaunchKernelEx(&cfg, k_pr_all<Op>, a, z));
+    PCtl hc;
+    MG_CUDA(cudaMemcpyAsync(&hc, a.ctl, sizeof(PCtl), cudaMemcpyDeviceToHost, s));
+    MG_CUDA(cudaStreamSynchronize(s));
+    return pr_outcome(g, hc, Op::kDataDriven, opt.max_iter > 0 ? opt.max_iter : 10000, info, final_cur);
 }
 
 static mg_status pr_setup(mg_graph *g, PArgs &a, bool weighted_or_adj, int32_t layout = MG_PR_LAYOUT_GATHER)
@@ -1586,7 +1874,8 @@ mg_status mg_pagerank(mg_graph *g, int32_t variant, const mg_opts *o, float *ran
         opt.pr_layout != MG_PR_LAYOUT_AUTO)
         return fail(MG_ERR_INVALID, "unknown PageRank layout %d", opt.pr_layout);
     PArgs a;
-    MG_TRY(pr_setup(g, a, false, opt.pr_layout));
+    const bool small = variant == MG_PR_TOPOLOGY && pr_small(g, opt, opt.pr_layout != MG_PR_LAYOUT_AUTO);
+    MG_TRY(pr_setup(g, a, false, small ? MG_PR_LAYOUT_GATHER : opt.pr_layout));
     cudaStream_t s = g->stream;
     const int grid = a.nblocks;
     const bool ref = variant == MG_PR_TOPOLOGY_REF || variant == MG_PR_DATA_REF;
@@ -1598,6 +1887,18 @@ mg_status mg_pagerank(mg_graph *g, int32_t variant, const mg_opts *o, float *ran
     float x0 = ref ? 0.0f : (g->nv > 0 ? 1.0f / g->nv : 0.0f);
     k_pr_ctl_init<<<1, 32, 0, s>>>(a.ctl, g->nv, max_iter, d, tol, dang0, 0.0);
     int cur = 0;
+    if (small) {
+        // one launch, the result in caller order included
+        float *out = nullptr;
+        if (g->relabeled) {
+            MG_TRY(dev_alloc(g->res_out[MG_RES_RANK], (size_t)g->nv * 4));
+            out = g->res_out[MG_RES_RANK].as<float>();
+        }
+        MG_TRY(pr_all<PrTopology>(g, a, opt, x0, out, info, &cur));
+        g->res[MG_RES_RANK] = out ? (const void *)out : a.x[cur];
+        MG_TRY(end_run(g, opt, info));
+        return copy_out(g, rank_out, g->res[MG_RES_RANK], (size_t)g->nv * 4);
+    }
     switch (variant) {
     case MG_PR_TOPOLOGY_REF:
         k_pr_init<PrTopologyRef><<<grid, THREADS, 0, s>>>(a, x0);
@@ -1680,9 +1981,13 @@ mg_status mg_wpagerank(mg_graph *g, const mg_opts *o, float *x_out, mg_run_info 
     // rows without out-edges are dangling (their mass is spread uniformly)
     float x0 = g->nv > 0 ? 1.0f / g->nv : 0.0f;
     k_pr_ctl_init<<<1, 32, 0, s>>>(a.ctl, g->nv, max_iter, d, tol, g->nv ? (double)g->n_dangling / g->nv : 0.0, 0.0);
-    k_pr_init<PrWeighted><<<grid, THREADS, 0, s>>>(a, x0);
     int cur = 0;
-    MG_TRY(pr_loop<PrWeighted>(g, a, opt, "wpr_pull", info, &cur));
+    if (pr_small(g, opt, false)) {
+        MG_TRY(pr_all<PrWeighted>(g, a, opt, x0, nullptr, info, &cur));
+    } else {
+        k_pr_init<PrWeighted><<<grid, THREADS, 0, s>>>(a, x0);
+        MG_TRY(pr_loop<PrWeighted>(g, a, opt, "wpr_pull", info, &cur));
+    }
     MG_CUDA(cudaMemcpyAsync(w->xkeep.p, a.x[cur], (size_t)g->nv * 4, cudaMemcpyDeviceToDevice, s));
     MG_TRY(to_caller(g, MG_RES_RANK, w->xkeep.p, 4, 1, &g->res[MG_RES_RANK]));
     MG_TRY(end_run(g, opt, info));
@@ -1722,9 +2027,13 @@ mg_status mg_wpagerank_backward(mg_graph *g, const float *g_host, const mg_opts 
     double2 *gsum = w->gsum.as<double2>();
     k_gvec_sums<<<g->num_sms, THREADS, 0, s>>>(g->nv, w->gvec_caller.as<float>(), gsum);
     k_adjoint_ctl_init<<<1, 32, 0, s>>>(a.ctl, g->nv, max_iter, d, tol, gsum, g->num_sms);
-    k_pr_init<PrAdjoint><<<grid, THREADS, 0, s>>>(a, 0.0f);
     int cur = 0;
-    MG_TRY(pr_loop<PrAdjoint>(g, a, opt, "wpr_adjoint", info, &cur));
+    if (pr_small(g, opt, false)) {
+        MG_TRY(pr_all<PrAdjoint>(g, a, opt, 0.0f, nullptr, info, &cur));
+    } else {
+        k_pr_init<PrAdjoint><<<grid, THREADS, 0, s>>>(a, 0.0f);
+        MG_TRY(pr_loop<PrAdjoint>(g, a, opt, "wpr_adjoint", info, &cur));
+    }
     float *lam = a.c[cur];
     MG_CUDA(cudaMemcpyAsync(w->lam_keep.p, lam, (size_t)g->nv * 4, cudaMemcpyDeviceToDevice, s));
     int sg = g->prof.slot("wpr_grad");
@@ -1759,10 +2068,20 @@ mg_status mgi::ppr_chunks(mg_graph *g)
     MG_TRY(dev_alloc(g->ppr_hchunk, std::max<size_t>(hc.size(), 3) * 4));
     MG_TRY(dev_alloc(g->ppr_hrows, std::max<size_t>(hr.size(), 1) * 4));
     MG_TRY(dev_alloc(g->ppr_hrow_chunk, hrc.size() * 4));
+    std::vector<int32_t> at;
+    for (size_t i = 0; i < hr.size(); i++) at.insert(at.end(), (size_t)(hrc[i + 1] - hrc[i]), (int32_t)i);
+    MG_TRY(dev_alloc(g->ppr_hchunk_at, std::max<size_t>(at.size(), 1) * 4));
+    if (!at.empty()) MG_CUDA(cudaMemcpyAsync(g->ppr_hchunk_at.p, at.data(), at.size() * 4, cudaMemcpyHostToDevice, s));
     if (!hc.empty()) MG_CUDA(cudaMemcpyAsync(g->ppr_hchunk.p, hc.data(), hc.size() * 4, cudaMemcpyHostToDevice, s));
     if (!hr.empty()) MG_CUDA(cudaMemcpyAsync(g->ppr_hrows.p, hr.data(), hr.size() * 4, cudaMemcpyHostToDevice, s));
     MG_CUDA(cudaMemcpyAsync(g->ppr_hrow_chunk.p, hrc.data(), hrc.size() * 4, cudaMemcpyHostToDevice, s));
     MG_CUDA(cudaStreamSynchronize(s));
+    // first of the short rows at the end (hub-first order: degrees fall by
+    // powers of two); a low-degree graph is all short rows
+    int32_t split = g->nv;
+    while (g->symmetric && split > 0 && pr[split] - pr[split - 1] < ALL_SHORT) split--;
+    if (!g->relabeled) split = (int64_t)g->ne <= (int64_t)8 * g->nv ? 0 : g->nv;
+    g->short_rows = split;
     g->ppr_nhchunks = (int32_t)(hc.size() / 3);
     g->ppr_nhrows = (int32_t)hr.size();
     return MG_OK;
