@@ -83,7 +83,7 @@ struct FCtl {
     int32_t alpha, beta;
     int32_t nlevels;      // BC: levels archived
     int32_t archive;      // 1: queue slices are appended (BFS/BC), 0: ping-pong (SSSP)
-    int32_t pad0;
+    int32_t qedges;         // out-edges of the current frontier (push phase only)
     long long nf_edges;      // out-edges of the next frontier (atomic)
     long long visited_edges; // out-edges of every vertex visited so far
     long long scanned;       // edges scanned (statistics, atomic)
@@ -324,6 +324,219 @@ __device__ __forceinline__ void push_level(const Args &a, const FCtl &c, LevelCn
     }
     warp_add64(&lc->nfe, dsum);
     if (lane == 0 && scanned) atomicAdd((unsigned long long *)&a.ctl->scanned, (unsigned long long)scanned);
+}
+
+// The end-of-level decision on a copy of the loop state, given the level's
+// counters; block 0 (write_lvl) also records the level offset.
+__device__ __forceinline__ int decide_local(const Args &a, FCtl &c, int32_t nq, int32_t nhcur, long long nfe_in,
+                                            bool write_lvl)
+{
+    int more = c.more;
+    if (more) {
+        if (c.mode == MODE_PULL) c.pull_iters++;
+        c.iter += 1;
+        if (c.archive && c.iter + 1 < a.n + 3) {
+            if (write_lvl) a.lvl_off[c.iter + 1] = c.nqoff + nq;
+            if (nq > 0) c.nlevels = c.iter + 1;
+        }
+        c.qoff = c.nqoff;
+        c.qsize = nq;
+        c.nqoff = c.archive ? (c.qoff + nq) : (c.qoff == 0 ? a.n : 0);
+        c.nq = 0;
+        c.hcur = nhcur;
+        c.nhcur = 0;
+        c.hpar ^= 1;
+        c.cur = (c.cur + 1) % 3;
+        const long long nfe = nfe_in;
+        c.visited_edges += nfe;
+        c.qedges = (int32_t)min(nfe, (long long)INT32_MAX);
+        c.nf_edges = 0;
+        if (nq == 0) {
+            more = 0;
+        } else {
+            if (c.dirmode == MG_DIR_PUSH) c.mode = MODE_PUSH;
+            else if (c.dirmode == MG_DIR_PULL) c.mode = MODE_PULL;
+            else if (c.archive) {
+                // Beamer: push -> pull when frontier edges exceed unvisited
+                // edges / alpha; pull -> push when the frontier is below n / beta
+                const long long unvisited = (long long)a.m - c.visited_edges;
+                if (c.mode == MODE_PUSH) {
+                    if (nfe * (long long)c.alpha > unvisited && nq > 64) c.mode = MODE_PULL;
+                } else {
+                    if ((long long)nq * c.beta < a.n) c.mode = MODE_PUSH;
+                }
+            } else {
+                // SSSP: pull when the frontier's edges are a large share of m
+                c.mode = (nfe * (long long)c.alpha > (long long)a.m) ? MODE_PULL : MODE_PUSH;
+            }
+            if (c.iter >= c.max_iter) { c.status = 1; more = 0; }
+        }
+        c.more = more;
+    }
+    return more;
+}
+
+// ----------------------------------------------------------------------------
+// push, one block: consecutive levels of a small frontier on a graph without
+// heavy vertices (a lattice, a road network: hundreds or thousands of levels
+// of a few hundred vertices).  A level of the whole grid is a barrier and a
+// chain of L2 round trips (atomics, loads that must see other blocks' writes)
+// whatever its size: 4.8 us for BFS and 9 us for BC on a 320 x 311 lattice.
+// One block needs neither: the frontier lies in shared memory with its row
+// offsets, a level's candidates are told apart in a shared hash table, path
+// counts are pulled by the new vertices instead of added atomically, and
+// labels and counts are read back through the block's own L1.  us per level,
+// grid -> block: BFS 4.8 -> 2.9 and BC 9.1 -> 5.6 at 230 vertices a level;
+// at 660 a level one SM's load rate makes it 7.5 and 14.5 against the grid's
+// 4.7 and 7.0, so the block takes over below CTA_ENTER and hands back above
+// CTA_Q.
+// ----------------------------------------------------------------------------
+constexpr int CTA_Q = 512;           // frontier entries held in shared memory
+constexpr int CTA_ENTER = 384;       // the block takes over at this many vertices
+constexpr int CTA_EDGES = 4096;      // and while the frontier has at most this many edges
+constexpr int CTA_HASH = 2 * CTA_EDGES;
+constexpr int CTA_LEVELS = 20000;    // levels before the grid meets again (a fraction of the barrier's time limit)
+
+struct CtaShared {
+    int32_t v[2][CTA_Q], b[2][CTA_Q];     // frontier: vertex, first edge
+    int32_t d[2][CTA_Q];                  // out-degree
+    int32_t slot[CTA_Q];                  // the new entries' hash slots
+    int32_t hash[CTA_HASH];
+    int32_t count;
+    int32_t nfe;                          // (at most CTA_EDGES vertices of fewer than 128 edges)
+};
+
+// Runs levels from the loop state c (shared memory, all threads of block 0
+// call) until the frontier outgrows the block, the traversal ends or the
+// direction switch picks pull; the queue archive, labels, visited bits and
+// level offsets are kept in global memory as the grid's levels keep them, the
+// frontier bitmaps (all zero on entry) hold the last frontier on return.
+template <class Op>
+__device__ __noinline__ void cta_push_levels(const Args &a, FCtl &c, CtaShared &s)
+{
+    static_assert(Op::kLevelSync, "labels are levels");
+    const int t = threadIdx.x;
+    for (int i = t; i < CTA_HASH; i += PTHREADS) s.hash[i] = -1;
+    for (int i = t; i < c.qsize; i += PTHREADS) {
+        const int32_t u = __ldcg(&a.queue[c.qoff + i]), b = a.row[u];
+        s.v[0][i] = u;
+        s.b[0][i] = b;
+        s.d[0][i] = a.row[u + 1] - b;
+    }
+    if (t == 0) {
+        s.count = 0;
+        s.nfe = 0;
+    }
+    __syncthreads();
+    int p = 0;
+    for (int lv = 0; lv < CTA_LEVELS; lv++) {
+        const int32_t it1 = c.iter + 1, n0 = c.qsize, out = c.nqoff;
+        // threads per vertex: 8, or fewer when the frontier fills the block
+        const int tpv = n0 <= 128 ? 8 : n0 <= 256 ? 4 : n0 <= 512 ? 2 : 1;
+        int32_t nfe = 0;
+        for (int i0 = (t & ~31) / tpv; i0 < n0; i0 += PTHREADS / tpv) {
+            const int i = i0 + (t & 31) / tpv;
+            const int32_t b = i < n0 ? s.b[p][i] : 0, d = i < n0 ? s.d[p][i] : 0;
+            const int32_t steps = (int32_t)__reduce_max_sync(0xffffffffu, (unsigned)((d + tpv - 1) / tpv));
+            // two edges a step, their loads together
+            for (int32_t k0 = 0; k0 < steps; k0 += 2) {
+                int32_t w[2], h[2], wb[2], wd[2];
+                bool fresh[2];
+#pragma unroll
+                for (int j = 0; j < 2; j++) {
+                    const int32_t k = (k0 + j) * tpv + t % tpv;
+                    w[j] = k < d ? __ldg(&a.col[b + k]) : -1;
+                }
+#pragma unroll
+                for (int j = 0; j < 2; j++) {
+                    fresh[j] = w[j] >= 0 && a.label[w[j]] == mgops::UNSET;
+                    wb[j] = fresh[j] ? __ldg(&a.row[w[j]]) : 0;
+                    wd[j] = fresh[j] ? __ldg(&a.row[w[j] + 1]) - wb[j] : 0;
+                }
+#pragma unroll
+                for (int j = 0; j < 2; j++) {
+                    if (fresh[j]) {
+                        h[j] = (int)(((uint32_t)w[j] * 2654435761u) >> 19) & (CTA_HASH - 1);
+                        int32_t old;
+                        while ((old = atomicCAS(&s.hash[h[j]], -1, w[j])) != -1 && old != w[j])
+                            h[j] = (h[j] + 1) & (CTA_HASH - 1);
+                        fresh[j] = old == -1;   // else another edge of this level has it
+                    }
+                    __syncwarp();
+                    const unsigned m = __ballot_sync(0xffffffffu, fresh[j]);
+                    if (m == 0) continue;
+                    int at = 0;
+                    if (mgd::lane() == 0) at = atomicAdd(&s.count, __popc(m));
+                    at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << mgd::lane()) - 1u));
+                    if (!fresh[j]) continue;
+                    a.queue[out + at] = w[j];
+                    atomicOr(&a.visited[w[j] >> 5], 1u << (w[j] & 31));
+                    nfe += wd[j];
+                    if (at < CTA_Q) {
+                        s.v[p ^ 1][at] = w[j];
+                        s.b[p ^ 1][at] = wb[j];
+                        s.d[p ^ 1][at] = wd[j];
+                        s.slot[at] = h[j];
+                    }                         // (else too many for the block: this is its last level)
+                }
+            }
+        }
+        __syncwarp();
+        nfe = (int32_t)__reduce_add_sync(0xffffffffu, (unsigned)nfe);
+        if (mgd::lane() == 0 && nfe) atomicAdd(&s.nfe, nfe);
+        __syncthreads();
+        const int32_t nq = s.count;
+        // path counts and labels of the new vertices: sums over the
+        // neighbours at this level.  (Labels are set after the candidates of
+        // the level are known, so the test above sees no label of its own.)
+        for (int i = t; i < nq; i += PTHREADS) {
+            const bool held = i < CTA_Q;
+            const int32_t w = held ? s.v[p ^ 1][i] : a.queue[out + i];
+            if constexpr (Op::kPathCounts) {
+                const bool own = held && a.trow == a.row;
+                const int32_t b = own ? s.b[p ^ 1][i] : __ldg(&a.trow[w]);
+                const int32_t d = own ? s.d[p ^ 1][i] : __ldg(&a.trow[w + 1]) - b;
+                mgops::PathCount sum = mgops::pc_zero();
+                for (int32_t k = b; k < b + d; k += 4) {
+                    int32_t u[4], lu[4];
+                    mgops::PathCount x[4];
+#pragma unroll
+                    for (int j = 0; j < 4; j++) u[j] = k + j < b + d ? __ldg(&a.tcol[k + j]) : w;
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        lu[j] = a.label[u[j]];
+                        x[j] = a.sigma[u[j]];
+                    }
+#pragma unroll
+                    for (int j = 0; j < 4; j++)
+                        if (u[j] != w && lu[j] == it1 - 1) sum = mgops::pc_add(sum, x[j], a.bc_ext != 0);
+                }
+                a.sigma[w] = sum;
+                if (!a.bc_ext && sum.m >= mgops::PC_PLAIN_MAX) *a.bc_ovf = 1;
+            }
+            if (held) s.hash[s.slot[i]] = -1;
+        }
+        if constexpr (Op::kPathCounts) __syncthreads();
+        for (int i = t; i < nq; i += PTHREADS) a.label[i < CTA_Q ? s.v[p ^ 1][i] : a.queue[out + i]] = it1;
+        if (t == 0) {
+            FCtl n = c;
+            atomicAdd((unsigned long long *)&a.ctl->scanned, (unsigned long long)n.qedges);
+            decide_local(a, n, nq, 0, (long long)s.nfe, true);
+            c = n;
+            s.count = 0;
+            s.nfe = 0;
+        }
+        p ^= 1;
+        __syncthreads();
+        if (c.more == 0 || c.mode != MODE_PUSH || c.qsize > CTA_Q || c.qedges > CTA_EDGES) break;
+    }
+    uint32_t *bm = bm_buf(a, c.cur);
+    if (c.more)
+        for (int i = t; i < c.qsize; i += PTHREADS) {
+            const int32_t u = a.queue[c.qoff + i];
+            atomicOr(&bm[u >> 5], 1u << (u & 31));
+        }
+    __syncthreads();
 }
 
 // ----------------------------------------------------------------------------
@@ -631,55 +844,6 @@ __device__ __forceinline__ void store_ctl(FCtl *p, const FCtl &c)
     for (int i = 0; i < (int)(sizeof(FCtl) / 8); i++) d[i] = s[i];
 }
 
-// The end-of-level decision on a copy of the loop state, given the level's
-// counters; block 0 (write_lvl) also records the level offset.
-__device__ __forceinline__ int decide_local(const Args &a, FCtl &c, int32_t nq, int32_t nhcur, long long nfe_in,
-                                            bool write_lvl)
-{
-    int more = c.more;
-    if (more) {
-        if (c.mode == MODE_PULL) c.pull_iters++;
-        c.iter += 1;
-        if (c.archive && c.iter + 1 < a.n + 3) {
-            if (write_lvl) a.lvl_off[c.iter + 1] = c.nqoff + nq;
-            if (nq > 0) c.nlevels = c.iter + 1;
-        }
-        c.qoff = c.nqoff;
-        c.qsize = nq;
-        c.nqoff = c.archive ? (c.qoff + nq) : (c.qoff == 0 ? a.n : 0);
-        c.nq = 0;
-        c.hcur = nhcur;
-        c.nhcur = 0;
-        c.hpar ^= 1;
-        c.cur = (c.cur + 1) % 3;
-        const long long nfe = nfe_in;
-        c.visited_edges += nfe;
-        c.nf_edges = 0;
-        if (nq == 0) {
-            more = 0;
-        } else {
-            if (c.dirmode == MG_DIR_PUSH) c.mode = MODE_PUSH;
-            else if (c.dirmode == MG_DIR_PULL) c.mode = MODE_PULL;
-            else if (c.archive) {
-                // Beamer: push -> pull when frontier edges exceed unvisited
-                // edges / alpha; pull -> push when the frontier is below n / beta
-                const long long unvisited = (long long)a.m - c.visited_edges;
-                if (c.mode == MODE_PUSH) {
-                    if (nfe * (long long)c.alpha > unvisited && nq > 64) c.mode = MODE_PULL;
-                } else {
-                    if ((long long)nq * c.beta < a.n) c.mode = MODE_PUSH;
-                }
-            } else {
-                // SSSP: pull when the frontier's edges are a large share of m
-                c.mode = (nfe * (long long)c.alpha > (long long)a.m) ? MODE_PULL : MODE_PUSH;
-            }
-            if (c.iter >= c.max_iter) { c.status = 1; more = 0; }
-        }
-        c.more = more;
-    }
-    return more;
-}
-
 // End of a level (one thread, no other thread touching the loop state):
 // next queue slice, direction switch, caps.  Works on a register copy (one
 // batch of parallel loads, one batch of stores).  Returns the continue flag.
@@ -723,6 +887,16 @@ __device__ __forceinline__ FCtl block_load_ctl(const FCtl *p)
     return c;
 }
 
+// the push phase's loop state back to global memory for the other kernels
+// (and blocks), all but the last word (the scanned-edges statistic, which
+// the push levels add to atomically)
+__device__ __forceinline__ void store_ctl_push(FCtl *p, const FCtl &c)
+{
+    int2 *d = reinterpret_cast<int2 *>(p);
+    const int2 *src = reinterpret_cast<const int2 *>(&c);
+    for (int i = 0; i < (int)(sizeof(FCtl) / 8) - 1; i++) __stcg(&d[i], src[i]);
+}
+
 // HEAVY: the graph may have vertices above PUSH_HEAVY out-edges (graphs that
 // have none run without the chunk code and its votes).
 template <class Op, bool HEAVY>
@@ -746,6 +920,24 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_sparse_levels(Args a)
             z->nhcur = 0;
             z->nfe = 0;
         }
+        if constexpr (!HEAVY && Op::kLevelSync) {
+            if (s_c.qsize <= CTA_ENTER && s_c.qedges <= CTA_EDGES) {
+                // block 0 alone from here on; the bitmaps start from zero
+                for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 3 * a.words; i += gridDim.x * blockDim.x)
+                    a.bm[i] = 0;
+                if (!mgd::grid_sync(a.bar, a.bar_err, a.bar_never)) break;
+                if (blockIdx.x == 0) {
+                    extern __shared__ __align__(16) unsigned char s_dyn[];
+                    cta_push_levels<Op>(a, s_c, *reinterpret_cast<CtaShared *>(s_dyn));
+                    if (threadIdx.x == 0) store_ctl_push(a.ctl, s_c);
+                }
+                if (!mgd::grid_sync(a.bar, a.bar_err, a.bar_never)) break;
+                const FCtl c1 = block_load_ctl(a.ctl);
+                if (threadIdx.x == 0) s_c = c1;
+                __syncthreads();
+                continue;
+            }
+        }
         push_level<Op, HEAVY>(a, s_c, lc);
         if (!mgd::grid_sync(a.bar, a.bar_err, a.bar_never)) break;
         if (threadIdx.x == 0) {
@@ -763,14 +955,7 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_sparse_levels(Args a)
             c.status = 3;
             c.more = 0;
         }
-        if (ran || c.status) {
-            // the loop state back to global memory for the other kernels,
-            // all but the last word (the scanned-edges statistic, which the
-            // push levels add to atomically)
-            int2 *d = reinterpret_cast<int2 *>(a.ctl);
-            const int2 *src = reinterpret_cast<const int2 *>(&c);
-            for (int i = 0; i < (int)(sizeof(FCtl) / 8) - 1; i++) d[i] = src[i];
-        }
+        if (ran || c.status) store_ctl_push(a.ctl, c);
     }
 }
 
@@ -824,6 +1009,7 @@ __global__ void __launch_bounds__(INIT_THREADS) k_init(Args a, int32_t src, cons
         c->qsize = q;
         c->nqoff = Op::kLevelSync ? q : a.n;
         c->visited_edges = (long long)s_ve;
+        c->qedges = (int32_t)min(s_ve, (unsigned long long)INT32_MAX);
         if (Op::kLevelSync) { a.lvl_off[0] = 0; a.lvl_off[1] = q; c->nlevels = 1; }
     }
 }
@@ -888,8 +1074,12 @@ mg_status ensure_ws(mg_graph *g)
         int per_sm = 0;
         if (g->relabeled)
             MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sparse_levels<Op, true>, PTHREADS, 0));
-        else
-            MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sparse_levels<Op, false>, PTHREADS, 0));
+        else {
+            MG_CUDA(cudaFuncSetAttribute(k_sparse_levels<Op, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)sizeof(CtaShared)));
+            MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sparse_levels<Op, false>, PTHREADS,
+                                                                  sizeof(CtaShared)));
+        }
         if (per_sm < 1) return fail(MG_ERR_CUDA, "persistent push kernel does not fit on an SM");
         cg = g->num_sms;
     }
@@ -903,7 +1093,7 @@ mg_status launch_sparse_levels(const Args &a, int grid, cudaStream_t st)
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3(PTHREADS);
-    cfg.dynamicSmemBytes = 0;
+    cfg.dynamicSmemBytes = a.has_heavy ? 0 : sizeof(CtaShared);
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;
