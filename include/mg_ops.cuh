@@ -116,22 +116,29 @@ constexpr double PC_PLAIN_MAX = 0x1p90;  // plain-mode ceiling (see above)
 __device__ __forceinline__ PathCount pc_zero() { return PathCount{0.0, 0, 0}; }
 __device__ __forceinline__ PathCount pc_one() { return PathCount{1.0, 0, 0}; }
 
-// a + b; in plain mode k is 0 on both sides and no renormalisation happens
+// a + b; in plain mode k is 0 on both sides and no renormalisation happens.
+// Mantissas are 0 or at least 1, so the tests and the scaling by 2^-512 work
+// on the high word (exponent) as integers: one FP64 instruction an add, where
+// comparing and scaling in FP64 took five (a warp's FP64 instruction holds
+// GB300's pipe for 16 cycles and more).
 __device__ __forceinline__ PathCount pc_add(PathCount a, PathCount b, bool ext)
 {
     if (!ext) return PathCount{a.m + b.m, 0, 0};
-    if (b.m == 0.0) return a;
-    if (a.m == 0.0) return b;
+    constexpr int32_t TOP_HI = (1023 + 512) << 20;  // high word of 2^512
+    if (__double2hiint(b.m) == 0) return a;
+    if (__double2hiint(a.m) == 0) return b;
     if (a.k < b.k) {
         const PathCount t = a;
         a = b;
         b = t;
     }
     const int32_t d = a.k - b.k;  // b is below a's ulp when d >= 2
-    double m = a.m + (d == 0 ? b.m : (d == 1 ? b.m * PC_DOWN : 0.0));
+    if (d >= 2) return a;
+    if (d == 1) b.m = __hiloint2double(__double2hiint(b.m) - (512 << 20), __double2loint(b.m));
+    double m = a.m + b.m;
     int32_t k = a.k;
-    if (m >= PC_TOP) {
-        m *= PC_DOWN;
+    if (__double2hiint(m) >= TOP_HI) {
+        m = __hiloint2double(__double2hiint(m) - (512 << 20), __double2loint(m));
         k += 1;
     }
     return PathCount{m, k, 0};

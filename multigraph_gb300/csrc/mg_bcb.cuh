@@ -301,6 +301,8 @@ __device__ __forceinline__ void mark_edge_block(const BbArgs &a, int32_t p, int3
 }
 
 // sparse level d (archive entries [b0, b1)): collect the candidate rows
+// (FLAT: no heavy entries)
+template <bool FLAT = false>
 __device__ __forceinline__ void bb_mark_phase(const BbArgs &a, const BbCtl &c, int32_t b0, int32_t b1, int32_t *ncand)
 {
     const int lane = mgd::lane();
@@ -317,7 +319,7 @@ __device__ __forceinline__ void bb_mark_phase(const BbArgs &a, const BbCtl &c, i
             f = a.amask[base + lane];
             start = __ldg(&a.row[u]);
             deg = __ldg(&a.row[u + 1]) - start;
-            if (deg > MARK_HEAVY) deg = 0;  // the grid-wide loop below
+            if (!FLAT && deg > MARK_HEAVY) deg = 0;  // the grid-wide loop below
         }
         const int incl = mgd::warp_scan_incl(deg);
         const int excl = incl - deg;
@@ -331,6 +333,7 @@ __device__ __forceinline__ void bb_mark_phase(const BbArgs &a, const BbCtl &c, i
             mark_edge_block(a, k < total ? p : 0, k < total ? p + 1 : 0, fo, ncand);
         }
     }
+    if (FLAT) return;
     // heavy frontier entries: every warp of the grid takes 32-edge slices
     const uint32_t *fcur = fm_of(a, c.cur);
     for (int32_t h = 0; h < c.nfh; h++) {
@@ -428,25 +431,40 @@ __device__ __forceinline__ void settle_row(const BbArgs &a, uint32_t *fnext, int
 // One thread, one row v with at most TDEG in-edges: per source s in the
 // sources that reach v at this level (at most TBITS of them, else false is
 // returned and the row goes to the warp path), the sum of sig over the
-// in-neighbours on s's frontier, in edge order as pull_span forms it.
+// in-neighbours on s's frontier, in edge order as pull_span forms it.  The
+// row's columns, their masks and a source's counts are loaded together.
+// *reached gets those sources.
 __device__ __forceinline__ bool pull_row_thread(const BbArgs &a, const uint32_t *fcur, uint32_t *fnext, int32_t v,
-                                                uint32_t want)
+                                                uint32_t want, uint32_t *reached)
 {
     const int32_t b = __ldg(&a.trow[v]), e = __ldg(&a.trow[v + 1]);
     if (e - b > TDEG) return false;
-    uint32_t newm = 0;
-    for (int32_t p = b; p < e; p++) newm |= fcur[__ldg(&a.tcol[p])];
+    int32_t u[TDEG];
+    uint32_t f[TDEG], newm = 0;
+#pragma unroll
+    for (int j = 0; j < TDEG; j++) u[j] = b + j < e ? __ldg(&a.tcol[b + j]) : -1;
+#pragma unroll
+    for (int j = 0; j < TDEG; j++) f[j] = u[j] >= 0 ? fcur[u[j]] : 0u;
+#pragma unroll
+    for (int j = 0; j < TDEG; j++) newm |= f[j];
     newm &= want;
     if (__popc(newm) > TBITS) return false;
+    *reached = newm;
     if (newm == 0) return true;
     uint32_t mm = newm;
-    while (mm) {  // the row's edges again per source (L1 hits)
+    while (mm) {
         const int s = __ffs(mm) - 1;
         mm &= mm - 1;
         mgops::PathCount acc = mgops::pc_zero();
-        for (int32_t p = b; p < e; p++) {
-            const int32_t u = __ldg(&a.tcol[p]);
-            if ((fcur[u] >> s) & 1u) acc = mgops::pc_add(acc, a.sig[(size_t)u * W + s], a.mode == M_EXT);
+#pragma unroll
+        for (int h = 0; h < TDEG; h += 4) {
+            mgops::PathCount x[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                x[j] = ((f[h + j] >> s) & 1u) ? a.sig[(size_t)u[h + j] * W + s] : mgops::pc_zero();
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                if ((f[h + j] >> s) & 1u) acc = mgops::pc_add(acc, x[j], a.mode == M_EXT);
         }
         a.sig[(size_t)v * W + s] = acc;
         if (a.mode != M_EXT && acc.m >= mgops::PC_PLAIN_MAX) a.ctl->ovf = 1;
@@ -477,7 +495,8 @@ __device__ __forceinline__ void bb_pull_phase(const BbArgs &a, const BbCtl &c, i
             if (lane < vpw && i < nrows) {
                 v = c.dense ? i : a.cand[i];
                 want = ~a.vis[v] & c.gmask;
-                if (want) deferred = !pull_row_thread(a, fcur, fnext, v, want);
+                uint32_t reached;
+                if (want) deferred = !pull_row_thread(a, fcur, fnext, v, want, &reached);
             }
             unsigned dm = __ballot_sync(0xffffffffu, deferred);
             while (dm) {
@@ -612,7 +631,10 @@ template <int M>
 __device__ __forceinline__ QT<M> back_term(const BbArgs &a, int32_t L, int32_t v, int s, int32_t ku)
 {
     QT<M> t = q_of<M>(a, L + 1)[(size_t)v * W + s];
-    if (M == M_EXT) t *= (QT<M>)mgops::pc_scale(ku - a.sig[(size_t)v * W + s].k);
+    if (M == M_EXT) {
+        const int32_t dk = ku - a.sig[(size_t)v * W + s].k;
+        if (dk != 0) t *= (QT<M>)mgops::pc_scale(dk);   // (one level in hundreds)
+    }
     return t;
 }
 
@@ -712,22 +734,28 @@ __device__ __forceinline__ void back_finish(const BbArgs &a, int32_t L, int32_t 
 // contributions are added in source order).
 template <int M>
 __device__ __forceinline__ bool back_entry_thread(const BbArgs &a, const uint32_t *nxt, int32_t L, int32_t u,
-                                                  uint32_t msk)
+                                                  uint32_t msk, int32_t b, int32_t e)
 {
     if (__popc(msk) > TBITS) return false;
-    const int32_t b = __ldg(&a.row[u]), e = __ldg(&a.row[u + 1]);
     if (e - b > TDEG) return false;
+    int32_t v[TDEG];
+    uint32_t f[TDEG];
+#pragma unroll
+    for (int j = 0; j < TDEG; j++) v[j] = b + j < e ? __ldg(&a.col[b + j]) : -1;
+#pragma unroll
+    for (int j = 0; j < TDEG; j++) f[j] = v[j] >= 0 ? nxt[v[j]] : 0u;
     float hi = 0.0f, lo = 0.0f;
     uint32_t mm = msk;
     while (mm) {
         const int s = __ffs(mm) - 1;
         mm &= mm - 1;
         const mgops::PathCount su = a.sig[(size_t)u * W + s];
-        QT<M> acc = 0;
-        for (int32_t p = b; p < e; p++) {
-            const int32_t v = __ldg(&a.col[p]);
-            if ((nxt[v] >> s) & 1u) acc += back_term<M>(a, L, v, s, su.k);
-        }
+        QT<M> t[TDEG], acc = 0;
+#pragma unroll
+        for (int j = 0; j < TDEG; j++) t[j] = ((f[j] >> s) & 1u) ? back_term<M>(a, L, v[j], s, su.k) : (QT<M>)0;
+#pragma unroll
+        for (int j = 0; j < TDEG; j++)
+            if ((f[j] >> s) & 1u) acc += t[j];
         const float dv = back_delta<M>(su, acc, q_of<M>(a, L)[(size_t)u * W + s]);
         if (__ldg(&a.src[s]) != u) pair_add(hi, lo, dv);
     }
@@ -757,7 +785,7 @@ __device__ __forceinline__ void bbb_pull_phase(const BbArgs &a, int32_t L)
             if (lane < vpw && i < hi) {
                 u = a.arch[i];
                 msk = a.amask[i];
-                deferred = !back_entry_thread<M>(a, nxt, L, u, msk);
+                deferred = !back_entry_thread<M>(a, nxt, L, u, msk, __ldg(&a.row[u]), __ldg(&a.row[u + 1]));
             }
             unsigned dm = __ballot_sync(0xffffffffu, deferred);
             while (dm) {
@@ -826,6 +854,136 @@ __device__ __forceinline__ void bbb_next_phase(const BbArgs &a, int32_t L)
     }
 }
 
+
+// ---------------------------------------------------------------------------
+// flat sweeps: graphs without heavy rows (no vertex of 128 edges), whole
+// sweeps in one persistent launch.  Masks of level l lie in fm[l % 3] forward
+// too.
+// ---------------------------------------------------------------------------
+// An entry a thread, 32 a warp, consecutive warps of entries on different
+// SMs: GB300's FP64 pipe takes a warp instruction in the same time whether
+// one lane is active or all (extended counts are FP64), and an entry spread
+// to a warp of its own kept it busy for 16 us a level (7,700 entries).
+__device__ __forceinline__ int flat_warp() { return (int)((threadIdx.x >> 5) * gridDim.x + blockIdx.x); }
+
+// Level d -> d+1 over nrows rows, the reached rows archived as they settle
+// (level d+1's entries from off_d1 on), their candidate bits and level d-1's
+// masks cleared on the way: nobody reads either in this phase.
+template <int M>
+__device__ __forceinline__ void bb_flat_phase(const BbArgs &a, const BbCtl &c, int32_t nrows, int32_t off_p,
+                                              int32_t off_d, int32_t off_d1, LvlCnt *k)
+{
+    const int lane = mgd::lane();
+    const int gtid = blockIdx.x * blockDim.x + threadIdx.x, gwarp = flat_warp();
+    const int nwarps = (gridDim.x * blockDim.x) >> 5;
+    const uint32_t *fcur = fmb_of(a, c.d);
+    uint32_t *fnext = fmb_of(a, c.d + 1), *fold = fmb_of(a, c.d + 2);
+    for (int32_t i = off_p + gtid; i < off_d; i += gridDim.x * blockDim.x) fold[__ldcg(&a.arch[i])] = 0;
+    unsigned long long nfe = 0;
+    for (int32_t base = gwarp * 32; base < nrows; base += nwarps * 32) {
+        const int32_t i = base + lane;
+        int32_t v = 0;
+        uint32_t want = 0, reached = 0;
+        bool deferred = false;
+        if (i < nrows) {
+            v = c.dense ? i : __ldcg(&a.cand[i]);
+            if (!c.dense) atomicAnd(&a.cbm[v >> 5], ~(1u << (v & 31)));
+            want = ~a.vis[v] & c.gmask;
+            if (want) deferred = !pull_row_thread(a, fcur, fnext, v, want, &reached);
+            if (deferred) reached = 0;
+        }
+        unsigned dm = __ballot_sync(0xffffffffu, deferred);
+        while (dm) {
+            const int j = __ffs(dm) - 1;
+            dm &= dm - 1;
+            const int32_t vj = __shfl_sync(0xffffffffu, v, j);
+            const uint32_t wj = __shfl_sync(0xffffffffu, want, j);
+            uint32_t newm;
+            const auto acc = pull_span<M>(a, fcur, c.d, __ldg(&a.trow[vj]), __ldg(&a.trow[vj + 1]), wj, newm);
+            if (newm) settle_row<M>(a, fnext, c.d, vj, newm, acc);
+            if (lane == j) reached = newm;
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, reached != 0);
+        if (m == 0) continue;
+        int at = 0;
+        if (lane == 0) at = atomicAdd(&k->nnew, __popc(m));
+        at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << lane) - 1u));
+        if (reached) {
+            const size_t o = (size_t)off_d1 + (size_t)at;
+            if (o < a.cap) {
+                a.arch[o] = v;
+                a.amask[o] = reached;
+            } else {
+                k->status = 2;
+            }
+            nfe += (unsigned long long)(__ldg(&a.row[v + 1]) - __ldg(&a.row[v]));
+        }
+    }
+    nfe = warp_sum_u64(nfe);
+    if (lane == 0 && nfe) atomicAdd(&k->nfe, nfe);
+}
+
+// A thread's first entry of a backward level, loaded ahead of the barrier
+// that opens the level
+struct FlatEntry {
+    int32_t u, b, e;
+    uint32_t msk;
+};
+
+__device__ __forceinline__ FlatEntry flat_load(const BbArgs &a, int32_t L)
+{
+    FlatEntry x{0, 0, 0, 0u};
+    if (L < 1) return x;
+    const int32_t lo = a.off[L], hi = a.off[L + 1];
+    const int32_t i = lo + flat_warp() * 32 + mgd::lane();
+    if (i < hi) {
+        x.u = a.arch[i];
+        x.msk = a.amask[i];
+        x.b = __ldg(&a.row[x.u]);
+        x.e = __ldg(&a.row[x.u + 1]);
+    }
+    return x;
+}
+
+// Backward level L; the entries' own masks go into fm[L % 3] for level L-1,
+// level L+2's are cleared (levels up to Ltop)
+template <int M>
+__device__ __forceinline__ void bbb_flat_phase(const BbArgs &a, int32_t L, int32_t Ltop, FlatEntry x)
+{
+    const int lane = mgd::lane();
+    const int gtid = blockIdx.x * blockDim.x + threadIdx.x, gwarp = flat_warp();
+    const int nwarps = (gridDim.x * blockDim.x) >> 5;
+    uint32_t *cur = fmb_of(a, L);
+    const uint32_t *nxt = fmb_of(a, L + 1);
+    const int32_t lo = a.off[L], hi = a.off[L + 1];
+    for (int32_t base = lo + gwarp * 32; base < hi; base += nwarps * 32) {
+        if (base != lo + gwarp * 32) {
+            x = FlatEntry{0, 0, 0, 0u};
+            if (base + lane < hi) {
+                x.u = a.arch[base + lane];
+                x.msk = a.amask[base + lane];
+                x.b = __ldg(&a.row[x.u]);
+                x.e = __ldg(&a.row[x.u + 1]);
+            }
+        }
+        const bool deferred = x.msk != 0 && !back_entry_thread<M>(a, nxt, L, x.u, x.msk, x.b, x.e);
+        if (x.msk) cur[x.u] = x.msk;
+        unsigned dm = __ballot_sync(0xffffffffu, deferred);
+        while (dm) {
+            const int j = __ffs(dm) - 1;
+            dm &= dm - 1;
+            const int32_t uj = __shfl_sync(0xffffffffu, x.u, j), bj = __shfl_sync(0xffffffffu, x.b, j),
+                          ej = __shfl_sync(0xffffffffu, x.e, j);
+            const uint32_t mj = __shfl_sync(0xffffffffu, x.msk, j);
+            const QT<M> sj = back_span<M>(a, nxt, L, a.col, bj, ej, mj, lane_scale<M>(a, uj, mj));
+            back_finish<M>(a, L, uj, mj, sj);
+        }
+    }
+    if (L + 2 <= Ltop) {
+        uint32_t *old = fmb_of(a, L + 2);
+        for (int32_t i = a.off[L + 2] + gtid; i < a.off[L + 3]; i += gridDim.x * blockDim.x) old[a.arch[i]] = 0;
+    }
+}
 
 // ---------------------------------------------------------------------------
 // mask-free levels (M_INT): eight lanes a row, four sources (16 bytes) a lane

@@ -43,7 +43,10 @@ template <bool EXT>
 __device__ __forceinline__ QT<EXT> bc_succ_term(const Args &a, const QT<EXT> *q, int32_t w, int32_t kv)
 {
     QT<EXT> t = __ldcg(&q[w]);
-    if (EXT) t *= (QT<EXT>)mgops::pc_scale(kv - a.sigma[w].k);
+    if (EXT) {
+        const int32_t dk = kv - a.sigma[w].k;
+        if (dk != 0) t *= (QT<EXT>)mgops::pc_scale(dk);   // (one level in hundreds)
+    }
     return t;
 }
 
@@ -178,13 +181,62 @@ __device__ __forceinline__ void bc_back_heavy_level(const Args &a, int32_t L, in
     }
 }
 
+// One level-(L-1) entry u (fewer than 128 edges [b, e)) by one thread, in
+// edge order; q read through L1 (the barrier before the level makes the
+// other blocks' values visible)
+template <bool EXT>
+__device__ __forceinline__ void bc_back_entry(const Args &a, int32_t L, int32_t u, int32_t b, int32_t e, int32_t src,
+                                              QT<EXT> *q, float *delta, float *bcacc)
+{
+    const mgops::PathCount su = a.sigma[u];
+    QT<EXT> acc = 0;
+    for (int32_t k = b; k < e; k += 4) {
+        int32_t w[4], lw[4], dk[4];
+        QT<EXT> x[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) w[j] = k + j < e ? __ldg(&a.col[k + j]) : u;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            lw[j] = a.label[w[j]];
+            x[j] = q[w[j]];
+            dk[j] = EXT ? su.k - a.sigma[w[j]].k : 0;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            if (w[j] != u && lw[j] == L) {
+                if (EXT && dk[j] != 0) x[j] *= (QT<EXT>)mgops::pc_scale(dk[j]);   // (one level in hundreds)
+                acc += x[j];
+            }
+    }
+    const float dv = (float)(su.m * (double)acc);
+    delta[u] = dv;
+    q[u] = (QT<EXT>)((1.0 + (double)dv) / su.m);
+    if (bcacc && u != src) bcacc[u] += dv;
+}
+
+// the same level over the whole grid: an entry a thread, 32 a warp (a warp
+// FP64 instruction costs the same for one lane as for all), the warps of
+// entries dealt out over the SMs.  3000 x 3000 lattice: 8.5 us a level with
+// an entry a warp -> 5.5.
+template <bool EXT>
+__device__ __forceinline__ void bc_back_level_flat(const Args &a, int32_t L, int32_t src, QT<EXT> *q, float *delta,
+                                                   float *bcacc)
+{
+    const int32_t b0 = a.lvl_off[L - 1], b1 = a.lvl_off[L];
+    const int32_t gw = (threadIdx.x >> 5) * gridDim.x + blockIdx.x, nwarps = (gridDim.x * blockDim.x) >> 5;
+    for (int32_t i = b0 + gw * 32 + mgd::lane(); i < b1; i += nwarps * 32) {
+        const int32_t u = a.queue[i];
+        bc_back_entry<EXT>(a, L, u, __ldg(&a.row[u]), __ldg(&a.row[u + 1]), src, q, delta, bcacc);
+    }
+}
+
 // Consecutive levels L .. of at most CTA_BACK entries by one block on a graph
 // without heavy vertices: a thread per entry, the next level's entries and
 // row offsets loaded ahead, a block barrier per level instead of a grid
 // barrier and L2 round trips (320 x 311 lattice, 230 entries a level: 11.7 ->
-// 4.0 us per level; at 1,100 a level 14 against the grid's 8, so the bound
-// lies between).  Sums in edge order.  All threads of block 0 call; stops
-// above L1.
+// 3.0 us per level, the grid's flat form 4.4; at 1,100 a level 14 against
+// 5.2, so the bound lies between).  All threads of block 0 call; stops above
+// L1.
 constexpr int CTA_BACK = 768;
 template <bool EXT>
 __device__ __noinline__ void cta_back_levels(const Args &a, int32_t L, int32_t L1, int32_t src, QT<EXT> *q,
@@ -203,38 +255,15 @@ __device__ __noinline__ void cta_back_levels(const Args &a, int32_t L, int32_t L
             re = __ldg(&a.row[v + 1]);
         }
     };
-    auto finish = [&](int32_t u, int32_t b, int32_t e) {
-        const mgops::PathCount su = a.sigma[u];
-        QT<EXT> acc = 0;
-        for (int32_t k = b; k < e; k += 4) {
-            int32_t w[4], lw[4];
-            QT<EXT> x[4];
-#pragma unroll
-            for (int j = 0; j < 4; j++) w[j] = k + j < e ? __ldg(&a.col[k + j]) : u;
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                lw[j] = a.label[w[j]];
-                x[j] = q[w[j]];
-                if (EXT) x[j] *= (QT<EXT>)mgops::pc_scale(su.k - a.sigma[w[j]].k);
-            }
-#pragma unroll
-            for (int j = 0; j < 4; j++)
-                if (w[j] != u && lw[j] == L) acc += x[j];
-        }
-        const float dv = (float)(su.m * (double)acc);
-        delta[u] = dv;
-        q[u] = (QT<EXT>)((1.0 + (double)dv) / su.m);
-        if (bcacc && u != src) bcacc[u] += dv;
-    };
     load(b0, b1);
     for (; L > L1; L--) {
         const int32_t cv = v, cb = rb, ce = re;
         const int32_t n0 = L - 1 > L1 ? a.lvl_off[L - 2] : 0, n1 = L - 1 > L1 ? b0 : 0;
         load(n0, n1);
-        if (cv >= 0) finish(cv, cb, ce);
+        if (cv >= 0) bc_back_entry<EXT>(a, L, cv, cb, ce, src, q, delta, bcacc);
         for (int32_t i = b0 + PTHREADS + t; i < b1; i += PTHREADS) {
             const int32_t u = a.queue[i];
-            finish(u, __ldg(&a.row[u]), __ldg(&a.row[u + 1]));
+            bc_back_entry<EXT>(a, L, u, __ldg(&a.row[u]), __ldg(&a.row[u + 1]), src, q, delta, bcacc);
         }
         b0 = n0;
         b1 = n1;
@@ -270,6 +299,9 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_bc_back_levels(Args a, BCtl *bc
                 L = L1 + 1;
                 continue;
             }
+            bc_back_level_flat<EXT>(a, L, src, q, delta, bcacc);
+            if (!mgd::grid_sync(a.bar, a.bar_err, a.bar_never)) return;
+            continue;
         }
         const int par = L & 1;
         if (blockIdx.x == 0 && threadIdx.x == 0) bc_ctl->hcnt[par ^ 1] = 0;

@@ -55,3 +55,30 @@ def test_row_bounds(count, direction):
     _check(g, og, (np.arange(count) * 97) % og.nv, direction=direction)
     g.free()
     h.free()
+
+
+@pytest.mark.parametrize("count", [1, 4, 5, 31, 33])
+@pytest.mark.parametrize("direction", [mg.DIR_AUTO, mg.DIR_PULL, mg.DIR_PUSH])
+def test_low_degree_rows(count, direction):
+    # a lattice with hubs of 8..127 edges (rows past the thread path) and a
+    # second component; sources close together, so rows meet many at a level
+    rng = np.random.default_rng(9)
+    v = np.arange(70 * 60).reshape(70, 60)
+    src = [v[:, :-1].ravel(), v[:-1].ravel()]
+    dst = [v[:, 1:].ravel(), v[1:].ravel()]
+    n = v.size
+    for k, d in enumerate([8, 9, 31, 32, 33, 100, 120]):
+        src.append(np.full(d, n + k))
+        dst.append(rng.choice(v.size, d, replace=False))
+    src.append(n + 7 + np.arange(20))
+    dst.append(n + 8 + np.arange(20))
+    h = mg.HostGraph.from_entries(n + 28, np.concatenate(src), np.concatenate(dst))
+    og = O.csr_from_arrays(*h.arrays())
+    assert og.ne <= 8 * og.nv and np.max(np.diff(h.arrays()[0])) < 128
+    g = mg.Graph(h)
+    sources = (np.arange(count) * 3 + 5) % og.nv
+    for _ in range(2):
+        _check(g, og, sources, direction=direction)
+    _check(g, og, [og.nv - 1, og.nv // 2], direction=direction)
+    g.free()
+    h.free()
