@@ -278,8 +278,11 @@ __device__ __noinline__ void cta_back_levels(const Args &a, int32_t L, int32_t L
 // level will use while the current level runs (its last readers finished
 // before the previous barrier).  A barrier timeout sets the error flag; the
 // host reads it and fails the run.
-template <bool EXT>
-__global__ void __launch_bounds__(PTHREADS, 1) k_bc_back_levels(Args a, BCtl *bc_ctl, QT<EXT> *q, float *delta,
+// Graphs with vertices of 128 edges (HEAVY) keep two blocks per SM: their
+// levels are few and large, and want the warps (R-MAT 22: 2.3 ms against
+// 3.4).
+template <bool EXT, bool HEAVY>
+__global__ void __launch_bounds__(PTHREADS, HEAVY ? 2 : 1) k_bc_back_levels(Args a, BCtl *bc_ctl, QT<EXT> *q, float *delta,
                                                                 float *bcacc, int32_t *heavy_list)
 {
     __shared__ int4 s_b;
@@ -288,7 +291,7 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_bc_back_levels(Args a, BCtl *bc
     __syncthreads();
     const int32_t L0 = s_b.x, src = s_b.y;
     for (int32_t L = L0; L >= 1; L--) {
-        if (!a.has_heavy) {
+        if constexpr (!HEAVY) {
             // a run of small levels is block 0's alone; the offsets are the
             // same for every block
             int32_t L1 = L;
@@ -302,20 +305,21 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_bc_back_levels(Args a, BCtl *bc
             bc_back_level_flat<EXT>(a, L, src, q, delta, bcacc);
             if (!mgd::grid_sync(a.bar, a.bar_err, a.bar_never)) return;
             continue;
+        } else {
+            const int par = L & 1;
+            if (blockIdx.x == 0 && threadIdx.x == 0) bc_ctl->hcnt[par ^ 1] = 0;
+            bc_back_level<EXT>(a, L, src, &bc_ctl->hcnt[par], q, delta, bcacc, heavy_list);
+            if (!mgd::grid_sync(a.bar, a.bar_err, a.bar_never)) return;
+            if (threadIdx.x == 0) s_nheavy = __ldcg(&bc_ctl->hcnt[par]);
+            __syncthreads();
+            const int32_t nheavy = s_nheavy;
+            // most levels list no heavy entry: every block sees the same count
+            // and skips the heavy phase and its barrier together (block 0's
+            // early clear of this counter then leaves it at the 0 it holds)
+            if (nheavy == 0) continue;
+            bc_back_heavy_level<EXT>(a, L, src, nheavy, q, delta, bcacc, heavy_list);
+            if (!mgd::grid_sync(a.bar, a.bar_err, a.bar_never)) return;
         }
-        const int par = L & 1;
-        if (blockIdx.x == 0 && threadIdx.x == 0) bc_ctl->hcnt[par ^ 1] = 0;
-        bc_back_level<EXT>(a, L, src, &bc_ctl->hcnt[par], q, delta, bcacc, heavy_list);
-        if (!mgd::grid_sync(a.bar, a.bar_err, a.bar_never)) return;
-        if (threadIdx.x == 0) s_nheavy = __ldcg(&bc_ctl->hcnt[par]);
-        __syncthreads();
-        const int32_t nheavy = s_nheavy;
-        // most levels list no heavy entry: every block sees the same count
-        // and skips the heavy phase and its barrier together (block 0's
-        // early clear of this counter then leaves it at the 0 it holds)
-        if (nheavy == 0) continue;
-        bc_back_heavy_level<EXT>(a, L, src, nheavy, q, delta, bcacc, heavy_list);
-        if (!mgd::grid_sync(a.bar, a.bar_err, a.bar_never)) return;
     }
 }
 
@@ -356,10 +360,8 @@ void free_frontier_ws(mg_graph *g)
 mg_status frontier_bfs_multi(mg_graph *g, const int32_t *srcs_host, int32_t nsrc, const mg_opts &opt,
                              mg_run_info *info)
 {
-    return frontier_run_impl<mgops::Bfs>(g, 0, srcs_host, nsrc, opt, info);
+    return frontier_run_impl<mgops::Bfs>(g, 0, srcs_host, nsrc, opt, info, MG_RES_LEVEL);
 }
-
-const void *frontier_label(mg_graph *g) { return g->fws ? g->fws->label.p : nullptr; }
 
 
 mg_status bc_backward(mg_graph *g, int32_t src, const mg_opts &opt, float *bcacc)
@@ -380,11 +382,16 @@ mg_status bc_backward(mg_graph *g, int32_t src, const mg_opts &opt, float *bcacc
     if (w->coop_back == 0) {
         int per_sm = 0;
         int per_sm_x = 0;
-        MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bc_back_levels<false>, PTHREADS, 0));
-        MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_x, k_bc_back_levels<true>, PTHREADS, 0));
+        if (a.has_heavy) {
+            MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bc_back_levels<false, true>, PTHREADS, 0));
+            MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_x, k_bc_back_levels<true, true>, PTHREADS, 0));
+        } else {
+            MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bc_back_levels<false, false>, PTHREADS, 0));
+            MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_x, k_bc_back_levels<true, false>, PTHREADS, 0));
+        }
         per_sm = std::min(per_sm, per_sm_x);
         if (per_sm < 1) return fail(MG_ERR_CUDA, "persistent backward kernel does not fit on an SM");
-        w->coop_back = g->num_sms;
+        w->coop_back = std::min(per_sm, a.has_heavy ? 2 : 1) * g->num_sms;
     }
     if (a.bc_ext) k_bc_q_init<true><<<grid, THREADS, 0, s>>>(g->nv, a.sigma, a.label, (double *)q, delta);
     else k_bc_q_init<false><<<grid, THREADS, 0, s>>>(g->nv, a.sigma, a.label, (float *)q, delta);
@@ -404,8 +411,14 @@ mg_status bc_backward(mg_graph *g, int32_t src, const mg_opts &opt, float *bcacc
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     P.begin(sb);
-    if (a.bc_ext) MG_CUDA(cudaLaunchKernelEx(&cfg, k_bc_back_levels<true>, a, bc, (double *)q, delta, bcacc, hl));
-    else MG_CUDA(cudaLaunchKernelEx(&cfg, k_bc_back_levels<false>, a, bc, (float *)q, delta, bcacc, hl));
+    if (a.bc_ext && a.has_heavy)
+        MG_CUDA(cudaLaunchKernelEx(&cfg, k_bc_back_levels<true, true>, a, bc, (double *)q, delta, bcacc, hl));
+    else if (a.bc_ext)
+        MG_CUDA(cudaLaunchKernelEx(&cfg, k_bc_back_levels<true, false>, a, bc, (double *)q, delta, bcacc, hl));
+    else if (a.has_heavy)
+        MG_CUDA(cudaLaunchKernelEx(&cfg, k_bc_back_levels<false, true>, a, bc, (float *)q, delta, bcacc, hl));
+    else
+        MG_CUDA(cudaLaunchKernelEx(&cfg, k_bc_back_levels<false, false>, a, bc, (float *)q, delta, bcacc, hl));
     P.end();
     int err = 0;
     MG_CUDA(cudaMemcpyAsync(&err, a.bar_err, 4, cudaMemcpyDeviceToHost, s));
@@ -432,8 +445,7 @@ mg_status mg_bfs(mg_graph *g, int32_t source, const mg_opts *o, int32_t *level_o
     mg_opts opt;
     MG_TRY(begin_run(g, o, opt, info));
     MG_TRY(check_source(g, source));
-    MG_TRY(frontier_run_impl<mgops::Bfs>(g, to_engine(g, source), nullptr, 0, opt, info));
-    MG_TRY(publish(g, MG_RES_LEVEL, g->fws->label.p, 4));
+    MG_TRY(frontier_run_impl<mgops::Bfs>(g, to_engine(g, source), nullptr, 0, opt, info, MG_RES_LEVEL));
     MG_TRY(end_run(g, opt, info));
     return copy_out(g, level_out, g->res[MG_RES_LEVEL], (size_t)g->nv * 4);
 }
@@ -443,8 +455,7 @@ mg_status mg_sssp(mg_graph *g, int32_t source, const mg_opts *o, int32_t *dist_o
     mg_opts opt;
     MG_TRY(begin_run(g, o, opt, info));
     MG_TRY(check_source(g, source));
-    MG_TRY(frontier_run_impl<mgops::Sssp>(g, to_engine(g, source), nullptr, 0, opt, info));
-    MG_TRY(publish(g, MG_RES_DIST, g->fws->label.p, 4));
+    MG_TRY(frontier_run_impl<mgops::Sssp>(g, to_engine(g, source), nullptr, 0, opt, info, MG_RES_DIST));
     MG_TRY(end_run(g, opt, info));
     return copy_out(g, dist_out, g->res[MG_RES_DIST], (size_t)g->nv * 4);
 }
@@ -456,10 +467,9 @@ mg_status mg_bc(mg_graph *g, int32_t source, const mg_opts *o, int32_t *level_ou
     MG_TRY(begin_run(g, o, opt, info));
     MG_TRY(check_source(g, source));
     const int32_t s = to_engine(g, source);
-    MG_TRY(frontier_run_impl<mgops::BcForward>(g, s, nullptr, 0, opt, info));
+    MG_TRY(frontier_run_impl<mgops::BcForward>(g, s, nullptr, 0, opt, info, MG_RES_LEVEL));
     MG_TRY(bc_backward(g, s, opt, nullptr));
     FrontierWS *w = g->fws;
-    MG_TRY(publish(g, MG_RES_LEVEL, w->label.p, 4));
     // path counts as FP64 values (infinity where a count exceeds the FP64 range)
     MG_TRY(dev_alloc(w->sigma_d, (size_t)std::max(g->nv, 1) * 8));
     k_pc_to_double<<<launch_grid(g, THREADS, 8), THREADS, 0, g->stream>>>(g->nv, w->sigma.as<mgops::PathCount>(),
@@ -503,7 +513,7 @@ mg_status mg_bc_multi(mg_graph *g, const int32_t *sources, int32_t nsrc, const m
     for (int32_t i = 0; i < nsrc; i++) {
         mg_run_info sub;
         const int32_t s = to_engine(g, sources[i]);
-        MG_TRY(frontier_run_impl<mgops::BcForward>(g, s, nullptr, 0, opt, &sub));
+        MG_TRY(frontier_run_impl<mgops::BcForward>(g, s, nullptr, 0, opt, &sub, -1));
         MG_TRY(bc_backward(g, s, opt, w->bc.as<float>()));
         iters += sub.iterations;
     }

@@ -130,6 +130,8 @@ struct LevelCnt {
     int32_t nq;
     int32_t nhcur;
     long long nfe;
+    int32_t fmin;        // least label on the frontier that enters the level (k_frontier_all, min-plus pulls)
+    int32_t pad[3];
 };
 
 __device__ __forceinline__ uint32_t *bm_buf(const Args &a, int idx) { return a.bm + (size_t)idx * a.words; }
@@ -629,30 +631,34 @@ template <class Op>
 using PullOp = std::conditional_t<Op::kPathCounts, PullCounts<Op>, PullRelax<Op>>;
 
 // min-plus pull levels: rows at or below this label cannot improve
-__device__ __forceinline__ int32_t sssp_bound(const Args &a)
+__device__ __forceinline__ int32_t sssp_bound(int32_t fmin, int32_t wmin)
 {
-    const int32_t f = *a.fmin;
-    return f >= INT32_MAX - a.wmin ? INT32_MAX : f + a.wmin;
+    return fmin >= INT32_MAX - wmin ? INT32_MAX : fmin + wmin;
 }
 
 // least label over the frontier queue (before a min-plus pull level)
-__global__ void __launch_bounds__(THREADS) k_fmin(Args a)
+__device__ __forceinline__ void frontier_min(const Args &a, const FCtl &c, int32_t *out)
 {
-    const FCtl c = *a.ctl;
-    if (c.mode != MODE_PULL || c.more == 0) return;
     int32_t mn = INT32_MAX;
     for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < c.qsize; i += gridDim.x * blockDim.x)
         mn = min(mn, a.label[a.queue[c.qoff + i]]);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mn = min(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-    if (mgd::lane() == 0 && mn < INT32_MAX) atomicMin(a.fmin, mn);
+    if (mgd::lane() == 0 && mn < INT32_MAX) atomicMin(out, mn);
 }
 
-template <class Op>
-__global__ void __launch_bounds__(THREADS) k_pull(Args a)
+__global__ void __launch_bounds__(THREADS) k_fmin(Args a)
 {
     const FCtl c = *a.ctl;
     if (c.mode != MODE_PULL || c.more == 0) return;
+    frontier_min(a, c, a.fmin);
+}
+
+// One pull level by blocks of NT threads; bound: min-plus rows at or below
+// this label cannot improve.
+template <class Op, int NT>
+__device__ __forceinline__ void pull_level(const Args &a, const FCtl &c, int32_t bound)
+{
     const int it1 = c.iter + 1;
     const int nextbuf = (c.cur + 1) % 3, sparebuf = (c.cur + 2) % 3;
     const uint32_t *fb = bm_buf(a, c.cur);
@@ -691,15 +697,15 @@ __global__ void __launch_bounds__(THREADS) k_pull(Args a)
         // degree-binned rows; reached rows marked in the next-frontier bitmap
         PullOp<Op> op{{a, bm_buf(a, nextbuf)}, fb, it1, false, 0};
         if constexpr (!Op::kLevelSync) op.all_in = (long long)c.qsize * 8 > a.n;
-        if constexpr (Op::kMinPlusBound) op.bound = sssp_bound(a);
+        if constexpr (Op::kMinPlusBound) op.bound = bound;
         mgd::bins_reduce(op, a.trow, a.tcol, a.twt, a.wrows, a.nwrows, a.nwlong, a.trows, a.ntrows);
         (void)gwarp;
         (void)nwarps;
     }
 
     // heavy rows: one CTA per 2048-edge chunk
-    __shared__ int32_t s_min[THREADS / 32];
-    __shared__ mgops::PathCount s_sum[THREADS / 32];
+    __shared__ int32_t s_min[NT / 32];
+    __shared__ mgops::PathCount s_sum[NT / 32];
     __shared__ int s_hit, s_skip;
     for (int32_t ch = blockIdx.x; ch < a.nhchunks; ch += gridDim.x) {
         int32_t v = a.hchunk[3 * ch], b = a.hchunk[3 * ch + 1], e = a.hchunk[3 * ch + 2];
@@ -711,7 +717,7 @@ __global__ void __launch_bounds__(THREADS) k_pull(Args a)
         // would drop this chunk's share of the row's path count
         if (threadIdx.x == 0) {
             if constexpr (!Op::kLevelSync) {
-                s_skip = Op::kMinPlusBound && a.label[v] <= sssp_bound(a);
+                s_skip = Op::kMinPlusBound && a.label[v] <= bound;
             } else {
                 const int32_t lv = __ldcg(&a.label[v]);
                 s_skip = lv != mgops::UNSET && lv != it1;
@@ -749,7 +755,7 @@ __global__ void __launch_bounds__(THREADS) k_pull(Args a)
         if (threadIdx.x == 0) {
             int32_t bm = Op::initialize();
             mgops::PathCount bs = mgops::pc_zero();
-            for (int w = 0; w < THREADS / 32; w++) {
+            for (int w = 0; w < NT / 32; w++) {
                 if constexpr (!Op::kLevelSync) Op::accumulate_nonAtomics(bm, s_min[w], it1);
                 if constexpr (Op::kPathCounts) bs = mgops::pc_add(bs, s_sum[w], ext);
             }
@@ -780,6 +786,14 @@ __global__ void __launch_bounds__(THREADS) k_pull(Args a)
     warp_add64(&a.ctl->scanned, scanned);
 }
 
+template <class Op>
+__global__ void __launch_bounds__(THREADS) k_pull(Args a)
+{
+    const FCtl c = *a.ctl;
+    if (c.mode != MODE_PULL || c.more == 0) return;
+    pull_level<Op, THREADS>(a, c, Op::kMinPlusBound ? sssp_bound(*a.fmin, a.wmin) : 0);
+}
+
 // ----------------------------------------------------------------------------
 // compact: after a pull sweep, the next frontier's bitmap -> queue slice,
 // edge count and heavy list.  A block takes every gridDim-th word of the
@@ -788,17 +802,16 @@ __global__ void __launch_bounds__(THREADS) k_pull(Args a)
 // reserves its queue slots with one atomicAdd; a warp goes through its words
 // a lane per vertex, so the row offsets come in coalesced.
 // ----------------------------------------------------------------------------
-__global__ void __launch_bounds__(THREADS) k_compact(Args a)
+template <int NT>
+__device__ __forceinline__ void compact_level(const Args &a, const FCtl &c, int32_t *nq, int32_t *nhcur, long long *nfe)
 {
-    const FCtl c = *a.ctl;
-    if (c.mode != MODE_PULL || c.more == 0) return;
-    constexpr int NW = THREADS / 32;
+    constexpr int NW = NT / 32;
     __shared__ int s_cnt[NW], s_base;
     const uint32_t *nb = bm_buf(a, (c.cur + 1) % 3);
     const int lane = mgd::lane(), warp = threadIdx.x >> 5;
     int4 *heavy = a.heavy + (size_t)(c.hpar ^ 1) * a.hcap;
     long long dsum = 0;
-    for (int64_t w0 = blockIdx.x; w0 < a.words; w0 += (int64_t)gridDim.x * THREADS) {
+    for (int64_t w0 = blockIdx.x; w0 < a.words; w0 += (int64_t)gridDim.x * NT) {
         const int64_t wi = w0 + (int64_t)(lane * NW + warp) * gridDim.x;
         const uint32_t bits = wi < a.words ? nb[wi] : 0u;
         const int total = __reduce_add_sync(0xffffffffu, __popc(bits));
@@ -809,7 +822,7 @@ __global__ void __launch_bounds__(THREADS) k_compact(Args a)
             base += k < warp ? s_cnt[k] : 0;
             all += s_cnt[k];
         }
-        if (threadIdx.x == 0 && all) s_base = atomicAdd(&a.ctl->nq, all);
+        if (threadIdx.x == 0 && all) s_base = atomicAdd(nq, all);
         __syncthreads();
         base += s_base;
         unsigned full = __ballot_sync(0xffffffffu, bits != 0);
@@ -826,11 +839,18 @@ __global__ void __launch_bounds__(THREADS) k_compact(Args a)
                 dsum += dg;
             }
             base += __popc(word);
-            if (a.has_heavy && __any_sync(0xffffffffu, dg > PUSH_HEAVY)) list_heavy(heavy, &a.ctl->nhcur, v, rb, dg);
+            if (a.has_heavy && __any_sync(0xffffffffu, dg > PUSH_HEAVY)) list_heavy(heavy, nhcur, v, rb, dg);
         }
         __syncthreads();   // s_cnt / s_base are reused
     }
-    warp_add64(&a.ctl->nf_edges, dsum);
+    warp_add64(nfe, dsum);
+}
+
+__global__ void __launch_bounds__(THREADS) k_compact(Args a)
+{
+    const FCtl c = *a.ctl;
+    if (c.mode != MODE_PULL || c.more == 0) return;
+    compact_level<THREADS>(a, c, &a.ctl->nq, &a.ctl->nhcur, &a.ctl->nf_edges);
 }
 
 // ----------------------------------------------------------------------------
@@ -897,6 +917,34 @@ __device__ __forceinline__ void store_ctl_push(FCtl *p, const FCtl &c)
     for (int i = 0; i < (int)(sizeof(FCtl) / 8) - 1; i++) __stcg(&d[i], src[i]);
 }
 
+// whether the next push levels are block 0's alone
+template <class Op, bool HEAVY>
+__device__ __forceinline__ bool block_phase_due(const FCtl &c)
+{
+    return !HEAVY && Op::kLevelSync && c.qsize <= CTA_ENTER && c.qedges <= CTA_EDGES;
+}
+
+// Block 0's levels while the others wait; false when a barrier failed
+template <class Op>
+__device__ __forceinline__ bool block_phase(const Args &a, FCtl &c)
+{
+    if constexpr (Op::kLevelSync) {
+        // the bitmaps start from zero
+        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 3 * a.words; i += gridDim.x * blockDim.x) a.bm[i] = 0;
+        if (!mgd::grid_sync(a.bar, a.bar_err, a.bar_never)) return false;
+        if (blockIdx.x == 0) {
+            extern __shared__ __align__(16) unsigned char s_dyn[];
+            cta_push_levels<Op>(a, c, *reinterpret_cast<CtaShared *>(s_dyn));
+            if (threadIdx.x == 0) store_ctl_push(a.ctl, c);
+        }
+        if (!mgd::grid_sync(a.bar, a.bar_err, a.bar_never)) return false;
+        const FCtl c1 = block_load_ctl(a.ctl);
+        if (threadIdx.x == 0) c = c1;
+        __syncthreads();
+    }
+    return true;
+}
+
 // HEAVY: the graph may have vertices above PUSH_HEAVY out-edges (graphs that
 // have none run without the chunk code and its votes).
 template <class Op, bool HEAVY>
@@ -920,23 +968,9 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_sparse_levels(Args a)
             z->nhcur = 0;
             z->nfe = 0;
         }
-        if constexpr (!HEAVY && Op::kLevelSync) {
-            if (s_c.qsize <= CTA_ENTER && s_c.qedges <= CTA_EDGES) {
-                // block 0 alone from here on; the bitmaps start from zero
-                for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 3 * a.words; i += gridDim.x * blockDim.x)
-                    a.bm[i] = 0;
-                if (!mgd::grid_sync(a.bar, a.bar_err, a.bar_never)) break;
-                if (blockIdx.x == 0) {
-                    extern __shared__ __align__(16) unsigned char s_dyn[];
-                    cta_push_levels<Op>(a, s_c, *reinterpret_cast<CtaShared *>(s_dyn));
-                    if (threadIdx.x == 0) store_ctl_push(a.ctl, s_c);
-                }
-                if (!mgd::grid_sync(a.bar, a.bar_err, a.bar_never)) break;
-                const FCtl c1 = block_load_ctl(a.ctl);
-                if (threadIdx.x == 0) s_c = c1;
-                __syncthreads();
-                continue;
-            }
+        if (block_phase_due<Op, HEAVY>(s_c)) {
+            if (!block_phase<Op>(a, s_c)) break;
+            continue;
         }
         push_level<Op, HEAVY>(a, s_c, lc);
         if (!mgd::grid_sync(a.bar, a.bar_err, a.bar_never)) break;
@@ -966,9 +1000,15 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_sparse_levels(Args a)
 // (several sources = one traversal of a disjoint union of graphs), a thread
 // each of one block (one thread walking 30 sources took 33 us)
 constexpr int INIT_THREADS = 256;
+struct StartArgs {
+    int32_t src;
+    const int32_t *srcs;
+    int32_t nsrc;
+    int dirmode, alpha, beta, max_iter;
+};
+
 template <class Op>
-__global__ void __launch_bounds__(INIT_THREADS) k_init(Args a, int32_t src, const int32_t *srcs, int32_t nsrc,
-                                                       int dirmode, int alpha, int beta, int max_iter)
+__device__ __forceinline__ void start_sources(const Args &a, const StartArgs &st)
 {
     __shared__ int s_q;
     __shared__ unsigned long long s_ve;
@@ -979,18 +1019,18 @@ __global__ void __launch_bounds__(INIT_THREADS) k_init(Args a, int32_t src, cons
         std::memset(c, 0, sizeof(FCtl));
         c->more = 1;
         c->archive = Op::kLevelSync;
-        c->max_iter = max_iter;
-        c->dirmode = dirmode;
-        c->alpha = alpha;
-        c->beta = beta;
-        c->mode = (dirmode == MG_DIR_PULL) ? MODE_PULL : MODE_PUSH;
+        c->max_iter = st.max_iter;
+        c->dirmode = st.dirmode;
+        c->alpha = st.alpha;
+        c->beta = st.beta;
+        c->mode = (st.dirmode == MG_DIR_PULL) ? MODE_PULL : MODE_PUSH;
         *a.fmin = INT32_MAX;
     }
     __syncthreads();
-    const int32_t count = srcs ? nsrc : 1;
-    for (int32_t i0 = threadIdx.x & ~31; i0 < count; i0 += INIT_THREADS) {
+    const int32_t count = st.srcs ? st.nsrc : 1;
+    for (int32_t i0 = threadIdx.x & ~31; i0 < count; i0 += blockDim.x) {
         const int32_t i = i0 + mgd::lane();
-        const int32_t s = i < count ? (srcs ? srcs[i] : src) : -1;
+        const int32_t s = i < count ? (st.srcs ? st.srcs[i] : st.src) : -1;
         int32_t b = 0, d = 0;
         if (s >= 0 && mgd::bm_set(a.visited, s)) {  // (a duplicate source is queued once)
             a.label[s] = Op::source_value();
@@ -1011,6 +1051,94 @@ __global__ void __launch_bounds__(INIT_THREADS) k_init(Args a, int32_t src, cons
         c->visited_edges = (long long)s_ve;
         c->qedges = (int32_t)min(s_ve, (unsigned long long)INT32_MAX);
         if (Op::kLevelSync) { a.lvl_off[0] = 0; a.lvl_off[1] = q; c->nlevels = 1; }
+    }
+}
+
+template <class Op>
+__global__ void __launch_bounds__(INIT_THREADS) k_init(Args a, StartArgs st)
+{
+    start_sources<Op>(a, st);
+}
+
+// The whole traversal of a small graph in one cooperative launch: start
+// values, push and pull levels, the result in caller order.  The loop of the
+// large form (k_sparse_levels, k_fmin, k_pull, k_compact, k_decide inside a
+// WHILE node) costs 15 to 20 us per switch between push and pull however
+// small the levels; here a pull level is two phases and two grid barriers.
+// BFS R-MAT 12: 97 -> 65 us on the device.
+template <class Op, bool HEAVY>
+__global__ void __launch_bounds__(PTHREADS, 1) k_frontier_all(Args a, StartArgs st, const int32_t *old2new,
+                                                              int32_t *out)
+{
+    __shared__ FCtl s_c;
+    __shared__ int32_t s_fmin;
+    const int gtid = blockIdx.x * PTHREADS + threadIdx.x, nthreads = gridDim.x * PTHREADS;
+    for (int32_t v = gtid; v < a.n; v += nthreads) {
+        a.label[v] = Op::initialize();
+        if (Op::kPathCounts) a.sigma[v] = mgops::pc_zero();
+    }
+    for (int32_t i = gtid; i < 3 * a.words; i += nthreads) a.bm[i] = 0;
+    for (int32_t i = gtid; i < a.words; i += nthreads) a.visited[i] = 0;
+    if (gtid < 4) {
+        a.cnt[gtid].nq = a.cnt[gtid].nhcur = 0;
+        a.cnt[gtid].nfe = 0;
+        a.cnt[gtid].fmin = INT32_MAX;
+    }
+    bool ok = mgd::grid_sync(a.bar, a.bar_err, a.bar_never);
+    if (ok && blockIdx.x == 0) start_sources<Op>(a, st);
+    ok = ok && mgd::grid_sync(a.bar, a.bar_err, a.bar_never);
+    if (ok) {
+        const FCtl c0 = block_load_ctl(a.ctl);
+        if (threadIdx.x == 0) s_c = c0;
+    }
+    __syncthreads();
+    for (int32_t lv = 0; ok && s_c.more; lv++) {
+        LevelCnt *lc = a.cnt + (lv & 3);
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            LevelCnt *z = a.cnt + ((lv + 2) & 3);
+            z->nq = 0;
+            z->nhcur = 0;
+            z->nfe = 0;
+            z->fmin = INT32_MAX;
+        }
+        if (s_c.mode == MODE_PUSH) {
+            if (block_phase_due<Op, HEAVY>(s_c)) {
+                ok = block_phase<Op>(a, s_c);
+                continue;
+            }
+            push_level<Op, HEAVY>(a, s_c, lc);
+        } else {
+            int32_t bound = 0;
+            if constexpr (Op::kMinPlusBound) {
+                frontier_min(a, s_c, &lc->fmin);
+                if (!(ok = mgd::grid_sync(a.bar, a.bar_err, a.bar_never))) break;
+                if (threadIdx.x == 0) s_fmin = __ldcg(&lc->fmin);
+                __syncthreads();
+                bound = sssp_bound(s_fmin, a.wmin);
+            }
+            pull_level<Op, PTHREADS>(a, s_c, bound);
+            if (!(ok = mgd::grid_sync(a.bar, a.bar_err, a.bar_never))) break;
+            compact_level<PTHREADS>(a, s_c, &lc->nq, &lc->nhcur, &lc->nfe);
+        }
+        if (!(ok = mgd::grid_sync(a.bar, a.bar_err, a.bar_never))) break;
+        if (threadIdx.x == 0) {
+            const int4 cnt = __ldcg(reinterpret_cast<const int4 *>(lc));  // nq, nhcur, nfe (lo, hi)
+            FCtl c = s_c;
+            const long long nfe = (long long)(((unsigned long long)(unsigned)cnt.w << 32) | (unsigned)cnt.z);
+            decide_local(a, c, cnt.x, cnt.y, nfe, blockIdx.x == 0);
+            s_c = c;
+        }
+        __syncthreads();
+    }
+    if (ok && out)
+        for (int32_t v = gtid; v < a.n; v += nthreads) out[v] = __ldcg(&a.label[__ldg(&old2new[v])]);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        FCtl c = s_c;
+        if (!ok || *(volatile int *)a.bar_err) {
+            c.status = 3;
+            c.more = 0;
+        }
+        store_ctl_push(a.ctl, c);
     }
 }
 
@@ -1105,6 +1233,44 @@ mg_status launch_sparse_levels(const Args &a, int grid, cudaStream_t st)
     return MG_OK;
 }
 
+// Graphs of up to this many edges run a traversal in one launch
+// (k_frontier_all); past them the pull kernels' twice as many resident warps
+// are worth the launches.  us, one launch / separate: BFS R-MAT 16 (1.8 M
+// edges) 77 / 111, R-MAT 18 (7.6 M) 163 / 144; SSSP 190 / 223 and 372 / 296.
+// A level-synchronous traversal of a graph without heavy vertices hardly ever
+// pulls: one launch at any size (BFS 1500 x 1400 lattice 9.1 / 10.2 ms).
+constexpr int64_t ONE_LAUNCH_EDGES_SYNC = 4 << 20, ONE_LAUNCH_EDGES_RELAX = 3 << 20;
+template <class Op>
+bool one_launch_pays(const mg_graph *g)
+{
+    if (Op::kLevelSync) return !g->relabeled || g->ne <= ONE_LAUNCH_EDGES_SYNC;
+    return g->ne <= ONE_LAUNCH_EDGES_RELAX;
+}
+
+template <class Op>
+mg_status launch_frontier_all(const Args &a, const StartArgs &st, int grid, const int32_t *old2new, int32_t *out,
+                              cudaStream_t s)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3(PTHREADS);
+    cfg.dynamicSmemBytes = a.has_heavy ? 0 : sizeof(CtaShared);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (a.has_heavy) {
+        MG_CUDA(cudaLaunchKernelEx(&cfg, k_frontier_all<Op, true>, a, st, old2new, out));
+    } else {
+        MG_CUDA(cudaFuncSetAttribute(k_frontier_all<Op, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)sizeof(CtaShared)));
+        MG_CUDA(cudaLaunchKernelEx(&cfg, k_frontier_all<Op, false>, a, st, old2new, out));
+    }
+    return MG_OK;
+}
+
 inline Args make_args(mg_graph *g)
 {
     FrontierWS *w = g->fws;
@@ -1148,11 +1314,53 @@ inline LoopKey key_of(const Args &a, const void *op_tag, int grid, int coop_grid
     return LoopKey().add(op_tag).add(a).add(grid).add(coop_grid);
 }
 
-// Forward traversal with operator Op from src (or from the nsrc sources in
-// srcs_host when it is non-null); results stay in the workspace.
+// result slot `which` in caller ids (mapped on the device before the run ends)
+inline mg_status publish(mg_graph *g, int which, const void *src, size_t elem)
+{
+    const void *p = nullptr;
+    MG_TRY(to_caller(g, which, src, elem, 1, &p));
+    g->res[which] = p;
+    return MG_OK;
+}
+
 template <class Op>
 mg_status frontier_run_impl(mg_graph *g, int32_t src, const int32_t *srcs_host, int32_t nsrc, const mg_opts &opt,
-                            mg_run_info *info)
+                            mg_run_info *info, int which);
+
+// what the loop state says after a run; an overflow of plain path counts
+// starts the run over with extended ones
+template <class Op>
+mg_status frontier_outcome(mg_graph *g, const Args &a, int32_t src, const int32_t *srcs_host, int32_t nsrc,
+                           const mg_opts &opt, int max_iter, mg_run_info *info, int which)
+{
+    cudaStream_t s = g->stream;
+    FCtl hc;
+    int32_t ovf = 0;
+    MG_CUDA(cudaMemcpyAsync(&hc, a.ctl, sizeof(FCtl), cudaMemcpyDeviceToHost, s));
+    if (Op::kPathCounts) MG_CUDA(cudaMemcpyAsync(&ovf, a.bc_ovf, 4, cudaMemcpyDeviceToHost, s));
+    MG_CUDA(cudaStreamSynchronize(s));
+    if (ovf && !g->bc_ext) {
+        // a path count passed FP64's comfortable range: this graph's BC runs
+        // use extended path counts from now on, starting with this one
+        g->bc_ext = true;
+        return frontier_run_impl<Op>(g, src, srcs_host, nsrc, opt, info, which);
+    }
+    if (info) {
+        info->iterations = hc.iter;
+        info->pull_iterations = hc.pull_iters;
+        info->edges_scanned = hc.scanned;
+    }
+    if (hc.status == 3) return fail(MG_ERR_CUDA, "grid barrier of the persistent push kernel timed out");
+    if (hc.status != 0) return fail(MG_ERR_ITER_LIMIT, "iteration cap %d reached", max_iter);
+    return MG_OK;
+}
+
+// Forward traversal with operator Op from src (or from the nsrc sources in
+// srcs_host when it is non-null); the labels in the workspace and, for
+// which >= 0, in caller order in the graph's result slot `which`.
+template <class Op>
+mg_status frontier_run_impl(mg_graph *g, int32_t src, const int32_t *srcs_host, int32_t nsrc, const mg_opts &opt,
+                            mg_run_info *info, int which)
 {
     static_assert(!Op::kLevelSync || Op::kFirstParent || Op::kPathCounts,
                   "a level-synchronous operator is first-parent (BFS) or carries path counts (BC)");
@@ -1172,14 +1380,34 @@ mg_status frontier_run_impl(mg_graph *g, int32_t src, const int32_t *srcs_host, 
     cudaStream_t s = g->stream;
     const size_t n = (size_t)g->nv;
     const int grid = launch_grid(g, THREADS, 8);
+    int max_iter = opt.max_iter > 0 ? opt.max_iter : (Op::kLevelSync ? g->nv + 2 : 4 * g->nv + 16);
+    int alpha = opt.alpha > 0 ? opt.alpha : (Op::kLevelSync ? 15 : 4), beta = opt.beta > 0 ? opt.beta : 18;
+    StartArgs st;
+    std::memset(&st, 0, sizeof(st));
+    st.src = src;
+    st.srcs = srcs_dev;
+    st.nsrc = nsrc;
+    st.dirmode = opt.direction;
+    st.alpha = alpha;
+    st.beta = beta;
+    st.max_iter = max_iter;
+    if (opt.exec == MG_EXEC_GRAPH && !opt.profile && one_launch_pays<Op>(g)) {
+        int32_t *out = nullptr;
+        if (which >= 0 && g->relabeled) {
+            MG_TRY(dev_alloc(g->res_out[which], std::max<size_t>(n, 1) * 4));
+            out = g->res_out[which].as<int32_t>();
+        }
+        MG_CUDA(cudaMemsetAsync(w->bar.p, 0, BAR_BYTES, s));
+        MG_TRY(launch_frontier_all<Op>(a, st, g->num_sms, g->old2new.as<int32_t>(), out, s));
+        if (which >= 0) g->res[which] = out ? (const void *)out : w->label.p;
+        return frontier_outcome<Op>(g, a, src, srcs_host, nsrc, opt, max_iter, info, which);
+    }
     if (n) k_label_init<Op><<<grid, THREADS, 0, s>>>(a.label, (int32_t)n);
     MG_CUDA(cudaMemsetAsync(a.bm, 0, 3 * (size_t)a.words * 4, s));
     MG_CUDA(cudaMemsetAsync(a.visited, 0, (size_t)a.words * 4, s));
     MG_CUDA(cudaMemsetAsync(w->bar.p, 0, BAR_BYTES, s));
     if (Op::kPathCounts) MG_CUDA(cudaMemsetAsync(a.sigma, 0, n * sizeof(mgops::PathCount), s));
-    int max_iter = opt.max_iter > 0 ? opt.max_iter : (Op::kLevelSync ? g->nv + 2 : 4 * g->nv + 16);
-    int alpha = opt.alpha > 0 ? opt.alpha : (Op::kLevelSync ? 15 : 4), beta = opt.beta > 0 ? opt.beta : 18;
-    k_init<Op><<<1, INIT_THREADS, 0, s>>>(a, src, srcs_dev, nsrc, opt.direction, alpha, beta, max_iter);
+    k_init<Op><<<1, INIT_THREADS, 0, s>>>(a, st);
     MG_CUDA(cudaGetLastError());
     const void *tag = &OpTag<Op>::id;
     const int coop = w->coop_grid[tag];
@@ -1214,35 +1442,8 @@ mg_status frontier_run_impl(mg_graph *g, int32_t src, const int32_t *srcs_host, 
     };
     MG_TRY(run_loop(opt.profile ? MG_EXEC_HOST : opt.exec, opt.profile != 0, s, w->lg[tag], key_of(a, tag, grid, coop),
                     body, &a.ctl->more, g->pinned_flag, max_iter + 2));
-    // status readback
-    FCtl hc;
-    int32_t ovf = 0;
-    MG_CUDA(cudaMemcpyAsync(&hc, a.ctl, sizeof(FCtl), cudaMemcpyDeviceToHost, s));
-    if (Op::kPathCounts) MG_CUDA(cudaMemcpyAsync(&ovf, a.bc_ovf, 4, cudaMemcpyDeviceToHost, s));
-    MG_CUDA(cudaStreamSynchronize(s));
-    if (ovf && !g->bc_ext) {
-        // a path count passed FP64's comfortable range: this graph's BC runs
-        // use extended path counts from now on, starting with this one
-        g->bc_ext = true;
-        return frontier_run_impl<Op>(g, src, srcs_host, nsrc, opt, info);
-    }
-    if (info) {
-        info->iterations = hc.iter;
-        info->pull_iterations = hc.pull_iters;
-        info->edges_scanned = hc.scanned;
-    }
-    if (hc.status == 3) return fail(MG_ERR_CUDA, "grid barrier of the persistent push kernel timed out");
-    if (hc.status != 0) return fail(MG_ERR_ITER_LIMIT, "iteration cap %d reached", max_iter);
-    return MG_OK;
-}
-
-// result slot `which` in caller ids (mapped on the device before the run ends)
-inline mg_status publish(mg_graph *g, int which, const void *src, size_t elem)
-{
-    const void *p = nullptr;
-    MG_TRY(to_caller(g, which, src, elem, 1, &p));
-    g->res[which] = p;
-    return MG_OK;
+    if (which >= 0) MG_TRY(publish(g, which, a.label, 4));
+    return frontier_outcome<Op>(g, a, src, srcs_host, nsrc, opt, max_iter, info, which);
 }
 
 // One whole run of a label operator through the C ABI's conventions:
@@ -1255,8 +1456,7 @@ mg_status frontier_operator_run(mg_graph *g, int32_t source, const mg_opts *o, i
     mg_opts opt;
     MG_TRY(begin_run(g, o, opt, info));
     if (source < 0 || source >= g->nv) return fail(MG_ERR_RANGE, "source %d out of range [0,%d)", source, g->nv);
-    MG_TRY(frontier_run_impl<Op>(g, to_engine(g, source), nullptr, 0, opt, info));
-    MG_TRY(publish(g, MG_RES_LEVEL, g->fws->label.p, 4));
+    MG_TRY(frontier_run_impl<Op>(g, to_engine(g, source), nullptr, 0, opt, info, MG_RES_LEVEL));
     MG_TRY(end_run(g, opt, info));
     return copy_out(g, label_out, g->res[MG_RES_LEVEL], (size_t)g->nv * 4);
 }
