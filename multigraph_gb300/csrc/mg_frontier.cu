@@ -14,12 +14,10 @@ namespace {
 // With path counts sigma = m * 2^(512 k), q is kept as (1 + delta) / m
 // (FP64) and a successor's term is scaled by 2^(512 (k_v - k_w)).
 // ----------------------------------------------------------------------------
-constexpr int32_t BACK_HEAVY = 4096;  // entries above this take a CTA each
-
 struct BCtl {
     int32_t L0;       // deepest level; levels L0 .. 1 finalise their predecessors
     int32_t src;      // source of this sweep (excluded from the BC sum)
-    int32_t hcnt[2];  // heavy entries listed at a level, by level parity
+    int32_t hcnt[2];  // chunks of long entries listed at a level, by level parity
 };
 
 // q and the successor sums: FP32 with plain counts (below 2^100, so
@@ -38,146 +36,160 @@ __global__ void k_bc_q_init(int32_t n, const mgops::PathCount *sigma, const int3
     }
 }
 
-// successor w's term of a level-(L-1) entry with scale kv
+// delta and q of one vertex from its successors' sum
 template <bool EXT>
-__device__ __forceinline__ QT<EXT> bc_succ_term(const Args &a, const QT<EXT> *q, int32_t w, int32_t kv)
+__device__ __forceinline__ void bc_finish_vertex(int32_t v, QT<EXT> s, mgops::PathCount su, float *delta, QT<EXT> *q,
+                                                 float *bc, int32_t src)
 {
-    QT<EXT> t = __ldcg(&q[w]);
-    if (EXT) {
-        const int32_t dk = kv - a.sigma[w].k;
-        if (dk != 0) t *= (QT<EXT>)mgops::pc_scale(dk);   // (one level in hundreds)
+    float dv;
+    if (!EXT && __double2hiint(su.m) < (1023 + 24) << 20) {
+        // a count below 2^24 is exact in FP32: one rounding in the product,
+        // and the quotient of the exact pair 1 + delta corrected by its
+        // remainder -- as formed in FP64 and rounded, off GB300's FP64 pipe
+        const float m = (float)su.m;
+        dv = m * (float)s;
+        const float hi = 1.0f + dv, bp = hi - 1.0f, lo = (1.0f - (hi - bp)) + (dv - bp);
+        const float q0 = __fdiv_rn(hi, m);
+        q[v] = (QT<EXT>)(q0 + __fdividef(fmaf(-q0, m, hi) + lo, m));
+    } else {
+        dv = (float)(su.m * (double)s);
+        q[v] = (QT<EXT>)((1.0 + (double)dv) / su.m);
     }
-    return t;
-}
-
-template <bool EXT>
-__device__ __forceinline__ void bc_finish_vertex(int32_t v, QT<EXT> s, const mgops::PathCount *sigma, float *delta,
-                                                 QT<EXT> *q, float *bc, int32_t src)
-{
-    const double m = sigma[v].m;
-    const float dv = (float)(m * (double)s);
     delta[v] = dv;
-    q[v] = (QT<EXT>)((1.0 + (double)dv) / m);
     if (bc && v != src) bc[v] += dv;
 }
 
-// Level L-1 entries pull (1+delta)/sigma from their level-L successors.
-// q of the successors was written by other blocks in the previous level,
-// so it is loaded through L2 (the persistent kernel runs every level in one
-// launch).  Entries above BACK_HEAVY are listed for bc_back_heavy_level.
-template <bool EXT>
-__device__ __forceinline__ void bc_back_level(const Args &a, int32_t L, int32_t src, int32_t *hcount, QT<EXT> *q,
-                                              float *delta, float *bcacc, int32_t *heavy_list)
-{
-    const int32_t b0 = a.lvl_off[L - 1], b1 = a.lvl_off[L];
-    const int lane = mgd::lane();
-    const int gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int nwarps = (gridDim.x * blockDim.x) >> 5;
-    // vpw entries per warp: 32, or fewer when the level would leave warps idle
-    int vpw = 32;
-    if (b1 - b0 < nwarps * 32) {
-        const int want = max(1, (b1 - b0) / nwarps);
-        vpw = 1;
-        while (vpw * 2 <= want) vpw *= 2;
-    }
-    if (vpw == 1) {
-        // one entry per warp: lanes stride its edges, a shuffle tree sums
-        for (int i = b0 + gwarp; i < b1; i += nwarps) {
-            const int32_t v = a.queue[i];
-            const int32_t b = a.row[v], e = a.row[v + 1];
-            if (e - b > BACK_HEAVY) {
-                if (lane == 0) heavy_list[atomicAdd(hcount, 1)] = v;
-                continue;
-            }
-            const int32_t kv = EXT ? a.sigma[v].k : 0;
-            QT<EXT> acc = 0;
-            for (int32_t p = b + lane; p < e; p += 32) {
-                const int32_t w = a.col[p];
-                if (a.label[w] == L) acc += bc_succ_term<EXT>(a, q, w, kv);
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-            if (lane == 0) bc_finish_vertex<EXT>(v, acc, a.sigma, delta, q, bcacc, src);
-        }
-        return;
-    }
-    for (int base = b0 + gwarp * vpw; base < b1; base += nwarps * vpw) {
-        int32_t v = -1, start = 0, deg = 0, kv = 0;
-        if (lane < vpw && base + lane < b1) {
-            v = a.queue[base + lane];
-            start = a.row[v];
-            deg = a.row[v + 1] - start;
-            if (EXT) kv = a.sigma[v].k;
-            if (deg > BACK_HEAVY) {
-                int h = atomicAdd(hcount, 1);
-                heavy_list[h] = v;
-                deg = 0;
-                v = -1;
-            }
-        }
-        int incl = mgd::warp_scan_incl(deg);
-        int excl = incl - deg;
-        int total = __shfl_sync(0xffffffffu, incl, 31);
-        QT<EXT> acc = 0;
-        for (int k0 = 0; k0 < total; k0 += 32) {
-            int k = k0 + lane;
-            int kk = k < total ? k : total - 1;
-            int own = mgd::owner_lane(excl, kk);
-            int32_t e = __shfl_sync(0xffffffffu, start, own) + (kk - __shfl_sync(0xffffffffu, excl, own));
-            const int32_t kown = __shfl_sync(0xffffffffu, kv, own);
-            QT<EXT> t = 0;
-            if (k < total) {
-                int32_t w = a.col[e];
-                if (a.label[w] == L) t = bc_succ_term<EXT>(a, q, w, kown);
-            } else {
-                own = -1;
-            }
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                int oo = __shfl_down_sync(0xffffffffu, own, o);
-                QT<EXT> ot = __shfl_down_sync(0xffffffffu, t, o);
-                if (lane + o < 32 && oo == own) t += ot;
-            }
-            int prev_own = __shfl_up_sync(0xffffffffu, own, 1);
-            bool head = (own >= 0) && (lane == 0 || prev_own != own);
-            unsigned heads = __ballot_sync(0xffffffffu, head);
-            while (heads) {
-                int hl = __ffs(heads) - 1;
-                heads &= heads - 1;
-                int ho = __shfl_sync(0xffffffffu, own, hl);
-                QT<EXT> ht = __shfl_sync(0xffffffffu, t, hl);
-                if (lane == ho) acc += ht;
-            }
-        }
-        if (v >= 0) bc_finish_vertex<EXT>(v, acc, a.sigma, delta, q, bcacc, src);
-    }
-}
+// Backward sweep of graphs with heavy vertices: few, large levels.  q is kept
+// in two arrays by level parity, zero where not yet formed: a level-l entry's
+// neighbours in array (l + 1) & 1 are its successors (level l + 1) and
+// vertices of level l - 1, whose q is still zero, so one gather an edge does
+// (the label test took a second, dependent one).  Entries of up to BACK_CHUNK
+// edges take eight lanes, four entries a warp, four gathers a lane in flight;
+// the others a warp per BACK_CHUNK-edge chunk, the last chunk of an entry
+// adding the partial sums up in order.  One warp for any entry of up to 4,096
+// edges took a level of R-MAT 20 up to 3 ms.  Backward sweep: R-MAT 16 154 ->
+// 49 us, R-MAT 20 1,200 to 4,000 -> 215, R-MAT 22 2,300 -> 800.
+constexpr int32_t BACK_CHUNK = 256;
 
-// heavy entries of the level: a CTA each, fixed-order block sum
+struct BackArgs {
+    int32_t *lvl_off;
+    void *q[2];
+    int4 *item;           // chunks of the level's long entries: vertex, begin, end, the entry's first chunk
+    int32_t *arrive;      // [items] chunks finished, at the entry's first chunk (zero between levels)
+    void *part;           // [items] partial sums
+    int32_t *nitems;      // [2] by level parity
+};
+
 template <bool EXT>
-__device__ __forceinline__ void bc_back_heavy_level(const Args &a, int32_t L, int32_t src, int32_t nheavy, QT<EXT> *q,
-                                                    float *delta, float *bcacc, const int32_t *heavy_list)
+__global__ void __launch_bounds__(PTHREADS, 1) k_bc_back_heavy(Args a, BCtl *bc_ctl, BackArgs k, float *delta,
+                                                               float *bcacc)
 {
-    __shared__ QT<EXT> s_part[32];
-    for (int32_t h = blockIdx.x; h < nheavy; h += gridDim.x) {
-        int32_t v = __ldcg(&heavy_list[h]);
-        int32_t b = a.row[v], e = a.row[v + 1];
-        const int32_t kv = EXT ? a.sigma[v].k : 0;
-        QT<EXT> acc = 0;
-        for (int32_t p = b + threadIdx.x; p < e; p += blockDim.x) {
-            int32_t w = a.col[p];
-            if (a.label[w] == L) acc += bc_succ_term<EXT>(a, q, w, kv);
+    constexpr unsigned FULL = 0xffffffffu;
+    __shared__ int4 s_b;
+    if (threadIdx.x == 0) s_b = __ldcg(reinterpret_cast<const int4 *>(bc_ctl));
+    __syncthreads();
+    const int32_t L0 = s_b.x, src = s_b.y;
+    const int lane = mgd::lane(), gl = lane & 7, grp = lane >> 3;
+    const int32_t gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
+    QT<EXT> *part = reinterpret_cast<QT<EXT> *>(k.part);
+    for (int32_t l = L0; l >= 0; l--) {
+        QT<EXT> *qo = reinterpret_cast<QT<EXT> *>(k.q[l & 1]);
+        const QT<EXT> *qi = reinterpret_cast<const QT<EXT> *>(k.q[(l + 1) & 1]);
+        const int32_t lo = a.lvl_off[l], hi = a.lvl_off[l + 1];
+        if (l == L0) {   // no successors
+            for (int32_t i = lo + gwarp * 32 + lane; i < hi; i += nwarps * 32) {
+                const int32_t u = a.queue[i];
+                bc_finish_vertex<EXT>(u, (QT<EXT>)0, a.sigma[u], delta, qo, bcacc, src);
+            }
+            if (!mgd::grid_sync(a.bar, a.bar_err, a.bar_never)) return;
+            continue;
         }
+        // one gathered term: the successor's q, scaled to the entry's count
+        auto term = [&](int32_t w, int32_t ku) {
+            QT<EXT> t = qi[w];
+            if (EXT) {
+                const int32_t dk = ku - a.sigma[w].k;
+                if (dk != 0) t *= (QT<EXT>)mgops::pc_scale(dk);
+            }
+            return t;
+        };
+        if (blockIdx.x == 0 && threadIdx.x == 0) k.nitems[(l + 1) & 1] = 0;
+        int32_t *nitems = &k.nitems[l & 1];
+        for (int32_t i0 = lo + gwarp * 4; i0 < hi; i0 += nwarps * 4) {
+            const int32_t i = i0 + grp;
+            int32_t u = 0, b = 0, e = 0;
+            if (i < hi) {
+                u = a.queue[i];
+                b = __ldg(&a.row[u]);
+                e = __ldg(&a.row[u + 1]);
+            }
+            // long entries to the chunk list (their groups' first lanes)
+            const int32_t nc = e - b > BACK_CHUNK && gl == 0 ? (e - b - 1) / BACK_CHUNK + 1 : 0;
+            if (__any_sync(FULL, nc > 0)) {
+                int32_t base = 0;
+                if (nc > 0) base = atomicAdd(nitems, nc);
+                unsigned lm = __ballot_sync(FULL, nc > 0);
+                while (lm) {
+                    const int j = __ffs(lm) - 1;
+                    lm &= lm - 1;
+                    const int32_t uj = __shfl_sync(FULL, u, j), bj = __shfl_sync(FULL, b, j), ej = __shfl_sync(FULL, e, j),
+                                  nj = __shfl_sync(FULL, nc, j), pj = __shfl_sync(FULL, base, j);
+                    for (int32_t c = lane; c < nj; c += 32)
+                        k.item[pj + c] = make_int4(uj, bj + c * BACK_CHUNK, min(ej, bj + (c + 1) * BACK_CHUNK), pj);
+                }
+            }
+            const bool row = i < hi && e - b <= BACK_CHUNK;
+            const mgops::PathCount su = row ? a.sigma[u] : mgops::pc_zero();
+            const int32_t len = row ? e - b : 0;
+            const int32_t rounds = (int32_t)__reduce_max_sync(FULL, (unsigned)((len + 31) >> 5));
+            QT<EXT> acc = 0;
+            for (int32_t r = 0; r < rounds; r++) {
+                QT<EXT> t[4];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = acc;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            QT<EXT> s = 0;
-            for (int w = 0; w < (int)(blockDim.x >> 5); w++) s += s_part[w];
-            bc_finish_vertex<EXT>(v, s, a.sigma, delta, q, bcacc, src);
+                for (int j = 0; j < 4; j++) {
+                    const int32_t p = r * 32 + j * 8 + gl;
+                    t[j] = p < len ? term(__ldcs(&a.col[b + p]), su.k) : (QT<EXT>)0;
+                }
+                acc += (t[0] + t[1]) + (t[2] + t[3]);
+            }
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) acc += __shfl_xor_sync(FULL, acc, o);
+            if (row && gl == 0) bc_finish_vertex<EXT>(u, acc, su, delta, qo, bcacc, src);
         }
-        __syncthreads();
+        if (!mgd::grid_sync(a.bar, a.bar_err, a.bar_never)) return;
+        const int32_t ni = __ldcg(nitems);
+        if (ni == 0) continue;   // (the same for every block: nobody adds to it in this phase)
+        for (int32_t c = gwarp; c < ni; c += nwarps) {
+            const int4 it = __ldcg(&k.item[c]);
+            const mgops::PathCount su = a.sigma[it.x];
+            QT<EXT> t[BACK_CHUNK / 32];
+#pragma unroll
+            for (int j = 0; j < BACK_CHUNK / 32; j++) {
+                const int32_t p = it.y + lane + 32 * j;
+                t[j] = p < it.z ? term(__ldcs(&a.col[p]), su.k) : (QT<EXT>)0;
+            }
+            QT<EXT> acc = ((t[0] + t[1]) + (t[2] + t[3])) + ((t[4] + t[5]) + (t[6] + t[7]));
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(FULL, acc, o);
+            const int32_t n = (__ldg(&a.row[it.x + 1]) - __ldg(&a.row[it.x]) - 1) / BACK_CHUNK + 1;
+            int last = 0;
+            if (lane == 0) {
+                __stcg(&part[c], acc);
+                __threadfence();
+                last = atomicAdd(&k.arrive[it.w], 1) == n - 1;
+            }
+            if (!__shfl_sync(FULL, last, 0)) continue;
+            __threadfence();
+            acc = 0;
+            for (int32_t x = it.w + lane; x < it.w + n; x += 32) acc += __ldcg(&part[x]);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(FULL, acc, o);
+            if (lane == 0) {
+                k.arrive[it.w] = 0;
+                bc_finish_vertex<EXT>(it.x, acc, su, delta, qo, bcacc, src);
+            }
+        }
+        if (!mgd::grid_sync(a.bar, a.bar_err, a.bar_never)) return;
     }
 }
 
@@ -208,10 +220,7 @@ __device__ __forceinline__ void bc_back_entry(const Args &a, int32_t L, int32_t 
                 acc += x[j];
             }
     }
-    const float dv = (float)(su.m * (double)acc);
-    delta[u] = dv;
-    q[u] = (QT<EXT>)((1.0 + (double)dv) / su.m);
-    if (bcacc && u != src) bcacc[u] += dv;
+    bc_finish_vertex<EXT>(u, acc, su, delta, q, bcacc, src);
 }
 
 // the same level over the whole grid: an entry a thread, 32 a warp (a warp
@@ -271,55 +280,29 @@ __device__ __noinline__ void cta_back_levels(const Args &a, int32_t L, int32_t L
     }
 }
 
-// Persistent backward sweep: every level in one cooperative launch, one or
-// two grid barriers per level (light entries | barrier | heavy entries |
-// barrier, the second half only when the level listed heavy entries).  Every block walks L = L0 .. 1 itself; the heavy-entry counter
-// alternates with the level's parity, and block 0 clears the one the next
-// level will use while the current level runs (its last readers finished
-// before the previous barrier).  A barrier timeout sets the error flag; the
-// host reads it and fails the run.
-// Graphs with vertices of 128 edges (HEAVY) keep two blocks per SM: their
-// levels are few and large, and want the warps (R-MAT 22: 2.3 ms against
-// 3.4).
-template <bool EXT, bool HEAVY>
-__global__ void __launch_bounds__(PTHREADS, HEAVY ? 2 : 1) k_bc_back_levels(Args a, BCtl *bc_ctl, QT<EXT> *q, float *delta,
-                                                                float *bcacc, int32_t *heavy_list)
+// Backward sweep of graphs without heavy vertices: every level in one
+// cooperative launch, runs of small levels by block 0.  A barrier timeout
+// sets the error flag; the host reads it and fails the run.
+template <bool EXT>
+__global__ void __launch_bounds__(PTHREADS, 1) k_bc_back_levels(Args a, BCtl *bc_ctl, QT<EXT> *q, float *delta,
+                                                                float *bcacc)
 {
     __shared__ int4 s_b;
-    __shared__ int s_nheavy;
     if (threadIdx.x == 0) s_b = __ldcg(reinterpret_cast<const int4 *>(bc_ctl));
     __syncthreads();
     const int32_t L0 = s_b.x, src = s_b.y;
     for (int32_t L = L0; L >= 1; L--) {
-        if constexpr (!HEAVY) {
-            // a run of small levels is block 0's alone; the offsets are the
-            // same for every block
-            int32_t L1 = L;
-            while (L1 >= 1 && L - L1 < CTA_LEVELS && a.lvl_off[L1] - a.lvl_off[L1 - 1] <= CTA_BACK) L1--;
-            if (L - L1 >= 4) {
-                if (blockIdx.x == 0) cta_back_levels<EXT>(a, L, L1, src, q, delta, bcacc);
-                if (!mgd::grid_sync(a.bar, a.bar_err, a.bar_never)) return;
-                L = L1 + 1;
-                continue;
-            }
-            bc_back_level_flat<EXT>(a, L, src, q, delta, bcacc);
-            if (!mgd::grid_sync(a.bar, a.bar_err, a.bar_never)) return;
-            continue;
+        // a run of small levels is block 0's alone; the offsets are the same
+        // for every block
+        int32_t L1 = L;
+        while (L1 >= 1 && L - L1 < CTA_LEVELS && a.lvl_off[L1] - a.lvl_off[L1 - 1] <= CTA_BACK) L1--;
+        if (L - L1 >= 4) {
+            if (blockIdx.x == 0) cta_back_levels<EXT>(a, L, L1, src, q, delta, bcacc);
+            L = L1 + 1;
         } else {
-            const int par = L & 1;
-            if (blockIdx.x == 0 && threadIdx.x == 0) bc_ctl->hcnt[par ^ 1] = 0;
-            bc_back_level<EXT>(a, L, src, &bc_ctl->hcnt[par], q, delta, bcacc, heavy_list);
-            if (!mgd::grid_sync(a.bar, a.bar_err, a.bar_never)) return;
-            if (threadIdx.x == 0) s_nheavy = __ldcg(&bc_ctl->hcnt[par]);
-            __syncthreads();
-            const int32_t nheavy = s_nheavy;
-            // most levels list no heavy entry: every block sees the same count
-            // and skips the heavy phase and its barrier together (block 0's
-            // early clear of this counter then leaves it at the 0 it holds)
-            if (nheavy == 0) continue;
-            bc_back_heavy_level<EXT>(a, L, src, nheavy, q, delta, bcacc, heavy_list);
-            if (!mgd::grid_sync(a.bar, a.bar_err, a.bar_never)) return;
+            bc_back_level_flat<EXT>(a, L, src, q, delta, bcacc);
         }
+        if (!mgd::grid_sync(a.bar, a.bar_err, a.bar_never)) return;
     }
 }
 
@@ -347,7 +330,7 @@ void free_frontier_ws(mg_graph *g)
     if (!g->fws) return;
     FrontierWS *w = g->fws;
     DevBuf *bufs[] = {&w->label, &w->sigma, &w->sigma_d, &w->bm, &w->visited, &w->queue, &w->heavy,
-                      &w->lvl_off, &w->ctl, &w->q, &w->delta, &w->bc, &w->bctl, &w->bheavy, &w->srcbuf, &w->bar,
+                      &w->lvl_off, &w->ctl, &w->q, &w->delta, &w->bc, &w->bctl, &w->bitem, &w->barrive, &w->bpart, &w->srcbuf, &w->bar,
                       &w->cnt};
     for (DevBuf *b : bufs) dev_free(*b);
     for (auto &kv : w->lg) kv.second.destroy();
@@ -368,35 +351,50 @@ mg_status bc_backward(mg_graph *g, int32_t src, const mg_opts &opt, float *bcacc
 {
     FrontierWS *w = g->fws;
     const size_t n = (size_t)std::max(g->nv, 1);
-    MG_TRY(dev_alloc(w->q, n * 8));
+    Args a = make_args(g);
+    // chunks of the long entries: at most this many a level
+    const size_t items = (size_t)g->ne / BACK_CHUNK + (size_t)g->ne / (BACK_CHUNK + 1) + 2;
+    MG_TRY(dev_alloc(w->q, n * 8 * (a.has_heavy ? 2 : 1)));
     MG_TRY(dev_alloc(w->delta, n * 4));
     MG_TRY(dev_alloc(w->bctl, sizeof(BCtl)));
-    MG_TRY(dev_alloc(w->bheavy, n * 4));
-    Args a = make_args(g);
     cudaStream_t s = g->stream;
     void *q = w->q.p;
     float *delta = w->delta.as<float>();
     BCtl *bc = w->bctl.as<BCtl>();
-    int32_t *hl = w->bheavy.as<int32_t>();
     const int grid = launch_grid(g, THREADS, 8);
-    if (w->coop_back == 0) {
-        int per_sm = 0;
-        int per_sm_x = 0;
-        if (a.has_heavy) {
-            MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bc_back_levels<false, true>, PTHREADS, 0));
-            MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_x, k_bc_back_levels<true, true>, PTHREADS, 0));
-        } else {
-            MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bc_back_levels<false, false>, PTHREADS, 0));
-            MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_x, k_bc_back_levels<true, false>, PTHREADS, 0));
-        }
-        per_sm = std::min(per_sm, per_sm_x);
-        if (per_sm < 1) return fail(MG_ERR_CUDA, "persistent backward kernel does not fit on an SM");
-        w->coop_back = std::min(per_sm, a.has_heavy ? 2 : 1) * g->num_sms;
+    if (!w->coop_back) {
+        int occ[4] = {0, 0, 0, 0};
+        MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[0], k_bc_back_levels<false>, PTHREADS, 0));
+        MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[1], k_bc_back_levels<true>, PTHREADS, 0));
+        MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[2], k_bc_back_heavy<false>, PTHREADS, 0));
+        MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[3], k_bc_back_heavy<true>, PTHREADS, 0));
+        if (std::min(std::min(occ[0], occ[1]), std::min(occ[2], occ[3])) < 1)
+            return fail(MG_ERR_CUDA, "persistent backward kernel does not fit on an SM");
+        w->coop_back = g->num_sms;
     }
-    if (a.bc_ext) k_bc_q_init<true><<<grid, THREADS, 0, s>>>(g->nv, a.sigma, a.label, (double *)q, delta);
-    else k_bc_q_init<false><<<grid, THREADS, 0, s>>>(g->nv, a.sigma, a.label, (float *)q, delta);
     k_bc_back_init<<<1, 32, 0, s>>>(a.ctl, bc, src);
     MG_CUDA(cudaMemsetAsync(w->bar.p, 0, BAR_BYTES, s));
+    BackArgs k;
+    std::memset(&k, 0, sizeof(k));
+    if (a.has_heavy) {
+        MG_TRY(dev_alloc(w->bitem, items * sizeof(int4)));
+        MG_TRY(dev_alloc(w->barrive, items * 4));
+        MG_TRY(dev_alloc(w->bpart, items * 8));
+        const size_t qb = n * (a.bc_ext ? 8 : 4);
+        k.q[0] = q;
+        k.q[1] = (char *)q + qb;
+        k.item = w->bitem.as<int4>();
+        k.arrive = w->barrive.as<int32_t>();
+        k.part = w->bpart.p;
+        k.nitems = bc->hcnt;
+        MG_CUDA(cudaMemsetAsync(q, 0, 2 * qb, s));
+        MG_CUDA(cudaMemsetAsync(delta, 0, n * 4, s));
+        MG_CUDA(cudaMemsetAsync(k.arrive, 0, items * 4, s));
+    } else if (a.bc_ext) {
+        k_bc_q_init<true><<<grid, THREADS, 0, s>>>(g->nv, a.sigma, a.label, (double *)q, delta);
+    } else {
+        k_bc_q_init<false><<<grid, THREADS, 0, s>>>(g->nv, a.sigma, a.label, (float *)q, delta);
+    }
     MG_CUDA(cudaGetLastError());
     // every level in one cooperative launch
     Profiler &P = g->prof;
@@ -411,14 +409,10 @@ mg_status bc_backward(mg_graph *g, int32_t src, const mg_opts &opt, float *bcacc
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     P.begin(sb);
-    if (a.bc_ext && a.has_heavy)
-        MG_CUDA(cudaLaunchKernelEx(&cfg, k_bc_back_levels<true, true>, a, bc, (double *)q, delta, bcacc, hl));
-    else if (a.bc_ext)
-        MG_CUDA(cudaLaunchKernelEx(&cfg, k_bc_back_levels<true, false>, a, bc, (double *)q, delta, bcacc, hl));
-    else if (a.has_heavy)
-        MG_CUDA(cudaLaunchKernelEx(&cfg, k_bc_back_levels<false, true>, a, bc, (float *)q, delta, bcacc, hl));
-    else
-        MG_CUDA(cudaLaunchKernelEx(&cfg, k_bc_back_levels<false, false>, a, bc, (float *)q, delta, bcacc, hl));
+    if (a.has_heavy && a.bc_ext) MG_CUDA(cudaLaunchKernelEx(&cfg, k_bc_back_heavy<true>, a, bc, k, delta, bcacc));
+    else if (a.has_heavy) MG_CUDA(cudaLaunchKernelEx(&cfg, k_bc_back_heavy<false>, a, bc, k, delta, bcacc));
+    else if (a.bc_ext) MG_CUDA(cudaLaunchKernelEx(&cfg, k_bc_back_levels<true>, a, bc, (double *)q, delta, bcacc));
+    else MG_CUDA(cudaLaunchKernelEx(&cfg, k_bc_back_levels<false>, a, bc, (float *)q, delta, bcacc));
     P.end();
     int err = 0;
     MG_CUDA(cudaMemcpyAsync(&err, a.bar_err, 4, cudaMemcpyDeviceToHost, s));

@@ -1168,7 +1168,7 @@ const char OpTag<Op>::id = 0;
 // ----------------------------------------------------------------------------
 struct FrontierWS {
     mgi::DevBuf label, sigma, sigma_d, bm, visited, queue, heavy, lvl_off, ctl;
-    mgi::DevBuf q, delta, bc, bctl, bheavy, srcbuf;
+    mgi::DevBuf q, delta, bc, bctl, bitem, barrive, bpart, srcbuf;
     mgi::DevBuf bar;        // grid barrier words + error flag of the persistent kernels
     mgi::DevBuf cnt;        // LevelCnt[4] of the persistent push phase
     std::map<const void *, int> coop_grid;      // resident blocks of k_sparse_levels<Op>, by operator tag

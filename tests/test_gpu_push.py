@@ -41,3 +41,33 @@ def test_many_sources_of_a_batch():
     for i, h in enumerate(hs):
         assert np.array_equal(levels[i], O.bfs(O.csr_from_arrays(*h.arrays()), i % h.nv)), i
     b.free()
+
+
+@pytest.mark.parametrize("deg", [129, 255, 256, 257, 512, 513, 4097, 40000])
+@pytest.mark.parametrize("flags", [mg.LOAD_SYM, mg.LOAD_NSYM], ids=["symmetric", "directed"])
+def test_bc_long_entries(deg, flags):
+    # BC over entries around the backward sweep's chunk bound: a hub over
+    # `deg` middle vertices that reach `deg` // 2 + 1 ends by two edges each,
+    # and a second, smaller hub on the way
+    mid = 1 + np.arange(deg)
+    end = 1 + deg + np.arange(deg // 2 + 1)
+    hub2 = 1 + deg + len(end)
+    some = end[:300]
+    src = np.concatenate([np.zeros(deg, np.int64), mid, mid, [0], np.full(len(some), hub2)])
+    dst = np.concatenate([mid, end[(mid - 1) // 2], end[mid % len(end)], [hub2], some])
+    h = mg.HostGraph.from_entries(hub2 + 1, src, dst, flags=flags)
+    rp, col, _ = h.arrays()
+    og = O.csr_from_arrays(*h.arrays())
+    g = mg.Graph(h)
+    for s in (0, 1, og.nv - 1):
+        (lv, sg, dl), _ = g.bc(s)
+        want = O.bc_f64(og, s)
+        assert np.array_equal(lv, want[0]) and np.array_equal(sg, want[1])
+        u = np.repeat(np.arange(og.nv), np.diff(rp))
+        ref = np.zeros(og.nv)
+        for at in range(int(lv[lv < 0x64646464].max()) - 1, -1, -1):
+            e = (lv[u] == at) & (lv[col] == at + 1)
+            np.add.at(ref, u[e], sg[u[e]] * (1.0 + ref[col[e]]) / sg[col[e]])
+        assert np.max(np.abs(dl - ref)) <= 1e-5 * max(1.0, np.max(np.abs(ref)))
+    g.free()
+    h.free()
