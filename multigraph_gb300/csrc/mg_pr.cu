@@ -21,7 +21,8 @@
 //               default to 32 / 512 / 2048, mg_autotune re-picks them);
 //   k_pr_apply  heavy rows summed chunk by chunk in order (thread per row),
 //               then the last block to finish sums every block's residual
-//               partials in slot order: convergence test, loop condition.
+//               partials in slot order: convergence test, loop condition
+//               (without heavy rows k_pr_light closes the sweep itself).
 // Sums are therefore deterministic (fixed order) run to run.
 // Algorithmic bytes per sweep: 4m (column ids) + 4(n+1) (offsets) + 12n
 // (old value read, new value and contribution written); in the gather
@@ -124,8 +125,7 @@ constexpr int SPARSE_ALPHA = 16;  // queue sweeps once active in-edges < m / SPA
 
 // ---------------------------------------------------------------------------
 // PageRank operators: the engine (k_pr_light / k_pr_apply / k_prd_*, k_pr_all)
-// is a template over one of these.  Row state that another block may have
-// written earlier in the same launch (k_pr_all) is read through L2.  Hooks:
+// is a template over one of these.  Hooks:
 //   apply(a, c, v, s, any, dang)  row v's update from its gathered sum s:
 //                                 writes the next iterate and contribution,
 //                                 returns |change|, sets any when the row
@@ -186,7 +186,7 @@ struct PrTopology {
                                                   float &dang)
     {
         const int cur = c.cur, nxt = cur ^ 1;
-        const float xo = __ldcg(&a.x[cur][v]);
+        const float xo = a.x[cur][v];
         const int32_t od = a.outrow[v + 1] - a.outrow[v];
         const float xn = c.base + c.damping * s;
         a.x[nxt][v] = xn;
@@ -230,7 +230,7 @@ struct PrWeighted {
                                                   float &dang)
     {
         const int cur = c.cur, nxt = cur ^ 1;
-        const float xo = __ldcg(&a.x[cur][v]);
+        const float xo = a.x[cur][v];
         const float xn = c.base + c.damping * s;
         a.x[nxt][v] = xn;
         const float Su = a.S[v];
@@ -252,7 +252,7 @@ struct PrAdjoint {
         const float Su = a.S[v];
         const float t = Su > 0.0f ? s / Su : c.lam_meanf;
         const float xn = a.gvec[v] + c.damping * t;
-        const float xo = __ldcg(&a.c[cur][v]);
+        const float xo = a.c[cur][v];
         a.c[nxt][v] = xn;
         dang = xn;  // sum of lambda for the mean
         return fabsf(xn - xo);
@@ -385,65 +385,6 @@ struct PrRowOp {
     }
 };
 
-template <class Op>
-__global__ void __launch_bounds__(THREADS) k_pr_light(PArgs a)
-{
-    // lets k_pr_apply (launched with programmatic dependent launch) be
-    // scheduled while this sweep runs; it waits for the sweep's completion
-    mgd::pdl_enter();
-    const PCtl c = *a.ctl;
-    if (c.more == 0 || c.sparse) return;
-    const int lane = mgd::lane();
-    const int gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int nwarps = (gridDim.x * blockDim.x) >> 5;
-    PrRowOp<Op> op{a, c};
-    (void)lane;
-    (void)gwarp;
-    (void)nwarps;
-    const int32_t *pwt = reinterpret_cast<const int32_t *>(a.pw);
-    mgd::bins_reduce(op, a.prow, a.pcol, pwt, a.wrows, a.nwrows, a.nwlong, a.trows, a.ntrows);
-    // heavy-row chunks, one per CTA, in batches of 8 * THREADS edges: each
-    // thread issues its 8 column loads, then its 8 gathers (one batch for
-    // the default 2048-edge chunks)
-    __shared__ float s_part[THREADS / 32];
-    for (int32_t ch = blockIdx.x; ch < a.nhchunks; ch += gridDim.x) {
-        int32_t v = a.hchunk[3 * ch], b = a.hchunk[3 * ch + 1], e = a.hchunk[3 * ch + 2];
-        if (a.P) {
-            // the same piece of the row's tail part: piece k of the full
-            // row covers tail positions [k * chunk, (k + 1) * chunk)
-            const int32_t k = (b - a.prow_full[v]) / a.chunk;
-            const int32_t tb = a.prow[v], te = a.prow[v + 1];
-            b = min(te, tb + k * a.chunk);
-            e = min(te, b + a.chunk);
-        }
-        float acc = 0.0f;
-        if (!pr_row_skipped<Op>(a, v)) {
-            for (int32_t b0 = b; b0 < e; b0 += 8 * THREADS) {
-                int32_t u[8];
-#pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    int32_t p = b0 + threadIdx.x + j * THREADS;
-                    u[j] = p < e ? __ldcs(&a.pcol[p]) : -1;  // streamed once: evict-first
-                }
-#pragma unroll
-                for (int j = 0; j < 8; j++)
-                    if (u[j] >= 0) acc += pr_gather<Op>(a, c.cur, b0 + threadIdx.x + j * THREADS, u[j]);
-            }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = acc;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            float s = 0.0f;
-            for (int w = 0; w < THREADS / 32; w++) s += s_part[w];
-            a.hpart[ch] = s;
-        }
-        __syncthreads();
-    }
-    block_partials<Op::kDataDriven>(a, blockIdx.x, op.resid, op.dangs, op.any, op.act, op.dfz);
-}
-
 // Sum of the partials of slots [s0, s1): lane-strided in slot order, then a
 // fixed shuffle tree and warp order (thread 0 gets T[0..3] and A).
 __device__ __forceinline__ void reduce_slots(const double *bpart, int s0, int s1, double T[NPART - 1], int &A)
@@ -553,6 +494,87 @@ __device__ __forceinline__ void close_sweep(const PArgs &a, const PCtl &c, int n
         }
         if (use_cond) cudaGraphSetConditional(h, more ? 1u : 0u);
     }
+}
+
+template <class Op>
+__global__ void __launch_bounds__(THREADS) k_pr_light(PArgs a)
+{
+    // lets k_pr_apply (launched with programmatic dependent launch) be
+    // scheduled while this sweep runs; it waits for the sweep's completion
+    mgd::pdl_enter();
+    const PCtl c = *a.ctl;
+    if (c.more == 0 || c.sparse) return;
+    const int lane = mgd::lane();
+    const int gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int nwarps = (gridDim.x * blockDim.x) >> 5;
+    PrRowOp<Op> op{a, c};
+    (void)lane;
+    (void)gwarp;
+    (void)nwarps;
+    const int32_t *pwt = reinterpret_cast<const int32_t *>(a.pw);
+    mgd::bins_reduce(op, a.prow, a.pcol, pwt, a.wrows, a.nwrows, a.nwlong, a.trows, a.ntrows);
+    // heavy-row chunks, one per CTA, in batches of 8 * THREADS edges: each
+    // thread issues its 8 column loads, then its 8 gathers (one batch for
+    // the default 2048-edge chunks)
+    __shared__ float s_part[THREADS / 32];
+    for (int32_t ch = blockIdx.x; ch < a.nhchunks; ch += gridDim.x) {
+        int32_t v = a.hchunk[3 * ch], b = a.hchunk[3 * ch + 1], e = a.hchunk[3 * ch + 2];
+        if (a.P) {
+            // the same piece of the row's tail part: piece k of the full
+            // row covers tail positions [k * chunk, (k + 1) * chunk)
+            const int32_t k = (b - a.prow_full[v]) / a.chunk;
+            const int32_t tb = a.prow[v], te = a.prow[v + 1];
+            b = min(te, tb + k * a.chunk);
+            e = min(te, b + a.chunk);
+        }
+        float acc = 0.0f;
+        if (!pr_row_skipped<Op>(a, v)) {
+            for (int32_t b0 = b; b0 < e; b0 += 8 * THREADS) {
+                int32_t u[8];
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    int32_t p = b0 + threadIdx.x + j * THREADS;
+                    u[j] = p < e ? __ldcs(&a.pcol[p]) : -1;  // streamed once: evict-first
+                }
+#pragma unroll
+                for (int j = 0; j < 8; j++)
+                    if (u[j] >= 0) acc += pr_gather<Op>(a, c.cur, b0 + threadIdx.x + j * THREADS, u[j]);
+            }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = acc;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            float s = 0.0f;
+            for (int w = 0; w < THREADS / 32; w++) s += s_part[w];
+            a.hpart[ch] = s;
+        }
+        __syncthreads();
+    }
+    block_partials<Op::kDataDriven>(a, blockIdx.x, op.resid, op.dangs, op.any, op.act, op.dfz);
+}
+
+// The whole sweep of a graph without heavy rows (and no segmented part): the
+// last block to finish closes it, so there is no k_pr_apply with nothing to
+// do (1000 x 1000 lattice, weighted: 31 -> 24 us a sweep).  With heavy rows,
+// letting the last of a row's chunks finish it costs more than the apply
+// kernel: a fence and an atomic a chunk took the weighted R-MAT 19 sweep from
+// 71 to 86 us.
+template <class Op>
+__global__ void __launch_bounds__(THREADS, 8) k_pr_light_close(PArgs a, cudaGraphConditionalHandle h, int use_cond)
+{
+    const PCtl c = *a.ctl;
+    if (c.more == 0) {
+        if (blockIdx.x == 0 && threadIdx.x == 0 && use_cond) cudaGraphSetConditional(h, 0u);
+        return;
+    }
+    if (c.sparse) return;
+    PrRowOp<Op> op{a, c};
+    mgd::bins_reduce(op, a.prow, a.pcol, reinterpret_cast<const int32_t *>(a.pw), a.wrows, a.nwrows, a.nwlong, a.trows,
+                     a.ntrows);
+    block_partials<Op::kDataDriven>(a, blockIdx.x, op.resid, op.dangs, op.any, op.act, op.dfz);
+    close_sweep<Op>(a, c, gridDim.x, h, use_cond);
 }
 
 // Row finish when every in-edge sits in a segment (no tail, no heavy-row
@@ -718,10 +740,10 @@ __global__ void __launch_bounds__(THREADS) k_pr_apply(PArgs a, cudaGraphConditio
 // straight from L2 took the R-MAT 16 sweep from 18 to 48 us.  Sums are
 // compensated as in the segmented layout.  After the barrier every block
 // adds up the 152 blocks' partial sums itself and comes to the same
-// decision.  Only for forms that are continuous in the sums' rounding
-// (normalised, weighted, adjoint): the data-driven form freezes and PR_T
-// holds a row by comparing its change with a threshold, where one last bit
-// can decide.  R-MAT 16: 30 -> 18 us per sweep, 320 x 311 lattice 18 -> 7 us.
+// decision.  Only for the normalised form: the data-driven form freezes and
+// PR_T holds a row by comparing its change with a threshold, where one last
+// bit can decide, and the weighted forms' order of additions shows in the
+// gradient (k_row_sums).  R-MAT 16: 30 -> 18 us per sweep, 320 x 311 lattice 18 -> 7 us.
 // ---------------------------------------------------------------------------
 constexpr int ALL_THREADS = 1024;
 constexpr int32_t ALL_CHUNK = 256;
@@ -745,14 +767,14 @@ struct PrAllArgs {
     int *bar_err;
     int bar_never;
     const int32_t *old2new; // null: engine ids are the caller's
-    float *out;             // result in caller order (null: left in x[cur] / c[cur])
+    float *out;             // result in caller order (null: left in x[cur])
     float x0;
 };
 
 template <class Op>
 __global__ void __launch_bounds__(ALL_THREADS, 1) k_pr_all(PArgs a, PrAllArgs z)
 {
-    static_assert(!Op::kDataDriven, "rows are never skipped here");
+    static_assert(!Op::kDataDriven && !Op::kWeights && !Op::kAdjoint, "the normalised form");
     constexpr unsigned FULL = 0xffffffffu;
     constexpr int NW = ALL_THREADS / 32;
     __shared__ PCtl s_c;
@@ -760,7 +782,6 @@ __global__ void __launch_bounds__(ALL_THREADS, 1) k_pr_all(PArgs a, PrAllArgs z)
     __shared__ int s_a[NW];
     const int lane = mgd::lane(), warp = threadIdx.x >> 5, gl = lane & 7, grp = lane >> 3;
     const int gwarp = blockIdx.x * NW + warp, nwarps = gridDim.x * NW;
-    const int32_t *pw = reinterpret_cast<const int32_t *>(a.pw);
     if (threadIdx.x == 0) s_c = *a.ctl;
     for (int32_t v = blockIdx.x * ALL_THREADS + threadIdx.x; v < a.n; v += gridDim.x * ALL_THREADS)
         pr_init_row<Op>(a, v, z.x0);
@@ -776,7 +797,6 @@ __global__ void __launch_bounds__(ALL_THREADS, 1) k_pr_all(PArgs a, PrAllArgs z)
             for (int j = 0; j < ALL_CHUNK / 32; j++) {
                 const int32_t p = b + lane + 32 * j;
                 t[j] = p < e ? cc[__ldg(&a.pcol[p])] : 0.0f;
-                if (Op::kWeights && p < e) t[j] *= __int_as_float(__ldg(&pw[p]));
             }
 #pragma unroll
             for (int j = 0; j < ALL_CHUNK / 32; j++) mgd::kahan_add(s, r, t[j]);
@@ -812,7 +832,6 @@ __global__ void __launch_bounds__(ALL_THREADS, 1) k_pr_all(PArgs a, PrAllArgs z)
                 for (int j = 0; j < 4; j++) {
                     const int32_t i = k * 32 + j * 8 + gl;
                     t[j] = i < len ? cc[__ldg(&a.pcol[b + i])] : 0.0f;
-                    if (Op::kWeights && i < len) t[j] *= __int_as_float(__ldg(&pw[b + i]));
                 }
 #pragma unroll
                 for (int j = 0; j < 4; j++) mgd::kahan_add(s, r, t[j]);
@@ -831,10 +850,7 @@ __global__ void __launch_bounds__(ALL_THREADS, 1) k_pr_all(PArgs a, PrAllArgs z)
             for (int32_t k = 0; k < len; k += 4) {
                 float t[4];
 #pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    t[j] = k + j < len ? cc[__ldg(&a.pcol[wb + k + j])] : 0.0f;
-                    if (Op::kWeights && k + j < len) t[j] *= __int_as_float(__ldg(&pw[wb + k + j]));
-                }
+                for (int j = 0; j < 4; j++) t[j] = k + j < len ? cc[__ldg(&a.pcol[wb + k + j])] : 0.0f;
 #pragma unroll
                 for (int j = 0; j < 4; j++) mgd::kahan_add(s, r, t[j]);
             }
@@ -891,13 +907,8 @@ __global__ void __launch_bounds__(ALL_THREADS, 1) k_pr_all(PArgs a, PrAllArgs z)
                 s_c.cur ^= 1;
                 s_c.resid = R;
                 s_c.any = any;
-                if (Op::kAdjoint) {
-                    s_c.lam_mean = D / a.n;
-                    s_c.lam_meanf = (float)s_c.lam_mean;
-                } else {
-                    s_c.dangling = D;
-                    s_c.base = (float)(base0 + basek * D);
-                }
+                s_c.dangling = D;
+                s_c.base = (float)(base0 + basek * D);
                 int more = Op::more(any, R, s_c.tol) ? 1 : 0;
                 if (more && s_c.iter >= s_c.max_iter) {
                     s_c.status = 1;
@@ -909,7 +920,7 @@ __global__ void __launch_bounds__(ALL_THREADS, 1) k_pr_all(PArgs a, PrAllArgs z)
         __syncthreads();
     }
     if (z.out && ok) {
-        const float *x = Op::kAdjoint ? a.c[s_c.cur] : a.x[s_c.cur];
+        const float *x = a.x[s_c.cur];
         for (int32_t i = blockIdx.x * ALL_THREADS + threadIdx.x; i < a.n; i += gridDim.x * ALL_THREADS)
             z.out[i] = __ldcg(&x[z.old2new ? __ldg(&z.old2new[i]) : i]);
     }
@@ -1122,84 +1133,176 @@ __global__ void k_adjoint_ctl_init(PCtl *c, int32_t n, int32_t max_iter, float d
     pctl_derive(c);
 }
 
-// Row totals over the degree bins of the pull rows (the graph is symmetric,
-// so they are the out-rows too) and CTA-sized chunks of the heavy rows, whose
-// partials k_row_total_heavy adds in order.  RowWeights: S[u] = sum_e w[e];
-// RowBack: the adjoint's row value t_u = sum_e w[e] lam[v] / S[u] and the
-// factor d x_u / S_u of its edges, ct[u] = (factor, t_u).  (A thread per row
-// for S kept one thread on a hub row: 1.3 ms on R-MAT 19; 30 us now.)
-struct RowWeights {
-    using T = float;
-    static constexpr bool kRowAware = false, kWeights = true;
-    float *S;
-    __device__ T identity() const { return 0.0f; }
-    __device__ bool skip(int32_t) const { return false; }
-    __device__ T edge(int32_t, int32_t, int32_t, int32_t w) const { return __int_as_float(w); }
-    __device__ T combine(T x, T y) const { return x + y; }
-    __device__ void flush() {}
-    __device__ void finish(int32_t u, T s) { S[u] = s; }
-};
-
-struct RowBack {
-    using T = float;
-    static constexpr bool kRowAware = false, kWeights = true;
-    const float *S, *x, *lam;
-    float damping;
-    float2 *ct;
-    __device__ T identity() const { return 0.0f; }
-    __device__ bool skip(int32_t) const { return false; }
-    __device__ T edge(int32_t, int32_t, int32_t v, int32_t w) const { return __int_as_float(w) * lam[v]; }
-    __device__ T combine(T x, T y) const { return x + y; }
-    __device__ void flush() {}
-    __device__ void finish(int32_t u, T s)
-    {
-        const float Su = S[u];
-        ct[u] = Su > 0.0f ? make_float2(damping * x[u] / Su, s / Su) : make_float2(0.0f, 0.0f);
-    }
-};
-
-template <class Op>
-__global__ void __launch_bounds__(THREADS) k_row_total(PArgs a, Op op)
+// Row totals of the weighted forms.  The order of their additions is part of
+// the result: an edge of a vertex with one or two light edges has a gradient
+// near zero that is a difference of nearly equal numbers times 1 / w, so the
+// last bit of S or of a row total shows there.  Rows of the thread bin take a
+// thread (S) or eight lanes / a warp (totals), the others a warp each, longest
+// bin first, loads well ahead of the additions.
+//
+// S[u] = w[b] + w[b + 1] + .. one after another.  Heavy rows: a block loads
+// the next 2,048 weights into shared memory while its first warp adds the
+// last ones from there, four a load, about four cycles an addition (one
+// thread loading and adding took 1.3 ms for a hub row of R-MAT 19, and a warp
+// shuffling them one by one 0.25).
+__global__ void __launch_bounds__(THREADS) k_row_sums(PArgs a, const float *__restrict__ w, float *S)
 {
-    const int32_t *pwt = reinterpret_cast<const int32_t *>(a.pw);
-    mgd::bins_reduce(op, a.prow, a.pcol, pwt, a.wrows, a.nwrows, a.nwlong, a.trows, a.ntrows);
-    __shared__ float s_part[THREADS / 32];
-    for (int32_t ch = blockIdx.x; ch < a.nhchunks; ch += gridDim.x) {
-        const int32_t u = a.hchunk[3 * ch], b = a.hchunk[3 * ch + 1], e = a.hchunk[3 * ch + 2];
-        float acc = 0.0f;
-        for (int32_t p = b + threadIdx.x; p < e; p += THREADS)
-            acc += op.edge(p, u, __ldcs(&a.pcol[p]), __ldcs(&pwt[p]));
+    constexpr unsigned FULL = 0xffffffffu;
+    constexpr int BATCH = 8 * THREADS;
+    __shared__ __align__(16) float s_w[2][BATCH];
+    const int lane = mgd::lane();
+    const int gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
+    for (int32_t i = blockIdx.x; i < a.nhrows; i += gridDim.x) {
+        const int32_t u = a.hrows[i], b = a.outrow[u], e = a.outrow[u + 1];
+        float s = 0.0f, x[8];
+        auto load = [&](int64_t p0) {
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (mgd::lane() == 0) s_part[threadIdx.x >> 5] = acc;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            float s = 0.0f;
-            for (int w = 0; w < THREADS / 32; w++) s += s_part[w];
-            a.hpart[ch] = s;
+            for (int j = 0; j < 8; j++) {
+                const int64_t p = p0 + threadIdx.x + j * THREADS;
+                x[j] = p < e ? __ldcs(&w[p]) : 0.0f;   // (adding +0 changes nothing)
+            }
+        };
+        load(b);
+        int buf = 0;
+        for (int64_t p0 = b; p0 < e; p0 += BATCH, buf ^= 1) {
+#pragma unroll
+            for (int j = 0; j < 8; j++) s_w[buf][threadIdx.x + j * THREADS] = x[j];
+            __syncthreads();
+            load(p0 + BATCH);
+            if (threadIdx.x < 32) {
+                const float4 *q = reinterpret_cast<const float4 *>(s_w[buf]);
+                const int n4 = (int)(min((int64_t)BATCH, e - p0) + 3) >> 2;
+                for (int k = 0; k < n4; k += 8) {   // (BATCH is a multiple of 32; past the row lie zeros)
+                    float4 f[8];
+#pragma unroll
+                    for (int j = 0; j < 8; j++) f[j] = q[k + j];
+#pragma unroll
+                    for (int j = 0; j < 8; j++) {
+                        s += f[j].x;
+                        s += f[j].y;
+                        s += f[j].z;
+                        s += f[j].w;
+                    }
+                }
+            }
         }
-        __syncthreads();
+        if (threadIdx.x == 0) S[u] = s;
+        __syncthreads();   // the buffers are reused
     }
-}
-
-template <class Op>
-__global__ void __launch_bounds__(THREADS) k_row_total_heavy(PArgs a, Op op)
-{
-    for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < a.nhrows; i += gridDim.x * blockDim.x) {
+    for (int32_t i = gwarp; i < a.nwrows; i += nwarps) {
+        const int32_t u = a.wrows[i], b = a.outrow[u], e = a.outrow[u + 1];
         float s = 0.0f;
-        for (int32_t k = a.hrow_chunk[i]; k < a.hrow_chunk[i + 1]; k++) s += a.hpart[k];
-        op.finish(a.hrows[i], s);
+        float x = b + lane < e ? __ldcs(&w[b + lane]) : 0.0f;
+        for (int32_t p = b; p < e; p += 32) {
+            const int64_t q = (int64_t)p + 32 + lane;
+            const float y = q < e ? __ldcs(&w[q]) : 0.0f;
+#pragma unroll
+            for (int k0 = 0; k0 < 32; k0 += 8) {
+                float f[8];
+#pragma unroll
+                for (int k = 0; k < 8; k++) f[k] = __shfl_sync(FULL, x, k0 + k);
+#pragma unroll
+                for (int k = 0; k < 8; k++) s += f[k];
+            }
+            x = y;
+        }
+        if (lane == 0) S[u] = s;
+    }
+    for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < a.ntrows; i += gridDim.x * blockDim.x) {
+        const int32_t u = a.trows[i], b = a.outrow[u], e = a.outrow[u + 1];
+        float s = 0.0f;
+        for (int32_t p = b; p < e; p += 8) {
+            float x[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++) x[k] = p + k < e ? __ldg(&w[p + k]) : 0.0f;
+#pragma unroll
+            for (int k = 0; k < 8; k++) s += x[k];
+        }
+        S[u] = s;
     }
 }
 
-template <class Op>
-mg_status row_totals(const mg_graph *g, const PArgs &a, const Op &op)
+// The adjoint's row value t_u = sum_e w[e] lam[v] / S[u] and the factor
+// d x_u / S_u of its edges, ct[u] = (factor, t_u): lane k of a warp adds edges
+// k, k + 32, .. in order, then an xor tree (of eight lanes for rows of up to
+// eight edges: the others' terms are zero).  Heavy rows: a block loads, its
+// first warp adds.
+__global__ void __launch_bounds__(THREADS) k_back_rows(PArgs a, const float *__restrict__ w, const float *__restrict__ S,
+                                                       const float *__restrict__ x, const float *__restrict__ lam,
+                                                       float damping, float2 *ct)
 {
-    k_row_total<Op><<<a.nblocks, THREADS, 0, g->stream>>>(a, op);
-    if (a.nhrows > 0)
-        k_row_total_heavy<Op><<<(a.nhrows + THREADS - 1) / THREADS, THREADS, 0, g->stream>>>(a, op);
-    MG_CUDA(cudaGetLastError());
-    return MG_OK;
+    constexpr unsigned FULL = 0xffffffffu;
+    const int lane = mgd::lane(), gl = lane & 7, grp = lane >> 3;
+    const int gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
+    auto finish = [&](int32_t u, float t) {
+        const float Su = S[u];
+        ct[u] = make_float2(Su > 0.0f ? damping * x[u] / Su : 0.0f, Su > 0.0f ? t / Su : 0.0f);
+    };
+    auto warp_row = [&](int32_t u) {
+        const int32_t b = a.outrow[u], e = a.outrow[u + 1];
+        float t = 0.0f;
+        int32_t p = b + lane;
+        for (; p + 224 < e; p += 256) {
+            float f[8], g[8];
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                f[j] = __ldcs(&w[p + 32 * j]);
+                g[j] = __ldg(&lam[__ldcs(&a.pcol[p + 32 * j])]);
+            }
+#pragma unroll
+            for (int j = 0; j < 8; j++) t = fmaf(f[j], g[j], t);
+        }
+        for (; p < e; p += 32) t = fmaf(__ldcs(&w[p]), __ldg(&lam[__ldcs(&a.pcol[p])]), t);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(FULL, t, o);
+        if (lane == 0) finish(u, t);
+    };
+    constexpr int BATCH = 8 * THREADS;
+    __shared__ float2 s_term[BATCH];
+    for (int32_t i = blockIdx.x; i < a.nhrows; i += gridDim.x) {
+        const int32_t u = a.hrows[i], b = a.outrow[u], e = a.outrow[u + 1];
+        float t = 0.0f;
+        for (int64_t p0 = b; p0 < e; p0 += BATCH) {
+            float2 x[8];
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                const int64_t p = p0 + threadIdx.x + j * THREADS;
+                x[j] = make_float2(0.0f, 0.0f);
+                if (p < e) x[j] = make_float2(__ldcs(&w[p]), __ldg(&lam[__ldcs(&a.pcol[p])]));
+            }
+            __syncthreads();   // the last batch has been added up
+#pragma unroll
+            for (int j = 0; j < 8; j++) s_term[threadIdx.x + j * THREADS] = x[j];
+            __syncthreads();
+            if (threadIdx.x < 32) {
+                const int n = (int)min((int64_t)BATCH, e - p0);
+#pragma unroll 8
+                for (int k = lane; k < n; k += 32) t = fmaf(s_term[k].x, s_term[k].y, t);
+            }
+        }
+        if (threadIdx.x < 32) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(FULL, t, o);
+            if (lane == 0) finish(u, t);
+        }
+    }
+    for (int32_t i = gwarp; i < a.nwrows; i += nwarps) warp_row(a.wrows[i]);
+    for (int32_t i0 = gwarp * 4; i0 < a.ntrows; i0 += nwarps * 4) {
+        const int32_t i = i0 + grp;
+        const int32_t u = i < a.ntrows ? a.trows[i] : -1;
+        const int32_t b = u >= 0 ? a.outrow[u] : 0, e = u >= 0 ? a.outrow[u + 1] : 0;
+        if (__any_sync(FULL, e - b > 8)) {
+            for (int k = 0; k < 4; k++) {
+                const int32_t uk = __shfl_sync(FULL, u, 8 * k);
+                if (uk >= 0) warp_row(uk);
+            }
+            continue;
+        }
+        float t = b + gl < e ? fmaf(__ldg(&w[b + gl]), __ldg(&lam[__ldg(&a.pcol[b + gl])]), 0.0f) : 0.0f;
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(FULL, t, o);
+        if (u >= 0 && gl == 0) finish(u, t);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1643,6 +1746,9 @@ static mg_status pr_loop(mg_graph *g, PArgs &a, const mg_opts &opt, const char *
             // every row finishes in k_pr_seg, which also closes the sweep
             k_pr_seg<Op><<<grid, THREADS, 0, st>>>(a, h, use_cond);
             P.end();
+        } else if (!a.P && a.nhchunks == 0) {
+            k_pr_light_close<Op><<<grid, THREADS, 0, st>>>(a, h, use_cond);
+            P.end();
         } else {
             k_pr_light<Op><<<grid, THREADS, 0, st>>>(a);
             P.end();
@@ -1936,12 +2042,7 @@ mg_status mg_wpagerank(mg_graph *g, const mg_opts *o, float *x_out, mg_run_info 
     MG_TRY(dev_alloc(w->xkeep, n * 4));
     if (w->wT_version != g->fw_version) {
         // out-weight sums and transposed weights, once per set of weights
-        a.prow = g->row.as<int32_t>();
-        a.pcol = g->col.as<int32_t>();
-        a.pw = g->fw.as<float>();
-        MG_TRY(row_totals(g, a, RowWeights{a.S}));
-        a.prow = g->trow;
-        a.pcol = g->tcol;
+        k_row_sums<<<grid, THREADS, 0, s>>>(a, g->fw.as<float>(), a.S);
         const int egrid = launch_grid(g, THREADS, 16);
         if (w->tpos_version != g->col_version) {
             // the reverse positions are found in the caller's CSR (ascending
@@ -1982,12 +2083,8 @@ mg_status mg_wpagerank(mg_graph *g, const mg_opts *o, float *x_out, mg_run_info 
     float x0 = g->nv > 0 ? 1.0f / g->nv : 0.0f;
     k_pr_ctl_init<<<1, 32, 0, s>>>(a.ctl, g->nv, max_iter, d, tol, g->nv ? (double)g->n_dangling / g->nv : 0.0, 0.0);
     int cur = 0;
-    if (pr_small(g, opt, false)) {
-        MG_TRY(pr_all<PrWeighted>(g, a, opt, x0, nullptr, info, &cur));
-    } else {
-        k_pr_init<PrWeighted><<<grid, THREADS, 0, s>>>(a, x0);
-        MG_TRY(pr_loop<PrWeighted>(g, a, opt, "wpr_pull", info, &cur));
-    }
+    k_pr_init<PrWeighted><<<grid, THREADS, 0, s>>>(a, x0);
+    MG_TRY(pr_loop<PrWeighted>(g, a, opt, "wpr_pull", info, &cur));
     MG_CUDA(cudaMemcpyAsync(w->xkeep.p, a.x[cur], (size_t)g->nv * 4, cudaMemcpyDeviceToDevice, s));
     MG_TRY(to_caller(g, MG_RES_RANK, w->xkeep.p, 4, 1, &g->res[MG_RES_RANK]));
     MG_TRY(end_run(g, opt, info));
@@ -2020,7 +2117,7 @@ mg_status mg_wpagerank_backward(mg_graph *g, const float *g_host, const mg_opts 
     a.pcol = g->col.as<int32_t>();
     a.pw = g->fw.as<float>();
     a.gvec = w->gvec.as<float>();
-    MG_TRY(row_totals(g, a, RowWeights{a.S}));
+    k_row_sums<<<grid, THREADS, 0, s>>>(a, g->fw.as<float>(), a.S);
     float d = opt.damping > 0 ? opt.damping : 0.85f;
     float tol = opt.tol > 0 ? opt.tol : 1e-6f;
     int max_iter = opt.max_iter > 0 ? opt.max_iter : 10000;
@@ -2028,17 +2125,14 @@ mg_status mg_wpagerank_backward(mg_graph *g, const float *g_host, const mg_opts 
     k_gvec_sums<<<g->num_sms, THREADS, 0, s>>>(g->nv, w->gvec_caller.as<float>(), gsum);
     k_adjoint_ctl_init<<<1, 32, 0, s>>>(a.ctl, g->nv, max_iter, d, tol, gsum, g->num_sms);
     int cur = 0;
-    if (pr_small(g, opt, false)) {
-        MG_TRY(pr_all<PrAdjoint>(g, a, opt, 0.0f, nullptr, info, &cur));
-    } else {
-        k_pr_init<PrAdjoint><<<grid, THREADS, 0, s>>>(a, 0.0f);
-        MG_TRY(pr_loop<PrAdjoint>(g, a, opt, "wpr_adjoint", info, &cur));
-    }
+    k_pr_init<PrAdjoint><<<grid, THREADS, 0, s>>>(a, 0.0f);
+    MG_TRY(pr_loop<PrAdjoint>(g, a, opt, "wpr_adjoint", info, &cur));
     float *lam = a.c[cur];
     MG_CUDA(cudaMemcpyAsync(w->lam_keep.p, lam, (size_t)g->nv * 4, cudaMemcpyDeviceToDevice, s));
     int sg = g->prof.slot("wpr_grad");
     g->prof.begin(sg);
-    MG_TRY(row_totals(g, a, RowBack{a.S, w->xkeep.as<float>(), w->lam_keep.as<float>(), d, w->ct.as<float2>()}));
+    k_back_rows<<<grid, THREADS, 0, s>>>(a, g->fw.as<float>(), a.S, w->xkeep.as<float>(), w->lam_keep.as<float>(), d,
+                                         w->ct.as<float2>());
     MG_TRY(edge_grad_to_caller(g, w->ct.as<float2>(), w->lam_keep.as<float>(), w->grad_caller.as<float>()));
     g->prof.end();
     const void *lam_out = nullptr;
