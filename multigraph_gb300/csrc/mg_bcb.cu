@@ -691,9 +691,11 @@ mg_status bc_batched(mg_graph *g, const int32_t *src_engine, int32_t nsrc, const
             MG_TRY(run_loop(exec_mode, opt.profile != 0, s, w->bwd, key_b, bwd, &a.ctl->more, g->pinned_flag,
                             max_levels + 2));
         }
+        static_assert(sizeof(BbCtl) <= 512, "pinned_flag holds 512 bytes");
+        MG_CUDA(cudaMemcpyAsync(g->pinned_flag, a.ctl, sizeof(BbCtl), cudaMemcpyDeviceToHost, s));
+        MG_TRY(run_status_wait(g));
         BbCtl hc;
-        MG_CUDA(cudaMemcpyAsync(&hc, a.ctl, sizeof(hc), cudaMemcpyDeviceToHost, s));
-        MG_CUDA(cudaStreamSynchronize(s));
+        std::memcpy(&hc, g->pinned_flag, sizeof(hc));
         if (hc.status == 1) return fail(MG_ERR_ITER_LIMIT, "batched BC: level cap %d reached", max_levels);
         if (hc.status == 3) return fail(MG_ERR_CUDA, "batched BC: grid barrier of a persistent sweep timed out");
         if (hc.status != 0) return fail(MG_ERR_CUDA, "batched BC: level archive overflow");

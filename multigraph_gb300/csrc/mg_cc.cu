@@ -271,6 +271,20 @@ __global__ void k_cc_compress(int32_t n, int32_t *parent)
         parent[v] = cc_find_near(parent, v);
 }
 
+// arena labels of a batch -> minimum vertex ids within each graph: the offset
+// of a vertex's graph by binary search over the graphs (cached)
+__global__ void k_local_labels(int32_t n, int32_t graphs, const int32_t *voff, int32_t *label)
+{
+    for (int32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
+        int32_t lo = 0, hi = graphs - 1;   // last graph starting at or before v
+        while (lo < hi) {
+            const int32_t mid = (lo + hi + 1) >> 1;
+            if (__ldg(&voff[mid]) <= v) lo = mid; else hi = mid - 1;
+        }
+        label[v] -= __ldg(&voff[lo]);
+    }
+}
+
 }  // namespace
 
 struct CcWS {
@@ -377,10 +391,12 @@ mg_status mg_cc(mg_graph *g, const mg_opts *o, int32_t *label_out, mg_run_info *
 {
     mg_opts opt;
     MG_TRY(begin_run(g, o, opt, info));
+    const size_t bytes = (size_t)g->nv * 4;
+    HostPages pages(g, {{label_out, nullptr, bytes}});
     MG_TRY(cc_run(g, info));
     MG_TRY(cc_to_caller(g, g->cws->parent.as<int32_t>(), &g->res[MG_RES_LABEL]));
-    MG_TRY(end_run(g, opt, info));
-    return copy_out(g, label_out, g->res[MG_RES_LABEL], (size_t)g->nv * 4);
+    pages.wait();
+    return end_run(g, opt, info, {{label_out, g->res[MG_RES_LABEL], bytes}});
 }
 
 mg_status mg_batch_create(const mg_host_graph *const *graphs, int32_t count, int32_t device, mg_batch **out)
@@ -442,9 +458,11 @@ mg_status mg_batch_bfs(mg_batch *b, const int32_t *sources, const mg_opts *o, in
     mg_graph *g = b->dg;
     mg_opts opt;
     MG_TRY(begin_run(g, o, opt, info));
+    const size_t bytes = (size_t)g->nv * 4;
+    HostPages pages(g, {{levels_out, nullptr, bytes}});
     MG_TRY(frontier_bfs_multi(g, srcs.data(), (int32_t)srcs.size(), opt, info));
-    MG_TRY(end_run(g, opt, info));
-    return copy_out(g, levels_out, g->res[MG_RES_LEVEL], (size_t)g->nv * 4);
+    pages.wait();
+    return end_run(g, opt, info, {{levels_out, g->res[MG_RES_LEVEL], bytes}});
 }
 
 mg_status mg_batch_cc(mg_batch *b, const mg_opts *o, int32_t *labels_out, mg_run_info *info)
@@ -454,14 +472,19 @@ mg_status mg_batch_cc(mg_batch *b, const mg_opts *o, int32_t *labels_out, mg_run
     mg_graph *g = b->dg;
     mg_opts opt;
     MG_TRY(begin_run(g, o, opt, info));
+    const size_t bytes = (size_t)g->nv * 4;
+    HostPages pages(g, {{labels_out, nullptr, bytes}});
     MG_TRY(cc_run(g, info, &b->voff));
-    MG_TRY(cc_to_caller(g, g->cws->parent.as<int32_t>(), &g->res[MG_RES_LABEL]));
-    MG_TRY(end_run(g, opt, info));
-    if (!labels_out) return MG_OK;
-    MG_TRY(copy_out(g, labels_out, g->res[MG_RES_LABEL], (size_t)g->nv * 4));
-    for (size_t i = 0; i + 1 < b->voff.size(); i++)
-        for (int32_t v = b->voff[i]; v < b->voff[i + 1]; v++) labels_out[v] -= b->voff[i];
-    return MG_OK;
+    const void *labels = nullptr;
+    MG_TRY(cc_to_caller(g, g->cws->parent.as<int32_t>(), &labels));
+    if (labels_out && g->nv > 0 && b->local_nv.size() > 1) {
+        // per-graph labels (the label buffer is rewritten by every run)
+        k_local_labels<<<launch_grid(g, THREADS, 8), THREADS, 0, g->stream>>>(
+            g->nv, (int32_t)b->local_nv.size(), g->cws->voff.as<int32_t>(), (int32_t *)labels);
+        MG_CUDA(cudaGetLastError());
+    }
+    pages.wait();
+    return end_run(g, opt, info, {{labels_out, labels, bytes}});
 }
 
 }  // extern "C"

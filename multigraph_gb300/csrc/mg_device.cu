@@ -19,7 +19,11 @@
 
 #include "mg_device.cuh"
 
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include <algorithm>
+#include <system_error>
 #include <utility>
 #include <cstring>
 #include <memory>
@@ -188,12 +192,57 @@ int launch_grid(const mg_graph *g, int threads, int per_sm)
     return g->num_sms * per_sm;
 }
 
-mg_status copy_out(mg_graph *g, void *host, const void *dev, size_t bytes)
+#ifndef MADV_POPULATE_WRITE
+#define MADV_POPULATE_WRITE 23   // Linux 5.14
+#endif
+
+HostPages::HostPages(mg_graph *graph, std::initializer_list<HostCopy> arrays) : g(graph)
 {
-    if (!host || bytes == 0) return MG_OK;
-    MG_CUDA(cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, g->stream));
+    constexpr size_t POPULATE_MIN = 1 << 20;
+    for (const HostCopy &c : arrays)
+        if (c.host && c.bytes >= POPULATE_MIN) todo.push_back(c);
+    g->pages = this;
+}
+
+void HostPages::start()
+{
+    constexpr size_t PER_THREAD = 16 << 20, MOST = 8;
+    const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+    for (const HostCopy &c : todo) {
+        const uintptr_t lo = (uintptr_t)c.host / page * page, hi = ((uintptr_t)c.host + c.bytes + page - 1) / page * page;
+        const size_t parts = std::min(MOST, (hi - lo + PER_THREAD - 1) / PER_THREAD);
+        const size_t step = ((hi - lo) / parts + page - 1) / page * page;
+        try {
+            for (uintptr_t p = lo; p < hi; p += step) {
+                const size_t len = std::min<uintptr_t>(step, hi - p);
+                threads.emplace_back([p, len] { (void)madvise((void *)p, len, MADV_POPULATE_WRITE); });
+            }
+        } catch (const std::system_error &) {
+            break;   // no thread to be had: the copy faults the pages in
+        }
+    }
+    todo.clear();
+}
+
+mg_status run_status_wait(mg_graph *g)
+{
+    if (g->pages) g->pages->start();
     MG_CUDA(cudaStreamSynchronize(g->stream));
     return MG_OK;
+}
+
+void HostPages::wait()
+{
+    start();
+    for (std::thread &t : threads) t.join();
+    threads.clear();
+}
+
+HostPages::~HostPages()
+{
+    todo.clear();   // (a run that failed early)
+    wait();
+    g->pages = nullptr;
 }
 
 mg_status begin_run(mg_graph *g, const mg_opts *o, mg_opts &opt, mg_run_info *info)
@@ -208,11 +257,13 @@ mg_status begin_run(mg_graph *g, const mg_opts *o, mg_opts &opt, mg_run_info *in
     return MG_OK;
 }
 
-mg_status end_run(mg_graph *g, const mg_opts &opt, mg_run_info *info)
+mg_status end_run(mg_graph *g, const mg_opts &opt, mg_run_info *info, std::initializer_list<HostCopy> out)
 {
     (void)opt;
     MG_CUDA(cudaEventRecord(g->ev1, g->stream));
-    MG_CUDA(cudaEventSynchronize(g->ev1));
+    for (const HostCopy &c : out)
+        if (c.host && c.bytes) MG_CUDA(cudaMemcpyAsync(c.host, c.dev, c.bytes, cudaMemcpyDeviceToHost, g->stream));
+    MG_CUDA(cudaStreamSynchronize(g->stream));
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail(MG_ERR_CUDA, "kernel error: %s", cudaGetErrorString(e));
     if (info) {
@@ -988,7 +1039,7 @@ mg_status mg_graph_upload(const mg_host_graph *h, int32_t device, mg_graph **out
     MG_CUDA(cudaEventCreate(&g->ev1));
     MG_CUDA(cudaEventCreateWithFlags(&g->ev_staged, cudaEventDisableTiming));
     MG_CUDA(cudaEventCreateWithFlags(&g->ev_consumed, cudaEventDisableTiming));
-    MG_CUDA(cudaMallocHost(&g->pinned_flag, 64));
+    MG_CUDA(cudaMallocHost(&g->pinned_flag, 512));
     MG_CUDA(cudaMallocHost(&g->sym_host, 64));
     HostLayout L;
     build_layout(*h, L);

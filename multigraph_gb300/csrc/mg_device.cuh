@@ -9,7 +9,9 @@
 
 #include <cstdlib>
 #include <functional>
+#include <initializer_list>
 #include <string>
+#include <thread>
 #include <vector>
 
 #define MG_CUDA(call)                                                                                 \
@@ -131,6 +133,10 @@ struct HubSplit {
 };
 }  // namespace mgi
 
+namespace mgi {
+class HostPages;
+}
+
 // ---------------------------------------------------------------------------
 // algorithm workspaces (defined in their translation units)
 // ---------------------------------------------------------------------------
@@ -212,6 +218,7 @@ struct mg_graph {
     PprWS *ppws = nullptr;
     WprWS *wpws = nullptr;
     mgi::Profiler prof;
+    mgi::HostPages *pages = nullptr; // the running call's result arrays
     int32_t *pinned_flag = nullptr; // pinned host word for host-loop readbacks
     // result pointers for mg_result_device
     const void *res[8] = {nullptr};
@@ -225,8 +232,39 @@ void free_bc_ws(mg_graph *g);
 void free_ppr_ws(mg_graph *g);
 void free_wpr_ws(mg_graph *g);
 mg_status begin_run(mg_graph *g, const mg_opts *o, mg_opts &opt, mg_run_info *info);
-mg_status end_run(mg_graph *g, const mg_opts &opt, mg_run_info *info);
-mg_status copy_out(mg_graph *g, void *host, const void *dev, size_t bytes);
+// End of a run: its end event, the results to the host (null host pointers
+// are skipped), one synchronisation, the run's time.
+struct HostCopy {
+    void *host;
+    const void *dev;
+    size_t bytes;
+};
+mg_status end_run(mg_graph *g, const mg_opts &opt, mg_run_info *info, std::initializer_list<HostCopy> out = {});
+// Pages of the host result arrays brought in by helper threads while this
+// thread waits for the GPU (the arrays' bytes stay as they are).  A fresh
+// array's pages would otherwise fault in one by one under the copy: the 62 MB
+// gradient of R-MAT 19 took 2.9 ms, of which 0.4 ms are the link's.  start()
+// comes once the run's work is enqueued (the helpers hold the address space's
+// lock, which launches and pageable copies need too: begun earlier, they
+// delayed the run by 0.8 ms); every wait for a run's status calls it through
+// run_status_wait.  Arrays below POPULATE_MIN are not worth a thread;
+// page-locked ones have their pages already, which costs a helper one walk
+// over the page tables.
+class HostPages {
+public:
+    HostPages(mg_graph *g, std::initializer_list<HostCopy> arrays);
+    ~HostPages();
+    HostPages(const HostPages &) = delete;
+    HostPages &operator=(const HostPages &) = delete;
+    void start();
+    void wait();   // the pages are there (or the system call does not exist)
+private:
+    mg_graph *g;
+    std::vector<HostCopy> todo;
+    std::vector<std::thread> threads;
+};
+// wait for the graph's stream, its result pages coming in meanwhile
+mg_status run_status_wait(mg_graph *g);
 int launch_grid(const mg_graph *g, int threads, int per_sm);
 // failure injection for tests (MG_FAIL_BARRIER=1): the persistent kernels'
 // barriers never complete, their bounded waits run out and the run reports

@@ -414,10 +414,9 @@ mg_status bc_backward(mg_graph *g, int32_t src, const mg_opts &opt, float *bcacc
     else if (a.bc_ext) MG_CUDA(cudaLaunchKernelEx(&cfg, k_bc_back_levels<true>, a, bc, (double *)q, delta, bcacc));
     else MG_CUDA(cudaLaunchKernelEx(&cfg, k_bc_back_levels<false>, a, bc, (float *)q, delta, bcacc));
     P.end();
-    int err = 0;
-    MG_CUDA(cudaMemcpyAsync(&err, a.bar_err, 4, cudaMemcpyDeviceToHost, s));
-    MG_CUDA(cudaStreamSynchronize(s));
-    if (err) return fail(MG_ERR_CUDA, "grid barrier of the persistent backward kernel timed out");
+    MG_CUDA(cudaMemcpyAsync(g->pinned_flag, a.bar_err, 4, cudaMemcpyDeviceToHost, s));
+    MG_TRY(run_status_wait(g));
+    if (*g->pinned_flag) return fail(MG_ERR_CUDA, "grid barrier of the persistent backward kernel timed out");
     (void)opt;
     return MG_OK;
 }
@@ -439,9 +438,11 @@ mg_status mg_bfs(mg_graph *g, int32_t source, const mg_opts *o, int32_t *level_o
     mg_opts opt;
     MG_TRY(begin_run(g, o, opt, info));
     MG_TRY(check_source(g, source));
+    const size_t bytes = (size_t)g->nv * 4;
+    HostPages pages(g, {{level_out, nullptr, bytes}});
     MG_TRY(frontier_run_impl<mgops::Bfs>(g, to_engine(g, source), nullptr, 0, opt, info, MG_RES_LEVEL));
-    MG_TRY(end_run(g, opt, info));
-    return copy_out(g, level_out, g->res[MG_RES_LEVEL], (size_t)g->nv * 4);
+    pages.wait();
+    return end_run(g, opt, info, {{level_out, g->res[MG_RES_LEVEL], bytes}});
 }
 
 mg_status mg_sssp(mg_graph *g, int32_t source, const mg_opts *o, int32_t *dist_out, mg_run_info *info)
@@ -449,9 +450,11 @@ mg_status mg_sssp(mg_graph *g, int32_t source, const mg_opts *o, int32_t *dist_o
     mg_opts opt;
     MG_TRY(begin_run(g, o, opt, info));
     MG_TRY(check_source(g, source));
+    const size_t bytes = (size_t)g->nv * 4;
+    HostPages pages(g, {{dist_out, nullptr, bytes}});
     MG_TRY(frontier_run_impl<mgops::Sssp>(g, to_engine(g, source), nullptr, 0, opt, info, MG_RES_DIST));
-    MG_TRY(end_run(g, opt, info));
-    return copy_out(g, dist_out, g->res[MG_RES_DIST], (size_t)g->nv * 4);
+    pages.wait();
+    return end_run(g, opt, info, {{dist_out, g->res[MG_RES_DIST], bytes}});
 }
 
 mg_status mg_bc(mg_graph *g, int32_t source, const mg_opts *o, int32_t *level_out, double *sigma_out,
@@ -461,6 +464,8 @@ mg_status mg_bc(mg_graph *g, int32_t source, const mg_opts *o, int32_t *level_ou
     MG_TRY(begin_run(g, o, opt, info));
     MG_TRY(check_source(g, source));
     const int32_t s = to_engine(g, source);
+    const size_t n4 = (size_t)g->nv * 4;
+    HostPages pages(g, {{level_out, nullptr, n4}, {sigma_out, nullptr, 2 * n4}, {delta_out, nullptr, n4}});
     MG_TRY(frontier_run_impl<mgops::BcForward>(g, s, nullptr, 0, opt, info, MG_RES_LEVEL));
     MG_TRY(bc_backward(g, s, opt, nullptr));
     FrontierWS *w = g->fws;
@@ -471,10 +476,10 @@ mg_status mg_bc(mg_graph *g, int32_t source, const mg_opts *o, int32_t *level_ou
     MG_CUDA(cudaGetLastError());
     MG_TRY(publish(g, MG_RES_SIGMA, w->sigma_d.p, 8));
     MG_TRY(publish(g, MG_RES_DELTA, w->delta.p, 4));
-    MG_TRY(end_run(g, opt, info));
-    MG_TRY(copy_out(g, level_out, g->res[MG_RES_LEVEL], (size_t)g->nv * 4));
-    MG_TRY(copy_out(g, sigma_out, g->res[MG_RES_SIGMA], (size_t)g->nv * 8));
-    return copy_out(g, delta_out, g->res[MG_RES_DELTA], (size_t)g->nv * 4);
+    pages.wait();
+    return end_run(g, opt, info, {{level_out, g->res[MG_RES_LEVEL], n4},
+                                  {sigma_out, g->res[MG_RES_SIGMA], 2 * n4},
+                                  {delta_out, g->res[MG_RES_DELTA], n4}});
 }
 
 mg_status mg_bc_multi(mg_graph *g, const int32_t *sources, int32_t nsrc, const mg_opts *o, float *bc_out,
@@ -485,6 +490,8 @@ mg_status mg_bc_multi(mg_graph *g, const int32_t *sources, int32_t nsrc, const m
     if (nsrc < 0 || (nsrc > 0 && !sources)) return fail(MG_ERR_INVALID, "invalid sources");
     for (int32_t i = 0; i < nsrc; i++)
         if (sources[i] < 0 || sources[i] >= g->nv) return fail(MG_ERR_RANGE, "source %d out of range", sources[i]);
+    const size_t bytes = (size_t)g->nv * 4;
+    HostPages pages(g, {{bc_out, nullptr, bytes}});
     if (g->symmetric) {
         // 32 sources per traversal (mg_bcb.cu)
         std::vector<int32_t> eng((size_t)nsrc);
@@ -494,9 +501,10 @@ mg_status mg_bc_multi(mg_graph *g, const int32_t *sources, int32_t nsrc, const m
         MG_TRY(publish(g, MG_RES_BC, bcd, 4));
         mg_run_info keep;
         if (info) keep = *info;
-        MG_TRY(end_run(g, opt, info));
+        pages.wait();
+        MG_TRY(end_run(g, opt, info, {{bc_out, g->res[MG_RES_BC], bytes}}));
         if (info) { info->iterations = keep.iterations; info->pull_iterations = keep.pull_iterations; }
-        return copy_out(g, bc_out, g->res[MG_RES_BC], (size_t)g->nv * 4);
+        return MG_OK;
     }
     // directed graphs: one forward/backward traversal per source
     MG_TRY(ensure_ws<mgops::BcForward>(g));
@@ -512,9 +520,10 @@ mg_status mg_bc_multi(mg_graph *g, const int32_t *sources, int32_t nsrc, const m
         iters += sub.iterations;
     }
     MG_TRY(publish(g, MG_RES_BC, w->bc.p, 4));
-    MG_TRY(end_run(g, opt, info));
+    pages.wait();
+    MG_TRY(end_run(g, opt, info, {{bc_out, g->res[MG_RES_BC], bytes}}));
     if (info) info->iterations = iters;
-    return copy_out(g, bc_out, g->res[MG_RES_BC], (size_t)g->nv * 4);
+    return MG_OK;
 }
 
 }  // extern "C"

@@ -1334,11 +1334,16 @@ mg_status frontier_outcome(mg_graph *g, const Args &a, int32_t src, const int32_
                            const mg_opts &opt, int max_iter, mg_run_info *info, int which)
 {
     cudaStream_t s = g->stream;
+    // (page-locked: the loop state, then the overflow word)
+    static_assert(sizeof(FCtl) <= 256, "pinned_flag holds 512 bytes");
+    int32_t *hovf = g->pinned_flag + 64;
+    *hovf = 0;
+    MG_CUDA(cudaMemcpyAsync(g->pinned_flag, a.ctl, sizeof(FCtl), cudaMemcpyDeviceToHost, s));
+    if (Op::kPathCounts) MG_CUDA(cudaMemcpyAsync(hovf, a.bc_ovf, 4, cudaMemcpyDeviceToHost, s));
+    MG_TRY(run_status_wait(g));
     FCtl hc;
-    int32_t ovf = 0;
-    MG_CUDA(cudaMemcpyAsync(&hc, a.ctl, sizeof(FCtl), cudaMemcpyDeviceToHost, s));
-    if (Op::kPathCounts) MG_CUDA(cudaMemcpyAsync(&ovf, a.bc_ovf, 4, cudaMemcpyDeviceToHost, s));
-    MG_CUDA(cudaStreamSynchronize(s));
+    std::memcpy(&hc, g->pinned_flag, sizeof(hc));
+    const int32_t ovf = *hovf;
     if (ovf && !g->bc_ext) {
         // a path count passed FP64's comfortable range: this graph's BC runs
         // use extended path counts from now on, starting with this one
@@ -1456,9 +1461,11 @@ mg_status frontier_operator_run(mg_graph *g, int32_t source, const mg_opts *o, i
     mg_opts opt;
     MG_TRY(begin_run(g, o, opt, info));
     if (source < 0 || source >= g->nv) return fail(MG_ERR_RANGE, "source %d out of range [0,%d)", source, g->nv);
+    const size_t bytes = (size_t)g->nv * 4;
+    HostPages pages(g, {{label_out, nullptr, bytes}});
     MG_TRY(frontier_run_impl<Op>(g, to_engine(g, source), nullptr, 0, opt, info, MG_RES_LEVEL));
-    MG_TRY(end_run(g, opt, info));
-    return copy_out(g, label_out, g->res[MG_RES_LEVEL], (size_t)g->nv * 4);
+    pages.wait();
+    return end_run(g, opt, info, {{label_out, g->res[MG_RES_LEVEL], bytes}});
 }
 
 }  // namespace

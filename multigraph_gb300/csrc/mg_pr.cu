@@ -1777,9 +1777,11 @@ static mg_status pr_loop(mg_graph *g, PArgs &a, const mg_opts &opt, const char *
     const LoopKey key = LoopKey().add(Op::kSlot).add(a).add(grid).add(apply_grid).add(a.P ? g->hub.gen : 0ull);
     MG_TRY(run_loop(opt.profile ? MG_EXEC_HOST : opt.exec, opt.profile != 0, s, g->pws->lg[Op::kSlot], key, body,
                     &a.ctl->more, g->pinned_flag, max_iter + 2));
+    static_assert(sizeof(PCtl) <= 512, "pinned_flag holds 512 bytes");
+    MG_CUDA(cudaMemcpyAsync(g->pinned_flag, a.ctl, sizeof(PCtl), cudaMemcpyDeviceToHost, s));
+    MG_TRY(run_status_wait(g));
     PCtl hc;
-    MG_CUDA(cudaMemcpyAsync(&hc, a.ctl, sizeof(PCtl), cudaMemcpyDeviceToHost, s));
-    MG_CUDA(cudaStreamSynchronize(s));
+    std::memcpy(&hc, g->pinned_flag, sizeof(hc));
     if (a.P) MG_TRY(hub_check(g));
     return pr_outcome(g, hc, Op::kDataDriven, max_iter, info, final_cur);
 }
@@ -1835,9 +1837,11 @@ static mg_status pr_all(mg_graph *g, const PArgs &a, const mg_opts &opt, float x
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     MG_CUDA(cudaLaunchKernelEx(&cfg, k_pr_all<Op>, a, z));
+    static_assert(sizeof(PCtl) <= 512, "pinned_flag holds 512 bytes");
+    MG_CUDA(cudaMemcpyAsync(g->pinned_flag, a.ctl, sizeof(PCtl), cudaMemcpyDeviceToHost, s));
+    MG_TRY(run_status_wait(g));
     PCtl hc;
-    MG_CUDA(cudaMemcpyAsync(&hc, a.ctl, sizeof(PCtl), cudaMemcpyDeviceToHost, s));
-    MG_CUDA(cudaStreamSynchronize(s));
+    std::memcpy(&hc, g->pinned_flag, sizeof(hc));
     return pr_outcome(g, hc, Op::kDataDriven, opt.max_iter > 0 ? opt.max_iter : 10000, info, final_cur);
 }
 
@@ -1979,6 +1983,8 @@ mg_status mg_pagerank(mg_graph *g, int32_t variant, const mg_opts *o, float *ran
     if (opt.pr_layout != MG_PR_LAYOUT_GATHER && opt.pr_layout != MG_PR_LAYOUT_SEGMENTED &&
         opt.pr_layout != MG_PR_LAYOUT_AUTO)
         return fail(MG_ERR_INVALID, "unknown PageRank layout %d", opt.pr_layout);
+    const size_t bytes = (size_t)g->nv * 4;
+    HostPages pages(g, {{rank_out, nullptr, bytes}});
     PArgs a;
     const bool small = variant == MG_PR_TOPOLOGY && pr_small(g, opt, opt.pr_layout != MG_PR_LAYOUT_AUTO);
     MG_TRY(pr_setup(g, a, false, small ? MG_PR_LAYOUT_GATHER : opt.pr_layout));
@@ -2002,8 +2008,8 @@ mg_status mg_pagerank(mg_graph *g, int32_t variant, const mg_opts *o, float *ran
         }
         MG_TRY(pr_all<PrTopology>(g, a, opt, x0, out, info, &cur));
         g->res[MG_RES_RANK] = out ? (const void *)out : a.x[cur];
-        MG_TRY(end_run(g, opt, info));
-        return copy_out(g, rank_out, g->res[MG_RES_RANK], (size_t)g->nv * 4);
+        pages.wait();
+        return end_run(g, opt, info, {{rank_out, g->res[MG_RES_RANK], bytes}});
     }
     switch (variant) {
     case MG_PR_TOPOLOGY_REF:
@@ -2024,14 +2030,16 @@ mg_status mg_pagerank(mg_graph *g, int32_t variant, const mg_opts *o, float *ran
         break;
     }
     MG_TRY(to_caller(g, MG_RES_RANK, a.x[cur], 4, 1, &g->res[MG_RES_RANK]));
-    MG_TRY(end_run(g, opt, info));
-    return copy_out(g, rank_out, g->res[MG_RES_RANK], (size_t)g->nv * 4);
+    pages.wait();
+    return end_run(g, opt, info, {{rank_out, g->res[MG_RES_RANK], bytes}});
 }
 
 mg_status mg_wpagerank(mg_graph *g, const mg_opts *o, float *x_out, mg_run_info *info)
 {
     mg_opts opt;
     MG_TRY(begin_run(g, o, opt, info));
+    const size_t bytes = (size_t)g->nv * 4;
+    HostPages pages(g, {{x_out, nullptr, bytes}});
     PArgs a;
     MG_TRY(pr_setup(g, a, true));
     PrWS *w = g->pws;
@@ -2087,8 +2095,8 @@ mg_status mg_wpagerank(mg_graph *g, const mg_opts *o, float *x_out, mg_run_info 
     MG_TRY(pr_loop<PrWeighted>(g, a, opt, "wpr_pull", info, &cur));
     MG_CUDA(cudaMemcpyAsync(w->xkeep.p, a.x[cur], (size_t)g->nv * 4, cudaMemcpyDeviceToDevice, s));
     MG_TRY(to_caller(g, MG_RES_RANK, w->xkeep.p, 4, 1, &g->res[MG_RES_RANK]));
-    MG_TRY(end_run(g, opt, info));
-    return copy_out(g, x_out, g->res[MG_RES_RANK], (size_t)g->nv * 4);
+    pages.wait();
+    return end_run(g, opt, info, {{x_out, g->res[MG_RES_RANK], bytes}});
 }
 
 mg_status mg_wpagerank_backward(mg_graph *g, const float *g_host, const mg_opts *o, float *grad_w_out,
@@ -2098,6 +2106,7 @@ mg_status mg_wpagerank_backward(mg_graph *g, const float *g_host, const mg_opts 
     MG_TRY(begin_run(g, o, opt, info));
     if (!g_host && g->nv > 0) return fail(MG_ERR_INVALID, "null loss weights");
     if (!g->pws || !g->pws->xkeep.p || !g->pws->wT.p) return fail(MG_ERR_INVALID, "run mg_wpagerank first");
+    HostPages pages(g, {{grad_w_out, nullptr, (size_t)g->ne * 4}, {lambda_out, nullptr, (size_t)g->nv * 4}});
     PArgs a;
     MG_TRY(pr_setup(g, a, true));
     PrWS *w = g->pws;
@@ -2137,9 +2146,9 @@ mg_status mg_wpagerank_backward(mg_graph *g, const float *g_host, const mg_opts 
     g->prof.end();
     const void *lam_out = nullptr;
     MG_TRY(to_caller(g, MG_RES_DELTA, w->lam_keep.p, 4, 1, &lam_out));
-    MG_TRY(end_run(g, opt, info));
-    MG_TRY(copy_out(g, lambda_out, lam_out, (size_t)g->nv * 4));
-    return copy_out(g, grad_w_out, w->grad_caller.p, (size_t)g->ne * 4);
+    pages.wait();
+    return end_run(g, opt, info, {{lambda_out, lam_out, (size_t)g->nv * 4},
+                                  {grad_w_out, w->grad_caller.p, (size_t)g->ne * 4}});
 }
 
 }  // extern "C"
@@ -2214,8 +2223,10 @@ static mg_status ppr_pass(mg_graph *g, const PPArgs &a, const int32_t *seeds_dev
     const int slot = (LPR == 1 ? 0 : LPR == 2 ? 1 : LPR == 4 ? 2 : 3) * 2 + (DANG ? 1 : 0);
     MG_TRY(run_loop(opt.profile ? MG_EXEC_HOST : opt.exec, opt.profile != 0, s, w->lg[slot], key, body, &a.ctl->more,
                     g->pinned_flag, max_iter + 2));
-    MG_CUDA(cudaMemcpyAsync(&hc, a.ctl, sizeof(PPCtl), cudaMemcpyDeviceToHost, s));
-    MG_CUDA(cudaStreamSynchronize(s));
+    static_assert(sizeof(PPCtl) <= 512, "pinned_flag holds 512 bytes");
+    MG_CUDA(cudaMemcpyAsync(g->pinned_flag, a.ctl, sizeof(PPCtl), cudaMemcpyDeviceToHost, s));
+    MG_TRY(run_status_wait(g));
+    std::memcpy(&hc, g->pinned_flag, sizeof(hc));
     return MG_OK;
 }
 
@@ -2237,6 +2248,7 @@ mg_status mg_ppr_batch(mg_graph *g, const int32_t *seeds, int32_t nseeds, const 
     if (nseeds < 0 || (nseeds > 0 && !seeds)) return fail(MG_ERR_INVALID, "invalid seeds");
     for (int32_t i = 0; i < nseeds; i++)
         if (seeds[i] < 0 || seeds[i] >= g->nv) return fail(MG_ERR_RANGE, "seed %d out of range", seeds[i]);
+    HostPages pages(g, {{out, nullptr, (size_t)nseeds * g->nv * 4}});
     if (!g->ppws) g->ppws = new PprWS();
     PprWS *w = g->ppws;
     const size_t n = (size_t)std::max(g->nv, 1);
@@ -2294,8 +2306,9 @@ mg_status mg_ppr_batch(mg_graph *g, const int32_t *seeds, int32_t nseeds, const 
             w->out.as<float>() + (size_t)s0 * g->nv);
         MG_CUDA(cudaGetLastError());
     }
-    MG_TRY(end_run(g, opt, info));
+    pages.wait();
+    MG_TRY(end_run(g, opt, info, {{out, w->out.p, (size_t)nseeds * g->nv * 4}}));
     if (info) { info->iterations = total_iters; info->residual = max_resid; }
-    return copy_out(g, out, w->out.p, (size_t)nseeds * g->nv * 4);
+    return MG_OK;
 }
 }  // extern "C"
