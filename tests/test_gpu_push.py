@@ -71,3 +71,29 @@ def test_bc_long_entries(deg, flags):
         assert np.max(np.abs(dl - ref)) <= 1e-5 * max(1.0, np.max(np.abs(ref)))
     g.free()
     h.free()
+
+
+@pytest.mark.parametrize("direction", [mg.DIR_AUTO, mg.DIR_PULL])
+def test_sssp_large_weights(direction):
+    # three layers, edges forward only: every path's sum is in range, an
+    # unreached vertex's label plus a weight would wrap
+    rng = np.random.default_rng(12)
+    a, b, c = np.arange(300), np.arange(300, 700), np.arange(700, 1000)
+    src = np.concatenate([rng.choice(a, 4000), rng.choice(b, 4000)])
+    dst = np.concatenate([rng.choice(b, 4000), rng.choice(c, 4000)])
+    wt = rng.integers(500_000_000, 800_000_000, 8000)
+    h = mg.HostGraph.from_entries(1000, src, dst, wt, flags=mg.LOAD_NSYM)
+    og = O.csr_from_arrays(*h.arrays())
+    src = np.repeat(np.arange(og.nv), np.diff(og.csc_v))
+    g = mg.Graph(h)
+    for s in (0, 7, 400, og.nv - 1):
+        far = np.full(og.nv, 1 << 40)
+        far[s] = 0
+        for _ in range(2):
+            np.minimum.at(far, og.csc_e, far[src] + og.csc_ev)
+        expect = np.where(far < 1 << 40, far, 1684300900)
+        assert far[far < 1 << 40].max() < 1684300900
+        for exec_ in (mg.EXEC_GRAPH, mg.EXEC_HOST):
+            assert np.array_equal(g.sssp(s, direction=direction, exec=exec_)[0], expect)
+    g.free()
+    h.free()
