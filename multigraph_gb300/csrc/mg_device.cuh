@@ -105,6 +105,7 @@ mg_status run_loop(int exec_mode, bool profile, cudaStream_t stream, LoopGraph &
 // memory; partial sums per (row, segment) pair; ids past the last segment
 // stay in an int32 tail (offsets toff) gathered through L2
 namespace mgi {
+constexpr int HUB_WIN = 512;   // piece sums the row finish stages in shared memory a warp (32 rows)
 struct HubSplit {
     bool valid = false;      // built for the current pull columns
     bool use = false;        // the split is in use (enough covered edges)
@@ -123,6 +124,7 @@ struct HubSplit {
     DevBuf pch;              // int32 [nparts+1]: each part's chunks (claimed by its CTA's warps)
     DevBuf cb;               // int32 [nchunks+1]: chunk boundaries (group indices)
     DevBuf pair_off;         // int32 [n+1]: row v's pieces in P
+    DevBuf porder;           // uint16 [npieces]: a sorted window's pieces' places in row order (graphs without a tail)
     DevBuf P;                // float [npieces+1]: piece sums of the current sweep (+ padding slot)
     DevBuf toff, tcol;       // tail rows: offsets [n+1], int32 ids
     DevBuf fin;              // int32 [nfw]: the rows the finish sums a warp each
@@ -130,6 +132,7 @@ struct HubSplit {
     // host copies for re-splitting the work among the CTAs
     std::vector<int32_t> hglam, hsegg;  // steps of every group; first group of every segment
     std::vector<double> w;            // every group's cost weight
+    double w0 = 0.0;                  // their total as first modelled, in cycles
 };
 }  // namespace mgi
 

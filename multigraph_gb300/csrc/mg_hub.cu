@@ -20,13 +20,24 @@
 //                     P[pair_off[v] .. pair_off[v+1]), segments ascending),
 //                     summed by the row's finish; pslot gives each packed
 //                     piece its place in P;
+//   sorted windows  : where the row finish copies 32 rows' piece sums to
+//                     shared memory anyway (at most HUB_WIN pieces, no warp
+//                     row, no tail), the window's P is ordered by (segment,
+//                     length, row) instead and porder gives each place its
+//                     piece's place in row order.  A group's pieces are
+//                     neighbours in that order, so the sweep's stores of
+//                     their sums share sectors: one sector a piece's sum was
+//                     what short groups cost (R-MAT 21: 0.96 sectors stored
+//                     a piece -> 0.34; a group 155 cycles of its SM where a
+//                     step takes 19).
 //   tail            : in-edges from ids beyond the last segment (graphs
 //                     with more than SEG_MAX segments' worth of vertices),
 //                     int32 ids gathered through L2 by the degree-binned
 //                     sweep.
 // One sweep: k_hub_sweep gives each CTA a contiguous range of groups (an
-// even share of the groups' cost weights: steps plus a fixed cost per group
-// at first, re-weighted by mg_autotune from measured per-CTA times), stages
+// even share of the groups' cost weights: a model of steps, groups, stored
+// sectors and staged segments at first, re-weighted by mg_autotune from
+// measured per-CTA times), stages
 // the contributions c[s*H, (s+1)*H) of every segment its range enters, and
 // its warps claim chunks of consecutive groups from a shared-memory counter
 // and stream them: a lane adds its four pieces' edges in order from shared
@@ -52,14 +63,18 @@ namespace {
 
 constexpr int32_t SEG_H = 57344;    // vertices per segment: 224 KB of FP32 contributions
 constexpr int32_t SEG_MAX = 64;     // segments at most; ids beyond stay in the L2 tail
-constexpr int32_t PIECE_MAX = 64;   // edges per piece at most
+constexpr int32_t PIECE_MAX = 32;   // edges per piece at most
 constexpr int32_t GROUP = 128;      // pieces per warp group: four per lane
 constexpr int HUB_THREADS = 1024;   // one CTA per SM (shared memory bound)
 constexpr int HUB_UNROLL = 4;       // steps (256-byte warp loads) in flight per warp
 constexpr int STAGE_BATCH = 4;      // 16-byte loads in flight per thread while staging a segment
-constexpr int64_t GROUP_COST = 16;  // a group's fixed cost in steps, for balancing CTA ranges
-constexpr int64_t CHUNK_COST = 64;  // a chunk's cost (steps + GROUP_COST per group): the unit warps claim
-                                    // (R-MAT 22 sweep: 128 -> 129-140 us, 64 -> 122 us, 32 -> 124-127, 16 -> 129-131)
+// what a CTA takes for its groups, in cycles of its SM (for the initial split
+// of the groups among the CTAs)
+constexpr double STEP_COST = 18.7;     // a step: 128 gathers from shared memory
+constexpr double GROUP_COST = 25.0;    // a group's slots, claim and switch
+constexpr double SECTOR_COST = 1.05;   // a 32-byte sector of P that a group's stores touch
+constexpr double STAGE_COST = 9000.0;  // a segment staged
+constexpr double CHUNK_COST = 600.0;   // a chunk, the unit that warps claim
 // the row finish sums rows with more than FIN_WARP pieces a warp each, the
 // rest a thread each (8-lane groups for rows of 5-64 pieces walked their
 // rows one after another and were slower)
@@ -210,8 +225,8 @@ static std::atomic<uint64_t> g_hub_builds{0};
 void hub_free(mg_graph *g)
 {
     HubSplit &h = g->hub;
-    DevBuf *bufs[] = {&h.hdat, &h.goff, &h.pslot, &h.cpart, &h.pseg, &h.pch, &h.cb, &h.ctime, &h.pair_off, &h.P, &h.toff,
-                      &h.tcol, &h.fin};
+    DevBuf *bufs[] = {&h.hdat, &h.goff, &h.pslot, &h.cpart, &h.pseg, &h.pch, &h.cb, &h.ctime, &h.pair_off, &h.porder,
+                      &h.P, &h.toff, &h.tcol, &h.fin};
     for (DevBuf *b : bufs) dev_free(*b);
     h = HubSplit();
 }
@@ -240,14 +255,10 @@ static mg_status hub_split(mg_graph *g)
         }
         out[parts] = hi;
     };
-    // the weight of an average group, for sizing chunks: CHUNK_COST is in
-    // units of the initial weights (steps)
-    double w0 = 0.0, wn = 0.0;
-    for (int32_t q = 0; q < ngroups; q++) {
-        w0 += (double)h.hglam[q] + (double)GROUP_COST;
-        wn += h.w[q];
-    }
-    const double chunk_w = (double)CHUNK_COST * (w0 > 0.0 ? wn / w0 : 1.0);
+    // CHUNK_COST in units of the weights as they are now
+    double wn = 0.0;
+    for (int32_t q = 0; q < ngroups; q++) wn += h.w[q];
+    const double chunk_w = CHUNK_COST * (h.w0 > 0.0 ? wn / h.w0 : 1.0);
     std::vector<int32_t> cta_lo((size_t)G + 1);
     cut(0, ngroups, G, cta_lo.data());
     std::vector<int32_t> cpart((size_t)G + 1, 0), pseg, pch, cb;
@@ -297,8 +308,15 @@ struct HubHost {
     int32_t H = 0, nseg = 0, nfw = 0;
     int64_t covered = 0, npieces = 0;
     std::vector<uint16_t> hdat;
+    std::vector<uint16_t> porder;
+    std::vector<float> cost;   // of every group, in cycles
     std::vector<int32_t> goff, pslot, glam, segg, pair_off, toff, tcol, fin;
 };
+
+// A bucket's q-th piece's place in its group: consecutive pieces (ascending
+// rows) go to consecutive lanes, so that a lane's j-th total is stored beside
+// its neighbours' j-th.
+inline int32_t group_place(int64_t q) { return (int32_t)((q % 32) * 4 + (q % GROUP) / 32); }
 
 static mg_status build_hub(const std::vector<int32_t> &prow, const std::vector<int32_t> &pcol, int32_t n, int64_t m,
                            int nt, HubHost &o)
@@ -317,7 +335,7 @@ static mg_status build_hub(const std::vector<int32_t> &prow, const std::vector<i
     for (int t = 1; t < nt; t++) {
         const int64_t goal = m * t / nt;
         rlo[t] = (int32_t)(std::lower_bound(prow.begin(), prow.end(), (int32_t)goal) - prow.begin());
-        rlo[t] = std::min(std::max(rlo[t], rlo[t - 1]), n);
+        rlo[t] = std::min(std::max((rlo[t] + 31) & ~31, rlo[t - 1]), n);   // whole windows
     }
     auto run = [&](const std::function<void(int)> &fn) {
         std::vector<std::thread> th;
@@ -397,21 +415,49 @@ static mg_status build_hub(const std::vector<int32_t> &prow, const std::vector<i
     std::vector<uint16_t> hdat((size_t)goff64[ngroups] * GROUP, (uint16_t)H);
     std::vector<int32_t> pslot((size_t)ngroups * GROUP, (int32_t)npieces);
     std::vector<int32_t> tcol((size_t)toff[n]);
+    std::vector<uint16_t> porder(toff[n] == 0 ? (size_t)npieces : 0);
     // pass 2: every row's pieces into their buckets, every edge into its
-    // piece's step and lane
+    // piece's step and lane, a window of 32 rows at a time
     run([&](int t) {
         std::vector<int64_t> next(tb.begin() + (size_t)t * NB, tb.begin() + (size_t)(t + 1) * NB);
-        int32_t cnt[SEG_MAX], full[SEG_MAX], e[SEG_MAX];
+        int32_t cnts[32][SEG_MAX], full[SEG_MAX], e[SEG_MAX];
         int64_t qfull[SEG_MAX], qrem[SEG_MAX];
+        std::vector<uint32_t> key;       // the window's pieces: (segment, length descending, place in row order)
+        std::vector<int32_t> at;         // their places in P from the window's first
+        int32_t base = 0;
         for (int32_t v = rlo[t]; v < rlo[t + 1]; v++) {
-            std::memset(cnt, 0, sizeof(int32_t) * nseg);
-            int32_t tp = toff[v];
-            for (int32_t p = prow[v]; p < prow[v + 1]; p++) {
-                const int32_t c = pcol[p];
-                if (c < cover) cnt[c / H]++;
-                else tcol[tp++] = c;
+            if (v % 32 == 0) {
+                const int32_t vend = std::min(v + 32, n);
+                base = pair_off[v];
+                key.clear();
+                at.clear();
+                bool sorted = toff[n] == 0 && pair_off[vend] - base <= HUB_WIN;
+                for (int32_t u = v; u < vend; u++) {
+                    int32_t *cnt = cnts[u - v];
+                    std::memset(cnt, 0, sizeof(int32_t) * nseg);
+                    int32_t tp = toff[u];
+                    for (int32_t p = prow[u]; p < prow[u + 1]; p++) {
+                        const int32_t c = pcol[p];
+                        if (c < cover) cnt[c / H]++;
+                        else tcol[tp++] = c;
+                    }
+                    sorted = sorted && npc[u] <= FIN_WARP;
+                    if (!sorted) continue;
+                    for (int sg = 0; sg < nseg; sg++)
+                        for (int32_t left = cnt[sg]; left > 0; left -= L)
+                            key.push_back((uint32_t)sg << 16 | (uint32_t)(L - std::min(left, L)) << 9 |
+                                          (uint32_t)key.size());
+                }
+                at.resize((size_t)(pair_off[vend] - base));
+                if (sorted) std::sort(key.begin(), key.end());
+                for (size_t i = 0; i < at.size(); i++) {
+                    const int32_t k = sorted ? (int32_t)(key[i] & 511u) : (int32_t)i;
+                    at[k] = (int32_t)i;
+                    if (!porder.empty()) porder[(size_t)base + i] = (uint16_t)k;
+                }
             }
-            int32_t slot = pair_off[v];   // the row's pieces: segments ascending, pieces in order
+            const int32_t *cnt = cnts[v % 32];
+            int32_t piece = pair_off[v] - base;   // the row's pieces: segments ascending, pieces in order
             for (int sg = 0; sg < nseg; sg++) {
                 e[sg] = 0;
                 if (!cnt[sg]) continue;
@@ -419,11 +465,13 @@ static mg_status build_hub(const std::vector<int32_t> &prow, const std::vector<i
                 const int32_t rem = cnt[sg] % L;
                 int64_t &nf = next[(size_t)sg * (L + 1) + L];
                 qfull[sg] = nf;
-                for (int32_t i = 0; i < full[sg]; i++) pslot[(size_t)(nf++)] = slot++;
+                for (int32_t i = 0; i < full[sg]; i++, nf++)
+                    pslot[(size_t)(nf / GROUP * GROUP + group_place(nf))] = base + at[piece++];
                 if (rem) {
                     int64_t &nr = next[(size_t)sg * (L + 1) + rem];
                     qrem[sg] = nr;
-                    pslot[(size_t)(nr++)] = slot++;
+                    pslot[(size_t)(nr / GROUP * GROUP + group_place(nr))] = base + at[piece++];
+                    nr++;
                 }
             }
             for (int32_t p = prow[v]; p < prow[v + 1]; p++) {
@@ -434,13 +482,29 @@ static mg_status build_hub(const std::vector<int32_t> &prow, const std::vector<i
                 e[sg]++;
                 const int64_t q = i < full[sg] ? qfull[sg] + i : qrem[sg];
                 const int64_t grp = q / GROUP;
-                hdat[(size_t)(goff64[grp] * GROUP + (int64_t)k * GROUP + q % GROUP)] = (uint16_t)(c - sg * H);
+                hdat[(size_t)(goff64[grp] * GROUP + (int64_t)k * GROUP + group_place(q))] = (uint16_t)(c - sg * H);
             }
         }
     });
+    // pass 3: every group's cost
+    o.cost.resize((size_t)ngroups);
+    run([&](int t) {
+        for (int32_t q = (int32_t)((int64_t)ngroups * t / nt); q < (int32_t)((int64_t)ngroups * (t + 1) / nt); q++) {
+            int32_t sectors = 0;
+            for (int j = 0; j < 4; j++)
+                for (int l = 0; l < 32; l++) {
+                    const int32_t *s = &pslot[(size_t)q * GROUP + 4 * l + j];
+                    if (l == 0 || s[0] / 8 != s[-4] / 8) sectors++;
+                }
+            o.cost[q] = (float)(STEP_COST * glam[q] + GROUP_COST + SECTOR_COST * sectors);
+        }
+    });
+    for (int sg = 1; sg < nseg; sg++)   // a CTA that goes on into the segment stages it
+        if (segg[sg] < segg[sg + 1]) o.cost[segg[sg]] += (float)STAGE_COST;
     o.hdat.swap(hdat);
     o.goff.swap(goff);
     o.pslot.swap(pslot);
+    o.porder.swap(porder);
     o.glam.swap(glam);
     o.segg.swap(segg);
     o.pair_off.swap(pair_off);
@@ -485,8 +549,9 @@ mg_status hub_prepare(mg_graph *g)
     const int32_t ngroups = (int32_t)o.glam.size();
     h.hglam = o.glam;
     h.hsegg = o.segg;
-    h.w.assign((size_t)ngroups, 0.0);
-    for (int32_t q = 0; q < ngroups; q++) h.w[q] = (double)o.glam[q] + (double)GROUP_COST;
+    h.w.assign(o.cost.begin(), o.cost.end());
+    h.w0 = 0.0;
+    for (double x : h.w) h.w0 += x;
     h.grid = g->num_sms;
     MG_TRY(dev_alloc(h.ctime, (size_t)h.grid * 8));
     MG_TRY(hub_split(g));
@@ -499,6 +564,7 @@ mg_status hub_prepare(mg_graph *g)
     MG_TRY(up(h.goff, o.goff.data(), o.goff.size() * 4));
     MG_TRY(up(h.pslot, o.pslot.data(), o.pslot.size() * 4));
     MG_TRY(up(h.pair_off, o.pair_off.data(), o.pair_off.size() * 4));
+    MG_TRY(up(h.porder, o.porder.data(), o.porder.size() * 2));
     MG_TRY(up(h.toff, o.toff.data(), o.toff.size() * 4));
     MG_TRY(up(h.tcol, o.tcol.data(), o.tcol.size() * 4));
     MG_TRY(up(h.fin, o.fin.data(), o.fin.size() * 4));   // at least 16 bytes even when empty
@@ -521,7 +587,7 @@ bool hub_covers_all(const mg_graph *g) { return (int64_t)g->nv <= (int64_t)SEG_M
 // Re-split the sweep's work from the last sweep's per-CTA clock counts:
 // every group's weight is scaled by its CTA's measured time over the
 // CTA's share of the weight (normalised to the mean), so groups whose real
-// cost the initial model (steps + GROUP_COST) misjudges move to other CTAs.
+// cost the initial model misjudges move to other CTAs.
 mg_status hub_rebalance(mg_graph *g)
 {
     HubSplit &h = g->hub;
@@ -641,7 +707,7 @@ extern "C" mg_status mg_selftest_segmented_layout(int32_t nv, int64_t ne, const 
     MG_TRY(build_hub(prow, pcol, nv, ne, threads, a));
     MG_TRY(build_hub(prow, pcol, nv, ne, 1, b));
     if (a.use != b.use || a.covered != b.covered || a.npieces != b.npieces || a.hdat != b.hdat || a.goff != b.goff ||
-        a.pslot != b.pslot || a.glam != b.glam || a.segg != b.segg || a.pair_off != b.pair_off || a.toff != b.toff ||
+        a.pslot != b.pslot || a.porder != b.porder || a.glam != b.glam || a.segg != b.segg || a.pair_off != b.pair_off || a.toff != b.toff ||
         a.tcol != b.tcol || a.fin != b.fin)
         return fail(MG_ERR_INTERNAL, "segmented layout differs between %d threads and one", threads);
     if (!a.use) return MG_OK;
@@ -686,6 +752,27 @@ extern "C" mg_status mg_selftest_segmented_layout(int32_t nv, int64_t ne, const 
     }
     for (int64_t p = 0; p < np; p++)
         if (seen[p] != 1) return fail(MG_ERR_INTERNAL, "segmented layout: slot %lld unused", (long long)p);
+    // sorted windows back in row order: porder is a permutation of each, and
+    // the identity where the row finish reads P directly
+    if (a.porder.size() != (a.tcol.empty() ? (size_t)np : 0))
+        return fail(MG_ERR_INTERNAL, "segmented layout: window order size");
+    for (int32_t vb = 0; vb < nv && !a.porder.empty(); vb += 32) {
+        const int32_t ve = std::min(vb + 32, nv), base = a.pair_off[vb], len = a.pair_off[ve] - base;
+        bool sorted = len <= HUB_WIN;
+        for (int32_t v = vb; v < ve; v++) sorted = sorted && a.pair_off[v + 1] - a.pair_off[v] <= FIN_WARP;
+        const std::vector<int32_t> s0(pseg.begin() + base, pseg.begin() + base + len),
+            l0(plen.begin() + base, plen.begin() + base + len);
+        const std::vector<int64_t> x0(psum.begin() + base, psum.begin() + base + len);
+        std::vector<int32_t> used((size_t)len, 0);
+        for (int32_t i = 0; i < len; i++) {
+            const int32_t k = a.porder[(size_t)base + i];
+            if (k >= len || used[k]++ || (!sorted && k != i))
+                return fail(MG_ERR_INTERNAL, "segmented layout: order of the window of row %d", vb);
+            pseg[base + k] = s0[i];
+            plen[base + k] = l0[i];
+            psum[base + k] = x0[i];
+        }
+    }
     // every row: its pieces (segments ascending, full pieces first) hold
     // exactly its covered in-edges; its tail holds the rest in row order
     std::vector<int32_t> fin;

@@ -98,6 +98,7 @@ struct PArgs {
     // chunks keep their full-row numbering (prow_full, chunk)
     const float *P;
     const int32_t *pair_off;
+    const uint16_t *porder;  // sorted windows (mg_hub.cu): each place's piece in row order
     const int32_t *prow_full;
     int32_t chunk;
     int32_t seg_only;        // every in-edge sits in a segment: rows finish in k_pr_seg
@@ -624,11 +625,11 @@ __global__ void __launch_bounds__(THREADS, 8) k_pr_seg(PArgs a, cudaGraphConditi
     // every other row a thread each, rows in order (the warp rows skipped):
     // a warp takes 32 consecutive rows, copies their piece sums (one
     // contiguous window of P) into shared memory with coalesced loads, and
-    // each lane sums its row from there; windows longer than SEG_WIN (rows
-    // near the hubs) are read from P directly.  Same adds in the same order
-    // either way.
-    constexpr int SEG_WIN = 512;
-    __shared__ float s_win[THREADS / 32][SEG_WIN];
+    // each lane sums its row from there; windows longer than HUB_WIN (rows
+    // near the hubs) are read from P directly.  A window without a warp row is
+    // sorted by segment in P (mg_hub.cu) and put back in row order on the way
+    // in.  Same adds in the same order every way.
+    __shared__ float s_win[THREADS / 32][mgi::HUB_WIN];
     float *win = s_win[threadIdx.x >> 5];
     for (int32_t vb = gwarp * 32; vb < a.n; vb += nwarps * 32) {
         const int32_t v = vb + lane;
@@ -638,8 +639,22 @@ __global__ void __launch_bounds__(THREADS, 8) k_pr_seg(PArgs a, cudaGraphConditi
         const int32_t last = min(a.n - vb, 32) - 1;
         const int32_t base = __shfl_sync(0xffffffffu, p0, 0), wend = __shfl_sync(0xffffffffu, p1, last);
         const int32_t len = wend - base;
-        const bool in_win = len <= SEG_WIN;
-        if (in_win) {
+        const bool in_win = len <= mgi::HUB_WIN;
+        const bool sorted = in_win && !__any_sync(0xffffffffu, p1 - p0 > a.fin_warp);
+        if (sorted) {
+            int32_t i = lane;
+            for (; i + 96 < len; i += 128) {
+                const int k0 = __ldcs(&a.porder[base + i]), k1 = __ldcs(&a.porder[base + i + 32]),
+                          k2 = __ldcs(&a.porder[base + i + 64]), k3 = __ldcs(&a.porder[base + i + 96]);
+                const float f0 = __ldcg(&a.P[base + i]), f1 = __ldcg(&a.P[base + i + 32]),
+                            f2 = __ldcg(&a.P[base + i + 64]), f3 = __ldcg(&a.P[base + i + 96]);
+                win[k0] = f0;
+                win[k1] = f1;
+                win[k2] = f2;
+                win[k3] = f3;
+            }
+            for (; i < len; i += 32) win[__ldcs(&a.porder[base + i])] = __ldcg(&a.P[base + i]);
+        } else if (in_win) {
             int32_t i = lane;
             for (; i + 96 < len; i += 128) {
                 const float f0 = __ldcg(&a.P[base + i]), f1 = __ldcg(&a.P[base + i + 32]),
@@ -1904,6 +1919,7 @@ static mg_status pr_setup(mg_graph *g, PArgs &a, bool weighted_or_adj, int32_t l
             a.pcol = g->hub.tcol.as<int32_t>();
             a.P = g->hub.P.as<float>();
             a.pair_off = g->hub.pair_off.as<int32_t>();
+            a.porder = g->hub.porder.as<uint16_t>();
             if (g->hub.ntail == 0) {
                 // rows finish in k_pr_seg; k_pr_apply only reduces
                 a.seg_only = 1;
