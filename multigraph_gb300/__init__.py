@@ -121,6 +121,7 @@ def _load_lib():
         "mg_autotune": ([vp, i32, i32, C.c_char_p, P(Opts)], i32),
         "mg_pagerank_noalloc": ([vp, vp, i32, i32, f32, f32, i32, vp, vp, P(i32), P(C.c_double)], i32),
         "mg_selftest_segmented_layout": ([i32, i64, vp, vp, i32, P(i64)], i32),
+        "mg_selftest_segmented_build": ([vp, P(i64)], i32),
     }
     for name, (args, res) in sig.items():
         fn = getattr(L, name)
@@ -152,7 +153,7 @@ EXPORTED = [
     "mg_graph_stream", "mg_graph_set_float_weights", "mg_opts_default", "mg_result_device", "mg_bfs", "mg_sssp",
     "mg_cc", "mg_bc", "mg_bc_multi", "mg_pagerank", "mg_ppr_batch", "mg_wpagerank", "mg_wpagerank_backward",
     "mg_batch_create", "mg_batch_free", "mg_batch_bfs", "mg_batch_cc", "mg_autotune", "mg_pagerank_noalloc",
-    "mg_selftest_segmented_layout",
+    "mg_selftest_segmented_layout", "mg_selftest_segmented_build",
 ]
 NOALLOC_MAX_VERTICES = 1 << 20
 
@@ -181,6 +182,15 @@ def selftest_segmented_layout(row_ptr, col, threads: int = 4) -> int:
     pieces = C.c_int64(0)
     _check(lib.mg_selftest_segmented_layout(len(rp) - 1, len(cl), rp.ctypes.data, cl.ctypes.data if len(cl) else None,
                                             threads, C.byref(pieces)), "mg_selftest_segmented_layout")
+    return pieces.value
+
+
+def selftest_segmented_build(graph: "Graph") -> int:
+    """PageRank's segmented layout as the device builds it for `graph`,
+    against the host's byte for byte (mg_selftest_segmented_build); returns
+    the number of pieces, raises MGError where they differ."""
+    pieces = C.c_int64(0)
+    _check(lib.mg_selftest_segmented_build(graph._h, C.byref(pieces)), "mg_selftest_segmented_build")
     return pieces.value
 
 

@@ -58,6 +58,7 @@
 #include <cstring>
 #include <functional>
 #include <thread>
+#include <type_traits>
 
 namespace {
 
@@ -216,11 +217,455 @@ __global__ void __launch_bounds__(HUB_THREADS, 1) k_hub_sweep(HubArgs a)
     if (threadIdx.x == 0) a.ctime[blockIdx.x] = clock64() - t_start;
 }
 
+// A bucket's q-th piece's place in its group: consecutive pieces (ascending
+// rows) go to consecutive lanes, so that a lane's j-th total is stored beside
+// its neighbours' j-th.
+__host__ __device__ inline int32_t group_place(int64_t q) { return (int32_t)((q % 32) * 4 + (q % GROUP) / 32); }
+
+// ---------------------------------------------------------------------------
+// The layout built on the device.  T = chunks of contiguous windows of 32
+// rows, even in rows + edges, a warp each: pass 1 counts every (row, segment)
+// and adds up the chunk's buckets, a scan over the chunks gives every chunk
+// its places in every bucket (rows ascending, whichever warp runs when), pass
+// 2 counts again and writes.  A window's rows are counted flat, 32 edges of
+// any of its rows at a time.  Rows of more than HB_ROW edges would keep one
+// warp busy for milliseconds: they are cut into subs of HB_ROW edges, a warp
+// each.  Built on the host, from the columns copied back, the layout took
+// most of the 434 ms of R-MAT 22's first PageRank call (here 20).
+// ---------------------------------------------------------------------------
+constexpr int32_t HB_CHUNKS = 4096;
+constexpr int32_t HB_ROW = 2048;
+constexpr int HB_WARPS = 4;
+
+struct HubBuild {
+    const int32_t *prow, *pcol;
+    int32_t n, nseg, cover, chunks;
+    int32_t nb;          // buckets: nseg * (PIECE_MAX + 1)
+    int32_t ncol;        // columns of a row's counts: the segments, then the tail
+    int32_t stride;      // ncol made odd (rows in shared memory, a lane each)
+    uint32_t *table;     // [chunks][nb + 3] bucket counts, then pieces, tail edges, warp rows; scanned in place
+    uint32_t *total;     // [nb + 3]
+    const uint32_t *place;   // [nb] each bucket's first place
+    int32_t *hid;        // [n] a long row's number + 1, or 0
+    int32_t *nlong;      // [2] long rows; their subs
+    int2 *lrow;          // long rows: (row, first sub)
+    int32_t *sub;        // subs: the long row's number
+    uint32_t *subcnt;    // [subs][ncol] counts, then the sub's first index in the row's segment
+    uint32_t *lcnt;      // [long rows][ncol] counts
+    uint32_t *lplace;    // [long rows][2][ncol] first places: full pieces (the tail's edges), the rest
+    const int32_t *goff;
+    int32_t *pair_off, *toff, *tcol, *fin, *pslot;
+    uint16_t *hdat, *porder;
+    int32_t ntail, npieces;
+};
+
+__device__ __forceinline__ int32_t hb_segment(const HubBuild &b, int32_t c) { return c < b.cover ? c / SEG_H : b.nseg; }
+
+__global__ void __launch_bounds__(256) k_hb_long(HubBuild b)
+{
+    for (int32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < b.n; v += gridDim.x * blockDim.x) {
+        const int32_t d = b.prow[v + 1] - b.prow[v];
+        int32_t id = 0;
+        if (d > HB_ROW) {
+            const int32_t ns = (d + HB_ROW - 1) / HB_ROW;
+            id = atomicAdd(&b.nlong[0], 1) + 1;
+            const int32_t first = atomicAdd(&b.nlong[1], ns);
+            b.lrow[id - 1] = make_int2(v, first);
+            for (int32_t s = 0; s < ns; s++) b.sub[first + s] = id - 1;
+        }
+        b.hid[v] = id;
+    }
+}
+
+__global__ void __launch_bounds__(HB_WARPS * 32) k_hb_sub_count(HubBuild b)
+{
+    __shared__ uint32_t s_cnt[HB_WARPS][SEG_MAX + 1];
+    uint32_t *cnt = s_cnt[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    const int32_t nsub = b.nlong[1];
+    for (int32_t s = blockIdx.x * HB_WARPS + (threadIdx.x >> 5); s < nsub; s += gridDim.x * HB_WARPS) {
+        for (int k = lane; k < b.ncol; k += 32) cnt[k] = 0;
+        __syncwarp();
+        const int2 r = b.lrow[b.sub[s]];
+        const int32_t p0 = b.prow[r.x] + (s - r.y) * HB_ROW, p1 = min(p0 + HB_ROW, b.prow[r.x + 1]);
+#pragma unroll 4
+        for (int32_t p = p0 + lane; p < p1; p += 32) atomicAdd(&cnt[hb_segment(b, __ldg(&b.pcol[p]))], 1u);
+        __syncwarp();
+        for (int k = lane; k < b.ncol; k += 32) b.subcnt[(size_t)s * b.ncol + k] = cnt[k];
+        __syncwarp();
+    }
+}
+
+__global__ void __launch_bounds__(128) k_hb_long_scan(HubBuild b)
+{
+    const int k = threadIdx.x;
+    const int32_t nl = b.nlong[0];
+    if (k >= b.ncol) return;
+    for (int32_t i = blockIdx.x; i < nl; i += gridDim.x) {
+        const int2 r = b.lrow[i];
+        const int32_t ns = (b.prow[r.x + 1] - b.prow[r.x] + HB_ROW - 1) / HB_ROW;
+        uint32_t run = 0;
+        for (int32_t s = 0; s < ns; s++) {
+            uint32_t *c = &b.subcnt[(size_t)(r.y + s) * b.ncol + k];
+            const uint32_t x = *c;
+            *c = run;
+            run += x;
+        }
+        b.lcnt[(size_t)i * b.ncol + k] = run;
+    }
+}
+
+// first row of chunk t: rows + edges in even shares, whole windows
+__device__ __forceinline__ int32_t hb_chunk_row(const HubBuild &b, int32_t t)
+{
+    if (t >= b.chunks) return b.n;
+    const long long goal = ((long long)b.prow[b.n] + b.n) * t / b.chunks;
+    int32_t lo = 0, hi = b.n;
+    while (lo < hi) {
+        const int32_t mid = lo + (hi - lo) / 2;
+        if ((long long)b.prow[mid] + mid < goal) lo = mid + 1;
+        else hi = mid;
+    }
+    return min((lo + 31) & ~31, b.n);
+}
+
+// the window's rows, a lane each, and their edges but the long rows' in one
+// list: lane l's at [off, off + deg) of it
+struct HubWindow {
+    int32_t v, start, id, off, total;
+};
+
+__device__ __forceinline__ HubWindow hb_window(const HubBuild &b, int32_t vb, int lane)
+{
+    HubWindow w;
+    w.v = vb + lane;
+    const bool act = w.v < b.n;
+    w.start = act ? b.prow[w.v] : 0;
+    w.id = act ? b.hid[w.v] : 0;
+    const int32_t deg = act && w.id == 0 ? b.prow[w.v + 1] - w.start : 0;
+    const int incl = mgd::warp_scan_incl(deg);
+    w.off = incl - deg;
+    w.total = __shfl_sync(0xffffffffu, incl, 31);
+    return w;
+}
+
+// fn(row's lane, column id, whether there is one), in edge order, 32 at a time
+template <class Fn>
+__device__ __forceinline__ void hb_edges(const HubBuild &b, const HubWindow &w, int lane, Fn fn)
+{
+    constexpr int AHEAD = 4;
+    for (int32_t i = 0; i < w.total; i += 32 * AHEAD) {
+        int32_t r[AHEAD], c[AHEAD];
+#pragma unroll
+        for (int j = 0; j < AHEAD; j++) {
+            const int32_t k = i + 32 * j + lane;
+            r[j] = mgd::owner_lane(w.off, min(k, w.total - 1));
+            const int32_t p = __shfl_sync(0xffffffffu, w.start, r[j]) + k - __shfl_sync(0xffffffffu, w.off, r[j]);
+            c[j] = k < w.total ? __ldg(&b.pcol[p]) : -1;
+        }
+#pragma unroll
+        for (int j = 0; j < AHEAD; j++)
+            if (i + 32 * j < w.total) fn(r[j], c[j]);
+    }
+}
+
+__device__ __forceinline__ void hb_count(const HubBuild &b, const HubWindow &w, int lane, uint32_t *cnt)
+{
+    for (int k = lane; k < 32 * b.stride; k += 32) cnt[k] = 0;
+    __syncwarp();
+    hb_edges(b, w, lane, [&](int32_t r, int32_t c) {
+        if (c >= 0) atomicAdd(&cnt[r * b.stride + hb_segment(b, c)], 1u);
+    });
+    unsigned longs = __ballot_sync(0xffffffffu, w.id > 0);
+    while (longs) {
+        const int r = __ffs(longs) - 1;
+        longs &= longs - 1;
+        const int32_t id = __shfl_sync(0xffffffffu, w.id, r) - 1;
+        for (int k = lane; k < b.ncol; k += 32) cnt[r * b.stride + k] = b.lcnt[(size_t)id * b.ncol + k];
+    }
+    __syncwarp();
+}
+
+__device__ __forceinline__ int32_t hb_pieces(const HubBuild &b, const uint32_t *row)
+{
+    int32_t np = 0;
+    for (int sg = 0; sg < b.nseg; sg++) np += (int32_t)((row[sg] + PIECE_MAX - 1) / PIECE_MAX);
+    return np;
+}
+
+__global__ void __launch_bounds__(HB_WARPS * 32) k_hb_count(HubBuild b)
+{
+    extern __shared__ uint32_t s_hb[];
+    const int lane = threadIdx.x & 31;
+    uint32_t *cnt = s_hb + (size_t)(threadIdx.x >> 5) * (32 * b.stride + b.nb), *hist = cnt + 32 * b.stride;
+    const int32_t t = blockIdx.x * HB_WARPS + (threadIdx.x >> 5);
+    if (t >= b.chunks) return;
+    for (int k = lane; k < b.nb; k += 32) hist[k] = 0;
+    const int32_t v0 = hb_chunk_row(b, t), v1 = hb_chunk_row(b, t + 1);
+    uint32_t pieces = 0, tail = 0, fin = 0;
+    for (int32_t vb = v0; vb < v1; vb += 32) {
+        const HubWindow w = hb_window(b, vb, lane);
+        hb_count(b, w, lane, cnt);
+        const uint32_t *row = cnt + lane * b.stride;
+        uint32_t np = 0;
+        for (int sg = 0; sg < b.nseg; sg++) {
+            const uint32_t full = row[sg] / PIECE_MAX, rem = row[sg] % PIECE_MAX;
+            if (full) atomicAdd(&hist[sg * (PIECE_MAX + 1) + PIECE_MAX], full);
+            if (rem) atomicAdd(&hist[sg * (PIECE_MAX + 1) + rem], 1u);
+            np += full + (rem > 0);
+        }
+        pieces += np;
+        tail += row[b.nseg];
+        fin += np > (uint32_t)FIN_WARP;
+        __syncwarp();
+    }
+    uint32_t *out = b.table + (size_t)t * (b.nb + 3);
+    for (int k = lane; k < b.nb; k += 32) out[k] = hist[k];
+    pieces = __reduce_add_sync(0xffffffffu, pieces);
+    tail = __reduce_add_sync(0xffffffffu, tail);
+    fin = __reduce_add_sync(0xffffffffu, fin);
+    if (lane == 0) {
+        out[b.nb] = pieces;
+        out[b.nb + 1] = tail;
+        out[b.nb + 2] = fin;
+    }
+}
+
+// exclusive scan of every column of the table: 32 columns a block, the rows
+// in 32 slices
+__global__ void __launch_bounds__(1024) k_hb_scan(HubBuild b)
+{
+    __shared__ uint32_t s_sum[32][33];
+    const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+    const int32_t w = b.nb + 3, k = blockIdx.x * 32 + x;
+    const int32_t per = (b.chunks + 31) / 32, t0 = min(y * per, b.chunks), t1 = min(t0 + per, b.chunks);
+    uint32_t sum = 0;
+    if (k < w)
+#pragma unroll 8
+        for (int32_t t = t0; t < t1; t++) sum += b.table[(size_t)t * w + k];
+    s_sum[y][x] = sum;
+    __syncthreads();
+    if (k >= w) return;
+    uint32_t run = 0;
+    for (int j = 0; j < y; j++) run += s_sum[j][x];
+    for (int32_t t = t0; t < t1; t++) {
+        uint32_t *c = &b.table[(size_t)t * w + k];
+        const uint32_t v = *c;
+        *c = run;
+        run += v;
+    }
+    if (y == 31) b.total[k] = run;
+}
+
+__global__ void __launch_bounds__(256) k_hb_fill(uint32_t *p, uint32_t x, long long count)
+{
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < count; i += (long long)gridDim.x * blockDim.x)
+        p[i] = x;
+}
+
+__device__ __forceinline__ void hb_slot(const HubBuild &b, uint32_t q, int32_t slot)
+{
+    b.pslot[(size_t)(q / GROUP) * GROUP + group_place(q)] = slot;
+}
+
+// the e-th of a row's edges from segment sg, whose pieces start at qf (full) and qr
+__device__ __forceinline__ void hb_put(const HubBuild &b, uint32_t e, uint32_t count, uint32_t qf, uint32_t qr, int32_t sg,
+                                       int32_t c)
+{
+    const uint32_t i = e / PIECE_MAX, k = e % PIECE_MAX;
+    const uint32_t q = i < count / PIECE_MAX ? qf + i : qr;
+    const size_t grp = q / GROUP;
+    b.hdat[((size_t)__ldg(&b.goff[grp]) + k) * GROUP + group_place(q)] = (uint16_t)(c - sg * SEG_H);
+}
+
+__global__ void __launch_bounds__(HB_WARPS * 32) k_hb_place(HubBuild b)
+{
+    extern __shared__ uint32_t s_hb[];
+    constexpr unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int mat = 32 * b.stride;
+    uint32_t *cnt = s_hb + (size_t)(threadIdx.x >> 5) * (3 * mat + 2 * mgi::HUB_WIN), *qf = cnt + mat, *qr = qf + mat;
+    uint32_t *key = qr + mat, *at = key + mgi::HUB_WIN;
+    const int32_t t = blockIdx.x * HB_WARPS + (threadIdx.x >> 5);
+    if (t >= b.chunks) return;
+    uint32_t *next = b.table + (size_t)t * (b.nb + 3);   // this warp's own
+    for (int k = lane; k < b.nb; k += 32) next[k] += b.place[k];
+    int32_t base = (int32_t)next[b.nb], tbase = (int32_t)next[b.nb + 1], fbase = (int32_t)next[b.nb + 2];
+    __syncwarp();
+    const int32_t v0 = hb_chunk_row(b, t), v1 = hb_chunk_row(b, t + 1);
+    for (int32_t vb = v0; vb < v1; vb += 32) {
+        const HubWindow w = hb_window(b, vb, lane);
+        const bool act = w.v < b.n;
+        hb_count(b, w, lane, cnt);
+        uint32_t *row = cnt + lane * b.stride;
+        const int32_t np = hb_pieces(b, row), nt = (int32_t)row[b.nseg];
+        const int32_t pincl = mgd::warp_scan_incl(np), tincl = mgd::warp_scan_incl(nt);
+        const int32_t len = __shfl_sync(FULL, pincl, 31);
+        const int32_t tlen = __shfl_sync(FULL, tincl, 31);
+        int32_t piece = pincl - np;   // the row's next piece, in row order
+        if (act) {
+            b.pair_off[w.v] = base + piece;
+            b.toff[w.v] = tbase + tincl - nt;
+        }
+        const unsigned fins = __ballot_sync(FULL, np > FIN_WARP);
+        if (np > FIN_WARP) b.fin[fbase + __popc(fins & ((1u << lane) - 1u))] = w.v;
+        const bool sorted = b.ntail == 0 && len <= mgi::HUB_WIN && fins == 0;
+        if (sorted) {
+            int32_t i = piece;
+            for (int sg = 0; sg < b.nseg; sg++)
+                for (int32_t left = (int32_t)row[sg]; left > 0; left -= PIECE_MAX, i++)
+                    key[i] = (uint32_t)sg << 16 | (uint32_t)(PIECE_MAX - min(left, PIECE_MAX)) << 9 | (uint32_t)i;
+            int size = 32;
+            while (size < len) size *= 2;   // at most HUB_WIN
+            for (int k = len + lane; k < size; k += 32) key[k] = FULL;
+            __syncwarp();
+            for (int up = 2; up <= size; up *= 2)
+                for (int d = up / 2; d > 0; d /= 2) {
+                    for (int k = lane; k < size / 2; k += 32) {
+                        const int x = 2 * d * (k / d) + k % d, y = x + d;
+                        const uint32_t kx = key[x], ky = key[y];
+                        if ((kx > ky) == ((x & up) == 0)) {
+                            key[x] = ky;
+                            key[y] = kx;
+                        }
+                    }
+                    __syncwarp();
+                }
+            for (int k = lane; k < len; k += 32) {
+                const uint32_t o = key[k] & 511u;
+                at[o] = (uint32_t)k;
+                b.porder[base + k] = (uint16_t)o;
+            }
+            __syncwarp();
+        } else if (b.ntail == 0) {
+            for (int32_t k = lane; k < len; k += 32) b.porder[base + k] = (uint16_t)k;
+        }
+        // every piece's place in its bucket, rows ascending
+        for (int sg = 0; sg < b.nseg; sg++) {
+            const uint32_t count = row[sg], full = count / PIECE_MAX, rem = count % PIECE_MAX;
+            uint32_t *nk = next + sg * (PIECE_MAX + 1);
+            if (__any_sync(FULL, full > 0)) {
+                const uint32_t incl = (uint32_t)mgd::warp_scan_incl((int)full);
+                const uint32_t q = nk[PIECE_MAX] + incl - full;
+                qf[lane * b.stride + sg] = q;
+                for (uint32_t i = 0; i < full; i++, piece++) hb_slot(b, q + i, base + (sorted ? (int32_t)at[piece] : piece));
+                __syncwarp();
+                if (lane == 31) nk[PIECE_MAX] += incl;
+            }
+            const unsigned same = __match_any_sync(FULL, rem);
+            if (rem) {
+                const int rank = __popc(same & ((1u << lane) - 1u));
+                const uint32_t q = nk[rem] + rank;
+                qr[lane * b.stride + sg] = q;
+                hb_slot(b, q, base + (sorted ? (int32_t)at[piece] : piece));
+                piece++;
+            }
+            __syncwarp();
+            if (rem && lane == 31 - __clz(same)) nk[rem] += __popc(same);
+            // a row that is not long has at most HB_ROW edges: its count in
+            // the upper half, the edges written so far in the lower
+            if (w.id == 0) row[sg] = count << 16;
+        }
+        qf[lane * b.stride + b.nseg] = (uint32_t)(tbase + tincl - nt);
+        if (w.id == 0) row[b.nseg] = (uint32_t)nt << 16;
+        __syncwarp();
+        hb_edges(b, w, lane, [&](int32_t r, int32_t c) {
+            const int32_t sg = c < 0 ? 0 : hb_segment(b, c);
+            const unsigned same = __match_any_sync(FULL, c < 0 ? -1 : r << 8 | sg);
+            const int at0 = r * b.stride + sg;
+            const uint32_t rc = cnt[at0];
+            const uint32_t e = (rc & 0xffffu) + __popc(same & ((1u << lane) - 1u));
+            __syncwarp();
+            if (c >= 0) {
+                if (lane == 31 - __clz(same)) cnt[at0] = rc + __popc(same);
+                if (sg == b.nseg) b.tcol[qf[at0] + e] = c;
+                else hb_put(b, e, rc >> 16, qf[at0], qr[at0], sg, c);
+            }
+            __syncwarp();
+        });
+        unsigned longs = __ballot_sync(FULL, w.id > 0);
+        while (longs) {
+            const int r = __ffs(longs) - 1;
+            longs &= longs - 1;
+            const int32_t id = __shfl_sync(FULL, w.id, r) - 1;
+            uint32_t *lp = b.lplace + (size_t)id * 2 * b.ncol;
+            for (int k = lane; k < b.ncol; k += 32) {
+                lp[k] = qf[r * b.stride + k];
+                lp[b.ncol + k] = qr[r * b.stride + k];
+            }
+        }
+        __syncwarp();
+        base += len;
+        tbase += tlen;
+        fbase += __popc(fins);
+    }
+    if (t == b.chunks - 1 && lane == 0) {
+        b.pair_off[b.n] = base;
+        b.toff[b.n] = tbase;
+    }
+}
+
+// the long rows' edges, a sub a warp
+__global__ void __launch_bounds__(HB_WARPS * 32) k_hb_sub_place(HubBuild b)
+{
+    constexpr unsigned FULL = 0xffffffffu;
+    __shared__ uint32_t s_e[HB_WARPS][SEG_MAX + 1];
+    uint32_t *pos = s_e[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    const int32_t nsub = b.nlong[1];
+    for (int32_t s = blockIdx.x * HB_WARPS + (threadIdx.x >> 5); s < nsub; s += gridDim.x * HB_WARPS) {
+        const int32_t id = b.sub[s];
+        const int2 r = b.lrow[id];
+        const uint32_t *count = b.lcnt + (size_t)id * b.ncol, *lp = b.lplace + (size_t)id * 2 * b.ncol;
+        for (int k = lane; k < b.ncol; k += 32) pos[k] = b.subcnt[(size_t)s * b.ncol + k];
+        __syncwarp();
+        const int32_t p0 = b.prow[r.x] + (s - r.y) * HB_ROW, p1 = min(p0 + HB_ROW, b.prow[r.x + 1]);
+        for (int32_t p = p0 + lane; p - lane < p1; p += 32) {
+            const int32_t c = p < p1 ? __ldg(&b.pcol[p]) : -1;
+            const int32_t sg = c < 0 ? 0 : hb_segment(b, c);
+            const unsigned same = __match_any_sync(FULL, c < 0 ? -1 : sg);
+            const uint32_t first = pos[sg], e = first + __popc(same & ((1u << lane) - 1u));
+            __syncwarp();
+            if (c >= 0) {
+                if (lane == 31 - __clz(same)) pos[sg] = first + __popc(same);
+                if (sg == b.nseg) b.tcol[lp[sg] + e] = c;
+                else hb_put(b, e, __ldg(&count[sg]), lp[sg], lp[b.ncol + sg], sg, c);
+            }
+            __syncwarp();
+        }
+        __syncwarp();
+    }
+}
+
+// the sectors of P that each group's stores touch
+__global__ void __launch_bounds__(256) k_hb_sectors(const int4 *pslot, int32_t ngroups, uint16_t *out)
+{
+    const int lane = threadIdx.x & 31;
+    for (int32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; q < ngroups; q += (gridDim.x * blockDim.x) >> 5) {
+        const int4 s = pslot[(size_t)q * 32 + lane];
+        int sectors = 0;
+        for (const int32_t x : {s.x, s.y, s.z, s.w}) {
+            const int32_t before = __shfl_up_sync(0xffffffffu, x / 8, 1);
+            sectors += __popc(__ballot_sync(0xffffffffu, lane == 0 || before != x / 8));
+        }
+        if (lane == 0) out[q] = (uint16_t)sectors;
+    }
+}
+
 }  // namespace
 
 namespace mgi {
 
 static std::atomic<uint64_t> g_hub_builds{0};
+
+static double group_cost(int32_t steps, int32_t sectors) { return STEP_COST * steps + GROUP_COST + SECTOR_COST * sectors; }
+
+// a CTA that goes on into a segment stages it: on the segment's first group
+static void stage_cost(const std::vector<int32_t> &segg, std::vector<double> &w)
+{
+    for (size_t sg = 1; sg + 1 < segg.size(); sg++)
+        if (segg[sg] < segg[sg + 1]) w[segg[sg]] += STAGE_COST;
+}
 
 void hub_free(mg_graph *g)
 {
@@ -297,8 +742,8 @@ static mg_status hub_split(mg_graph *g)
     return MG_OK;
 }
 
-// Build the segmented layout from a pull CSR on the host (prow [n+1], pcol
-// [m], engine ids): row-parallel passes over the edges (count, then write)
+// The layout from a pull CSR on the host (prow [n+1], pcol [m], engine ids),
+// what the device's builder is checked against: row-parallel passes over the edges (count, then write)
 // on nt threads, each a contiguous row range whose pieces take consecutive
 // places in every (segment, length) bucket, so buckets come out rows
 // ascending and the layout does not depend on nt.  o.use stays false when a
@@ -309,14 +754,8 @@ struct HubHost {
     int64_t covered = 0, npieces = 0;
     std::vector<uint16_t> hdat;
     std::vector<uint16_t> porder;
-    std::vector<float> cost;   // of every group, in cycles
     std::vector<int32_t> goff, pslot, glam, segg, pair_off, toff, tcol, fin;
 };
-
-// A bucket's q-th piece's place in its group: consecutive pieces (ascending
-// rows) go to consecutive lanes, so that a lane's j-th total is stored beside
-// its neighbours' j-th.
-inline int32_t group_place(int64_t q) { return (int32_t)((q % 32) * 4 + (q % GROUP) / 32); }
 
 static mg_status build_hub(const std::vector<int32_t> &prow, const std::vector<int32_t> &pcol, int32_t n, int64_t m,
                            int nt, HubHost &o)
@@ -486,21 +925,6 @@ static mg_status build_hub(const std::vector<int32_t> &prow, const std::vector<i
             }
         }
     });
-    // pass 3: every group's cost
-    o.cost.resize((size_t)ngroups);
-    run([&](int t) {
-        for (int32_t q = (int32_t)((int64_t)ngroups * t / nt); q < (int32_t)((int64_t)ngroups * (t + 1) / nt); q++) {
-            int32_t sectors = 0;
-            for (int j = 0; j < 4; j++)
-                for (int l = 0; l < 32; l++) {
-                    const int32_t *s = &pslot[(size_t)q * GROUP + 4 * l + j];
-                    if (l == 0 || s[0] / 8 != s[-4] / 8) sectors++;
-                }
-            o.cost[q] = (float)(STEP_COST * glam[q] + GROUP_COST + SECTOR_COST * sectors);
-        }
-    });
-    for (int sg = 1; sg < nseg; sg++)   // a CTA that goes on into the segment stages it
-        if (segg[sg] < segg[sg + 1]) o.cost[segg[sg]] += (float)STAGE_COST;
     o.hdat.swap(hdat);
     o.goff.swap(goff);
     o.pslot.swap(pslot);
@@ -520,8 +944,20 @@ static mg_status build_hub(const std::vector<int32_t> &prow, const std::vector<i
     return MG_OK;
 }
 
-// Build the segmented layout from the pull CSR (copied back from the
-// device), upload it and split the sweep's work among the CTAs.
+namespace {
+// device buffers for the time of a build
+struct BuildBufs {
+    DevBuf table, total, place, hid, nlong, lrow, sub, subcnt, lcnt, lplace, sectors;
+    ~BuildBufs()
+    {
+        for (DevBuf *b : {&table, &total, &place, &hid, &nlong, &lrow, &sub, &subcnt, &lcnt, &lplace, &sectors}) dev_free(*b);
+    }
+};
+}  // namespace
+
+// Build the segmented layout from the pull CSR on the device and split the
+// sweep's work among the CTAs (first PageRank call with the layout built on
+// the host -> here: R-MAT 22 434 -> 20 ms, R-MAT 20 69 -> 5, R-MAT 19 29 -> 3).
 mg_status hub_prepare(mg_graph *g)
 {
     HubSplit &h = g->hub;
@@ -535,47 +971,117 @@ mg_status hub_prepare(mg_graph *g)
         h.valid = true;
         return MG_OK;
     }
-    std::vector<int32_t> prow((size_t)n + 1), pcol((size_t)m);
-    MG_CUDA(cudaMemcpyAsync(prow.data(), g->trow, ((size_t)n + 1) * 4, cudaMemcpyDeviceToHost, s));
-    MG_CUDA(cudaMemcpyAsync(pcol.data(), g->tcol, (size_t)m * 4, cudaMemcpyDeviceToHost, s));
+    constexpr int32_t L = PIECE_MAX;
+    HubBuild b;
+    std::memset(&b, 0, sizeof(b));
+    b.prow = g->trow;
+    b.pcol = g->tcol;
+    b.n = n;
+    b.nseg = std::min<int32_t>(SEG_MAX, (n + SEG_H - 1) / SEG_H);
+    b.cover = (int32_t)std::min<int64_t>(n, (int64_t)b.nseg * SEG_H);
+    b.chunks = std::min(HB_CHUNKS, (n + 31) / 32);
+    b.nb = b.nseg * (L + 1);
+    b.ncol = b.nseg + 1;
+    b.stride = b.ncol | 1;
+    const size_t nlong = (size_t)(m / HB_ROW) + 1, nsub = 2 * nlong, tw = (size_t)b.nb + 3;
+    BuildBufs t;
+    auto make = [&](DevBuf &buf, size_t bytes, auto *&ptr) -> mg_status {
+        MG_TRY(dev_alloc(buf, std::max<size_t>(bytes, 16) + 16));
+        ptr = buf.as<std::remove_reference_t<decltype(*ptr)>>();
+        return MG_OK;
+    };
+    MG_TRY(make(t.table, (size_t)b.chunks * tw * 4, b.table));
+    MG_TRY(make(t.total, tw * 4, b.total));
+    MG_TRY(make(t.place, (size_t)b.nb * 4, b.place));
+    MG_TRY(make(t.hid, (size_t)n * 4, b.hid));
+    MG_TRY(make(t.nlong, 8, b.nlong));
+    MG_TRY(make(t.lrow, nlong * 8, b.lrow));
+    MG_TRY(make(t.sub, nsub * 4, b.sub));
+    MG_TRY(make(t.subcnt, nsub * b.ncol * 4, b.subcnt));
+    MG_TRY(make(t.lcnt, nlong * b.ncol * 4, b.lcnt));
+    MG_TRY(make(t.lplace, nlong * 2 * b.ncol * 4, b.lplace));
+    const int grid = launch_grid(g, 256, 4), wgrid = (b.chunks + HB_WARPS - 1) / HB_WARPS;
+    const size_t sm_count = (size_t)HB_WARPS * (32 * b.stride + b.nb) * 4,
+                 sm_place = (size_t)HB_WARPS * (3 * 32 * b.stride + 2 * HUB_WIN) * 4;
+    MG_CUDA(cudaFuncSetAttribute(k_hb_count, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_count));
+    MG_CUDA(cudaFuncSetAttribute(k_hb_place, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_place));
+    MG_CUDA(cudaMemsetAsync(b.nlong, 0, 8, s));
+    k_hb_long<<<grid, 256, 0, s>>>(b);
+    k_hb_sub_count<<<grid, HB_WARPS * 32, 0, s>>>(b);
+    k_hb_long_scan<<<grid, 128, 0, s>>>(b);
+    k_hb_count<<<wgrid, HB_WARPS * 32, sm_count, s>>>(b);
+    k_hb_scan<<<(int)((tw + 31) / 32), 1024, 0, s>>>(b);
+    MG_CUDA(cudaGetLastError());
+    std::vector<uint32_t> total(tw), place((size_t)b.nb, 0);
+    MG_CUDA(cudaMemcpyAsync(total.data(), b.total, tw * 4, cudaMemcpyDeviceToHost, s));
     MG_CUDA(cudaStreamSynchronize(s));
-    HubHost o;
-    MG_TRY(build_hub(prow, pcol, n, m, host_threads(0), o));
-    h.covered = o.covered;
-    if (!o.use) {
+    const int64_t npieces = total[b.nb], ntail = total[b.nb + 1];
+    h.covered = m - ntail;
+    // the segmented pull pays when a quarter of the edges or more are covered
+    if (h.covered * 4 < m) {
         h.valid = true;
         return MG_OK;
     }
-    const int32_t ngroups = (int32_t)o.glam.size();
-    h.hglam = o.glam;
-    h.hsegg = o.segg;
-    h.w.assign(o.cost.begin(), o.cost.end());
+    // buckets in order: segments ascending, lengths descending; each padded
+    // to whole groups
+    h.hglam.clear();
+    h.hsegg.assign((size_t)b.nseg + 1, 0);
+    std::vector<int32_t> goff(1, 0);
+    int64_t steps = 0;
+    for (int32_t sg = 0; sg < b.nseg; sg++) {
+        h.hsegg[sg] = (int32_t)h.hglam.size();
+        for (int32_t lam = L; lam >= 1; lam--) {
+            const size_t k = (size_t)sg * (L + 1) + lam;
+            place[k] = (uint32_t)(h.hglam.size() * GROUP);
+            for (uint32_t q = 0; q < (total[k] + GROUP - 1) / GROUP; q++) {
+                h.hglam.push_back(lam);
+                steps += lam;
+                goff.push_back((int32_t)steps);
+            }
+        }
+    }
+    const int32_t ngroups = (int32_t)h.hglam.size();
+    h.hsegg[b.nseg] = ngroups;
+    if (npieces >= INT32_MAX || steps >= INT32_MAX) return fail(MG_ERR_RANGE, "segmented PageRank layout too large");
+    b.ntail = (int32_t)ntail;
+    b.npieces = (int32_t)npieces;
+    h.nfw = (int32_t)total[b.nb + 2];
+    const size_t words = (size_t)steps * GROUP / 2, slots = (size_t)ngroups * GROUP;
+    MG_TRY(make(h.hdat, words * 4, b.hdat));
+    MG_TRY(make(h.goff, goff.size() * 4, b.goff));
+    MG_TRY(make(h.pslot, slots * 4, b.pslot));
+    MG_TRY(make(h.pair_off, ((size_t)n + 1) * 4, b.pair_off));
+    MG_TRY(make(h.porder, ntail == 0 ? (size_t)npieces * 2 : 0, b.porder));
+    MG_TRY(make(h.toff, ((size_t)n + 1) * 4, b.toff));
+    MG_TRY(make(h.tcol, (size_t)ntail * 4, b.tcol));
+    MG_TRY(make(h.fin, (size_t)h.nfw * 4, b.fin));
+    MG_TRY(dev_alloc(h.P, (size_t)(npieces + 1) * 4));
+    uint16_t *sectors = nullptr;
+    MG_TRY(make(t.sectors, (size_t)ngroups * 2, sectors));
+    MG_CUDA(cudaMemcpyAsync(t.place.p, place.data(), place.size() * 4, cudaMemcpyHostToDevice, s));
+    MG_CUDA(cudaMemcpyAsync(h.goff.p, goff.data(), goff.size() * 4, cudaMemcpyHostToDevice, s));
+    k_hb_fill<<<grid, 256, 0, s>>>(h.hdat.as<uint32_t>(), (uint32_t)SEG_H << 16 | (uint32_t)SEG_H, (long long)words);
+    k_hb_fill<<<grid, 256, 0, s>>>(h.pslot.as<uint32_t>(), (uint32_t)npieces, (long long)slots);
+    k_hb_place<<<wgrid, HB_WARPS * 32, sm_place, s>>>(b);
+    k_hb_sub_place<<<grid, HB_WARPS * 32, 0, s>>>(b);
+    k_hb_sectors<<<grid, 256, 0, s>>>(h.pslot.as<int4>(), ngroups, sectors);
+    MG_CUDA(cudaGetLastError());
+    std::vector<uint16_t> sec((size_t)ngroups);
+    MG_CUDA(cudaMemcpyAsync(sec.data(), sectors, sec.size() * 2, cudaMemcpyDeviceToHost, s));
+    MG_CUDA(cudaStreamSynchronize(s));
+    h.w.resize((size_t)ngroups);
+    for (int32_t q = 0; q < ngroups; q++) h.w[q] = group_cost(h.hglam[q], sec[q]);
+    stage_cost(h.hsegg, h.w);
     h.w0 = 0.0;
     for (double x : h.w) h.w0 += x;
     h.grid = g->num_sms;
     MG_TRY(dev_alloc(h.ctime, (size_t)h.grid * 8));
     MG_TRY(hub_split(g));
-    auto up = [&](DevBuf &b, const void *src, size_t bytes) -> mg_status {
-        MG_TRY(dev_alloc(b, std::max<size_t>(bytes, 16) + 16));
-        if (bytes) MG_CUDA(cudaMemcpyAsync(b.p, src, bytes, cudaMemcpyHostToDevice, s));
-        return MG_OK;
-    };
-    MG_TRY(up(h.hdat, o.hdat.data(), o.hdat.size() * 2));
-    MG_TRY(up(h.goff, o.goff.data(), o.goff.size() * 4));
-    MG_TRY(up(h.pslot, o.pslot.data(), o.pslot.size() * 4));
-    MG_TRY(up(h.pair_off, o.pair_off.data(), o.pair_off.size() * 4));
-    MG_TRY(up(h.porder, o.porder.data(), o.porder.size() * 2));
-    MG_TRY(up(h.toff, o.toff.data(), o.toff.size() * 4));
-    MG_TRY(up(h.tcol, o.tcol.data(), o.tcol.size() * 4));
-    MG_TRY(up(h.fin, o.fin.data(), o.fin.size() * 4));   // at least 16 bytes even when empty
-    MG_TRY(dev_alloc(h.P, (size_t)(o.npieces + 1) * 4));
-    MG_CUDA(cudaStreamSynchronize(s));
-    h.H = o.H;
-    h.nseg = o.nseg;
+    h.H = SEG_H;
+    h.nseg = b.nseg;
     h.ngroups = ngroups;
-    h.npieces = o.npieces;
-    h.ntail = o.toff[n];
-    h.nfw = o.nfw;
+    h.npieces = npieces;
+    h.ntail = ntail;
     h.fin_warp = FIN_WARP;
     h.use = true;
     h.valid = true;
@@ -681,6 +1187,50 @@ mg_status hub_launch(mg_graph *g, const float *c0, const float *c1, const int32_
 mg_status hub_check(mg_graph *) { return MG_OK; }
 
 }  // namespace mgi
+
+// ---------------------------------------------------------------------------
+// The layout that the device built for g, against the host's, byte for byte.
+// ---------------------------------------------------------------------------
+extern "C" mg_status mg_selftest_segmented_build(mg_graph *g, int64_t *pieces_out)
+{
+    using namespace mgi;
+    clear_error();
+    if (!g || !pieces_out) return fail(MG_ERR_INVALID, "null argument");
+    MG_CUDA(cudaSetDevice(g->device));
+    *pieces_out = 0;
+    MG_TRY(hub_prepare(g));
+    HubSplit &h = g->hub;
+    const int32_t n = g->nv;
+    const int64_t m = g->ne;
+    if (n < 4 || m == 0) return h.use ? fail(MG_ERR_INTERNAL, "segmented layout of nothing") : MG_OK;
+    std::vector<int32_t> prow((size_t)n + 1), pcol((size_t)m);
+    MG_CUDA(cudaMemcpy(prow.data(), g->trow, prow.size() * 4, cudaMemcpyDeviceToHost));
+    MG_CUDA(cudaMemcpy(pcol.data(), g->tcol, pcol.size() * 4, cudaMemcpyDeviceToHost));
+    HubHost o;
+    MG_TRY(build_hub(prow, pcol, n, m, host_threads(0), o));
+    if (o.use != h.use || o.covered != h.covered) return fail(MG_ERR_INTERNAL, "segmented build: covered edges");
+    if (!o.use) return MG_OK;
+    if (o.nseg != h.nseg || o.npieces != h.npieces || o.glam != h.hglam || o.segg != h.hsegg || o.nfw != h.nfw ||
+        (int64_t)o.tcol.size() != h.ntail)
+        return fail(MG_ERR_INTERNAL, "segmented build: sizes");
+    auto same = [&](const DevBuf &d, const auto &v, const char *what) -> mg_status {
+        std::vector<char> got(v.size() * sizeof(v[0]));
+        if (!got.empty()) MG_CUDA(cudaMemcpy(got.data(), d.p, got.size(), cudaMemcpyDeviceToHost));
+        if (!got.empty() && std::memcmp(got.data(), v.data(), got.size()))
+            return fail(MG_ERR_INTERNAL, "segmented build: %s", what);
+        return MG_OK;
+    };
+    MG_TRY(same(h.goff, o.goff, "group offsets"));
+    MG_TRY(same(h.pair_off, o.pair_off, "piece offsets"));
+    MG_TRY(same(h.toff, o.toff, "tail offsets"));
+    MG_TRY(same(h.tcol, o.tcol, "tail"));
+    MG_TRY(same(h.fin, o.fin, "warp rows"));
+    MG_TRY(same(h.porder, o.porder, "window order"));
+    MG_TRY(same(h.pslot, o.pslot, "slots"));
+    MG_TRY(same(h.hdat, o.hdat, "ids"));
+    *pieces_out = o.npieces;
+    return MG_OK;
+}
 
 // ---------------------------------------------------------------------------
 // Host-only check of the segmented layout (no GPU): builds it from a host

@@ -1,7 +1,8 @@
 """The segmented PageRank layout's windows of 32 rows -- sorted ones, ones of
 more than 512 pieces, ones with a warp row (more than 32 pieces), the last
 one of a row count off 32, a layout with a tail -- against the FP64 oracle for
-the same sweeps (1e-6 max-abs, the contract)."""
+the same sweeps (1e-6 max-abs, the contract); and the layout that the device
+builds against the host's."""
 import numpy as np
 import pytest
 
@@ -21,6 +22,8 @@ def _make(kind):
         deg[64:96] = 500
     elif kind == "warp":        # a warp row in a window of short rows
         deg[64] = 1500
+    elif kind == "rows":        # rows at the bounds of the build's subs, and far above them
+        deg[[5, 70, 71, 72, 73, 900, 5000]] = [2047, 2048, 2049, 4096, 4097, 40000, 90001]
     elif kind == "tail":        # more vertices than the segments hold
         n = 57344 * 64 + 37
         deg = rng.integers(0, 2, n)
@@ -33,7 +36,7 @@ def _make(kind):
     return mg.HostGraph.from_entries(n, src, dst)
 
 
-@pytest.mark.parametrize("kind", ["short", "long", "edge", "warp", "tail"])
+@pytest.mark.parametrize("kind", ["short", "long", "edge", "warp", "rows", "tail"])
 def test_windows(kind):
     h = _make(kind)
     og = O.csr_from_arrays(*h.arrays())
@@ -44,5 +47,23 @@ def test_windows(kind):
         if ref is None:
             ref, _ = O.pr_norm_f64(og, 0.85, 0.0, info.iterations)
         assert np.max(np.abs(x.astype(np.float64) - ref)) < 1e-6
+    g.free()
+    h.free()
+
+
+@pytest.mark.parametrize("kind", ["short", "long", "edge", "warp", "rows", "tail", "directed", "small"])
+def test_device_build(kind):
+    # the layout built on the device, byte for byte the host's
+    if kind == "directed":
+        rng = np.random.default_rng(4)
+        s = np.concatenate([rng.integers(0, 90000, 400000), rng.integers(0, 90000, 5000), np.full(7000, 3)])
+        d = np.concatenate([rng.integers(0, 90000, 400000), np.full(5000, 77), rng.integers(0, 90000, 7000)])
+        h = mg.HostGraph.from_entries(90000, s, d, flags=mg.LOAD_NSYM)
+    elif kind == "small":
+        h = mg.HostGraph.rmat(7, 4, seed=2)
+    else:
+        h = _make(kind)
+    g = mg.Graph(h)
+    assert mg.selftest_segmented_build(g) > 0
     g.free()
     h.free()
