@@ -231,11 +231,13 @@ __host__ __device__ inline int32_t group_place(int64_t q) { return (int32_t)((q 
 // any of its rows at a time.  Rows of more than HB_ROW edges would keep one
 // warp busy for milliseconds: they are cut into subs of HB_ROW edges, a warp
 // each.  Built on the host, from the columns copied back, the layout took
-// most of the 434 ms of R-MAT 22's first PageRank call (here 20).
+// most of the 434 ms of R-MAT 22's first PageRank call (here 17).
 // ---------------------------------------------------------------------------
-constexpr int32_t HB_CHUNKS = 4096;
+// (R-MAT 22's first call with 2048, 4096, 8192 and 16384 chunks: 27, 20, 17 and 16 ms -- the more of
+// them, the closer in time the warps that fill one group)
+constexpr int32_t HB_CHUNKS = 8192;
 constexpr int32_t HB_ROW = 2048;
-constexpr int HB_WARPS = 4;
+constexpr int HB_WARPS = 2;   // a block: shared memory of 20-30 KB a warp decides how many an SM holds
 
 struct HubBuild {
     const int32_t *prow, *pcol;
@@ -540,31 +542,45 @@ __global__ void __launch_bounds__(HB_WARPS * 32) k_hb_place(HubBuild b)
         } else if (b.ntail == 0) {
             for (int32_t k = lane; k < len; k += 32) b.porder[base + k] = (uint16_t)k;
         }
-        // every piece's place in its bucket, rows ascending
-        for (int sg = 0; sg < b.nseg; sg++) {
-            const uint32_t count = row[sg], full = count / PIECE_MAX, rem = count % PIECE_MAX;
-            uint32_t *nk = next + sg * (PIECE_MAX + 1);
-            if (__any_sync(FULL, full > 0)) {
-                const uint32_t incl = (uint32_t)mgd::warp_scan_incl((int)full);
-                const uint32_t q = nk[PIECE_MAX] + incl - full;
-                qf[lane * b.stride + sg] = q;
-                for (uint32_t i = 0; i < full; i++, piece++) hb_slot(b, q + i, base + (sorted ? (int32_t)at[piece] : piece));
-                __syncwarp();
-                if (lane == 31) nk[PIECE_MAX] += incl;
-            }
-            const unsigned same = __match_any_sync(FULL, rem);
-            if (rem) {
-                const int rank = __popc(same & ((1u << lane) - 1u));
-                const uint32_t q = nk[rem] + rank;
-                qr[lane * b.stride + sg] = q;
-                hb_slot(b, q, base + (sorted ? (int32_t)at[piece] : piece));
-                piece++;
+        // every piece's place in its bucket, rows ascending; the buckets' next
+        // places are read BATCH segments at a time
+        constexpr int BATCH = 4;
+        for (int sb = 0; sb < b.nseg; sb += BATCH) {
+            uint32_t nfull[BATCH], nrem[BATCH];
+#pragma unroll
+            for (int j = 0; j < BATCH; j++) {
+                if (sb + j >= b.nseg) break;
+                const uint32_t *nk = next + (sb + j) * (PIECE_MAX + 1);
+                nfull[j] = nk[PIECE_MAX];
+                nrem[j] = nk[row[sb + j] % PIECE_MAX];
             }
             __syncwarp();
-            if (rem && lane == 31 - __clz(same)) nk[rem] += __popc(same);
-            // a row that is not long has at most HB_ROW edges: its count in
-            // the upper half, the edges written so far in the lower
-            if (w.id == 0) row[sg] = count << 16;
+#pragma unroll
+            for (int j = 0; j < BATCH; j++) {
+                const int sg = sb + j;
+                if (sg >= b.nseg) break;
+                const uint32_t count = row[sg], full = count / PIECE_MAX, rem = count % PIECE_MAX;
+                uint32_t *nk = next + sg * (PIECE_MAX + 1);
+                if (__any_sync(FULL, full > 0)) {
+                    const uint32_t incl = (uint32_t)mgd::warp_scan_incl((int)full);
+                    const uint32_t q = nfull[j] + incl - full;
+                    qf[lane * b.stride + sg] = q;
+                    for (uint32_t i = 0; i < full; i++, piece++)
+                        hb_slot(b, q + i, base + (sorted ? (int32_t)at[piece] : piece));
+                    if (lane == 31) nk[PIECE_MAX] = nfull[j] + incl;
+                }
+                const unsigned same = __match_any_sync(FULL, rem);
+                if (rem) {
+                    const uint32_t q = nrem[j] + __popc(same & ((1u << lane) - 1u));
+                    qr[lane * b.stride + sg] = q;
+                    hb_slot(b, q, base + (sorted ? (int32_t)at[piece] : piece));
+                    piece++;
+                    if (lane == 31 - __clz(same)) nk[rem] = nrem[j] + __popc(same);
+                }
+                // a row that is not long has at most HB_ROW edges: its count in
+                // the upper half, the edges written so far in the lower
+                if (w.id == 0) row[sg] = count << 16;
+            }
         }
         qf[lane * b.stride + b.nseg] = (uint32_t)(tbase + tincl - nt);
         if (w.id == 0) row[b.nseg] = (uint32_t)nt << 16;
@@ -957,7 +973,7 @@ struct BuildBufs {
 
 // Build the segmented layout from the pull CSR on the device and split the
 // sweep's work among the CTAs (first PageRank call with the layout built on
-// the host -> here: R-MAT 22 434 -> 20 ms, R-MAT 20 69 -> 5, R-MAT 19 29 -> 3).
+// the host -> here: R-MAT 22 434 -> 17 ms, R-MAT 20 69 -> 5, R-MAT 19 29 -> 3).
 mg_status hub_prepare(mg_graph *g)
 {
     HubSplit &h = g->hub;
