@@ -347,7 +347,7 @@ mg_status mg_pagerank_noalloc(const int32_t *d_row, const int32_t *d_col, int32_
  * threads and on one, require the two builds to be equal, and verify every
  * invariant the segmented sweep and the row finish rely on: each in-edge
  * below the segments' reach in exactly one piece of its (row, segment) pair,
- * pieces of at most 32 edges with the full ones first, groups of equal-
+ * pieces of at most 64 edges with the full ones first, groups of equal-
  * length pieces with padding that reads a zero, every piece in exactly one
  * slot of the row-major sums in segment order, the rest of a row's in-edges
  * in its tail, and the list of rows the finish sums a warp each.  Sums are

@@ -34,11 +34,11 @@
 //                     with more than SEG_MAX segments' worth of vertices),
 //                     int32 ids gathered through L2 by the degree-binned
 //                     sweep.
-// One sweep: k_hub_sweep gives each CTA a contiguous range of groups (an
-// even share of the groups' cost weights: a model of steps, groups, stored
-// sectors and staged segments at first, re-weighted by mg_autotune from
-// measured per-CTA times), stages
-// the contributions c[s*H, (s+1)*H) of every segment its range enters, and
+// One sweep: k_hub_sweep gives each CTA a contiguous range of groups (the
+// least largest load under the groups' cost weights and the segments to be
+// staged; the weights are a model of steps, groups and stored sectors at
+// first, re-weighted by mg_autotune from measured per-CTA times), stages the
+// contributions c[s*H, (s+1)*H) of every segment its range enters, and
 // its warps claim chunks of consecutive groups from a shared-memory counter
 // and stream them: a lane adds its four pieces' edges in order from shared
 // memory and stores the four totals to P.  Pieces never cross a group, so
@@ -64,13 +64,14 @@ namespace {
 
 constexpr int32_t SEG_H = 57344;    // vertices per segment: 224 KB of FP32 contributions
 constexpr int32_t SEG_MAX = 64;     // segments at most; ids beyond stay in the L2 tail
-constexpr int32_t PIECE_MAX = 32;   // edges per piece at most
+constexpr int32_t PIECE_MAX = 64;   // edges per piece at most
 constexpr int32_t GROUP = 128;      // pieces per warp group: four per lane
 constexpr int HUB_THREADS = 1024;   // one CTA per SM (shared memory bound)
 constexpr int HUB_UNROLL = 4;       // steps (256-byte warp loads) in flight per warp
 constexpr int STAGE_BATCH = 4;      // 16-byte loads in flight per thread while staging a segment
 // what a CTA takes for its groups, in cycles of its SM (for the initial split
 // of the groups among the CTAs)
+// (least squares over the CTAs of R-MAT 20 to 22: within 3-9 % of the measured cycles)
 constexpr double STEP_COST = 18.7;     // a step: 128 gathers from shared memory
 constexpr double GROUP_COST = 25.0;    // a group's slots, claim and switch
 constexpr double SECTOR_COST = 1.05;   // a 32-byte sector of P that a group's stores touch
@@ -676,13 +677,6 @@ static std::atomic<uint64_t> g_hub_builds{0};
 
 static double group_cost(int32_t steps, int32_t sectors) { return STEP_COST * steps + GROUP_COST + SECTOR_COST * sectors; }
 
-// a CTA that goes on into a segment stages it: on the segment's first group
-static void stage_cost(const std::vector<int32_t> &segg, std::vector<double> &w)
-{
-    for (size_t sg = 1; sg + 1 < segg.size(); sg++)
-        if (segg[sg] < segg[sg + 1]) w[segg[sg]] += STAGE_COST;
-}
-
 void hub_free(mg_graph *g)
 {
     HubSplit &h = g->hub;
@@ -692,11 +686,16 @@ void hub_free(mg_graph *g)
     h = HubSplit();
 }
 
-// Split the groups among the CTAs by the groups' cost weights h.w: each
-// CTA an even share of the total weight (contiguous groups), cut at
-// segment boundaries into parts and each part into chunks of about
-// CHUNK_COST that the CTA's warps claim one at a time.  The captured loops
-// that launch the sweep take the new split (the build number changes).
+// Split the groups among the CTAs by the groups' cost weights h.w:
+// contiguous ranges of the least largest load, cut at segment boundaries into
+// parts and each part into chunks of about CHUNK_COST that the CTA's warps
+// claim one at a time.  The captured loops that launch the sweep take the new
+// split (the build number changes).  Even shares of the weight, a staging
+// charged to each segment's first group, left CTAs that stage a segment for
+// its last few groups: a sweep of R-MAT 20 took 57-68 us by the accident of
+// where the cuts fell, 57 now (even shares with a group taken as 16 steps and
+// row-major piece sums: 63.5); R-MAT 20 of degree 6 45-55 -> 46 (48), R-MAT 19
+// 42-55 -> 43 (46), R-MAT 22 161-170 -> 160 (191).
 static mg_status hub_split(mg_graph *g)
 {
     HubSplit &h = g->hub;
@@ -720,8 +719,37 @@ static mg_status hub_split(mg_graph *g)
     double wn = 0.0;
     for (int32_t q = 0; q < ngroups; q++) wn += h.w[q];
     const double chunk_w = CHUNK_COST * (h.w0 > 0.0 ? wn / h.w0 : 1.0);
-    std::vector<int32_t> cta_lo((size_t)G + 1);
-    cut(0, ngroups, G, cta_lo.data());
+    // the least load T under which G CTAs, filled one after another, take all
+    // groups; a CTA pays for every segment that it stages, and leaves a
+    // segment that it has no room to stage to the next
+    const double stage = STAGE_COST * (h.w0 > 0.0 ? wn / h.w0 : 1.0);
+    std::vector<int32_t> cta_lo((size_t)G + 1, ngroups);
+    auto fill = [&](double T) {
+        int32_t at = 0;
+        for (int b = 0; b < G; b++) {
+            cta_lo[b] = at;
+            double room = T;
+            for (bool first = true; at < ngroups; first = false) {
+                const int32_t sg = (int32_t)(std::upper_bound(segg.begin(), segg.end(), at) - segg.begin()) - 1;
+                room -= stage;
+                int32_t e = (int32_t)(std::upper_bound(gcum.begin() + at, gcum.begin() + segg[sg + 1] + 1, gcum[at] + room) -
+                                      gcum.begin()) - 1;
+                e = std::max(e, first ? at + 1 : at);
+                if (e <= at) break;
+                room -= gcum[e] - gcum[at];
+                at = e;
+                if (at < segg[sg + 1]) break;
+            }
+        }
+        return at == ngroups;
+    };
+    double lo_t = 0.0, hi_t = gcum[ngroups] + stage * (double)segg.size();
+    for (int it = 0; it < 40; it++) {
+        const double T = 0.5 * (lo_t + hi_t);
+        (fill(T) ? hi_t : lo_t) = T;
+    }
+    fill(hi_t);
+    cta_lo[G] = ngroups;
     std::vector<int32_t> cpart((size_t)G + 1, 0), pseg, pch, cb;
     for (int b = 0; b < G; b++) {
         cpart[b] = (int32_t)pseg.size();
@@ -1087,7 +1115,6 @@ mg_status hub_prepare(mg_graph *g)
     MG_CUDA(cudaStreamSynchronize(s));
     h.w.resize((size_t)ngroups);
     for (int32_t q = 0; q < ngroups; q++) h.w[q] = group_cost(h.hglam[q], sec[q]);
-    stage_cost(h.hsegg, h.w);
     h.w0 = 0.0;
     for (double x : h.w) h.w0 += x;
     h.grid = g->num_sms;
