@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(THREADS, TP ? 4 : 1) k_bb_pull(BbArgs a)
     pdl_enter();
     const BbCtl c = *a.ctl;
     if (c.more == 0 || c.dense == 2) return;
-    bb_pull_phase<TP, M>(a, c, c.dense ? a.n : c.k.ncand);
+    bb_pull_phase<TP, M>(a, c, c.dense ? a.n : c.k.ncand, &a.ctl->k);
 }
 
 template <int M>
@@ -92,8 +92,8 @@ __global__ void __launch_bounds__(THREADS) k_bb_heavy(BbArgs a)
     pdl_enter();
     const BbCtl c = *a.ctl;
     if (c.more == 0) return;
-    if (M == M_INT && c.dense == 2) bb_gather_heavy_phase(a, c);
-    else bb_heavy_phase<M>(a, c);
+    if (M == M_INT && c.dense == 2) bb_gather_heavy_phase(a, c, &a.ctl->k);
+    else bb_heavy_phase<M>(a, c, &a.ctl->k);
 }
 
 // dense level without masks (M_INT)
@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(GTHREADS, GPER_SM) k_bb_gather(BbArgs a)
     pdl_enter();
     const BbCtl c = *a.ctl;
     if (c.more == 0 || c.dense != 2) return;
-    bb_gather_phase(a, c);
+    bb_gather_phase(a, c, &a.ctl->k);
 }
 
 // Archives level d+1 and, in the last block to finish, decides the next
@@ -122,10 +122,10 @@ __global__ void __launch_bounds__(THREADS) k_bb_compact(BbArgs a, cudaGraphCondi
     const LvlCnt k = n.k;
     const int32_t d = n.d;
     int32_t off_d2;
-    bb_decide(n, k, n.ovf, a.off[d + 1], off_d2, a.m, a.mode);
+    bb_decide(n, k, a.off[d + 1], off_d2, a.m, a.mode);
     a.off[d + 2] = off_d2;
     a.lnfe[d + 1] = k.nfe;
-    n.k = LvlCnt{0, 0, 0, 0, 0ull};
+    n.k = LvlCnt{};
     n.done = 0;
     *cp = n;
     if (use_cond) cudaGraphSetConditional(h, n.more ? 1u : 0u);
@@ -222,6 +222,8 @@ __device__ __forceinline__ LvlCnt load_cnt_l2(const LvlCnt *k)
     r.nfh_build = __ldcg(&k->nfh_build);
     r.status = __ldcg(&k->status);
     r.nfe = __ldcg(&k->nfe);
+    r.ovf = __ldcg(&k->ovf);
+    r.pad = 0;
     return r;
 }
 
@@ -242,15 +244,15 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_bb_levels(BbArgs a, int heavy)
         if (c.more == 0 || c.dense) break;
         ran = true;
         LvlCnt *k = a.pcnt + (lv & 3);
-        if (blockIdx.x == 0 && threadIdx.x == 0) a.pcnt[(lv + 2) & 3] = LvlCnt{0, 0, 0, 0, 0ull};
+        if (blockIdx.x == 0 && threadIdx.x == 0) a.pcnt[(lv + 2) & 3] = LvlCnt{};
         const int32_t b0 = s_off[0], b1 = s_off[1];
         bb_mark_phase(a, c, b0, b1, &k->ncand);
         if (!(ok = mgd::grid_sync(a.bar, a.bar_err))) break;
         const int32_t ncand = __ldcg(&k->ncand);
-        bb_pull_phase<TP, M>(a, c, ncand);
+        bb_pull_phase<TP, M>(a, c, ncand, k);
         if (!(ok = mgd::grid_sync(a.bar, a.bar_err))) break;
         if (heavy) {
-            bb_heavy_phase<M>(a, c);
+            bb_heavy_phase<M>(a, c, k);
             if (!(ok = mgd::grid_sync(a.bar, a.bar_err))) break;
         }
         bb_compact_phase(a, c, b0, b1, ncand, k);
@@ -258,7 +260,7 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_bb_levels(BbArgs a, int heavy)
         if (threadIdx.x == 0) {
             BbCtl n = c;
             int32_t off_d2;
-            bb_decide(n, load_cnt_l2(k), __ldcg(&a.ctl->ovf), b1, off_d2, a.m, M);
+            bb_decide(n, load_cnt_l2(k), b1, off_d2, a.m, M);
             if (blockIdx.x == 0) a.off[c.d + 2] = off_d2;
             s_c = n;
             s_off[0] = b1;
@@ -272,8 +274,7 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_bb_levels(BbArgs a, int heavy)
             n.status = 3;
             n.more = 0;
         }
-        n.ovf |= __ldcg(&a.ctl->ovf);
-        n.k = LvlCnt{0, 0, 0, 0, 0ull};
+        n.k = LvlCnt{};
         n.done = 0;
         *a.ctl = n;
     }
@@ -328,7 +329,7 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_bb_flat(BbArgs a)
         const BbCtl c = s_c;
         if (c.more == 0) break;
         LvlCnt *k = a.pcnt + (lv & 3);
-        if (blockIdx.x == 0 && threadIdx.x == 0) a.pcnt[(lv + 2) & 3] = LvlCnt{0, 0, 0, 0, 0ull};
+        if (blockIdx.x == 0 && threadIdx.x == 0) a.pcnt[(lv + 2) & 3] = LvlCnt{};
         const int32_t op = s_off[0], b0 = s_off[1], b1 = s_off[2];
         int32_t nrows = a.n;
         if (!c.dense) {
@@ -341,7 +342,7 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_bb_flat(BbArgs a)
         if (threadIdx.x == 0) {
             BbCtl n = c;
             int32_t off_d2;
-            bb_decide(n, load_cnt_l2(k), __ldcg(&a.ctl->ovf), b1, off_d2, a.m, M);
+            bb_decide(n, load_cnt_l2(k), b1, off_d2, a.m, M);
             if (blockIdx.x == 0) a.off[c.d + 2] = off_d2;
             s_c = n;
             s_off[0] = b0;
@@ -361,8 +362,7 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_bb_flat(BbArgs a)
             n.status = 3;
             n.more = 0;
         }
-        n.ovf |= __ldcg(&a.ctl->ovf);
-        n.k = LvlCnt{0, 0, 0, 0, 0ull};
+        n.k = LvlCnt{};
         n.done = 0;
         *a.ctl = n;
     }

@@ -108,13 +108,18 @@ constexpr int GTHREADS = 512;  // mask-free kernels: two blocks per SM at 64 reg
 constexpr int GPER_SM = 2;
 
 // what one forward level counts (atomics): candidates of a sparse level,
-// entries archived for the next level, their heavy entries and out-edges
+// entries archived for the next level, their heavy entries and out-edges,
+// whether a path count did not fit.  A persistent sweep's level has a slot of
+// its own for all of it: the next level's phases, which a faster block may
+// have begun, write another one, so every block decides from the same words.
 struct LvlCnt {
     int32_t ncand;
     int32_t nnew;
     int32_t nfh_build;
     int32_t status;            // 2: archive overflow
     unsigned long long nfe;
+    int32_t ovf;               // a path count reached the form's limit (ends the sweep)
+    int32_t pad;
 };
 
 struct BbCtl {
@@ -132,22 +137,22 @@ struct BbCtl {
     uint32_t gmask;     // lanes holding a source
     int32_t dense_levels;
     int32_t done;       // blocks finished (last-block-done step of the level's final kernel)
-    int32_t ovf;        // a plain-mode path count reached PC_PLAIN_MAX (ends the sweep)
+    int32_t ovf;        // a path count reached the form's limit (the sweep has ended for a rerun)
     int32_t pad;
     unsigned long long nfe_cur;  // out-edges of level d
     LvlCnt k;                    // this level's counters (per-level kernels)
 };
 
 // the next level from level d's counters; off_d2 = archive offset of level d+2
-__device__ __forceinline__ void bb_decide(BbCtl &n, const LvlCnt &k, int32_t ovf, int32_t off_d1, int32_t &off_d2,
-                                          int32_t m, int32_t mode)
+__device__ __forceinline__ void bb_decide(BbCtl &n, const LvlCnt &k, int32_t off_d1, int32_t &off_d2, int32_t m,
+                                          int32_t mode)
 {
     off_d2 = off_d1 + k.nnew;
     if (k.status) n.status = k.status;
-    if (k.nnew == 0 || n.status || ovf) {  // (a path-count overflow ends the sweep for a rerun)
+    if (k.nnew == 0 || n.status || k.ovf) {  // (a path-count overflow ends the sweep for a rerun)
         n.more = 0;
         n.nlevels = n.d + 1;
-        if (ovf) n.ovf = 1;
+        if (k.ovf) n.ovf = 1;
     } else if (n.d + 2 >= n.max_levels) {
         n.more = 0;
         n.status = 1;
@@ -410,16 +415,16 @@ __device__ __forceinline__ typename SumOf<M>::T pull_span(const BbArgs &a, const
 // row v reached at level d + 1 from the sources in newm
 template <int M>
 __device__ __forceinline__ void settle_row(const BbArgs &a, uint32_t *fnext, int32_t d, int32_t v, uint32_t newm,
-                                           typename SumOf<M>::T acc)
+                                           typename SumOf<M>::T acc, LvlCnt *k)
 {
     const int lane = mgd::lane();
     if ((newm >> lane) & 1u) {
         if constexpr (M == M_INT) {
             a.cnt[(d + 1) & 1][(size_t)v * W + lane] = (uint32_t)acc;
-            if (acc >= INT_LIMIT) a.ctl->ovf = 1;
+            if (acc >= INT_LIMIT) k->ovf = 1;
         } else {
             a.sig[(size_t)v * W + lane] = acc;
-            if (M == M_PLAIN && acc.m >= mgops::PC_PLAIN_MAX) a.ctl->ovf = 1;
+            if (M == M_PLAIN && acc.m >= mgops::PC_PLAIN_MAX) k->ovf = 1;
         }
     }
     if (lane == 0) {
@@ -435,7 +440,7 @@ __device__ __forceinline__ void settle_row(const BbArgs &a, uint32_t *fnext, int
 // row's columns, their masks and a source's counts are loaded together.
 // *reached gets those sources.
 __device__ __forceinline__ bool pull_row_thread(const BbArgs &a, const uint32_t *fcur, uint32_t *fnext, int32_t v,
-                                                uint32_t want, uint32_t *reached)
+                                                uint32_t want, uint32_t *reached, LvlCnt *k)
 {
     const int32_t b = __ldg(&a.trow[v]), e = __ldg(&a.trow[v + 1]);
     if (e - b > TDEG) return false;
@@ -467,7 +472,7 @@ __device__ __forceinline__ bool pull_row_thread(const BbArgs &a, const uint32_t 
                 if ((f[h + j] >> s) & 1u) acc = mgops::pc_add(acc, x[j], a.mode == M_EXT);
         }
         a.sig[(size_t)v * W + s] = acc;
-        if (a.mode != M_EXT && acc.m >= mgops::PC_PLAIN_MAX) a.ctl->ovf = 1;
+        if (a.mode != M_EXT && acc.m >= mgops::PC_PLAIN_MAX) k->ovf = 1;
     }
     a.vis[v] |= newm;
     fnext[v] = newm;
@@ -476,7 +481,7 @@ __device__ __forceinline__ bool pull_row_thread(const BbArgs &a, const uint32_t 
 
 // level d -> d+1 over nrows rows (every row when dense, else the candidates)
 template <bool TP, int M>
-__device__ __forceinline__ void bb_pull_phase(const BbArgs &a, const BbCtl &c, int32_t nrows)
+__device__ __forceinline__ void bb_pull_phase(const BbArgs &a, const BbCtl &c, int32_t nrows, LvlCnt *k)
 {
     const int lane = mgd::lane();
     const int gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -496,7 +501,7 @@ __device__ __forceinline__ void bb_pull_phase(const BbArgs &a, const BbCtl &c, i
                 v = c.dense ? i : a.cand[i];
                 want = ~a.vis[v] & c.gmask;
                 uint32_t reached;
-                if (want) deferred = !pull_row_thread(a, fcur, fnext, v, want, &reached);
+                if (want) deferred = !pull_row_thread(a, fcur, fnext, v, want, &reached, k);
             }
             unsigned dm = __ballot_sync(0xffffffffu, deferred);
             while (dm) {
@@ -508,7 +513,7 @@ __device__ __forceinline__ void bb_pull_phase(const BbArgs &a, const BbCtl &c, i
                 if (e - b > a.heavy_deg) continue;  // chunk path below
                 uint32_t newm;
                 const auto acc = pull_span<M>(a, fcur, c.d, b, e, wj, newm);
-                if (newm) settle_row<M>(a, fnext, c.d, vj, newm, acc);
+                if (newm) settle_row<M>(a, fnext, c.d, vj, newm, acc, k);
             }
         }
     } else {
@@ -520,7 +525,7 @@ __device__ __forceinline__ void bb_pull_phase(const BbArgs &a, const BbCtl &c, i
             if (e - b > a.heavy_deg) continue;  // chunk path below
             uint32_t newm;
             const auto acc = pull_span<M>(a, fcur, c.d, b, e, want, newm);
-            if (newm) settle_row<M>(a, fnext, c.d, v, newm, acc);
+            if (newm) settle_row<M>(a, fnext, c.d, v, newm, acc, k);
         }
     }
     for (int32_t ch = gwarp; ch < a.nhchunks; ch += nwarps) {
@@ -536,7 +541,7 @@ __device__ __forceinline__ void bb_pull_phase(const BbArgs &a, const BbCtl &c, i
 }
 
 template <int M>
-__device__ __forceinline__ void bb_heavy_phase(const BbArgs &a, const BbCtl &c)
+__device__ __forceinline__ void bb_heavy_phase(const BbArgs &a, const BbCtl &c, LvlCnt *k)
 {
     const int lane = mgd::lane();
     const int gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -547,14 +552,14 @@ __device__ __forceinline__ void bb_heavy_phase(const BbArgs &a, const BbCtl &c)
         uint32_t newm = 0;
         typename SumOf<M>::T acc{};
         const auto *part = reinterpret_cast<const typename SumOf<M>::T *>(a.hpart);
-        for (int32_t k = k0; k < k1; k++) {
-            const uint32_t hm = a.hmask[k];
+        for (int32_t ch = k0; ch < k1; ch++) {
+            const uint32_t hm = a.hmask[ch];
             newm |= hm;
             if (!((hm >> lane) & 1u)) continue;
-            if constexpr (M == M_INT) acc += part[(size_t)k * W + lane];
-            else acc = mgops::pc_add(acc, part[(size_t)k * W + lane], M == M_EXT);
+            if constexpr (M == M_INT) acc += part[(size_t)ch * W + lane];
+            else acc = mgops::pc_add(acc, part[(size_t)ch * W + lane], M == M_EXT);
         }
-        if (newm) settle_row<M>(a, fnext, c.d, v, newm, acc);
+        if (newm) settle_row<M>(a, fnext, c.d, v, newm, acc, k);
     }
 }
 
@@ -889,7 +894,7 @@ __device__ __forceinline__ void bb_flat_phase(const BbArgs &a, const BbCtl &c, i
             v = c.dense ? i : __ldcg(&a.cand[i]);
             if (!c.dense) atomicAnd(&a.cbm[v >> 5], ~(1u << (v & 31)));
             want = ~a.vis[v] & c.gmask;
-            if (want) deferred = !pull_row_thread(a, fcur, fnext, v, want, &reached);
+            if (want) deferred = !pull_row_thread(a, fcur, fnext, v, want, &reached, k);
             if (deferred) reached = 0;
         }
         unsigned dm = __ballot_sync(0xffffffffu, deferred);
@@ -900,7 +905,7 @@ __device__ __forceinline__ void bb_flat_phase(const BbArgs &a, const BbCtl &c, i
             const uint32_t wj = __shfl_sync(0xffffffffu, want, j);
             uint32_t newm;
             const auto acc = pull_span<M>(a, fcur, c.d, __ldg(&a.trow[vj]), __ldg(&a.trow[vj + 1]), wj, newm);
-            if (newm) settle_row<M>(a, fnext, c.d, vj, newm, acc);
+            if (newm) settle_row<M>(a, fnext, c.d, vj, newm, acc, k);
             if (lane == j) reached = newm;
         }
         const unsigned m = __ballot_sync(0xffffffffu, reached != 0);
@@ -1030,7 +1035,7 @@ struct Sum4 {
 // had not reached v, the row's masks updated (all eight lanes of the row's
 // group call)
 __device__ __forceinline__ void gather_settle(const BbArgs &a, uint32_t *fnext, int32_t d, int32_t v, uint32_t want,
-                                              const Sum4 &s, unsigned gmask)
+                                              const Sum4 &s, unsigned gmask, LvlCnt *cnt)
 {
     const int gl = threadIdx.x & (GL - 1);
     const unsigned long long x[4] = {s.x, s.y, s.z, s.w};
@@ -1046,7 +1051,7 @@ __device__ __forceinline__ void gather_settle(const BbArgs &a, uint32_t *fnext, 
             over |= x[k] >= INT_LIMIT;
         }
     }
-    if (over) a.ctl->ovf = 1;
+    if (over) cnt->ovf = 1;
     const uint32_t newm = __reduce_or_sync(gmask, m);
     if (gl == 0 && newm) {
         a.vis[v] |= newm;
@@ -1056,7 +1061,7 @@ __device__ __forceinline__ void gather_settle(const BbArgs &a, uint32_t *fnext, 
 
 __device__ __forceinline__ unsigned group_mask() { return 0xffu << (mgd::lane() & ~(GL - 1)); }
 
-__device__ __forceinline__ void bb_gather_phase(const BbArgs &a, const BbCtl &c)
+__device__ __forceinline__ void bb_gather_phase(const BbArgs &a, const BbCtl &c, LvlCnt *k)
 {
     constexpr int RPW = 32 / GL;
     const int gl = threadIdx.x & (GL - 1), grp = mgd::lane() / GL;
@@ -1091,7 +1096,7 @@ __device__ __forceinline__ void bb_gather_phase(const BbArgs &a, const BbCtl &c)
         const bool row = want != 0 && e - b <= GCHUNK;
         Sum4 s;
         gather_rows(val, a.tcol, b, row ? e : b, [&](const uint4 (&t)[GL]) { s.add(t); });
-        if (row) gather_settle(a, fnext, c.d, v, want, s, gm);
+        if (row) gather_settle(a, fnext, c.d, v, want, s, gm, k);
         v = vn;
         want = wn;
         b = bn;
@@ -1100,7 +1105,7 @@ __device__ __forceinline__ void bb_gather_phase(const BbArgs &a, const BbCtl &c)
 }
 
 // rows above GCHUNK edges: their chunks' sums
-__device__ __forceinline__ void bb_gather_heavy_phase(const BbArgs &a, const BbCtl &c)
+__device__ __forceinline__ void bb_gather_heavy_phase(const BbArgs &a, const BbCtl &c, LvlCnt *cnt)
 {
     constexpr int RPW = 32 / GL;
     const int gl = threadIdx.x & (GL - 1), grp = mgd::lane() / GL;
@@ -1127,7 +1132,7 @@ __device__ __forceinline__ void bb_gather_heavy_phase(const BbArgs &a, const BbC
             s.z += __shfl_xor_sync(0xffffffffu, s.z, o);
             s.w += __shfl_xor_sync(0xffffffffu, s.w, o);
         }
-        if (grp == 0) gather_settle(a, fnext, c.d, v, want, s, 0xffu);
+        if (grp == 0) gather_settle(a, fnext, c.d, v, want, s, 0xffu, cnt);
     }
 }
 
