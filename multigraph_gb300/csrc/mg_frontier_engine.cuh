@@ -518,7 +518,9 @@ __device__ __noinline__ void cta_push_levels(const Args &a, FCtl &c, CtaShared &
             }
             if (held) s.hash[s.slot[i]] = -1;
         }
-        if constexpr (Op::kPathCounts) __syncthreads();
+        // every warp has read s.count (thread 0 sets it back below) and, with
+        // path counts, every label test of the sums above is done
+        __syncthreads();
         for (int i = t; i < nq; i += PTHREADS) a.label[i < CTA_Q ? s.v[p ^ 1][i] : a.queue[out + i]] = it1;
         if (t == 0) {
             FCtl n = c;
