@@ -958,6 +958,9 @@ static mg_status upload_arrays(mg_graph *g, const mg_host_graph *h, const HostLa
     g->hub.valid = false;  // new pull columns
     g->col_version += 1;
     g->h_prow = L.prow;
+    g->short_pull = true;
+    for (size_t v = 0; v + 1 < L.prow.size() && g->short_pull; v++)
+        g->short_pull = L.prow[v + 1] - L.prow[v] < SHORT_PULL;
     g->symmetric = L.symmetric;
     g->weights_symmetric = L.wsym;
     g->n_dangling = L.n_dangling;

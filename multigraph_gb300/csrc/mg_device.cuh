@@ -105,6 +105,7 @@ mg_status run_loop(int exec_mode, bool profile, cudaStream_t stream, LoopGraph &
 // memory; partial sums per (row, segment) pair; ids past the last segment
 // stay in an int32 tail (offsets toff) gathered through L2
 namespace mgi {
+constexpr int32_t SHORT_PULL = 128;  // (out-degrees of 128 or more relabel a graph; in-degrees do not)
 constexpr int HUB_WIN = 512;   // piece sums the row finish stages in shared memory a warp (32 rows)
 struct HubSplit {
     bool valid = false;      // built for the current pull columns
@@ -187,6 +188,7 @@ struct mg_graph {
     int32_t hchunk_size = 0;       // edges per heavy chunk
     int32_t tbin = 0;              // rows up to this in-degree are in the thread bin
     std::vector<int32_t> h_prow;   // pull-side row offsets (engine order), for re-binning
+    bool short_pull = false;       // no pull row has SHORT_PULL in-edges or more
     int32_t n_dangling = 0;        // vertices with out-degree 0
     int32_t min_weight = 0;        // smallest integer edge weight
     // pull rows above 256 in-edges in 256-edge chunks (personalised PageRank,

@@ -112,6 +112,7 @@ struct Args {
     int4 *heavy;         // 2 * hcap chunks (parity): vertex, first edge, end
     int32_t hcap;
     int32_t has_heavy;   // some vertex may have more than PUSH_HEAVY out-edges
+    int32_t short_pull;  // no vertex has SHORT_PULL in-edges or more
     int32_t *lvl_off;
     FCtl *ctl;
     unsigned *bar;       // grid barrier words of the persistent kernels
@@ -944,11 +945,16 @@ __device__ __forceinline__ void store_ctl_push(FCtl *p, const FCtl &c)
     for (int i = 0; i < (int)(sizeof(FCtl) / 8) - 1; i++) __stcg(&d[i], src[i]);
 }
 
-// whether the next push levels are block 0's alone
+// Whether the next push levels are block 0's alone.  Path counts are summed
+// there over a new vertex's whole in-row by one thread: not on a directed
+// graph with long in-rows, of which its out-degrees say nothing (reaching a
+// vertex of two million in-edges: 220 ms by one thread, 0.4 ms in the grid's
+// levels, which touch the frontier's out-edges only).
 template <class Op, bool HEAVY>
-__device__ __forceinline__ bool block_phase_due(const FCtl &c)
+__device__ __forceinline__ bool block_phase_due(const Args &a, const FCtl &c)
 {
-    return !HEAVY && Op::kLevelSync && c.qsize <= CTA_ENTER && c.qedges <= CTA_EDGES;
+    return !HEAVY && Op::kLevelSync && (!Op::kPathCounts || a.short_pull) && c.qsize <= CTA_ENTER &&
+           c.qedges <= CTA_EDGES;
 }
 
 // Block 0's levels while the others wait; false when a barrier failed
@@ -995,7 +1001,7 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_sparse_levels(Args a)
             z->nhcur = 0;
             z->nfe = 0;
         }
-        if (block_phase_due<Op, HEAVY>(s_c)) {
+        if (block_phase_due<Op, HEAVY>(a, s_c)) {
             if (!block_phase<Op>(a, s_c)) break;
             continue;
         }
@@ -1129,7 +1135,7 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_frontier_all(Args a, StartArgs 
             z->fmin = INT32_MAX;
         }
         if (s_c.mode == MODE_PUSH) {
-            if (block_phase_due<Op, HEAVY>(s_c)) {
+            if (block_phase_due<Op, HEAVY>(a, s_c)) {
                 ok = block_phase<Op>(a, s_c);
                 continue;
             }
@@ -1324,6 +1330,7 @@ inline Args make_args(mg_graph *g)
     a.heavy = w->heavy.as<int4>();
     a.hcap = heavy_cap(g->ne);
     a.has_heavy = g->relabeled;  // (graphs with a degree of 128 or more are relabeled)
+    a.short_pull = g->short_pull;
     a.lvl_off = w->lvl_off.as<int32_t>();
     a.ctl = w->ctl.as<FCtl>();
     a.bar = w->bar.as<unsigned>();
