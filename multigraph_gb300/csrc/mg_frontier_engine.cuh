@@ -409,6 +409,14 @@ struct CtaShared {
     int32_t nfe;                          // (at most CTA_EDGES vertices of fewer than 128 edges)
 };
 
+// The block tells new vertices by their label and writes the level as the
+// label: the built-in operators' labels, whose start value is UNSET.  Another
+// level-synchronous operator may start its labels at any value (even at the
+// source's) and label by its own offer; the grid's levels claim by the visited
+// bitmap and run it.
+template <class Op>
+constexpr bool kBlockLevels = std::is_same<Op, mgops::Bfs>::value || std::is_same<Op, mgops::BcForward>::value;
+
 // Runs levels from the loop state c (shared memory, all threads of block 0
 // call) until the frontier outgrows the block, the traversal ends or the
 // direction switch picks pull; the queue archive, labels, visited bits and
@@ -417,7 +425,7 @@ struct CtaShared {
 template <class Op>
 __device__ __noinline__ void cta_push_levels(const Args &a, FCtl &c, CtaShared &s)
 {
-    static_assert(Op::kLevelSync, "labels are levels");
+    static_assert(kBlockLevels<Op>, "labels are levels, UNSET before");
     const int t = threadIdx.x;
     for (int i = t; i < CTA_HASH; i += PTHREADS) s.hash[i] = -1;
     for (int i = t; i < c.qsize; i += PTHREADS) {
@@ -745,7 +753,7 @@ __device__ __forceinline__ void pull_level(const Args &a, const FCtl &c, int32_t
                 s_skip = Op::kMinPlusBound && a.label[v] <= bound;
             } else {
                 const int32_t lv = __ldcg(&a.label[v]);
-                s_skip = lv != mgops::UNSET && lv != it1;
+                s_skip = lv != Op::initialize() && lv != it1;
             }
         }
         __syncthreads();
@@ -953,7 +961,7 @@ __device__ __forceinline__ void store_ctl_push(FCtl *p, const FCtl &c)
 template <class Op, bool HEAVY>
 __device__ __forceinline__ bool block_phase_due(const Args &a, const FCtl &c)
 {
-    return !HEAVY && Op::kLevelSync && (!Op::kPathCounts || a.short_pull) && c.qsize <= CTA_ENTER &&
+    return !HEAVY && kBlockLevels<Op> && (!Op::kPathCounts || a.short_pull) && c.qsize <= CTA_ENTER &&
            c.qedges <= CTA_EDGES;
 }
 
@@ -961,7 +969,7 @@ __device__ __forceinline__ bool block_phase_due(const Args &a, const FCtl &c)
 template <class Op>
 __device__ __forceinline__ bool block_phase(const Args &a, FCtl &c)
 {
-    if constexpr (Op::kLevelSync) {
+    if constexpr (kBlockLevels<Op>) {
         // the bitmaps start from zero
         for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 3 * a.words; i += gridDim.x * blockDim.x) a.bm[i] = 0;
         if (!mgd::grid_sync(a.bar, a.bar_err, a.bar_never)) return false;
