@@ -104,12 +104,15 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_bc_back_heavy(Args a, BCtl *bc_
             if (!mgd::grid_sync(a.bar, a.bar_err, a.bar_never)) return;
             continue;
         }
-        // one gathered term: the successor's q, scaled to the entry's count
+        // One gathered term: the successor's q, scaled to the entry's count.
+        // A successor's count is at least the entry's, so only scales down:
+        // a neighbour of a smaller scale is one level up, its q still zero,
+        // and must not be multiplied by an infinite 2^(512 dk).
         auto term = [&](int32_t w, int32_t ku) {
             QT<EXT> t = qi[w];
             if (EXT) {
                 const int32_t dk = ku - a.sigma[w].k;
-                if (dk != 0) t *= (QT<EXT>)mgops::pc_scale(dk);
+                if (dk < 0) t *= (QT<EXT>)mgops::pc_scale(dk);
             }
             return t;
         };
