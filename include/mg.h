@@ -178,8 +178,9 @@ typedef struct mg_opts {
     int32_t profile;       /* 1: host loop with cudaEvents around each kernel  */
     int32_t pr_layout;     /* PageRank pull sweep over unweighted graphs:      */
                            /* MG_PR_LAYOUT_AUTO (default: segmented where it   */
-                           /* applies, unless mg_autotune measured the gather  */
-                           /* layout faster on this graph),                    */
+                           /* applies; MG_PR_TOPOLOGY on small graphs in one   */
+                           /* launch without a layout; after mg_autotune       */
+                           /* whichever it measured faster on this graph),     */
                            /* MG_PR_LAYOUT_GATHER (L2 gathers over degree      */
                            /* bins) or MG_PR_LAYOUT_SEGMENTED (shared-memory   */
                            /* segments; gather where a quarter of the edges    */
@@ -307,7 +308,7 @@ mg_status mg_batch_cc(mg_batch *b, const mg_opts *o, int32_t *labels_out, mg_run
  * call).  MG_ALGO_PR tunes the pull layout instead: the heavy-row threshold,
  * the chunk size and the thread-bin cutoff of the degree bins, applied to
  * the graph itself (every pull kernel uses them; *tuned is left as passed,
- * `source` is ignored). */
+ * `source` is ignored), and what MG_PR_LAYOUT_AUTO takes on the graph. */
 enum { MG_ALGO_BFS = 0, MG_ALGO_SSSP = 1, MG_ALGO_BC = 2, MG_ALGO_CC = 3, MG_ALGO_PR = 4 };
 mg_status mg_autotune(mg_graph *dg, int32_t algo, int32_t source, const char *cache_path, mg_opts *tuned);
 

@@ -1097,6 +1097,7 @@ static void drop_workspaces(mg_graph *g)
     g->ppr_nhrows = 0;
     // a new layout has not been timed by mg_autotune
     g->pr_prefer_gather = false;
+    g->pr_no_one_launch = false;
 }
 
 mg_status mg_graph_commit(mg_graph *g)

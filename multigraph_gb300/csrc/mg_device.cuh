@@ -205,6 +205,7 @@ struct mg_graph {
     // log2 degree; results are mapped back before they leave the library
     bool relabeled = false;
     bool pr_prefer_gather = false; // mg_autotune measured the gather PageRank layout faster (MG_PR_LAYOUT_AUTO)
+    bool pr_no_one_launch = false; // mg_autotune measured the one-launch PageRank slower than the tuned layout
     mgi::DevBuf o_row, o_col, o_wt;        // the CSR in the caller's ids (as uploaded)
     mgi::DevBuf o_fw;                      // float weights in caller CSR order
     mgi::DevBuf old2new, new2old;          // int32 [nv]
@@ -297,6 +298,8 @@ mg_status edge_grad_to_caller(mg_graph *g, const float2 *ct, const float *val, f
 // bin cutoff) from the
 // host copy of the pull-side row offsets; drops the algorithm workspaces
 mg_status rebin(mg_graph *g, int32_t heavy, int32_t chunk, int32_t tbin);
+// whether the graph's size lets a default-layout PageRank run in one launch
+bool pr_one_launch_size(const mg_graph *g);
 // the table of rows above 256 in-edges (once per layout)
 mg_status ppr_chunks(mg_graph *g);
 // batched multi-source BC over engine-id sources (symmetric graphs); the

@@ -1801,13 +1801,12 @@ static mg_status pr_loop(mg_graph *g, PArgs &a, const mg_opts &opt, const char *
     return pr_outcome(g, hc, Op::kDataDriven, max_iter, info, final_cur);
 }
 
-// Whether a run takes the one-launch form.  A host-driven or profiled loop
-// and a layout the caller names keep their kernels.
+// Whether a run takes the one-launch form.  A host-driven or profiled loop, a
+// layout the caller names and one that mg_autotune measured faster on this
+// graph keep their kernels.
 static bool pr_small(const mg_graph *g, const mg_opts &opt, bool named_layout)
 {
-    const bool short_rows = !g->relabeled && (int64_t)g->ne <= (int64_t)8 * g->nv;  // (as ppr_chunks)
-    return opt.exec == MG_EXEC_GRAPH && !opt.profile && !named_layout && g->nv > 0 &&
-           g->ne <= (short_rows ? ALL_MAX_EDGES_SHORT : ALL_MAX_EDGES);
+    return opt.exec == MG_EXEC_GRAPH && !opt.profile && !named_layout && !g->pr_no_one_launch && pr_one_launch_size(g);
 }
 
 // the one-launch form, after the control block's start values; out: result
@@ -2168,6 +2167,12 @@ mg_status mg_wpagerank_backward(mg_graph *g, const float *g_host, const mg_opts 
 }
 
 }  // extern "C"
+
+bool mgi::pr_one_launch_size(const mg_graph *g)
+{
+    const bool short_rows = !g->relabeled && (int64_t)g->ne <= (int64_t)8 * g->nv;  // (as ppr_chunks)
+    return g->nv > 0 && g->ne <= (short_rows ? ALL_MAX_EDGES_SHORT : ALL_MAX_EDGES);
+}
 
 // heavy-row chunk table (built once per layout from the pull offsets)
 mg_status mgi::ppr_chunks(mg_graph *g)

@@ -16,7 +16,9 @@
 // direction, or heavy threshold / chunk edges / thread-bin cutoff for
 // PageRank, the winner's time, and for PageRank the layout that
 // MG_PR_LAYOUT_AUTO takes on the graph (gather or segmented, whichever ran
-// faster once the gather layout's bins were tuned).
+// faster once the gather layout's bins were tuned) and, on graphs small enough
+// for PageRank in one launch, whether that was faster still (1) or not (0; a
+// line without the word says nothing about it).
 
 #include "mg_device.cuh"
 
@@ -47,7 +49,8 @@ uint64_t graph_signature(mg_graph *g)
     return h;
 }
 
-bool cache_lookup(const char *path, uint64_t sig, int algo, mg_opts *o)
+// one_launch: PageRank's last word of the line, -1 where it has none
+bool cache_lookup(const char *path, uint64_t sig, int algo, mg_opts *o, int *one_launch = nullptr)
 {
     if (!path) return false;
     FILE *f = std::fopen(path, "r");
@@ -56,14 +59,15 @@ bool cache_lookup(const char *path, uint64_t sig, int algo, mg_opts *o)
     bool found = false;
     while (std::fgets(line, sizeof(line), f)) {
         unsigned long long s;
-        int a, alpha, beta, dir, lay = -1;
+        int a, alpha, beta, dir, lay = -1, one = -1;
         double ms;
-        const int k = std::sscanf(line, "%llx %d %d %d %d %lf %d", &s, &a, &alpha, &beta, &dir, &ms, &lay);
+        const int k = std::sscanf(line, "%llx %d %d %d %d %lf %d %d", &s, &a, &alpha, &beta, &dir, &ms, &lay, &one);
         if (k >= 5 && s == sig && a == algo) {
             o->alpha = alpha;
             o->beta = beta;
             o->direction = dir;
-            if (algo == MG_ALGO_PR && k == 7) o->pr_layout = lay;   // the layout MG_PR_LAYOUT_AUTO takes
+            if (algo == MG_ALGO_PR && k >= 7) o->pr_layout = lay;   // the layout MG_PR_LAYOUT_AUTO takes
+            if (one_launch) *one_launch = one;
             found = true;  // the last entry wins
         }
     }
@@ -71,13 +75,15 @@ bool cache_lookup(const char *path, uint64_t sig, int algo, mg_opts *o)
     return found;
 }
 
-void cache_store(const char *path, uint64_t sig, int algo, const mg_opts &o, double ms)
+void cache_store(const char *path, uint64_t sig, int algo, const mg_opts &o, double ms, int one_launch = -1)
 {
     if (!path) return;
     FILE *f = std::fopen(path, "a");
     if (!f) return;
-    std::fprintf(f, "%llx %d %d %d %d %.4f %d\n", (unsigned long long)sig, algo, o.alpha, o.beta, o.direction, ms,
+    std::fprintf(f, "%llx %d %d %d %d %.4f %d", (unsigned long long)sig, algo, o.alpha, o.beta, o.direction, ms,
                  o.pr_layout);
+    if (one_launch >= 0) std::fprintf(f, " %d", one_launch);
+    std::fprintf(f, "\n");
     std::fclose(f);
 }
 
@@ -99,12 +105,15 @@ static mg_status pr_median_ms(mg_graph *g, const mg_opts &o, double *ms)
 // gather layout's degree bins (timed with that layout), then whether the
 // segmented layout beats the tuned gather layout on this graph (the choice
 // of MG_PR_LAYOUT_AUTO); for the segmented layout also the split of the
-// sweep's work among the CTAs (mgi::hub_rebalance)
+// sweep's work among the CTAs (mgi::hub_rebalance).  On small graphs the
+// one-launch form, which AUTO takes there untuned, runs against the winner.
 mg_status tune_pr_layout(mg_graph *g, const char *cache_path, uint64_t sig, const mg_opts &base)
 {
     mg_opts cached = base;
     cached.pr_layout = -1;   // set by a cache line that records the layout
-    if (cache_lookup(cache_path, sig, MG_ALGO_PR, &cached)) {
+    int one = -1;
+    if (cache_lookup(cache_path, sig, MG_ALGO_PR, &cached, &one)) {
+        g->pr_no_one_launch = one == 0;
         if (cached.pr_layout == MG_PR_LAYOUT_GATHER || cached.pr_layout == MG_PR_LAYOUT_SEGMENTED)
             g->pr_prefer_gather = cached.pr_layout == MG_PR_LAYOUT_GATHER;
         return mgi::rebin(g, cached.alpha, cached.beta, cached.direction);
@@ -149,13 +158,21 @@ mg_status tune_pr_layout(mg_graph *g, const char *cache_path, uint64_t sig, cons
             else mgi::hub_weights(g, nullptr, &w0);
         }
         g->pr_prefer_gather = seg_ms > best_ms;
+        if (mgi::pr_one_launch_size(g)) {
+            o.pr_layout = MG_PR_LAYOUT_AUTO;
+            g->pr_no_one_launch = false;
+            double one_ms = 0.0;
+            MG_TRY(pr_median_ms(g, o, &one_ms));
+            one = one_ms <= std::min(seg_ms, best_ms);
+            g->pr_no_one_launch = one == 0;
+        }
     }
     mg_opts rec = base;
     rec.alpha = best.heavy;
     rec.beta = best.chunk;
     rec.direction = best.tbin;
     rec.pr_layout = g->pr_prefer_gather ? MG_PR_LAYOUT_GATHER : MG_PR_LAYOUT_SEGMENTED;
-    cache_store(cache_path, sig, MG_ALGO_PR, rec, best_ms);
+    cache_store(cache_path, sig, MG_ALGO_PR, rec, best_ms, one);
     return MG_OK;
 }
 
