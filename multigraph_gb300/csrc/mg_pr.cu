@@ -1335,9 +1335,11 @@ __global__ void __launch_bounds__(THREADS) k_back_rows(PArgs a, const float *__r
 // gather of eight edges a lane in 32 registers kept 55 KB.
 // R-MAT 20, 32 seeds: 527 -> 358 us per sweep (11.5 TB/s of gathers).
 //
-// Sums run in a fixed order that does not depend on LPR (pairwise over eight
-// consecutive edges, the eights compensated in order), so a hub's total does
-// not drift between sweeps.
+// Sums run in a fixed order that does not depend on LPR: pairwise over eight
+// consecutive edges, the eights compensated in order; a heavy row's chunks in
+// eight streams.  So a hub's total does not drift between sweeps, and a seed's
+// ranks do not depend on how many seeds share its pass.  The update takes a
+// total as a pair high + low and rounds once.
 // ---------------------------------------------------------------------------
 constexpr int32_t PPR_HEAVY = 256;
 constexpr int PPR_THREADS = 512;       // two blocks per SM at 64 registers
@@ -1424,22 +1426,50 @@ __device__ __forceinline__ PprLane ppr_lane(const PPArgs &a)
     return l;
 }
 
+// a gathered sum, high + low
+struct PprSum {
+    float4 hi, lo;
+};
+
+__device__ __forceinline__ float4 f4_neg(float4 a) { return make_float4(-a.x, -a.y, -a.z, -a.w); }
+
+__device__ __forceinline__ float4 f4_xor(float4 a, int o)
+{
+    return make_float4(__shfl_xor_sync(0xffffffffu, a.x, o), __shfl_xor_sync(0xffffffffu, a.y, o),
+                       __shfl_xor_sync(0xffffffffu, a.z, o), __shfl_xor_sync(0xffffffffu, a.w, o));
+}
+
+// a += b, the same value in either operand order (TwoSum)
+__device__ __forceinline__ void ppr_pair_add(PprSum &a, const PprSum &b)
+{
+    auto add = [](float &h, float &l, float x, float y) {
+        const float u = h + x, bp = u - h;
+        l = (l + y) + ((h - (u - bp)) + (x - bp));
+        h = u;
+    };
+    add(a.hi.x, a.lo.x, b.hi.x, b.lo.x);
+    add(a.hi.y, a.lo.y, b.hi.y, b.lo.y);
+    add(a.hi.z, a.lo.z, b.hi.z, b.lo.z);
+    add(a.hi.w, a.lo.w, b.hi.w, b.lo.w);
+}
+
 // row v's update from its gathered sum s (this lane's four seeds)
 template <int LPR, bool DANG>
-__device__ __forceinline__ void ppr_apply(const PPArgs &a, int cur, int32_t v, float4 s4, PprLane &l)
+__device__ __forceinline__ void ppr_apply(const PPArgs &a, int cur, int32_t v, const PprSum &sum, PprLane &l)
 {
     const int gl = threadIdx.x & (LPR - 1);
     const size_t at = (size_t)v * LPR + gl;
     const int32_t od = __ldg(&a.outrow[v + 1]) - __ldg(&a.outrow[v]);
     // the iterate is streamed; L2 is kept for the contributions
     const float4 xo4 = __ldcs(&a.X[cur][at]);
-    const float s[4] = {s4.x, s4.y, s4.z, s4.w}, xo[4] = {xo4.x, xo4.y, xo4.z, xo4.w};
+    const float s[4] = {sum.hi.x, sum.hi.y, sum.hi.z, sum.hi.w}, low[4] = {sum.lo.x, sum.lo.y, sum.lo.z, sum.lo.w};
+    const float xo[4] = {xo4.x, xo4.y, xo4.z, xo4.w};
     float xn[4], cn[4];
 #pragma unroll
     for (int k = 0; k < 4; k++) {
         float base = 0.0f;
         if (v == l.seed[k]) base = (1.0f - a.damping) + a.damping * (float)a.dang[gl * 4 + k];
-        xn[k] = base + a.damping * s[k];
+        xn[k] = fmaf(a.damping, s[k], fmaf(a.damping, low[k], base));
         cn[k] = od > 0 ? xn[k] / (float)od : 0.0f;
         mgd::kahan_add(l.r[k], l.rc[k], fabsf(xn[k] - xo[k]));
         if (DANG && od == 0) mgd::kahan_add(l.d[k], l.dc[k], xn[k]);
@@ -1453,7 +1483,7 @@ __device__ __forceinline__ void ppr_apply(const PPArgs &a, int cur, int32_t v, f
 // of their ranges; the next eight ids are loaded ahead of the current
 // gathers.
 template <int LPR>
-__device__ __forceinline__ float4 ppr_gather(const float4 *__restrict__ C, const int32_t *__restrict__ pcol, int32_t b,
+__device__ __forceinline__ PprSum ppr_gather(const float4 *__restrict__ C, const int32_t *__restrict__ pcol, int32_t b,
                                              int32_t e)
 {
     constexpr int IPL = 8 / LPR;   // ids a lane loads of eight
@@ -1482,7 +1512,7 @@ __device__ __forceinline__ float4 ppr_gather(const float4 *__restrict__ C, const
         f4_kahan(acc, low, f4_add(f4_add(f4_add(t[0], t[1]), f4_add(t[2], t[3])),
                                   f4_add(f4_add(t[4], t[5]), f4_add(t[6], t[7]))));
     }
-    return acc;
+    return PprSum{acc, f4_neg(low)};
 }
 
 // the block's residual and dangling sums of every seed to bpart[slot]
@@ -1532,8 +1562,8 @@ __global__ void __launch_bounds__(PPR_THREADS, PPR_PER_SM) k_ppr_sweep(PPArgs a)
         const int32_t ch = c0 + grp;
         const bool ok = ch < a.nhchunks;
         const int32_t b = ok ? __ldg(&a.hchunk[3 * ch + 1]) : 0, e = ok ? __ldg(&a.hchunk[3 * ch + 2]) : 0;
-        const float4 s = ppr_gather<LPR>(C, a.pcol, b, e);
-        if (ok) a.hpart[(size_t)ch * LPR + gl] = s;
+        const PprSum s = ppr_gather<LPR>(C, a.pcol, b, e);
+        if (ok) a.hpart[(size_t)ch * LPR + gl] = f4_add(s.hi, s.lo);
     }
     // the next rows' offsets are loaded ahead of the current rows' gathers
     int32_t v = gwarp * RPW + grp;
@@ -1542,7 +1572,7 @@ __global__ void __launch_bounds__(PPR_THREADS, PPR_PER_SM) k_ppr_sweep(PPArgs a)
         const int32_t vn = v + nwarps * RPW;
         const int32_t bn = vn < a.n ? __ldg(&a.prow[vn]) : 0, en = vn < a.n ? __ldg(&a.prow[vn + 1]) : 0;
         const bool row = v < a.n && e - b <= PPR_HEAVY;
-        const float4 s = ppr_gather<LPR>(C, a.pcol, b, row ? e : b);
+        const PprSum s = ppr_gather<LPR>(C, a.pcol, b, row ? e : b);
         if (row) ppr_apply<LPR, DANG>(a, cur, v, s, l);
         v = vn;
         b = bn;
@@ -1551,8 +1581,8 @@ __global__ void __launch_bounds__(PPR_THREADS, PPR_PER_SM) k_ppr_sweep(PPArgs a)
     ppr_block_partials<LPR, PPR_THREADS>(a, blockIdx.x, l);
 }
 
-// Closes a sweep: the heavy rows (a warp each: its lane groups take every
-// (32 / LPR)-th chunk, combined by a fixed xor tree), then the last block to
+// Closes a sweep: the heavy rows (a warp each: eight streams of every eighth
+// chunk whatever LPR, a lane group one or two, combined by a fixed tree), then the last block to
 // arrive adds up every block's residual and dangling sums (a warp per share
 // of the slots, fixed order) and updates the loop state.  (One warp adding
 // 2,432 slots one after another took 300 us of an 830 us sweep.)
@@ -1566,26 +1596,35 @@ __global__ void __launch_bounds__(PPR_CLOSE_THREADS, PPR_CLOSE_PER_SM) k_ppr_clo
         return;
     }
     constexpr int RPW = 32 / LPR, NW = PPR_CLOSE_THREADS / 32;
+    constexpr int STREAMS = 8, PER = RPW < STREAMS ? STREAMS / RPW : 1;   // streams of chunks; a lane group's
     const int cur = ctl->cur;
     const int gl = threadIdx.x & (LPR - 1), grp = mgd::lane() / LPR, warp = threadIdx.x >> 5;
     const int gwarp = blockIdx.x * NW + warp;
     PprLane l = ppr_lane<LPR>(a);
     for (int32_t i = gwarp; i < a.nhrows; i += gridDim.x * NW) {
-        const int32_t v = __ldg(&a.hrows[i]), k1 = __ldg(&a.hrow_chunk[i + 1]);
-        int32_t k = __ldg(&a.hrow_chunk[i]) + grp;
-        float4 s = make_float4(0.f, 0.f, 0.f, 0.f), low = s;
-        for (; k + 3 * RPW < k1; k += 4 * RPW) {
-            float4 t[4];
+        const int32_t v = __ldg(&a.hrows[i]), k0 = __ldg(&a.hrow_chunk[i]), k1 = __ldg(&a.hrow_chunk[i + 1]);
+        float4 s[PER], low[PER];
 #pragma unroll
-            for (int j = 0; j < 4; j++) t[j] = __ldcs(&a.hpart[(size_t)(k + j * RPW) * LPR + gl]);
-            f4_kahan(s, low, f4_add(f4_add(t[0], t[1]), f4_add(t[2], t[3])));
+        for (int p = 0; p < PER; p++) s[p] = low[p] = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int32_t k = k0 + grp; k < k1 && grp < STREAMS; k += 4 * STREAMS) {
+            float4 t[PER][4];
+#pragma unroll
+            for (int p = 0; p < PER; p++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const int32_t at = k + p * RPW + j * STREAMS;
+                    t[p][j] = at < k1 ? __ldcs(&a.hpart[(size_t)at * LPR + gl]) : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+#pragma unroll
+            for (int p = 0; p < PER; p++)
+                f4_kahan(s[p], low[p], f4_add(f4_add(t[p][0], t[p][1]), f4_add(t[p][2], t[p][3])));
         }
-        for (; k < k1; k += RPW) f4_kahan(s, low, __ldcs(&a.hpart[(size_t)k * LPR + gl]));
+        // the streams' totals, i and i + 4, then i and i + 2, then i and i + 1
+        PprSum x{s[0], f4_neg(low[0])};
+        if (PER == 2) ppr_pair_add(x, PprSum{s[PER - 1], f4_neg(low[PER - 1])});
 #pragma unroll
-        for (int o = LPR; o < 32; o <<= 1)
-            s = f4_add(s, make_float4(__shfl_xor_sync(0xffffffffu, s.x, o), __shfl_xor_sync(0xffffffffu, s.y, o),
-                                      __shfl_xor_sync(0xffffffffu, s.z, o), __shfl_xor_sync(0xffffffffu, s.w, o)));
-        if (grp == 0) ppr_apply<LPR, DANG>(a, cur, v, s, l);
+        for (int o = (PER == 2 ? 2 : 4) * LPR; o >= LPR; o >>= 1) ppr_pair_add(x, PprSum{f4_xor(x.hi, o), f4_xor(x.lo, o)});
+        if (grp == 0) ppr_apply<LPR, DANG>(a, cur, v, x, l);
     }
     ppr_block_partials<LPR, PPR_CLOSE_THREADS>(a, sweep_blocks + blockIdx.x, l);
     __shared__ int s_last;
