@@ -775,7 +775,7 @@ struct PrAllArgs {
     const int32_t *chunk, *chunk_at, *rows, *row_chunk;  // rows above ALL_CHUNK edges (mgi::ppr_chunks)
     int32_t nchunks;
     int32_t split;          // rows [0, split) take eight lanes, the others a thread each
-    int32_t *arrive;        // [rows] chunks finished (zero before the launch, only grows)
+    int32_t *arrive;        // [rows] chunks finished (zero before the launch and between sweeps)
     float *part;            // [chunks] partial sums
     double *bsum;           // [2][grid][3] blocks' sums by sweep parity
     unsigned *bar;          // grid barrier word (zero before the launch), error word
@@ -821,7 +821,8 @@ __global__ void __launch_bounds__(ALL_THREADS, 1) k_pr_all(PArgs a, PrAllArgs z)
             if (lane == 0) {
                 __stcg(&z.part[ch], s);
                 __threadfence();
-                last = (atomicAdd(&z.arrive[at], 1) + 1) % (k1 - k0) == 0;
+                last = atomicAdd(&z.arrive[at], 1) == k1 - k0 - 1;
+                if (last) z.arrive[at] = 0;   // (the next sweep adds to it behind the barrier)
             }
             if (__shfl_sync(FULL, last, 0)) {
                 __threadfence();
