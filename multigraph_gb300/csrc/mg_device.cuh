@@ -375,6 +375,24 @@ __device__ __forceinline__ float warp_sum_comp(float t, float r)
     return v + c;
 }
 
+// The same total as an exact pair high + low, the low parts of t - r kept.
+template <int G = 32>
+__device__ __forceinline__ float2 warp_pair_comp(float t, float r)
+{
+    float v = t, c = -r;
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) {
+        const float vo = __shfl_xor_sync(0xffffffffu, v, o);
+        const float co = __shfl_xor_sync(0xffffffffu, c, o);
+        const float u = v + vo;
+        const float bp = u - v;
+        const float e = (v - (u - bp)) + (vo - bp);
+        c = (c + co) + e;
+        v = u;
+    }
+    return make_float2(v, c);
+}
+
 // warp-bin rows below this many edges are summed by an 8-lane group (four
 // rows per warp in flight, mg_bins.cuh), longer ones by a whole warp
 constexpr int32_t SUBWARP_MAX = 128;
