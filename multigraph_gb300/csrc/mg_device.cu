@@ -196,32 +196,39 @@ int launch_grid(const mg_graph *g, int threads, int per_sm)
 #define MADV_POPULATE_WRITE 23   // Linux 5.14
 #endif
 
-HostPages::HostPages(mg_graph *graph, std::initializer_list<HostCopy> arrays) : g(graph)
+HostPages::HostPages(mg_graph *graph, std::initializer_list<HostCopy> arrays) noexcept : g(graph)
 {
     constexpr size_t POPULATE_MIN = 1 << 20;
-    for (const HostCopy &c : arrays)
-        if (c.host && c.bytes >= POPULATE_MIN) todo.push_back(c);
+    for (const HostCopy &c : arrays) {
+        if (!c.host || c.bytes < POPULATE_MIN || ntodo == ARRAYS) continue;
+        // (page-locked pages are there already, managed ones may be the device's)
+        cudaPointerAttributes at;
+        if (cudaPointerGetAttributes(&at, c.host) != cudaSuccess) (void)cudaGetLastError();
+        else if (at.type == cudaMemoryTypeUnregistered) todo[ntodo++] = c;
+    }
     g->pages = this;
 }
 
-void HostPages::start()
+void HostPages::start() noexcept
 {
-    constexpr size_t PER_THREAD = 16 << 20, MOST = 8;
+    constexpr size_t PER_THREAD = 16 << 20, MOST = PARTS;
     const size_t page = (size_t)sysconf(_SC_PAGESIZE);
-    for (const HostCopy &c : todo) {
+    for (int i = 0; i < ntodo; i++) {
+        const HostCopy &c = todo[i];
         const uintptr_t lo = (uintptr_t)c.host / page * page, hi = ((uintptr_t)c.host + c.bytes + page - 1) / page * page;
         const size_t parts = std::min(MOST, (hi - lo + PER_THREAD - 1) / PER_THREAD);
         const size_t step = ((hi - lo) / parts + page - 1) / page * page;
         try {
             for (uintptr_t p = lo; p < hi; p += step) {
                 const size_t len = std::min<uintptr_t>(step, hi - p);
-                threads.emplace_back([p, len] { (void)madvise((void *)p, len, MADV_POPULATE_WRITE); });
+                threads[nthreads] = std::thread([p, len] { (void)madvise((void *)p, len, MADV_POPULATE_WRITE); });
+                nthreads++;
             }
-        } catch (const std::system_error &) {
+        } catch (...) {
             break;   // no thread to be had: the copy faults the pages in
         }
     }
-    todo.clear();
+    ntodo = 0;
 }
 
 mg_status run_status_wait(mg_graph *g)
@@ -231,16 +238,16 @@ mg_status run_status_wait(mg_graph *g)
     return MG_OK;
 }
 
-void HostPages::wait()
+void HostPages::wait() noexcept
 {
     start();
-    for (std::thread &t : threads) t.join();
-    threads.clear();
+    for (int i = 0; i < nthreads; i++) threads[i].join();
+    nthreads = 0;
 }
 
 HostPages::~HostPages()
 {
-    todo.clear();   // (a run that failed early)
+    ntodo = 0;   // (a run that failed early)
     wait();
     g->pages = nullptr;
 }

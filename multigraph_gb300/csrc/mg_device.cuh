@@ -254,20 +254,22 @@ mg_status end_run(mg_graph *g, const mg_opts &opt, mg_run_info *info, std::initi
 // lock, which launches and pageable copies need too: begun earlier, they
 // delayed the run by 0.8 ms); every wait for a run's status calls it through
 // run_status_wait.  Arrays below POPULATE_MIN are not worth a thread;
-// page-locked ones have their pages already, which costs a helper one walk
-// over the page tables.
+// page-locked, managed and device memory is left alone.  Nothing here throws:
+// without a helper the copy faults the pages in.
 class HostPages {
 public:
-    HostPages(mg_graph *g, std::initializer_list<HostCopy> arrays);
+    HostPages(mg_graph *g, std::initializer_list<HostCopy> arrays) noexcept;
     ~HostPages();
     HostPages(const HostPages &) = delete;
     HostPages &operator=(const HostPages &) = delete;
-    void start();
-    void wait();   // the pages are there (or the system call does not exist)
+    void start() noexcept;
+    void wait() noexcept;   // the pages are there (or the system call does not exist)
 private:
+    static constexpr int ARRAYS = 3, PARTS = 8;   // result arrays of a call, helpers an array
     mg_graph *g;
-    std::vector<HostCopy> todo;
-    std::vector<std::thread> threads;
+    HostCopy todo[ARRAYS];
+    std::thread threads[ARRAYS * PARTS];
+    int ntodo = 0, nthreads = 0;
 };
 // wait for the graph's stream, its result pages coming in meanwhile
 mg_status run_status_wait(mg_graph *g);
