@@ -88,16 +88,16 @@ __device__ __forceinline__ void cc_union(int32_t *parent, int32_t a, int32_t b)
 
 constexpr int SAMPLE_ROUNDS = 2;
 constexpr int MODE_SAMPLES = 1024;
-constexpr int LINK_FIRST = 8;   // neighbours looked at by the first link of a relabeled graph (one or two sectors)
+using mgi::LINK_FIRST;
 
 // The first `link` neighbours below v start the tree: v hangs under the
 // least of them (a valid link: parent < v), a plain store.  With hub-first
 // ids that is the neighbour of the highest degree, so the trees are a few
 // links deep: on R-MAT 16 with shuffled-round ids, linking to the first two
 // neighbours in caller order by atomic unions took 123 us and flattening
-// the chains it made 70 us; this takes 3 + 5.  Without hub-first ids (a
-// lattice) the least neighbour would chain whole columns: link 0, every
-// vertex its own tree.
+// the chains it made 70 us; this takes 3 + 5.  Where the ids do not lead to
+// hubs (a lattice, also one with a hub or two) the least neighbour would chain
+// whole columns: link 0, every vertex its own tree.
 __global__ void k_cc_init(int32_t n, const int32_t *row, const int32_t *col, int32_t *parent, int link)
 {
     for (int32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
@@ -327,7 +327,7 @@ mg_status cc_run(mg_graph *g, mg_run_info *info, const std::vector<int32_t> *vof
     Profiler &P = g->prof;
     const int si = P.slot("cc_init"), sh = P.slot("cc_hook"), sc = P.slot("cc_compress");
     const bool sample = g->symmetric;
-    const bool hub_link = sample && g->relabeled;
+    const bool hub_link = sample && g->hub_link;
     P.begin(si);
     k_cc_init<<<grid, THREADS, 0, s>>>(g->nv, g->trow, g->tcol, parent, hub_link ? LINK_FIRST : sample ? 0 : 1);
     P.end();
@@ -340,8 +340,8 @@ mg_status cc_run(mg_graph *g, mg_run_info *info, const std::vector<int32_t> *vof
         }
         for (int r = 0; r < SAMPLE_ROUNDS; r++) {
             // each round links the trees and flattens them again, so no find
-            // walks a long chain: the roots among themselves on hub-first
-            // ids, else every vertex to its r-th neighbour
+            // walks a long chain: the roots among themselves on ids that lead
+            // to hubs, else every vertex to its r-th neighbour
             P.begin(ss);
             if (hub_link) k_cc_roots<<<grid, THREADS, 0, s>>>(g->nv, g->trow, g->tcol, parent);
             else k_cc_sample<<<grid, THREADS, 0, s>>>(g->nv, g->trow, g->tcol, r, parent);

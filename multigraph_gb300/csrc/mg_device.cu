@@ -299,6 +299,7 @@ struct HostLayout {
     int32_t n_dangling = 0, min_weight = 0;
     // hub-first relabeling (engine id = rank by descending log2 out-degree)
     bool relabel = false;
+    bool hub_link = false;
     std::vector<int32_t> new2old, old2new, row_new;
 };
 
@@ -368,6 +369,36 @@ static void build_bins(const std::vector<int32_t> &prow, int32_t n, int32_t heav
     L.tbin = tbin;
 }
 
+// Whether hub-first ids lead straight to the hubs: at least three quarters of
+// up to 1,024 vertices spread over the id range have a neighbour of a higher
+// degree class among their first LINK_FIRST.  The components' first link then
+// makes trees a few links deep.  One vertex of 128 edges relabels a graph, but
+// not every such graph is hub-first in this sense: on a lattice with one the
+// interior shares one class, in caller order, and the links chain whole columns
+// (median of CC in ms, linked / sampled: 1000 x 1000 with a vertex of 130 edges
+// 0.51 / 0.26, 2000 x 2000 1.9 / 0.43; R-MAT 16 0.059 / 0.077, R-MAT 20
+// 0.090 / 0.16).  R-MAT graphs of scale 9 to 20 come to 0.98 and more, such
+// lattices to 0.01, with a fifth of their edges gone to 0.5.
+static bool leads_to_hubs(const mg_host_graph &h, const std::vector<int32_t> &old2new, const std::vector<int32_t> &row_new)
+{
+    const int32_t n = h.nv, samples = std::min(n, 1024);
+    auto degree_class = [](int32_t d) {
+        int b = 0;
+        while (d > 1) { d >>= 1; b++; }
+        return b;
+    };
+    int32_t seen = 0, up = 0;
+    for (int32_t i = 0; i < samples; i++) {
+        const int32_t v = (int32_t)((int64_t)i * n / samples), b = h.v[v], d = h.v[v + 1] - b;
+        if (d == 0) continue;
+        int32_t first = n;   // the least engine id: the highest class among them
+        for (int32_t k = 0; k < std::min(d, mgi::LINK_FIRST); k++) first = std::min(first, old2new[h.e[b + k]]);
+        seen++;
+        up += degree_class(row_new[first + 1] - row_new[first]) > degree_class(d);
+    }
+    return up * 4 >= seen * 3;
+}
+
 static void build_layout(const mg_host_graph &h, HostLayout &L, int32_t heavy = HEAVY_DEG, int32_t chunk = HCHUNK,
                          int32_t tbin = TBIN)
 {
@@ -379,6 +410,7 @@ static void build_layout(const mg_host_graph &h, HostLayout &L, int32_t heavy = 
         hub_first_order(h, L.new2old, L.old2new);
         L.row_new.assign(n + 1, 0);
         for (int32_t i = 0; i < n; i++) L.row_new[i + 1] = L.row_new[i] + (h.v[L.new2old[i] + 1] - h.v[L.new2old[i]]);
+        L.hub_link = leads_to_hubs(h, L.old2new, L.row_new);
     }
     // transpose by counting sort (rows come out with ascending columns)
     std::vector<int32_t> tr(n + 1, 0), tc(m), tw(m);
@@ -931,6 +963,7 @@ static mg_status upload_arrays(mg_graph *g, const mg_host_graph *h, const HostLa
     }
     cudaStream_t s = g->stream;
     g->relabeled = L.relabel;
+    g->hub_link = L.hub_link;
     if (L.relabel) {
         g->h_old2new = L.old2new;
         MG_CUDA(cudaMemcpyAsync(g->old2new.p, L.old2new.data(), n * 4, cudaMemcpyHostToDevice, s));

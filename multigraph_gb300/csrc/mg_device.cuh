@@ -105,6 +105,7 @@ mg_status run_loop(int exec_mode, bool profile, cudaStream_t stream, LoopGraph &
 // memory; partial sums per (row, segment) pair; ids past the last segment
 // stay in an int32 tail (offsets toff) gathered through L2
 namespace mgi {
+constexpr int32_t LINK_FIRST = 8;    // neighbours looked at by the components' first link (one or two sectors)
 constexpr int32_t SHORT_PULL = 128;  // (out-degrees of 128 or more relabel a graph; in-degrees do not)
 constexpr int HUB_WIN = 512;   // piece sums the row finish stages in shared memory a warp (32 rows)
 struct HubSplit {
@@ -204,6 +205,7 @@ struct mg_graph {
     // hub-first relabeling: the engines run on ids ordered by descending
     // log2 degree; results are mapped back before they leave the library
     bool relabeled = false;
+    bool hub_link = false;         // most vertices see a higher degree class among their first neighbours (components)
     bool pr_prefer_gather = false; // mg_autotune measured the gather PageRank layout faster (MG_PR_LAYOUT_AUTO)
     bool pr_no_one_launch = false; // mg_autotune measured the one-launch PageRank slower than the tuned layout
     mgi::DevBuf o_row, o_col, o_wt;        // the CSR in the caller's ids (as uploaded)
