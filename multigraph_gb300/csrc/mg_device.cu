@@ -209,6 +209,18 @@ HostPages::HostPages(mg_graph *graph, std::initializer_list<HostCopy> arrays) no
     g->pages = this;
 }
 
+// whether some of eight pages spread over [lo, hi) has not been brought in yet
+static bool pages_missing(uintptr_t lo, uintptr_t hi, size_t page) noexcept
+{
+    for (int i = 0; i < 8; i++) {
+        unsigned char there = 0;
+        const uintptr_t p = lo + (hi - lo - page) / 7 * i / page * page;
+        if (mincore((void *)p, page, &there) != 0) return false;
+        if (!(there & 1)) return true;
+    }
+    return false;
+}
+
 void HostPages::start() noexcept
 {
     constexpr size_t PER_THREAD = 16 << 20, MOST = PARTS;
@@ -216,6 +228,7 @@ void HostPages::start() noexcept
     for (int i = 0; i < ntodo; i++) {
         const HostCopy &c = todo[i];
         const uintptr_t lo = (uintptr_t)c.host / page * page, hi = ((uintptr_t)c.host + c.bytes + page - 1) / page * page;
+        if (!pages_missing(lo, hi, page)) continue;
         const size_t parts = std::min(MOST, (hi - lo + PER_THREAD - 1) / PER_THREAD);
         const size_t step = ((hi - lo) / parts + page - 1) / page * page;
         try {

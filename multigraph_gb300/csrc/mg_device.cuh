@@ -255,7 +255,9 @@ mg_status end_run(mg_graph *g, const mg_opts &opt, mg_run_info *info, std::initi
 // comes once the run's work is enqueued (the helpers hold the address space's
 // lock, which launches and pageable copies need too: begun earlier, they
 // delayed the run by 0.8 ms); every wait for a run's status calls it through
-// run_status_wait.  Arrays below POPULATE_MIN are not worth a thread;
+// run_status_wait.  Arrays below POPULATE_MIN are not worth a thread, nor are
+// arrays written before (a helper's start and end cost 45 us where no GPU work
+// hides them, as after a host-driven loop; eight calls of mincore about 2);
 // page-locked, managed and device memory is left alone.  Nothing here throws:
 // without a helper the copy faults the pages in.
 class HostPages {
