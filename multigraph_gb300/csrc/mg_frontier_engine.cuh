@@ -59,8 +59,13 @@ constexpr int THREADS = 256;
 // block per SM: 152 arrivals at the grid barrier instead of 304, and 64
 // registers a thread instead of 32 with spills in the edge loops (lattice
 // BFS 5.8 -> 4.8 us a level at 100 K vertices, 8.5 -> 7.9 at 16.8 M; R-MAT
-// pushes 5-15 % faster)
+// pushes 5-15 % faster).  Graphs without heavy vertices whose rows average
+// more than DENSE_ROWS edges (random graphs) push few and large levels, where
+// twice the warps in flight are worth more: two blocks per SM (push levels of
+// a BFS, one block / two: 1 M vertices of degree 64 630 / 456 us, 4 M of degree
+// 16 1384 / 1143; of degree 8 and less one block is as fast or faster).
 constexpr int PTHREADS = 1024;
+constexpr int64_t DENSE_ROWS = 8;
 // grid barrier words (2 + GRID_SYNC_GROUPS), the barrier error flag, the BC
 // path-count overflow flag, rounded up
 constexpr size_t BAR_BYTES = 4 * (2 + mgd::GRID_SYNC_GROUPS + 1 + 7);
@@ -988,8 +993,9 @@ __device__ __forceinline__ bool block_phase(const Args &a, FCtl &c)
 
 // HEAVY: the graph may have vertices above PUSH_HEAVY out-edges (graphs that
 // have none run without the chunk code and its votes).
-template <class Op, bool HEAVY>
-__global__ void __launch_bounds__(PTHREADS, 1) k_sparse_levels(Args a)
+// PER_SM: blocks of it on an SM; with two, no levels are one block's alone.
+template <class Op, bool HEAVY, int PER_SM>
+__global__ void __launch_bounds__(PTHREADS, PER_SM) k_sparse_levels(Args a)
 {
     __shared__ FCtl s_c;
     __shared__ int4 s_cnt;
@@ -1009,9 +1015,11 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_sparse_levels(Args a)
             z->nhcur = 0;
             z->nfe = 0;
         }
-        if (block_phase_due<Op, HEAVY>(a, s_c)) {
-            if (!block_phase<Op>(a, s_c)) break;
-            continue;
+        if constexpr (PER_SM == 1) {
+            if (block_phase_due<Op, HEAVY>(a, s_c)) {
+                if (!block_phase<Op>(a, s_c)) break;
+                continue;
+            }
         }
         push_level<Op, HEAVY>(a, s_c, lc);
         if (!mgd::grid_sync(a.bar, a.bar_err, a.bar_never)) break;
@@ -1221,6 +1229,9 @@ namespace {
 
 using namespace mgi;
 
+// no vertex of 128 edges, rows of more than DENSE_ROWS edges on average
+inline bool dense_rows(const mg_graph *g) { return !g->relabeled && (int64_t)g->ne > DENSE_ROWS * g->nv; }
+
 template <class Op>
 mg_status ensure_ws(mg_graph *g)
 {
@@ -1242,35 +1253,39 @@ mg_status ensure_ws(mg_graph *g)
     if (cg == 0) {
         int per_sm = 0;
         if (g->relabeled)
-            MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sparse_levels<Op, true>, PTHREADS, 0));
+            MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sparse_levels<Op, true, 1>, PTHREADS, 0));
+        else if (dense_rows(g))
+            MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sparse_levels<Op, false, 2>, PTHREADS, 0));
         else {
-            MG_CUDA(cudaFuncSetAttribute(k_sparse_levels<Op, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            MG_CUDA(cudaFuncSetAttribute(k_sparse_levels<Op, false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)sizeof(CtaShared)));
-            MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sparse_levels<Op, false>, PTHREADS,
+            MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sparse_levels<Op, false, 1>, PTHREADS,
                                                                   sizeof(CtaShared)));
         }
         if (per_sm < 1) return fail(MG_ERR_CUDA, "persistent push kernel does not fit on an SM");
-        cg = g->num_sms;
+        cg = (dense_rows(g) ? std::min(per_sm, 2) : 1) * g->num_sms;
     }
     return MG_OK;
 }
 
 // cooperative launch (all blocks resident) of the persistent push phase
 template <class Op>
-mg_status launch_sparse_levels(const Args &a, int grid, cudaStream_t st)
+mg_status launch_sparse_levels(const mg_graph *g, const Args &a, int grid, cudaStream_t st)
 {
+    const bool dense = dense_rows(g);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3(PTHREADS);
-    cfg.dynamicSmemBytes = a.has_heavy ? 0 : sizeof(CtaShared);
+    cfg.dynamicSmemBytes = a.has_heavy || dense ? 0 : sizeof(CtaShared);
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (a.has_heavy) MG_CUDA(cudaLaunchKernelEx(&cfg, k_sparse_levels<Op, true>, a));
-    else MG_CUDA(cudaLaunchKernelEx(&cfg, k_sparse_levels<Op, false>, a));
+    if (a.has_heavy) MG_CUDA(cudaLaunchKernelEx(&cfg, k_sparse_levels<Op, true, 1>, a));
+    else if (dense) MG_CUDA(cudaLaunchKernelEx(&cfg, k_sparse_levels<Op, false, 2>, a));
+    else MG_CUDA(cudaLaunchKernelEx(&cfg, k_sparse_levels<Op, false, 1>, a));
     return MG_OK;
 }
 
@@ -1468,7 +1483,7 @@ mg_status frontier_run_impl(mg_graph *g, int32_t src, const int32_t *srcs_host, 
     BodyFn body = [&](cudaStream_t st, cudaGraphConditionalHandle h, int use_cond) -> mg_status {
         MG_CUDA(cudaMemsetAsync(a.cnt, 0, 4 * sizeof(LevelCnt), st));
         P.begin(sp);
-        MG_TRY(launch_sparse_levels<Op>(a, coop, st));
+        MG_TRY(launch_sparse_levels<Op>(g, a, coop, st));
         P.end();
         if (Op::kMinPlusBound) {
             P.begin(sf);
