@@ -1293,13 +1293,17 @@ mg_status launch_sparse_levels(const mg_graph *g, const Args &a, int grid, cudaS
 // (k_frontier_all); past them the pull kernels' twice as many resident warps
 // are worth the launches.  us, one launch / separate: BFS R-MAT 16 (1.8 M
 // edges) 77 / 111, R-MAT 18 (7.6 M) 163 / 144; SSSP 190 / 223 and 372 / 296.
-// A level-synchronous traversal of a graph without heavy vertices hardly ever
-// pulls: one launch at any size (BFS 1500 x 1400 lattice 9.1 / 10.2 ms).
-constexpr int64_t ONE_LAUNCH_EDGES_SYNC = 4 << 20, ONE_LAUNCH_EDGES_RELAX = 3 << 20;
+// Without heavy vertices the levels are more even and the line for
+// level-synchronous operators lies higher.  BFS of random graphs: 1 M vertices
+// of degree 16 (16.8 M edges) 157 / 230, 4 M of degree 8 (33 M) 483 / 446, 1 M
+// of degree 64 (67 M; only pushed, 653 / 503), 4 M of degree 16 (67 M) 483 /
+// 423; lattices, ms: 1500 x 1400 (8.6 M) 9.1 / 10.2, 3000 x 3000 (36 M) 28.2 /
+// 28.4.
+constexpr int64_t ONE_LAUNCH_EDGES_SYNC = 4 << 20, ONE_LAUNCH_EDGES_FLAT = 16 << 20, ONE_LAUNCH_EDGES_RELAX = 3 << 20;
 template <class Op>
 bool one_launch_pays(const mg_graph *g)
 {
-    if (Op::kLevelSync) return !g->relabeled || g->ne <= ONE_LAUNCH_EDGES_SYNC;
+    if (Op::kLevelSync) return g->ne <= (g->relabeled ? ONE_LAUNCH_EDGES_SYNC : ONE_LAUNCH_EDGES_FLAT);
     return g->ne <= ONE_LAUNCH_EDGES_RELAX;
 }
 
