@@ -88,7 +88,7 @@ struct FCtl {
     int32_t alpha, beta;
     int32_t nlevels;      // BC: levels archived
     int32_t archive;      // 1: queue slices are appended (BFS/BC), 0: ping-pong (SSSP)
-    int32_t qedges;         // out-edges of the current frontier (push phase only)
+    int32_t qedges;         // out-edges of the current frontier
     long long nf_edges;      // out-edges of the next frontier (atomic)
     long long visited_edges; // out-edges of every vertex visited so far
     long long scanned;       // edges scanned (statistics, atomic)
@@ -576,23 +576,30 @@ struct PullEmit {
 // unreached or earlier-relaxed vertices never spoil a label, labels still
 // converge to the same fixed point, and one dependent load per edge goes away.
 //
-// Min-plus operators take every reached in-neighbour's offer at any frontier:
-// the bitmap test puts a dependent load in front of every label (device time
-// of SSSP with the test where the frontier is sparse -> without: R-MAT 22 1.69
-// -> 1.48 ms, R-MAT 20 0.51 -> 0.48, R-MAT 18 0.32 -> 0.30).  An unreached one
-// is told by its initial label, to which no weight is added, so that no sum of
-// the two can wrap.
+// Min-plus operators take every reached in-neighbour's offer at any frontier
+// that the direction switch pulls for (it holds a quarter of the edges by
+// default): the bitmap test puts a dependent load in front of every label
+// (device time of SSSP with the test where the frontier has few vertices ->
+// without: R-MAT 22 1.69 -> 1.48 ms, R-MAT 20 0.51 -> 0.48, R-MAT 18 0.32 ->
+// 0.30).  Where the caller has every level pulled, most frontiers are small and
+// most edges end at the bitmap, which stays in L1: k_pull has a form with the
+// test for that (ALL false; SSSP of 1 M vertices of degree 64 so pulled, with
+// the test / without, 3.5 / 4.1 ms; a test on the level's size inside the one
+// form cost the switched runs 4 %).  An unreached neighbour is told by its
+// initial label, to which no weight is added, so that no sum of the two can
+// wrap.
 //
 // Min-plus operators (kMinPlusBound) skip rows whose label is at most (least
 // frontier label + least weight): every offer is label[u] + w from a
 // frontier vertex u, or from a vertex whose edges an earlier level already
 // relaxed, so such a row cannot improve this level.  On R-MAT the hubs
 // settle first, so the later pull levels read a fraction of the edges.
-template <class Op>
+template <class Op, bool ALL>
 __device__ __forceinline__ bool pull_offer(const Args &a, const uint32_t *fb, bool all_in, int32_t u, int32_t w,
                                            int32_t &offer)
 {
     if constexpr (Op::kMinPlusBound) {
+        if (!ALL && !all_in && !mgd::bm_test(fb, u)) return false;
         const int32_t label = a.label[u];
         if (label == Op::initialize()) return false;
         offer = Op::get_partial_result(label, w);
@@ -603,7 +610,14 @@ __device__ __forceinline__ bool pull_offer(const Args &a, const uint32_t *fb, bo
     return true;
 }
 
+// whether a relaxed level with the test folds every in-neighbour's offer
 template <class Op>
+__device__ __forceinline__ bool pull_all_in(const Args &a, const FCtl &c)
+{
+    return (long long)c.qsize * 8 > a.n || (Op::kMinPlusBound && (long long)c.qedges * 4 > a.m);
+}
+
+template <class Op, bool ALL>
 struct PullRelax : PullEmit {
     using T = int32_t;
     static constexpr bool kRowAware = Op::kMinPlusBound;
@@ -617,7 +631,7 @@ struct PullRelax : PullEmit {
     __device__ T edge(int32_t, int32_t, int32_t u, int32_t w) const
     {
         int32_t offer;
-        return pull_offer<Op>(a, fb, all_in, u, w, offer) ? offer : Op::initialize();
+        return pull_offer<Op, ALL>(a, fb, all_in, u, w, offer) ? offer : Op::initialize();
     }
     __device__ T combine(T x, T y) const
     {
@@ -665,8 +679,8 @@ struct PullCounts : PullEmit {
     }
 };
 
-template <class Op>
-using PullOp = std::conditional_t<Op::kPathCounts, PullCounts<Op>, PullRelax<Op>>;
+template <class Op, bool ALL>
+using PullOp = std::conditional_t<Op::kPathCounts, PullCounts<Op>, PullRelax<Op, ALL>>;
 
 // min-plus pull levels: rows at or below this label cannot improve
 __device__ __forceinline__ int32_t sssp_bound(int32_t fmin, int32_t wmin)
@@ -693,8 +707,8 @@ __global__ void __launch_bounds__(THREADS) k_fmin(Args a)
 }
 
 // One pull level by blocks of NT threads; bound: min-plus rows at or below
-// this label cannot improve.
-template <class Op, int NT>
+// this label cannot improve; ALL: min-plus without the bitmap test.
+template <class Op, bool ALL, int NT>
 __device__ __forceinline__ void pull_level(const Args &a, const FCtl &c, int32_t bound)
 {
     const int it1 = c.iter + 1;
@@ -733,8 +747,8 @@ __device__ __forceinline__ void pull_level(const Args &a, const FCtl &c, int32_t
         }
     } else {
         // degree-binned rows; reached rows marked in the next-frontier bitmap
-        PullOp<Op> op{{a, bm_buf(a, nextbuf)}, fb, it1, false, 0};
-        if constexpr (!Op::kLevelSync) op.all_in = (long long)c.qsize * 8 > a.n;
+        PullOp<Op, ALL> op{{a, bm_buf(a, nextbuf)}, fb, it1, false, 0};
+        if constexpr (!Op::kLevelSync && !ALL) op.all_in = pull_all_in<Op>(a, c);
         if constexpr (Op::kMinPlusBound) op.bound = bound;
         mgd::bins_reduce(op, a.trow, a.tcol, a.twt, a.wrows, a.nwrows, a.nwlong, a.trows, a.ntrows);
         (void)gwarp;
@@ -769,12 +783,12 @@ __device__ __forceinline__ void pull_level(const Args &a, const FCtl &c, int32_t
         mgops::PathCount ssum = mgops::pc_zero();
         const bool ext = a.bc_ext != 0;
         int hit = 0;
-        const bool all_in = !Op::kLevelSync && (long long)c.qsize * 8 > a.n;  // as PullRelax
+        const bool all_in = !Op::kLevelSync && !ALL && pull_all_in<Op>(a, c);  // as PullRelax
         for (int32_t p = b + threadIdx.x; p < e; p += blockDim.x) {
             int32_t u = __ldcs(&a.tcol[p]);  // streamed once: evict-first
             if constexpr (!Op::kLevelSync) {
                 int32_t offer;
-                if (pull_offer<Op>(a, fb, all_in, u, Op::kWeighted ? __ldcs(&a.twt[p]) : 0, offer)) {
+                if (pull_offer<Op, ALL>(a, fb, all_in, u, Op::kWeighted ? __ldcs(&a.twt[p]) : 0, offer)) {
                     hit = 1;
                     Op::accumulate_nonAtomics(best, offer, it1);
                 }
@@ -827,12 +841,12 @@ __device__ __forceinline__ void pull_level(const Args &a, const FCtl &c, int32_t
     warp_add64(&a.ctl->scanned, scanned);
 }
 
-template <class Op>
+template <class Op, bool ALL>
 __global__ void __launch_bounds__(THREADS) k_pull(Args a)
 {
     const FCtl c = *a.ctl;
     if (c.mode != MODE_PULL || c.more == 0) return;
-    pull_level<Op, THREADS>(a, c, Op::kMinPlusBound ? sssp_bound(*a.fmin, a.wmin) : 0);
+    pull_level<Op, ALL, THREADS>(a, c, Op::kMinPlusBound ? sssp_bound(*a.fmin, a.wmin) : 0);
 }
 
 // ----------------------------------------------------------------------------
@@ -1165,7 +1179,7 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_frontier_all(Args a, StartArgs 
                 __syncthreads();
                 bound = sssp_bound(s_fmin, a.wmin);
             }
-            pull_level<Op, PTHREADS>(a, s_c, bound);
+            pull_level<Op, Op::kMinPlusBound, PTHREADS>(a, s_c, bound);
             if (!(ok = mgd::grid_sync(a.bar, a.bar_err, a.bar_never))) break;
             compact_level<PTHREADS>(a, s_c, &lc->nq, &lc->nhcur, &lc->nfe);
         }
@@ -1484,6 +1498,7 @@ mg_status frontier_run_impl(mg_graph *g, int32_t src, const int32_t *srcs_host, 
     const int sc = P.slot("frontier_compact");
     const int sf = Op::kMinPlusBound ? P.slot((t + "_fmin").c_str()) : -1;
     const int sd = P.slot("frontier_decide");
+    const bool every_offer = Op::kMinPlusBound && opt.direction != MG_DIR_PULL;   // k_pull's form
     BodyFn body = [&](cudaStream_t st, cudaGraphConditionalHandle h, int use_cond) -> mg_status {
         MG_CUDA(cudaMemsetAsync(a.cnt, 0, 4 * sizeof(LevelCnt), st));
         P.begin(sp);
@@ -1495,7 +1510,8 @@ mg_status frontier_run_impl(mg_graph *g, int32_t src, const int32_t *srcs_host, 
             P.end();
         }
         P.begin(sl);
-        k_pull<Op><<<grid, THREADS, 0, st>>>(a);
+        if (every_offer) k_pull<Op, Op::kMinPlusBound><<<grid, THREADS, 0, st>>>(a);
+        else k_pull<Op, false><<<grid, THREADS, 0, st>>>(a);
         P.end();
         P.begin(sc);
         k_compact<<<grid, THREADS, 0, st>>>(a);
@@ -1506,8 +1522,8 @@ mg_status frontier_run_impl(mg_graph *g, int32_t src, const int32_t *srcs_host, 
         MG_CUDA(cudaGetLastError());
         return MG_OK;
     };
-    MG_TRY(run_loop(opt.profile ? MG_EXEC_HOST : opt.exec, opt.profile != 0, s, w->lg[tag], key_of(a, tag, grid, coop),
-                    body, &a.ctl->more, g->pinned_flag, max_iter + 2));
+    MG_TRY(run_loop(opt.profile ? MG_EXEC_HOST : opt.exec, opt.profile != 0, s, w->lg[tag],
+                    key_of(a, tag, grid, coop).add(every_offer), body, &a.ctl->more, g->pinned_flag, max_iter + 2));
     if (which >= 0) MG_TRY(publish(g, which, a.label, 4));
     return frontier_outcome<Op>(g, a, src, srcs_host, nsrc, opt, max_iter, info, which);
 }
