@@ -576,7 +576,20 @@ __global__ void __launch_bounds__(THREADS) k_pr_light(PArgs a)
 // do (1000 x 1000 lattice, weighted: 31 -> 24 us a sweep).  With heavy rows,
 // letting the last of a row's chunks finish it costs more than the apply
 // kernel: a fence and an atomic a chunk took the weighted R-MAT 19 sweep from
-// 71 to 86 us.
+// 71 to 86 us.  With longer rows (above eight edges on average) the weighted
+// forms lose more to the 32 registers that eight blocks an SM leave than the
+// launch costs: us a sweep with the apply kernel / closed here, forward, random
+// graphs of 256 K vertices of degree 16 41 / 47, 1 M of degree 16 116 / 123;
+// adjoint, 200 K rows of 120 edges in a band (24 M) 62 / 71, 1 M of degree 16
+// (16.8 M) 142 / 131.  (With six blocks an SM the forward stays at 126, the
+// band's adjoint at 77.)
+template <class Op>
+bool light_closes(const mg_graph *g)
+{
+    constexpr int64_t ADJOINT_EDGES = 16 << 20;
+    return !Op::kWeights || (int64_t)g->ne <= (int64_t)8 * g->nv || (Op::kAdjoint && g->ne <= ADJOINT_EDGES);
+}
+
 template <class Op>
 __global__ void __launch_bounds__(THREADS, 8) k_pr_light_close(PArgs a, cudaGraphConditionalHandle h, int use_cond)
 {
@@ -1822,7 +1835,7 @@ static mg_status pr_loop(mg_graph *g, PArgs &a, const mg_opts &opt, const char *
             // every row finishes in k_pr_seg, which also closes the sweep
             k_pr_seg<Op><<<grid, THREADS, 0, st>>>(a, h, use_cond);
             P.end();
-        } else if (!a.P && a.nhchunks == 0) {
+        } else if (!a.P && a.nhchunks == 0 && light_closes<Op>(g)) {
             k_pr_light_close<Op><<<grid, THREADS, 0, st>>>(a, h, use_cond);
             P.end();
         } else {
