@@ -688,7 +688,7 @@ void hub_free(mg_graph *g)
 
 // Split the groups among the CTAs by the groups' cost weights h.w:
 // contiguous ranges of the least largest load, cut at segment boundaries into
-// parts and each part into chunks of about CHUNK_COST that the CTA's warps
+// parts and each part into chunks of up to CHUNK_COST that the CTA's warps
 // claim one at a time.  The captured loops that launch the sweep take the new
 // split (the build number changes).  Even shares of the weight, a staging
 // charged to each segment's first group, left CTAs that stage a segment for
@@ -705,16 +705,6 @@ static mg_status hub_split(mg_graph *g)
     const std::vector<int32_t> &segg = h.hsegg;
     std::vector<double> gcum((size_t)ngroups + 1, 0.0);
     for (int32_t q = 0; q < ngroups; q++) gcum[q + 1] = gcum[q] + h.w[q];
-    auto cut = [&](int32_t lo, int32_t hi, int parts, int32_t *out) {
-        // out[0..parts]: boundaries in [lo, hi] of equal weight
-        out[0] = lo;
-        for (int k = 1; k < parts; k++) {
-            const double goal = gcum[lo] + (gcum[hi] - gcum[lo]) * k / parts;
-            int32_t b = (int32_t)(std::lower_bound(gcum.begin() + lo, gcum.begin() + hi, goal) - gcum.begin());
-            out[k] = std::min(std::max(b, out[k - 1]), hi);
-        }
-        out[parts] = hi;
-    };
     // CHUNK_COST in units of the weights as they are now
     double wn = 0.0;
     for (int32_t q = 0; q < ngroups; q++) wn += h.w[q];
@@ -760,12 +750,14 @@ static mg_status hub_split(mg_graph *g)
             const int32_t e = std::min(hi, segg[sg + 1]);
             pseg.push_back(sg);
             pch.push_back((int32_t)cb.size());
-            const double cost = gcum[e] - gcum[lo];
-            const int nch = (int)std::max<int64_t>(1, std::min<int64_t>(e - lo, (int64_t)std::ceil(cost / chunk_w)));
-            std::vector<int32_t> bnd((size_t)nch + 1);
-            cut(lo, e, nch, bnd.data());
-            for (int k = 0; k < nch; k++)
-                if (bnd[k] < bnd[k + 1]) cb.push_back(bnd[k]);
+            // A chunk takes groups while they stay within CHUNK_COST and
+            // within a warp's even share of the part: a warp with two groups
+            // of a part that has fewer groups than the CTA warps doubles the
+            // part's time (cuts of equal weight, groups of 64 steps: a band of
+            // 200 K rows 36 us a sweep, 26 so; directed R-MAT 18 21, 19)
+            const double most = std::min(chunk_w, (gcum[e] - gcum[lo]) / (HUB_THREADS / 32));
+            for (int32_t q = lo; q < e; q++)
+                if (q == lo || gcum[q + 1] - gcum[cb.back()] > most) cb.push_back(q);
             lo = e;
         }
     }
