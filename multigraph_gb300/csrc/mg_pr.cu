@@ -795,10 +795,11 @@ constexpr int32_t ALL_CHUNK = 256;
 constexpr int32_t ALL_SHORT = 16;
 // Up to this many edges; past them the other layouts' sweeps, whose blocks
 // are resident twice as densely, are the faster ones.  us per sweep, here /
-// segmented / gather: R-MAT 17 (3.7 M edges) 25 / 32 / 36, R-MAT 19 of edge
-// factor 6 (6.0 M) 35 / 38 / 39, R-MAT 18 (7.6 M) 40 / 39 / 42, R-MAT 19
-// (15.5 M) 84 / 41 / 57.  Graphs of short rows only: 1500 x 1400 lattice
-// (8.6 M) 21 / 48 / 30.
+// segmented / gather: R-MAT 17 (3.7 M edges) 24 / 32 / 36, of edge factor 24
+// (5.4 M) 31 / 33 / 39, R-MAT 19 of edge factor 6 (6.0 M) 33 / 34 / 39, R-MAT
+// 18 (7.6 M) 40 / 35 / 42, R-MAT 19 (15.5 M) 84 / 41 / 57.  Graphs of short
+// rows only: 1400 x 1400 lattice (8.0 M) 19 / 43 / 29, 1700 x 1700 (11.8 M)
+// 39 / 53 / 47.
 constexpr int64_t ALL_MAX_EDGES = 6 << 20, ALL_MAX_EDGES_SHORT = 12 << 20;
 
 struct PrAllArgs {
