@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_bc_back_heavy(Args a, BCtl *bc_
                     const int32_t uj = __shfl_sync(FULL, u, j), bj = __shfl_sync(FULL, b, j), ej = __shfl_sync(FULL, e, j),
                                   nj = __shfl_sync(FULL, nc, j), pj = __shfl_sync(FULL, base, j);
                     for (int32_t c = lane; c < nj; c += 32)
-                        k.item[pj + c] = make_int4(uj, bj + c * BACK_CHUNK, min(ej, bj + (c + 1) * BACK_CHUNK), pj);
+                        k.item[pj + c] = make_int4(uj, bj + c * BACK_CHUNK, bj + min(ej - bj, (c + 1) * BACK_CHUNK), pj);
                 }
             }
             const bool row = i < hi && e - b <= BACK_CHUNK;
@@ -168,8 +168,8 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_bc_back_heavy(Args a, BCtl *bc_
             QT<EXT> t[BACK_CHUNK / 32];
 #pragma unroll
             for (int j = 0; j < BACK_CHUNK / 32; j++) {
-                const int32_t p = it.y + lane + 32 * j;
-                t[j] = p < it.z ? term(__ldcs(&a.col[p]), su.k) : (QT<EXT>)0;
+                const int32_t p = lane + 32 * j;
+                t[j] = p < it.z - it.y ? term(__ldcs(&a.col[it.y + p]), su.k) : (QT<EXT>)0;
             }
             QT<EXT> acc = ((t[0] + t[1]) + (t[2] + t[3])) + ((t[4] + t[5]) + (t[6] + t[7]));
 #pragma unroll

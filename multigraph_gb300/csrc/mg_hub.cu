@@ -240,6 +240,16 @@ constexpr int32_t HB_CHUNKS = 8192;
 constexpr int32_t HB_ROW = 2048;
 constexpr int HB_WARPS = 2;   // a block: shared memory of 20-30 KB a warp decides how many an SM holds
 
+// A long row [begin, end) in subs: their number; sub s's first edge and length.
+// (No sum passes end, which may be the last int32.)
+__host__ __device__ inline int32_t hb_subs(int32_t begin, int32_t end) { return (end - begin - 1) / HB_ROW + 1; }
+__host__ __device__ inline int32_t hb_sub_begin(int32_t begin, int32_t s) { return begin + s * HB_ROW; }
+__host__ __device__ inline int32_t hb_sub_len(int32_t begin, int32_t end, int32_t s)
+{
+    const int32_t left = end - hb_sub_begin(begin, s);
+    return left < HB_ROW ? left : HB_ROW;
+}
+
 struct HubBuild {
     const int32_t *prow, *pcol;
     int32_t n, nseg, cover, chunks;
@@ -270,7 +280,7 @@ __global__ void __launch_bounds__(256) k_hb_long(HubBuild b)
         const int32_t d = b.prow[v + 1] - b.prow[v];
         int32_t id = 0;
         if (d > HB_ROW) {
-            const int32_t ns = (d + HB_ROW - 1) / HB_ROW;
+            const int32_t ns = hb_subs(b.prow[v], b.prow[v + 1]);
             id = atomicAdd(&b.nlong[0], 1) + 1;
             const int32_t first = atomicAdd(&b.nlong[1], ns);
             b.lrow[id - 1] = make_int2(v, first);
@@ -290,9 +300,10 @@ __global__ void __launch_bounds__(HB_WARPS * 32) k_hb_sub_count(HubBuild b)
         for (int k = lane; k < b.ncol; k += 32) cnt[k] = 0;
         __syncwarp();
         const int2 r = b.lrow[b.sub[s]];
-        const int32_t p0 = b.prow[r.x] + (s - r.y) * HB_ROW, p1 = min(p0 + HB_ROW, b.prow[r.x + 1]);
+        const int32_t begin = b.prow[r.x], len = hb_sub_len(begin, b.prow[r.x + 1], s - r.y);
+        const int32_t *col = b.pcol + hb_sub_begin(begin, s - r.y);
 #pragma unroll 4
-        for (int32_t p = p0 + lane; p < p1; p += 32) atomicAdd(&cnt[hb_segment(b, __ldg(&b.pcol[p]))], 1u);
+        for (int32_t i = lane; i < len; i += 32) atomicAdd(&cnt[hb_segment(b, __ldg(&col[i]))], 1u);
         __syncwarp();
         for (int k = lane; k < b.ncol; k += 32) b.subcnt[(size_t)s * b.ncol + k] = cnt[k];
         __syncwarp();
@@ -306,7 +317,7 @@ __global__ void __launch_bounds__(128) k_hb_long_scan(HubBuild b)
     if (k >= b.ncol) return;
     for (int32_t i = blockIdx.x; i < nl; i += gridDim.x) {
         const int2 r = b.lrow[i];
-        const int32_t ns = (b.prow[r.x + 1] - b.prow[r.x] + HB_ROW - 1) / HB_ROW;
+        const int32_t ns = hb_subs(b.prow[r.x], b.prow[r.x + 1]);
         uint32_t run = 0;
         for (int32_t s = 0; s < ns; s++) {
             uint32_t *c = &b.subcnt[(size_t)(r.y + s) * b.ncol + k];
@@ -636,9 +647,10 @@ __global__ void __launch_bounds__(HB_WARPS * 32) k_hb_sub_place(HubBuild b)
         const uint32_t *count = b.lcnt + (size_t)id * b.ncol, *lp = b.lplace + (size_t)id * 2 * b.ncol;
         for (int k = lane; k < b.ncol; k += 32) pos[k] = b.subcnt[(size_t)s * b.ncol + k];
         __syncwarp();
-        const int32_t p0 = b.prow[r.x] + (s - r.y) * HB_ROW, p1 = min(p0 + HB_ROW, b.prow[r.x + 1]);
-        for (int32_t p = p0 + lane; p - lane < p1; p += 32) {
-            const int32_t c = p < p1 ? __ldg(&b.pcol[p]) : -1;
+        const int32_t begin = b.prow[r.x], len = hb_sub_len(begin, b.prow[r.x + 1], s - r.y);
+        const int32_t *col = b.pcol + hb_sub_begin(begin, s - r.y);
+        for (int32_t i = lane; i - lane < len; i += 32) {
+            const int32_t c = i < len ? __ldg(&col[i]) : -1;
             const int32_t sg = c < 0 ? 0 : hb_segment(b, c);
             const unsigned same = __match_any_sync(FULL, c < 0 ? -1 : sg);
             const uint32_t first = pos[sg], e = first + __popc(same & ((1u << lane) - 1u));
@@ -1286,6 +1298,20 @@ extern "C" mg_status mg_selftest_segmented_layout(int32_t nv, int64_t ne, const 
     for (int64_t p = 0; p < ne; p++)
         if (col[p] < 0 || col[p] >= nv) return fail(MG_ERR_INVALID, "column id out of range at %lld", (long long)p);
     *pieces_out = 0;
+    // the device build's subs tile a long row, wherever it lies
+    const int32_t ends[][2] = {{0, HB_ROW + 1}, {5, 5 + 2 * HB_ROW}, {INT32_MAX - 5000, INT32_MAX},
+                               {INT32_MAX - 2 * HB_ROW - 1, INT32_MAX - 1}, {0, INT32_MAX}};
+    for (const auto &r : ends) {
+        int64_t at = r[0];
+        const int32_t ns = hb_subs(r[0], r[1]);
+        for (int32_t s = 0; s < ns; s++) {
+            const int32_t len = hb_sub_len(r[0], r[1], s);
+            if (hb_sub_begin(r[0], s) != at || len < 1 || len > HB_ROW)
+                return fail(MG_ERR_INTERNAL, "segmented build: sub %d of the row at %d", s, r[0]);
+            at += len;
+        }
+        if (at != r[1]) return fail(MG_ERR_INTERNAL, "segmented build: subs of the row at %d", r[0]);
+    }
     if (nv < 4 || ne == 0) return MG_OK;
     const std::vector<int32_t> prow(row, row + nv + 1), pcol(col, col + ne);
     HubHost a, b;
