@@ -1430,7 +1430,7 @@ mg_status frontier_outcome(mg_graph *g, const Args &a, int32_t src, const int32_
         info->pull_iterations = hc.pull_iters;
         info->edges_scanned = hc.scanned;
     }
-    if (hc.status == 3) return fail(MG_ERR_CUDA, "grid barrier of the persistent push kernel timed out");
+    if (hc.status == 3) return fail(MG_ERR_CUDA, "grid barrier of a persistent traversal kernel timed out");
     if (hc.status != 0) return fail(MG_ERR_ITER_LIMIT, "iteration cap %d reached", max_iter);
     return MG_OK;
 }

@@ -269,7 +269,7 @@ struct HubBuild {
     const int32_t *goff;
     int32_t *pair_off, *toff, *tcol, *fin, *pslot;
     uint16_t *hdat, *porder;
-    int32_t ntail, npieces;
+    int32_t ntail;
 };
 
 __device__ __forceinline__ int32_t hb_segment(const HubBuild &b, int32_t c) { return c < b.cover ? c / SEG_H : b.nseg; }
@@ -1092,7 +1092,6 @@ mg_status hub_prepare(mg_graph *g)
     h.hsegg[b.nseg] = ngroups;
     if (npieces >= INT32_MAX || steps >= INT32_MAX) return fail(MG_ERR_RANGE, "segmented PageRank layout too large");
     b.ntail = (int32_t)ntail;
-    b.npieces = (int32_t)npieces;
     h.nfw = (int32_t)total[b.nb + 2];
     const size_t words = (size_t)steps * GROUP / 2, slots = (size_t)ngroups * GROUP;
     MG_TRY(make(h.hdat, words * 4, b.hdat));

@@ -520,13 +520,7 @@ __global__ void __launch_bounds__(THREADS) k_pr_light(PArgs a)
     mgd::pdl_enter();
     const PCtl c = *a.ctl;
     if (c.more == 0 || c.sparse) return;
-    const int lane = mgd::lane();
-    const int gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int nwarps = (gridDim.x * blockDim.x) >> 5;
     PrRowOp<Op> op{a, c};
-    (void)lane;
-    (void)gwarp;
-    (void)nwarps;
     const int32_t *pwt = reinterpret_cast<const int32_t *>(a.pw);
     mgd::bins_reduce(op, a.prow, a.pcol, pwt, a.wrows, a.nwrows, a.nwlong, a.trows, a.ntrows);
     // heavy-row chunks, one per CTA, in batches of 8 * THREADS edges: each
@@ -781,14 +775,15 @@ __global__ void __launch_bounds__(THREADS) k_pr_apply(PArgs a, cudaGraphConditio
 // Contributions are gathered through L1 (the barrier's fence makes the other
 // blocks' values visible there): the hubs' few sectors read by every edge
 // straight from L2 took the R-MAT 16 sweep from 18 to 48 us.  Sums are
-// compensated and kept as exact pairs, so an update rounds once.  After the barrier every block
-// adds up the 152 blocks' partial sums itself and comes to the same
-// decision.  Only for the normalised form: the data-driven form freezes and
+// compensated and kept as exact pairs, so an update rounds once.  After the
+// barrier every block adds up the 152 blocks' partial sums itself and comes to
+// the same decision.  Only for the normalised form: the data-driven form freezes and
 // PR_T holds a row by comparing its change with a threshold, where one last
 // bit can decide, and the weighted forms' order of additions shows in the
 // gradient (k_row_sums).  R-MAT 16: 30 -> 18 us per sweep, 320 x 311 lattice 18 -> 7 us.
-// Error against 64 bits over 24 graphs of up to 6 M edges (relative rms):
-// 4.8e-8 the other layouts, 4.0e-8 here.
+// Error against 64 bits (relative rms, geometric mean over R-MAT 9 to 16):
+// 4.0e-8 the segmented layout, 6.1e-8 the gather layout, less than either here
+// (R-MAT 16 2.9e-8 and 3.7e-8 segmented).
 // ---------------------------------------------------------------------------
 constexpr int ALL_THREADS = 1024;
 constexpr int32_t ALL_CHUNK = 256;
@@ -803,7 +798,7 @@ constexpr int32_t ALL_SHORT = 16;
 constexpr int64_t ALL_MAX_EDGES = 6 << 20, ALL_MAX_EDGES_SHORT = 12 << 20;
 
 struct PrAllArgs {
-    const int32_t *chunk, *chunk_at, *rows, *row_chunk;  // rows above ALL_CHUNK edges (mgi::ppr_chunks)
+    const int32_t *chunk, *chunk_at, *row_chunk;         // rows above ALL_CHUNK edges (mgi::ppr_chunks)
     int32_t nchunks;
     int32_t split;          // rows [0, split) take eight lanes, the others a thread each
     int32_t *arrive;        // [rows] chunks finished (zero before the launch and between sweeps)
@@ -1902,7 +1897,7 @@ static mg_status pr_all(mg_graph *g, const PArgs &a, const mg_opts &opt, float x
     MG_TRY(dev_alloc(w->bsum, (size_t)grid * 2 * 3 * 8));
     MG_TRY(dev_alloc(w->bar, 64));
     z.chunk = g->ppr_hchunk.as<int32_t>(); z.chunk_at = g->ppr_hchunk_at.as<int32_t>();
-    z.rows = g->ppr_hrows.as<int32_t>(); z.row_chunk = g->ppr_hrow_chunk.as<int32_t>();
+    z.row_chunk = g->ppr_hrow_chunk.as<int32_t>();
     z.nchunks = g->ppr_nhchunks;
     z.split = g->short_rows;
     z.arrive = w->arrive.as<int32_t>();
@@ -1995,7 +1990,7 @@ static mg_status pr_setup(mg_graph *g, PArgs &a, bool weighted_or_adj, int32_t l
             a.pair_off = g->hub.pair_off.as<int32_t>();
             a.porder = g->hub.porder.as<uint16_t>();
             if (g->hub.ntail == 0) {
-                // rows finish in k_pr_seg; k_pr_apply only reduces
+                // rows finish in k_pr_seg, which closes the sweep
                 a.seg_only = 1;
                 a.fin = g->hub.fin.as<int32_t>();
                 a.nfw = g->hub.nfw;
