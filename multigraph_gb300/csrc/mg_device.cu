@@ -1011,7 +1011,7 @@ static mg_status upload_arrays(mg_graph *g, const mg_host_graph *h, const HostLa
     g->hub.valid = false;  // new pull columns
     g->col_version += 1;
     g->h_prow = L.prow;
-    g->short_pull = true;
+    g->short_pull = (int64_t)g->ne <= (int64_t)8 * g->nv;
     for (size_t v = 0; v + 1 < L.prow.size() && g->short_pull; v++)
         g->short_pull = L.prow[v + 1] - L.prow[v] < SHORT_PULL;
     g->symmetric = L.symmetric;

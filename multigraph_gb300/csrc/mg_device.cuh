@@ -189,7 +189,7 @@ struct mg_graph {
     int32_t hchunk_size = 0;       // edges per heavy chunk
     int32_t tbin = 0;              // rows up to this in-degree are in the thread bin
     std::vector<int32_t> h_prow;   // pull-side row offsets (engine order), for re-binning
-    bool short_pull = false;       // no pull row has SHORT_PULL in-edges or more
+    bool short_pull = false;       // pull rows average at most eight in-edges, none has SHORT_PULL or more
     int32_t n_dangling = 0;        // vertices with out-degree 0
     int32_t min_weight = 0;        // smallest integer edge weight
     // pull rows above 256 in-edges in 256-edge chunks (personalised PageRank,

@@ -117,7 +117,7 @@ struct Args {
     int4 *heavy;         // 2 * hcap chunks (parity): vertex, first edge, end
     int32_t hcap;
     int32_t has_heavy;   // some vertex may have more than PUSH_HEAVY out-edges
-    int32_t short_pull;  // no vertex has SHORT_PULL in-edges or more
+    int32_t short_pull;  // the graph's in-rows are short (mg_graph)
     int32_t *lvl_off;
     FCtl *ctl;
     unsigned *bar;       // grid barrier words of the persistent kernels
@@ -973,10 +973,13 @@ __device__ __forceinline__ void store_ctl_push(FCtl *p, const FCtl &c)
 }
 
 // Whether the next push levels are block 0's alone.  Path counts are summed
-// there over a new vertex's whole in-row by one thread: not on a directed
-// graph with long in-rows, of which its out-degrees say nothing (reaching a
-// vertex of two million in-edges: 220 ms by one thread, 0.4 ms in the grid's
-// levels, which touch the frontier's out-edges only).
+// there over a new vertex's whole in-row by one thread: not on graphs whose
+// rows average more than eight edges (a level of 4,096 edges pulls thousands of
+// whole rows: BC of 256 K vertices of degree 16 345 us with it, 218 without;
+// the push levels of 1 M of degree 64 464 and 73), nor on a directed graph
+// with a long in-row, of which its out-degrees say nothing (reaching a vertex
+// of two million in-edges: 220 ms by one thread, 0.4 ms in the grid's levels,
+// which touch the frontier's out-edges only).
 template <class Op, bool HEAVY>
 __device__ __forceinline__ bool block_phase_due(const Args &a, const FCtl &c)
 {
