@@ -707,7 +707,9 @@ void hub_free(mg_graph *g)
 // its last few groups: a sweep of R-MAT 20 took 57-68 us by the accident of
 // where the cuts fell, 57 now (even shares with a group taken as 16 steps and
 // row-major piece sums: 63.5); R-MAT 20 of degree 6 45-55 -> 46 (48), R-MAT 19
-// 42-55 -> 43 (46), R-MAT 22 161-170 -> 160 (191).
+// 42-55 -> 43 (46), R-MAT 22 161-170 -> 160 (191).  With chunks bounded by a
+// warp's share as well (below), k_hub_sweep alone: R-MAT 18 22 -> 17 us, 19 26 ->
+// 23, 20 37.5 -> 35, of degree 6 28 -> 23, 21 61 -> 54.5, 22 as it was (107).
 static mg_status hub_split(mg_graph *g)
 {
     HubSplit &h = g->hub;
